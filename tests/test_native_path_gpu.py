@@ -1,0 +1,112 @@
+r"""The operators' native host path (``_native``) against their Python autograd functions: same outputs, same
+gradients, same errors, and the calls it leaves to Python."""
+import pytest
+import torch
+
+from triton_helpers_b200 import _lib
+from triton_helpers_b200.layers.fully_fused_mlp import FullyFusedMLP, fully_fused_mlp
+from triton_helpers_b200.layers.hash_encoding import HashEncoding, hash_encoding
+from triton_helpers_b200.layers.hash_encoding.helpers import level_geometry
+from triton_helpers_b200.layers.neural_field import hash_encoded_mlp
+from triton_helpers_b200.layers.reversible_mlp import ReversibleMLP
+
+pytestmark = pytest.mark.gpu
+
+
+def both(call, leaves):
+    r"""``call``'s output and the gradients of ``leaves``: native, then Python."""
+    results = []
+    for deferred in (False, True):
+        _lib.native().defer(deferred)
+        try:
+            y = call()
+            assert "Backward" in y.grad_fn.name() and isinstance(y.grad_fn, torch.autograd.function.BackwardCFunction) == deferred
+            g = torch.Generator(device="cuda").manual_seed(5)
+            go = torch.randn(y.shape, device="cuda", generator=g).to(y.dtype)
+            results.append((y.detach(), *torch.autograd.grad(y, leaves, go)))
+        finally:
+            _lib.native().defer(False)
+    return results
+
+
+def close(native, python, rel):
+    for a, b in zip(native, python):
+        assert a.shape == b.shape and a.dtype == b.dtype
+        assert float((a.double() - b.double()).norm() / b.double().norm().clamp_min(1e-30)) <= rel
+
+
+@pytest.mark.parametrize("shape,dtype", [((1, 3), torch.float32), ((257, 2), torch.float16), ((5, 40, 3), torch.float32)])
+@pytest.mark.parametrize("own_primes", [False, True])
+def test_hash_encoding(shape, dtype, own_primes):
+    layer = HashEncoding(2**12, 8, shape[-1], 2, 16, 128).cuda().to(dtype)
+    layer.pi = layer.pi.long()
+    x = torch.rand(*shape, device="cuda")
+    pi = torch.tensor([1, 7919, 104729], device="cuda") if own_primes else None
+    call = lambda: hash_encoding(x, layer.embeddings, None, pi, 2**12, 16, 128, 8)  # noqa: E731
+    native, python = both(call, [layer.embeddings])
+    assert torch.equal(native[0], python[0])
+    close(native, python, 1e-5 if dtype == torch.float32 else 5e-3)
+
+
+@pytest.mark.parametrize("rows,bias,depth,activation,dtype", [(1, True, 1, "relu", torch.float16), (300, True, 3, "silu", torch.bfloat16),
+                                                              (129, False, 2, "none", torch.float16)])  # fmt: skip
+def test_fused_mlp(rows, bias, depth, activation, dtype):
+    layer = FullyFusedMLP(16, 32, 8, depth, activation, bias=bias).cuda().to(dtype)
+    x = torch.randn(1, rows, 16, device="cuda").to(dtype).requires_grad_(True)
+    native, python = both(lambda: layer(x), [x, *layer.parameters()])
+    assert torch.equal(native[0], python[0])
+    close(native, python, 2e-3 if dtype == torch.float16 else 1e-2)
+
+
+@pytest.mark.parametrize("rows,bias", [(1, False), (333, True)])
+def test_reversible_mlp(rows, bias):
+    layer = ReversibleMLP(64, 3, 32, bias=bias).cuda().half()
+    x = torch.randn(rows, 64, device="cuda").half().requires_grad_(True)
+    native, python = both(lambda: layer(x), [x, *layer.parameters()])
+    assert torch.equal(native[0], python[0])
+    close(native, python, 2e-3)
+
+
+@pytest.mark.parametrize("rows,depth", [(1, 1), (1000, 2)])
+def test_hash_encoded_mlp(rows, depth):
+    table = (torch.randn(level_geometry(16, 2**12, 3, 16, 128).total_rows, 2, device="cuda") * 0.1).half().requires_grad_(True)
+    mlp = FullyFusedMLP(32, 64, 16, depth, bias=False).cuda().half()
+    x = torch.rand(rows, 3, device="cuda")
+    leaves = [table, mlp.w_in, mlp.w_out] + ([mlp.w_hid] if depth > 1 else [])
+    native, python = both(lambda: hash_encoded_mlp(x, table, mlp.w_in, mlp.w_out, mlp.w_hid, None, 2**12, 16, 128, 16), leaves)
+    assert torch.equal(native[0], python[0])
+    close(native, python, 1e-2)
+
+
+def test_what_the_native_path_leaves_to_python():
+    layer = FullyFusedMLP(16, 32, 8, 2).cuda().half()
+    x = torch.randn(1, 64, 16, device="cuda").half()
+    args = (layer.w_in, layer.b_in, layer.w_out, layer.b_out, layer.w_hid, layer.b_hid, "relu")
+    fast = _lib.native().fully_fused_mlp
+    assert fast(x, *args) is not NotImplemented
+    with torch.autocast("cuda"):
+        assert fast(x, *args) is NotImplemented
+    with _lib.KernelTimer() as timer:
+        assert fast(x, *args) is NotImplemented
+        layer(x)
+    assert timer.summary()["th_mlp_fwd"][0] == 1 and fast(x, *args) is not NotImplemented
+    assert fast(x.cpu(), *args) is NotImplemented and fast(x[..., ::2], *args) is NotImplemented
+    with pytest.raises(AssertionError, match="Input dimension mismatch"):
+        layer(x[..., :8])
+    # a graph is gone after one backward pass, and a parameter changed in between is noticed
+    y = layer(x)
+    y.sum().backward()
+    with pytest.raises(RuntimeError, match="second time"):
+        y.sum().backward()
+    y = layer(x)
+    with torch.no_grad():
+        layer.w_in.add_(1)
+    with pytest.raises(RuntimeError, match="inplace operation"):
+        y.sum().backward()
+    # frozen input, one live parameter: only its gradient arrives
+    for p in layer.parameters():
+        p.requires_grad_(False)
+    layer.w_out.requires_grad_(True)
+    y = fully_fused_mlp(x, *args)
+    y.sum().backward()
+    assert layer.w_in.grad is not None and x.grad is None  # w_in.grad: from the first pass above

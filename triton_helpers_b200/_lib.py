@@ -4,6 +4,9 @@ The library is the only compute path: there is no Triton, eager-PyTorch or CPU f
 If the shared object has not been built, loading raises with the build command; every
 non-zero return code of an entry point becomes a ``RuntimeError`` carrying
 ``th_last_error_string()``.
+
+``native()`` is the compiled host path of the operators (``csrc/torch_binding.cpp``): autograd nodes in C++
+that call the same entry points.
 """
 import ctypes
 from ctypes import c_char_p, c_float, c_int, c_int32, c_int64, c_void_p
@@ -15,6 +18,7 @@ import torch
 from torch import Tensor
 
 LIB_PATH = Path(__file__).resolve().parent / "csrc" / "libth_b200.so"
+NATIVE_PATH = Path(__file__).resolve().parent / "_native.so"
 
 DTYPE_CODE = {torch.float32: 0, torch.float16: 1, torch.bfloat16: 2}
 ACTIVATION_CODE = {"none": 0, "relu": 1, "silu": 2, "relu2": 3}
@@ -122,11 +126,13 @@ class KernelTimer:
     def __enter__(self):
         global _ACTIVE_TIMER
         _ACTIVE_TIMER = self
+        native().defer(True)  # the events are recorded around the ctypes calls
         return self
 
     def __exit__(self, *exc):
         global _ACTIVE_TIMER
         _ACTIVE_TIMER = None
+        native().defer(False)
         return False
 
     def summary(self):
@@ -179,6 +185,23 @@ def lib() -> _Library:
         fn.restype = restype
         fn.argtypes = argtypes
     return _Library(handle)
+
+
+@lru_cache(maxsize=1)
+def native():
+    r"""The extension module ``triton_helpers_b200._native``.  Its functions take the arguments of the public
+    operators and answer ``NotImplemented`` when the call is one they leave to Python."""
+    if not NATIVE_PATH.exists():
+        raise RuntimeError(
+            f"{NATIVE_PATH} is missing: build the extension with `python -m triton_helpers_b200.build` "
+            "(there is no fallback path)"
+        )
+    from . import _native
+    from .layers.hash_encoding.helpers import level_geometry
+    from .layers.hash_encoding.kernel import host_primes
+
+    _native.configure(level_geometry, host_primes)
+    return _native
 
 
 def check(code: int, what: str) -> None:

@@ -2,12 +2,15 @@ r"""Builds ``libth_b200.so`` in-tree with nvcc for sm_100a (no other architectur
 
 ``python -m triton_helpers_b200.build`` compiles every ``csrc/*.cu`` to an object file (in
 parallel, one nvcc process per file) and links them into
-``triton_helpers_b200/csrc/libth_b200.so``.  Objects are rebuilt only when their source or a
-header is newer.  nvcc cross-compiles, so no GPU is needed to build.
+``triton_helpers_b200/csrc/libth_b200.so``; ``csrc/torch_binding.cpp`` is compiled with g++ against
+torch's headers and linked with that library into the Python module ``triton_helpers_b200/_native.so``.
+Objects are rebuilt only when their source or a header is newer.  nvcc cross-compiles, so no GPU is
+needed to build.
 """
 import os
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 from typing import List
@@ -15,6 +18,7 @@ from typing import List
 CSRC = Path(__file__).resolve().parent / "csrc"
 INCLUDE = Path(__file__).resolve().parent.parent / "include"
 LIB_PATH = CSRC / "libth_b200.so"
+NATIVE_PATH = CSRC.parent / "_native.so"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -42,6 +46,27 @@ def _compile(src: Path, obj: Path, verbose: bool) -> None:
     subprocess.run(cmd, check=True)
 
 
+def _build_native(force: bool, verbose: bool) -> None:
+    r"""The autograd nodes in C++ (``csrc/torch_binding.cpp``), next to the package's Python files."""
+    import torch
+    from torch.utils.cpp_extension import include_paths, library_paths
+
+    src = CSRC / "torch_binding.cpp"
+    if not force and NATIVE_PATH.exists() and NATIVE_PATH.stat().st_mtime >= max(src.stat().st_mtime, _newest_header()):
+        return
+    cuda_home = Path(os.environ.get("CUDA_HOME", "/usr/local/cuda"))
+    includes = [*include_paths(), str(cuda_home / "include"), sysconfig.get_paths()["include"], str(INCLUDE)]
+    cmd = [
+        "g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+        *(f"-I{path}" for path in dict.fromkeys(includes)), str(src), "-o", str(NATIVE_PATH),
+        f"-L{CSRC}", "-lth_b200", "-Wl,-rpath,$ORIGIN/csrc",
+        *(f"-L{path}" for path in library_paths()), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python",
+    ]  # fmt: skip
+    if verbose:
+        print(" ".join(cmd), flush=True)
+    subprocess.run(cmd, check=True)
+
+
 def build(force: bool = False, verbose: bool = False) -> Path:
     sources: List[Path] = sorted(CSRC.glob("*.cu"))
     if not sources:
@@ -60,6 +85,7 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         if verbose:
             print(" ".join(cmd), flush=True)
         subprocess.run(cmd, check=True)
+    _build_native(force, verbose)
     return LIB_PATH
 
 

@@ -223,6 +223,10 @@ def fully_fused_mlp(
         - w_hid: :math:`(depth \cdot D_{hidden}, D_{hidden})`, b_hid: :math:`(depth, D_{hidden})`
     """
     activation = ensure_str(activation)
+    if not fp16_acc:
+        out = _lib.native().fully_fused_mlp(x, w_in, b_in, w_out, b_out, w_hid, b_hid, activation)
+        if out is not NotImplemented:
+            return out
     return _fully_fused_mlp.apply(x, w_in, b_in, w_out, b_out, w_hid, b_hid, activation, fp16_acc)
 
 

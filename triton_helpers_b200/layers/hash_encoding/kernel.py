@@ -310,6 +310,11 @@ def hash_encoding(
         ``coord`` - :math:`(..., D)`, ``embeddings`` - :math:`(E, D_e)`, ``features`` - :math:`(..., D_f)`,
         ``pi`` - :math:`(D,)`, output - :math:`(..., L \times D_e + D_f)`.
     """
+    out = _lib.native().hash_encoding(
+        coord, embeddings, features, pi, max_entries_per_level, min_res, max_res, levels, divider, bwd_divider, scale
+    )
+    if out is not NotImplemented:
+        return out
     return HashEncoding.apply(
         coord, embeddings, pi, features, max_entries_per_level, min_res, max_res, levels, divider, bwd_divider, scale
     )

@@ -178,6 +178,12 @@ def hash_encoded_mlp(
     r"""``fully_fused_mlp(hash_encoding(coord, embeddings, ...), w_in, None, w_out, None, w_hid, None, activation)``
     in one kernel per direction.  Arguments are those of the two functions (bias-free network); output
     ``(..., D_out)``.  Raises ``FieldUnsupported`` for configurations the fused kernels do not cover."""
+    activation = ensure_str(activation)
+    out = _lib.native().hash_encoded_mlp(
+        coord, embeddings, w_in, w_out, w_hid, pi, max_entries_per_level, min_res, max_res, levels, activation, scale
+    )
+    if out is not NotImplemented:
+        return out
     return HashEncodedMLP.apply(
-        coord, embeddings, w_in, w_out, w_hid, pi, max_entries_per_level, min_res, max_res, levels, ensure_str(activation), scale
+        coord, embeddings, w_in, w_out, w_hid, pi, max_entries_per_level, min_res, max_res, levels, activation, scale
     )

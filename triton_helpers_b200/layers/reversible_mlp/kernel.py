@@ -173,4 +173,7 @@ def reversible_mlp(
         - b_f1, b_g1: :math:`(blocks, D_{hidden})`; b_f2, b_g2: :math:`(blocks, H)`; all or none
     """
     activation = ensure_str(activation)
+    out = _lib.native().reversible_mlp(x, w_f1, w_f2, w_g1, w_g2, b_f1, b_f2, b_g1, b_g2, activation)
+    if out is not NotImplemented:
+        return out
     return _reversible_mlp.apply(x, w_f1, w_f2, w_g1, w_g2, b_f1, b_f2, b_g1, b_g2, activation)
