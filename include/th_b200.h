@@ -114,6 +114,30 @@ int th_hash_bwd(const void *coords_dev, int64_t coord_stride_n, int64_t coord_st
                 const int32_t *level_res_host, const int64_t *level_rows_host, const int64_t *level_offset_host,
                 const int64_t *primes_host, float scale, int level_begin, int level_end, void *stream);
 
+/*
+ * The same two operations on a spatially ordered batch.  th_hash_order sorts the points along a space-filling curve
+ * (in buckets, about one per point) and writes 16 bytes per point to order_dev: up to three coordinates, divided by
+ * `scale`, and the point's row as uint32.  th_hash_fwd_ordered / th_hash_bwd_ordered walk the batch in that order,
+ * which lets neighbours share table rows on chip; outputs and gradients stay in the caller's row order
+ * (keep_order = 0) or are in the order of order_dev as well (keep_order = 1).  Values are those of th_hash_fwd;
+ * gradients differ from th_hash_bwd's in the order of the sums.  order_dev: 16 * n_points bytes; scratch_dev:
+ * th_hash_order_scratch_bytes, free once the work queued by th_hash_order is done.  Both 16-byte aligned.
+ * th_hash_order_pays: 1 where the ordering is measured to pay for itself, for a forward pass alone (backward = 0) or a
+ * forward and a backward pass.  No counterpart in the reference.
+ */
+int th_hash_order_pays(int64_t n_points, int n_dims, int backward);
+int64_t th_hash_order_scratch_bytes(int64_t n_points, int n_dims);
+int th_hash_order(const void *coords_dev, int64_t coord_stride_n, int64_t coord_stride_d, int coord_dtype, int64_t n_points,
+                  int n_dims, float scale, void *order_dev, void *scratch_dev, int64_t scratch_bytes, void *stream);
+int th_hash_fwd_ordered(const void *order_dev, int keep_order, const void *table_dev, int table_dtype, void *out_dev,
+                        int64_t out_stride_n, int64_t n_points, int n_dims, int n_feats, int n_levels,
+                        const int32_t *level_res_host, const int64_t *level_rows_host, const int64_t *level_offset_host,
+                        const int64_t *primes_host, int level_begin, int level_end, void *stream);
+int th_hash_bwd_ordered(const void *order_dev, int keep_order, const void *grad_out_dev, int64_t go_stride_n,
+                        void *grad_table_dev, int table_dtype, int64_t n_points, int n_dims, int n_feats, int n_levels,
+                        const int32_t *level_res_host, const int64_t *level_rows_host, const int64_t *level_offset_host,
+                        const int64_t *primes_host, int level_begin, int level_end, void *stream);
+
 /* Device-side status word of the encoding kernels: 0 = fine, 1 = a shared-memory accumulation of the
  * backward pass (compare-and-swap loop, bounded) gave up and dropped an update.  Synchronises the device.
  * No counterpart in the reference. */

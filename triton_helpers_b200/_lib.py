@@ -46,6 +46,22 @@ SIGNATURES = {
         [c_void_p, c_int64, c_int64, c_int, c_void_p, c_void_p, c_int64, c_int, c_int, _I32P, _I64P, _I64P,
          c_float, c_void_p],
     ),
+    "th_hash_order_pays": (c_int, [c_int64, c_int, c_int]),
+    "th_hash_order_scratch_bytes": (c_int64, [c_int64, c_int]),
+    "th_hash_order": (
+        c_int,
+        [c_void_p, c_int64, c_int64, c_int, c_int64, c_int, c_float, c_void_p, c_void_p, c_int64, c_void_p],
+    ),
+    "th_hash_fwd_ordered": (
+        c_int,
+        [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int64, c_int64, c_int, c_int, c_int, _I32P, _I64P, _I64P, _I64P,
+         c_int, c_int, c_void_p],
+    ),
+    "th_hash_bwd_ordered": (
+        c_int,
+        [c_void_p, c_int, c_void_p, c_int64, c_void_p, c_int, c_int64, c_int, c_int, c_int, _I32P, _I64P, _I64P, _I64P,
+         c_int, c_int, c_void_p],
+    ),
     "th_hash_status": (c_int, []),
     "th_field_fwd": (
         c_int,
@@ -117,7 +133,7 @@ class KernelTimer:
     queued.  ``summary()`` synchronises and returns ``{entry point: (calls, total ms)}``.
     """
 
-    LAUNCHING = ("th_field_fwd", "th_field_bwd", "th_hash_fwd", "th_hash_bwd", "th_mlp_fwd", "th_mlp_fwd_mse", "th_mlp_bwd", "th_rev_fwd", "th_rev_bwd",
+    LAUNCHING = ("th_field_fwd", "th_field_bwd", "th_hash_fwd", "th_hash_bwd", "th_hash_order", "th_hash_fwd_ordered", "th_hash_bwd_ordered", "th_mlp_fwd", "th_mlp_fwd_mse", "th_mlp_bwd", "th_rev_fwd", "th_rev_bwd",
                  "th_mse_grad", "th_adam_step", "th_scale_cast")  # fmt: skip
 
     def __init__(self):

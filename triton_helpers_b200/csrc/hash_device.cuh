@@ -85,6 +85,17 @@ __device__ __forceinline__ bool load_coords(const CoordView &cv, long long n_poi
     return i < n_points;
 }
 
+// One point of a spatially ordered batch (hash_order.cu): its coordinates, already divided by the scale, and
+// the row it has in the caller's arrays.
+template <int D>
+__device__ __forceinline__ uint32_t load_ordered(const float4 *order, long long i, float (&x)[D]) {
+    const float4 p = __ldg(order + i);
+    x[0] = p.x;
+    if constexpr (D > 1) x[1] = p.y;
+    if constexpr (D > 2) x[2] = p.z;
+    return __float_as_uint(p.w);
+}
+
 // ---- per-level index / weight arithmetic ----------------------------------------------------
 
 template <int D>
@@ -492,6 +503,82 @@ int make_coord_view(CoordView &cv, const void *coords, int64_t stride_n, int64_t
     cv.stride_d = stride_d;
     cv.dtype = dtype;
     cv.packed_f32 = dtype == TH_F32 && stride_d == 1 && stride_n == n_dims && aligned_to(coords, 16);
+    return TH_OK;
+}
+
+// Level passes.  Rows of a level are visited at random, so a launch runs at cache speed only while
+// the levels it touches stay resident in L2.  When the levels of [l0, l1) add up to more than
+// kPassBytes and the batch is large, the range is cut into consecutive passes of at most kPassBytes
+// each (a single level larger than that is a pass of its own).  Measured with 2^22 rows x 16 B per
+// level and 2^22 points: four such levels in one launch 2.6 ms backward / 1.2 ms forward, the same
+// four as one launch each 0.95 / 0.83 ms.  The reference exposes the same idea as its `divider`
+// argument; here it is automatic and `level_begin/level_end` passes of the caller still work.
+constexpr size_t kPassBytes = static_cast<size_t>(72) << 20;
+constexpr int64_t kPassMinPoints = 1 << 16;
+
+struct LevelPasses {
+    int count = 0;
+    int begin[TH_MAX_LEVELS];
+    int end[TH_MAX_LEVELS];
+};
+
+// A pass takes at least `least` levels (1, or what makes whole 32-byte sectors of a row of outputs), if the range has them.
+inline LevelPasses plan_level_passes(const LevelParams &P, int64_t n, int l0, int l1, size_t row_bytes, int least = 1) {
+    LevelPasses passes;
+    size_t total = 0;
+    for (int l = l0; l < l1; ++l) total += static_cast<size_t>(P.rows[l]) * row_bytes;
+    if (total <= kPassBytes || n < kPassMinPoints) {
+        passes.count = 1;
+        passes.begin[0] = l0;
+        passes.end[0] = l1;
+        return passes;
+    }
+    int a = l0;
+    while (a < l1) {
+        size_t bytes = static_cast<size_t>(P.rows[a]) * row_bytes;
+        int b = a + 1;
+        while (b < l1 && (b % least != 0 || bytes + static_cast<size_t>(P.rows[b]) * row_bytes <= kPassBytes)) {
+            bytes += static_cast<size_t>(P.rows[b]) * row_bytes;
+            ++b;
+        }
+        passes.begin[passes.count] = a;
+        passes.end[passes.count] = b;
+        ++passes.count;
+        a = b;
+    }
+    return passes;
+}
+
+// ---- spatially ordered batches (hash_order.cu) ----
+
+template <int F>
+constexpr int kPointsPerTile = F > 4 ? 512 : 1024;  // points the backward pass sorts together: what 48 KB of shared memory hold
+
+// Expands (dtype, D, F) into a template instantiation.
+#define TH_DISPATCH_F(T, D, CALL)                                                      \
+    switch (n_feats) {                                                                 \
+        case 1: return CALL(T, D, 1);                                                  \
+        case 2: return CALL(T, D, 2);                                                  \
+        case 4: return CALL(T, D, 4);                                                  \
+        case 8: return CALL(T, D, 8);                                                  \
+        default: return fail(TH_ERR_UNSUPPORTED, "n_feats %d not in {1, 2, 4, 8}", n_feats); \
+    }
+#define TH_DISPATCH_D(T, CALL)                    \
+    switch (n_dims) {                             \
+        case 1: TH_DISPATCH_F(T, 1, CALL)         \
+        case 2: TH_DISPATCH_F(T, 2, CALL)         \
+        default: TH_DISPATCH_F(T, 3, CALL)        \
+    }
+#define TH_DISPATCH(CALL)                                                                  \
+    switch (table_dtype) {                                                                 \
+        case TH_F32: TH_DISPATCH_D(float, CALL)                                            \
+        case TH_F16: TH_DISPATCH_D(__half, CALL)                                           \
+        case TH_BF16: TH_DISPATCH_D(__nv_bfloat16, CALL)                                   \
+        default: return fail(TH_ERR_BAD_ARG, "unknown table dtype %d", table_dtype);       \
+    }
+
+inline int check_range(int n_levels, int l0, int l1) {
+    if (l0 < 0 || l1 > n_levels || l0 >= l1) return fail(TH_ERR_BAD_ARG, "level range [%d, %d) outside [0, %d)", l0, l1, n_levels);
     return TH_OK;
 }
 

@@ -33,29 +33,38 @@ namespace {
 
 // ---- forward --------------------------------------------------------------------------------
 
-template <typename T, int D, int F, int LG>
+// ORDERED: the points come from a spatially ordered batch; output rows are the caller's (`keep_order` 0) or in order too.
+template <typename T, int D, int F, int LG, bool ORDERED>
 __global__ void __launch_bounds__(kThreads)
-hash_fwd_kernel(const __grid_constant__ LevelParams P, const CoordView cv, const T *__restrict__ table,
-                T *__restrict__ out, long long out_stride, long long n_points, int level_begin, int level_end,
-                int vector_ok) {
+hash_fwd_kernel(const __grid_constant__ LevelParams P, const CoordView cv, const float4 *__restrict__ order, int keep_order,
+                const T *__restrict__ table, T *__restrict__ out, long long out_stride, long long n_points, int level_begin,
+                int level_end, int vector_ok) {
     constexpr int kPoints = kThreads / 2;
     constexpr int kSide = 1 << (D - 1);   // corners per lane
     constexpr int kCount = LG * F;        // outputs per level group
     constexpr int kFirst = (kCount + 1) / 2;  // written by lane 0 of the pair; the rest by lane 1
-    __shared__ __align__(16) float stage[kPoints * D];
     float x[D];
-    const bool live = load_coords<D, 2>(cv, n_points, blockIdx.x, x, stage);
-    // dead pairs of the last CTA stay in the loop: the pair shuffle below needs both lanes
-    if (P.scale != 1.f) {
+    long long i = static_cast<long long>(blockIdx.x) * kPoints + (threadIdx.x >> 1);
+    bool live = i < n_points;
+    if constexpr (ORDERED) {
+        if (live) {
+            const uint32_t row = load_ordered<D>(order, i, x);
+            if (!keep_order) i = row;
+        }
+    } else {
+        __shared__ __align__(16) float stage[kPoints * D];
+        live = load_coords<D, 2>(cv, n_points, blockIdx.x, x, stage);
+        // dead pairs of the last CTA stay in the loop: the pair shuffle below needs both lanes
+        if (P.scale != 1.f) {
 #pragma unroll
-        for (int d = 0; d < D; ++d) x[d] = __fdiv_rn(x[d], P.scale);
+            for (int d = 0; d < D; ++d) x[d] = __fdiv_rn(x[d], P.scale);
+        }
     }
     if (!live) {
 #pragma unroll
         for (int d = 0; d < D; ++d) x[d] = 0.f;
     }
     const int side = threadIdx.x & 1;
-    const long long i = static_cast<long long>(blockIdx.x) * kPoints + (threadIdx.x >> 1);
     T *out_row = out + (live ? i : 0) * out_stride;
 
     // gridDim.y CTAs share a point tile and take every gridDim.y-th level group each
@@ -397,63 +406,27 @@ dim3 point_level_grid(int64_t n, int l0, int l1, int levels_per_group) {
     return dim3(static_cast<unsigned>(tiles), static_cast<unsigned>(split), 1);
 }
 
-// Level passes.  Rows of a level are visited at random, so a launch runs at cache speed only while
-// the levels it touches stay resident in L2.  When the levels of [l0, l1) add up to more than
-// kPassBytes and the batch is large, the range is cut into consecutive passes of at most kPassBytes
-// each (a single level larger than that is a pass of its own).  Measured with 2^22 rows x 16 B per
-// level and 2^22 points: four such levels in one launch 2.6 ms backward / 1.2 ms forward, the same
-// four as one launch each 0.95 / 0.83 ms.  The reference exposes the same idea as its `divider`
-// argument; here it is automatic and `level_begin/level_end` passes of the caller still work.
-constexpr size_t kPassBytes = static_cast<size_t>(72) << 20;
-constexpr int64_t kPassMinPoints = 1 << 16;
-
-struct LevelPasses {
-    int count = 0;
-    int begin[TH_MAX_LEVELS];
-    int end[TH_MAX_LEVELS];
-};
-
-LevelPasses plan_level_passes(const LevelParams &P, int64_t n, int l0, int l1, size_t row_bytes) {
-    LevelPasses passes;
-    size_t total = 0;
-    for (int l = l0; l < l1; ++l) total += static_cast<size_t>(P.rows[l]) * row_bytes;
-    if (total <= kPassBytes || n < kPassMinPoints) {
-        passes.count = 1;
-        passes.begin[0] = l0;
-        passes.end[0] = l1;
-        return passes;
-    }
-    int a = l0;
-    while (a < l1) {
-        size_t bytes = static_cast<size_t>(P.rows[a]) * row_bytes;
-        int b = a + 1;
-        while (b < l1 && bytes + static_cast<size_t>(P.rows[b]) * row_bytes <= kPassBytes) {
-            bytes += static_cast<size_t>(P.rows[b]) * row_bytes;
-            ++b;
-        }
-        passes.begin[passes.count] = a;
-        passes.end[passes.count] = b;
-        ++passes.count;
-        a = b;
-    }
-    return passes;
-}
-
 template <typename T, int D, int F>
-int launch_fwd(const LevelParams &P, const CoordView &cv, const void *table, void *out, int64_t out_stride,
+int launch_fwd(const LevelParams &P, const CoordView &cv, const float4 *order, int keep_order, const void *table, void *out, int64_t out_stride,
                int64_t n, int l0, int l1, cudaStream_t stream) {
     const int vec = aligned_to(out, 16) && (out_stride * sizeof(T)) % 16 == 0;
     const T *tb = static_cast<const T *>(table);
     T *o = static_cast<T *>(out);
-    const LevelPasses passes = plan_level_passes(P, n, l0, l1, F * sizeof(T));
+    // Ordered points write their rows in random order: passes that fill whole sectors of a row (2^22 clustered points, rows
+    // of 4 x 16 float32, one 64 MB level per pass 2.70 ms, two 1.51 ms).
+    const int least = order && F * sizeof(T) < 32 ? static_cast<int>(32 / (F * sizeof(T))) : 1;
+    const LevelPasses passes = plan_level_passes(P, n, l0, l1, F * sizeof(T), least);
     for (int p = 0; p < passes.count; ++p) {
         const int a = passes.begin[p], b = passes.end[p];
         const int lg = pick_level_group(a, b, F);
         const dim3 grid = point_level_grid(n, a, b, lg);
         switch (lg) {
-            case 4: hash_fwd_kernel<T, D, F, 4><<<grid, kThreads, 0, stream>>>(P, cv, tb, o, out_stride, n, a, b, vec); break;
-            case 2: hash_fwd_kernel<T, D, F, 2><<<grid, kThreads, 0, stream>>>(P, cv, tb, o, out_stride, n, a, b, vec); break;
-            default: hash_fwd_kernel<T, D, F, 1><<<grid, kThreads, 0, stream>>>(P, cv, tb, o, out_stride, n, a, b, vec); break;
+            case 4: order ? hash_fwd_kernel<T, D, F, 4, true><<<grid, kThreads, 0, stream>>>(P, cv, order, keep_order, tb, o, out_stride, n, a, b, vec)
+                          : hash_fwd_kernel<T, D, F, 4, false><<<grid, kThreads, 0, stream>>>(P, cv, order, 0, tb, o, out_stride, n, a, b, vec); break;
+            case 2: order ? hash_fwd_kernel<T, D, F, 2, true><<<grid, kThreads, 0, stream>>>(P, cv, order, keep_order, tb, o, out_stride, n, a, b, vec)
+                          : hash_fwd_kernel<T, D, F, 2, false><<<grid, kThreads, 0, stream>>>(P, cv, order, 0, tb, o, out_stride, n, a, b, vec); break;
+            default: order ? hash_fwd_kernel<T, D, F, 1, true><<<grid, kThreads, 0, stream>>>(P, cv, order, keep_order, tb, o, out_stride, n, a, b, vec)
+                          : hash_fwd_kernel<T, D, F, 1, false><<<grid, kThreads, 0, stream>>>(P, cv, order, 0, tb, o, out_stride, n, a, b, vec); break;
         }
         if (int rc = launch_status("hash_fwd_kernel launch")) return rc;
     }
@@ -517,34 +490,6 @@ int launch_bwd(const LevelParams &P, const CoordView &cv, const void *go, int64_
     return TH_OK;
 }
 
-// Expands (dtype, D, F) into a template instantiation.
-#define TH_DISPATCH_F(T, D, CALL)                                                      \
-    switch (n_feats) {                                                                 \
-        case 1: return CALL(T, D, 1);                                                  \
-        case 2: return CALL(T, D, 2);                                                  \
-        case 4: return CALL(T, D, 4);                                                  \
-        case 8: return CALL(T, D, 8);                                                  \
-        default: return fail(TH_ERR_UNSUPPORTED, "n_feats %d not in {1, 2, 4, 8}", n_feats); \
-    }
-#define TH_DISPATCH_D(T, CALL)                    \
-    switch (n_dims) {                             \
-        case 1: TH_DISPATCH_F(T, 1, CALL)         \
-        case 2: TH_DISPATCH_F(T, 2, CALL)         \
-        default: TH_DISPATCH_F(T, 3, CALL)        \
-    }
-#define TH_DISPATCH(CALL)                                                                  \
-    switch (table_dtype) {                                                                 \
-        case TH_F32: TH_DISPATCH_D(float, CALL)                                            \
-        case TH_F16: TH_DISPATCH_D(__half, CALL)                                           \
-        case TH_BF16: TH_DISPATCH_D(__nv_bfloat16, CALL)                                   \
-        default: return fail(TH_ERR_BAD_ARG, "unknown table dtype %d", table_dtype);       \
-    }
-
-int check_range(int n_levels, int l0, int l1) {
-    if (l0 < 0 || l1 > n_levels || l0 >= l1) return fail(TH_ERR_BAD_ARG, "level range [%d, %d) outside [0, %d)", l0, l1, n_levels);
-    return TH_OK;
-}
-
 }  // namespace
 
 int hash_status_word() {
@@ -575,7 +520,7 @@ extern "C" int th_hash_fwd(const void *coords_dev, int64_t coord_stride_n, int64
     if (!aligned_to(table_dev, row_bytes < 16 ? row_bytes : 16)) return fail(TH_ERR_ALIGNMENT, "table rows must be aligned to min(row bytes, 16)");
     if (out_stride_n < static_cast<int64_t>(n_levels) * n_feats) return fail(TH_ERR_BAD_ARG, "out_stride_n smaller than n_levels * n_feats");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-#define TH_CALL_FWD(T, D, F) launch_fwd<T, D, F>(P, cv, table_dev, out_dev, out_stride_n, n_points, level_begin, level_end, s)
+#define TH_CALL_FWD(T, D, F) launch_fwd<T, D, F>(P, cv, nullptr, 0, table_dev, out_dev, out_stride_n, n_points, level_begin, level_end, s)
     TH_DISPATCH(TH_CALL_FWD)
 #undef TH_CALL_FWD
 }
@@ -601,6 +546,29 @@ extern "C" int th_hash_bwd(const void *coords_dev, int64_t coord_stride_n, int64
 #define TH_CALL_BWD(T, D, F) launch_bwd<T, D, F>(P, cv, grad_out_dev, go_stride_n, grad_table_dev, n_points, level_begin, level_end, s)
     TH_DISPATCH(TH_CALL_BWD)
 #undef TH_CALL_BWD
+}
+
+extern "C" int th_hash_fwd_ordered(const void *order_dev, int keep_order, const void *table_dev, int table_dtype, void *out_dev, int64_t out_stride_n,
+                                   int64_t n_points, int n_dims, int n_feats, int n_levels, const int32_t *level_res_host,
+                                   const int64_t *level_rows_host, const int64_t *level_offset_host, const int64_t *primes_host, int level_begin,
+                                   int level_end, void *stream) {
+    if (n_points < 0) return fail(TH_ERR_BAD_ARG, "negative n_points");
+    LevelParams P;
+    if (int rc = fill_params(P, n_dims, n_levels, level_res_host, level_rows_host, level_offset_host, primes_host, 1.f)) return rc;
+    if (!level_offset_host) return fail(TH_ERR_BAD_ARG, "null level offsets");
+    if (int rc = check_range(n_levels, level_begin, level_end)) return rc;
+    if (n_points == 0) return TH_OK;
+    if (!order_dev || !table_dev || !out_dev) return fail(TH_ERR_BAD_ARG, "null order, table or output");
+    const size_t row_bytes = n_feats * dtype_bytes(table_dtype);
+    if (!aligned_to(order_dev, 16)) return fail(TH_ERR_ALIGNMENT, "the order must be 16-byte aligned");
+    if (!aligned_to(table_dev, row_bytes < 16 ? row_bytes : 16)) return fail(TH_ERR_ALIGNMENT, "table rows must be aligned to min(row bytes, 16)");
+    if (out_stride_n < static_cast<int64_t>(n_levels) * n_feats) return fail(TH_ERR_BAD_ARG, "out_stride_n smaller than n_levels * n_feats");
+    const CoordView cv{};
+    const float4 *order = static_cast<const float4 *>(order_dev);
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+#define TH_CALL_FWD(T, D, F) launch_fwd<T, D, F>(P, cv, order, keep_order, table_dev, out_dev, out_stride_n, n_points, level_begin, level_end, s)
+    TH_DISPATCH(TH_CALL_FWD)
+#undef TH_CALL_FWD
 }
 
 namespace th {

@@ -300,16 +300,40 @@ CoordArgs coord_args(const Tensor &coords, int64_t dims) {
     return a;
 }
 
-void hash_forward(const EncodeCall &c, const CoordArgs &x, const Tensor &table, const Tensor &out, void *stream) {
+// The batch along a space-filling curve, 16 bytes per point
+Tensor point_order(const EncodeCall &c, const CoordArgs &x, void *stream) {
+    Tensor order = empty_like_shape({c.n, 4}, at::kFloat, x.keep.device());
+    const int64_t bytes = th_hash_order_scratch_bytes(c.n, static_cast<int>(c.dims));
+    const Tensor scratch = empty_like_shape({bytes}, at::kByte, x.keep.device());
+    check(th_hash_order(ptr(x.keep), x.stride_n, x.stride_d, dtype_code(x.keep.scalar_type()), c.n, static_cast<int>(c.dims), c.scale, ptr(order),
+                        ptr(scratch), bytes, stream),
+          "th_hash_order");
+    return order;
+}
+
+// `order`: the batch's order, or an undefined tensor
+void hash_forward(const EncodeCall &c, const CoordArgs &x, const Tensor &order, const Tensor &table, const Tensor &out, void *stream) {
     const Geometry &g = *c.geo;
+    if (order.defined()) {
+        check(th_hash_fwd_ordered(ptr(order), 0, ptr(table), dtype_code(table.scalar_type()), ptr(out), c.feats * g.levels, c.n,
+                                  static_cast<int>(c.dims), static_cast<int>(c.feats), g.levels, g.res, g.rows, g.offsets, c.primes.v, 0, g.levels, stream),
+              "th_hash_fwd_ordered");
+        return;
+    }
     check(th_hash_fwd(ptr(x.keep), x.stride_n, x.stride_d, dtype_code(x.keep.scalar_type()), ptr(table), dtype_code(table.scalar_type()),
                       ptr(out), c.feats * g.levels, c.n, static_cast<int>(c.dims), static_cast<int>(c.feats), g.levels, g.res, g.rows, g.offsets,
                       c.primes.v, c.scale, 0, g.levels, stream),
           "th_hash_fwd");
 }
 
-void hash_backward(const EncodeCall &c, const CoordArgs &x, const Rows &go, const Tensor &grad_table, void *stream) {
+void hash_backward(const EncodeCall &c, const CoordArgs &x, const Tensor &order, const Rows &go, const Tensor &grad_table, void *stream) {
     const Geometry &g = *c.geo;
+    if (order.defined()) {
+        check(th_hash_bwd_ordered(ptr(order), 0, ptr(go.keep), go.stride, ptr(grad_table), dtype_code(grad_table.scalar_type()), c.n,
+                                  static_cast<int>(c.dims), static_cast<int>(c.feats), g.levels, g.res, g.rows, g.offsets, c.primes.v, 0, g.levels, stream),
+              "th_hash_bwd_ordered");
+        return;
+    }
     check(th_hash_bwd(ptr(x.keep), x.stride_n, x.stride_d, dtype_code(x.keep.scalar_type()), ptr(go.keep), go.stride, ptr(grad_table),
                       dtype_code(grad_table.scalar_type()), c.n, static_cast<int>(c.dims), static_cast<int>(c.feats), g.levels, g.res, g.rows,
                       g.offsets, c.primes.v, c.scale, 0, g.levels, stream),
@@ -319,9 +343,11 @@ void hash_backward(const EncodeCall &c, const CoordArgs &x, const Rows &go, cons
 struct HashEncodingNode : public Node {
     EncodeCall call;
     SavedVariable coords, table;
+    Tensor order;
 
     std::string name() const override { return "HashEncodingBackward"; }
     void release_variables() override {
+        order.reset();
         coords.reset_data();
         table.reset_data();
     }
@@ -336,7 +362,7 @@ struct HashEncodingNode : public Node {
         const Rows rows = rows_or_copy(go, call.feats * call.geo->levels);
         Tensor de = empty_like_shape(t.sizes(), t.scalar_type(), t.device());
         de.zero_();
-        hash_backward(call, coord_args(x, call.dims), rows, de, current_stream());
+        hash_backward(call, coord_args(x, call.dims), order, rows, de, current_stream());
         out[0] = std::move(de);
         return out;
     }
@@ -397,7 +423,11 @@ PyObject *py_hash_encoding(PyObject *, PyObject *const *args, Py_ssize_t n_args)
             at::AutoDispatchBelowADInplaceOrView below;
             c10::cuda::CUDAGuard guard(coords.device());
             out = empty_like_shape(with_last(coords, call.feats * call.geo->levels), table.scalar_type(), table.device());
-            hash_forward(call, coord_args(coords, call.dims), table, out, current_stream());
+            const CoordArgs x = coord_args(coords, call.dims);
+            void *stream = current_stream();
+            Tensor order = th_hash_order_pays(call.n, static_cast<int>(call.dims), grad) ? point_order(call, x, stream) : Tensor();
+            hash_forward(call, x, order, table, out, stream);
+            if (grad) node->order = std::move(order);
         }
         if (grad) torch::autograd::set_history(out, node);
     }

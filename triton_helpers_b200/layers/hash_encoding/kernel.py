@@ -117,7 +117,27 @@ class _Launch:
         )
 
 
-def _launch_backward(launch: "_Launch", do: Tensor, de: Tensor, D_in: int, D_embed: int, levels: int, begin: int, end: int):
+    def order(self, backward: bool) -> Optional[Tensor]:
+        r"""The batch along a space-filling curve (16 bytes per point) where that pays, else ``None``."""
+        D = self.coords2d.shape[1]
+        lib = _lib.lib()
+        if not lib.th_hash_order_pays(self.n, D, int(backward)):
+            return None
+        device = self.coords2d.device
+        order = torch.empty(self.n, 4, dtype=torch.float32, device=device)
+        scratch = torch.empty(lib.th_hash_order_scratch_bytes(self.n, D), dtype=torch.uint8, device=device)
+        with torch.cuda.device(device):
+            _lib.check(
+                lib.th_hash_order(*self.coord_args, self.n, D, self.scale, order.data_ptr(), scratch.data_ptr(), scratch.numel(),
+                                  _lib.stream_ptr(device)),
+                "th_hash_order",
+            )  # fmt: skip
+        return order
+
+
+def _launch_backward(
+    launch: "_Launch", do: Tensor, de: Tensor, D_in: int, D_embed: int, levels: int, begin: int, end: int, order: Optional[Tensor] = None
+):
     r"""``th_hash_bwd`` for levels ``[begin, end)``: adds into the (zero-initialised) table gradient ``de``."""
     D_out = do.shape[-1]
     go = _flatten_rows(do, D_out)
@@ -128,6 +148,15 @@ def _launch_backward(launch: "_Launch", do: Tensor, de: Tensor, D_in: int, D_emb
     go_stride = go.stride(0) if go.shape[0] > 1 else D_out
     device = de.device
     with torch.cuda.device(device):
+        if order is not None:
+            _lib.check(
+                _lib.lib().th_hash_bwd_ordered(
+                    order.data_ptr(), 0, go.data_ptr(), go_stride, de.data_ptr(), _lib.dtype_code(de), launch.n, D_in, D_embed,
+                    levels, launch.res, launch.rows, launch.offsets, launch.primes, begin, end, _lib.stream_ptr(device),
+                ),
+                "th_hash_bwd_ordered",
+            )  # fmt: skip
+            return
         _lib.check(
             _lib.lib().th_hash_bwd(
                 *launch.coord_args, go.data_ptr(), go_stride, de.data_ptr(), _lib.dtype_code(de),
@@ -231,9 +260,18 @@ class HashEncoding(torch.autograd.Function):
         D_out = D_embed * levels + D_feature
         o = embeddings.new_empty(*coords.shape[:-1], D_out)
         step = divider if divider is not None else levels
+        order = launch.order(any(ctx.needs_input_grad)) if divider is None and bwd_divider is None else None
         with torch.cuda.device(device):
             stream = _lib.stream_ptr(device)
-            for begin in range(0, levels, step):
+            if order is not None:
+                _lib.check(
+                    _lib.lib().th_hash_fwd_ordered(
+                        order.data_ptr(), 0, table.data_ptr(), _lib.dtype_code(table), o.data_ptr(), D_out, launch.n, D_in, D_embed,
+                        levels, launch.res, launch.rows, launch.offsets, launch.primes, 0, levels, stream,
+                    ),
+                    "th_hash_fwd_ordered",
+                )  # fmt: skip
+            for begin in range(0, levels if order is None else 0, step):
                 _lib.check(
                     _lib.lib().th_hash_fwd(
                         *launch.coord_args, table.data_ptr(), _lib.dtype_code(table), o.data_ptr(), D_out,
@@ -247,6 +285,7 @@ class HashEncoding(torch.autograd.Function):
 
         ctx.save_for_backward(coords, embeddings, pi)
         ctx.prime_values = launch.prime_values  # the backward pass needs no second look at `pi`
+        ctx.order = order if any(ctx.needs_input_grad) else None
         ctx.max_entries_per_level = max_entries_per_level
         ctx.min_res = min_res
         ctx.max_res = max_res
@@ -270,7 +309,7 @@ class HashEncoding(torch.autograd.Function):
         de = torch.zeros(embeddings.shape, dtype=embeddings.dtype, device=embeddings.device)
         step = ctx.bwd_divider if ctx.bwd_divider is not None else levels
         for begin in range(0, levels, step):
-            _launch_backward(launch, do, de, D_in, D_embed, levels, begin, begin + step)
+            _launch_backward(launch, do, de, D_in, D_embed, levels, begin, begin + step, ctx.order)
         return None, de, None, None, None, None, None, None, None, None, None
 
     @staticmethod
