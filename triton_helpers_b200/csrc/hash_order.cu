@@ -506,16 +506,17 @@ int launch_bwd_ordered(const LevelParams &P, const float4 *order, int keep_order
 
 using namespace th;
 
-// Where the order pays (B200, microseconds of all kernels, unordered -> ordered, sorting included).  A batch needs enough
-// points for several of them to meet in a cell of the middle levels, which takes fewer in two dimensions than in three;
-// clustered batches gain earlier (65 536 points: 96 -> 76) but are not known here.
-//   forward + backward, D = 3, 2 features: 2^16 uniform 70 -> 76, 2^17 122 -> 132, 2^18 233 -> 224, 2^19 346 -> 336,
-//     2^21 1328 -> 1112, 300 001 clustered 294 -> 210;  D = 2: 2^15 31 -> 31, 2^16 63 -> 41, 200 003 175 -> 90
-//   forward alone (sorting costs 14 us at 2^18, 55 at 2^21): 2^18 89 -> 85, 2^19 136 -> 122, 2^20 247 -> 171, 2^21 552 -> 404
-extern "C" int th_hash_order_pays(int64_t n_points, int n_dims, int backward) {
+// Where the order pays (B200, forward + backward with the sorting, unordered time / ordered time, uniform points):
+//   D = 3, 16 levels: 2^16 0.83-0.91, 2^17 0.83-1.11, 2^18 0.90-1.14, 2^19 0.95-1.18, 2^20 1.01-1.29, 2^21 1.03-1.20; clustered
+//     points, which the host cannot tell, gain more (300 001: 1.40, 2^22: 1.61)
+//   D = 2, rows of 16 bytes: 2^16 0.98, 2^17 1.19-1.47, 2^18 1.17-1.19, 2^20 1.11-1.31; smaller rows: from 2^18 on 0.79-1.07, because
+//     hash_bwd_coarse_kernel holds more of the levels there
+// Forward alone (sorting costs 14 us at 2^18 points, 55 at 2^21): D = 3 2^18 0.77-1.04, 2^19 1.06-1.18, 2^20 1.09-1.48; D = 2 with
+//   16-byte rows 2^18 0.99-1.37, 2^19 1.14-2.26, smaller rows 0.67-1.07 at every size.
+extern "C" int th_hash_order_pays(int64_t n_points, int n_dims, int row_bytes, int backward) {
     if (n_points >= (1ll << 31)) return 0;
-    if (!backward) return n_points >= (1 << 19);
-    return n_points >= (n_dims <= 2 ? 1 << 16 : 1 << 18);
+    if (n_dims >= 3) return n_points >= (1 << 19);
+    return row_bytes >= 16 && n_points >= (backward ? 1 << 17 : 1 << 18);
 }
 
 extern "C" int64_t th_hash_order_scratch_bytes(int64_t n_points, int n_dims) {

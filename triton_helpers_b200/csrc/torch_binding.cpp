@@ -425,7 +425,7 @@ PyObject *py_hash_encoding(PyObject *, PyObject *const *args, Py_ssize_t n_args)
             out = empty_like_shape(with_last(coords, call.feats * call.geo->levels), table.scalar_type(), table.device());
             const CoordArgs x = coord_args(coords, call.dims);
             void *stream = current_stream();
-            Tensor order = th_hash_order_pays(call.n, static_cast<int>(call.dims), grad) ? point_order(call, x, stream) : Tensor();
+            Tensor order = th_hash_order_pays(call.n, static_cast<int>(call.dims), static_cast<int>(call.feats * table.element_size()), grad) ? point_order(call, x, stream) : Tensor();
             hash_forward(call, x, order, table, out, stream);
             if (grad) node->order = std::move(order);
         }
