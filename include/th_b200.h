@@ -138,6 +138,18 @@ int th_hash_bwd_ordered(const void *order_dev, int keep_order, const void *grad_
                         const int32_t *level_res_host, const int64_t *level_rows_host, const int64_t *level_offset_host,
                         const int64_t *primes_host, int level_begin, int level_end, void *stream);
 
+/* th_hash_fwd / th_hash_bwd over all levels of a float32 table with 16-bit activations: outputs rounded to out_dtype,
+ * gradients read in go_dtype (TH_F16 or TH_BF16).  What a cast next to the call would compute, without its pass over the
+ * rows.  n_dims 2 or 3, n_feats 2 or 4, tables 16-byte aligned.  No counterpart in the reference. */
+int th_hash_fwd_cast(const void *coords_dev, int64_t coord_stride_n, int64_t coord_stride_d, int coord_dtype,
+                     const float *table_dev, void *out_dev, int out_dtype, int64_t out_stride_n, int64_t n_points, int n_dims,
+                     int n_feats, int n_levels, const int32_t *level_res_host, const int64_t *level_rows_host,
+                     const int64_t *level_offset_host, const int64_t *primes_host, float scale, void *stream);
+int th_hash_bwd_cast(const void *coords_dev, int64_t coord_stride_n, int64_t coord_stride_d, int coord_dtype,
+                     const void *grad_out_dev, int go_dtype, int64_t go_stride_n, float *grad_table_dev, int64_t n_points,
+                     int n_dims, int n_feats, int n_levels, const int32_t *level_res_host, const int64_t *level_rows_host,
+                     const int64_t *level_offset_host, const int64_t *primes_host, float scale, void *stream);
+
 /* Device-side status word of the encoding kernels: 0 = fine, 1 = a shared-memory accumulation of the
  * backward pass (compare-and-swap loop, bounded) gave up and dropped an update.  Synchronises the device.
  * No counterpart in the reference. */
@@ -189,6 +201,16 @@ int th_mlp_fwd_mse(const void *x_dev, int64_t x_stride, const void *w_in_dev, co
                    void *out_dev, int64_t out_stride, const void *target_dev, int64_t target_stride, void *grad_dev,
                    int64_t grad_stride, float *loss_sum_dev, float grad_scale, int64_t rows, int d_in, int d_hidden,
                    int d_out, int depth, int activation, int dtype, void *stream);
+
+/* The same for rows in the order of a spatially ordered batch (order_dev of th_hash_order; null: rows in their own order):
+ * row r is compared with the target of point r of the order.  target_dtype: the network's, or TH_F32 (the difference is
+ * then formed with the unrounded target).  *loss_sum_dev receives the squared
+ * errors times loss_scale; the prediction is not kept. */
+int th_mlp_fwd_mse_ordered(const void *x_dev, int64_t x_stride, const void *w_in_dev, const void *b_in_dev, const void *w_hid_dev,
+                           const void *b_hid_dev, const void *w_out_dev, const void *b_out_dev, const void *target_dev,
+                           int64_t target_stride, int target_dtype, const void *order_dev, void *grad_dev, int64_t grad_stride,
+                           float *loss_sum_dev, float loss_scale, float grad_scale, int64_t rows, int d_in, int d_hidden, int d_out,
+                           int depth, int activation, int dtype, void *stream);
 
 /* Device-side status word of the tensor-core MLP kernels (th_mlp_*, th_field_*): 0 = fine, non-zero =
  * one of their bounded waits ran out (the kernel then returned early and its results are invalid).
@@ -351,6 +373,15 @@ int th_mse_grad(const void *pred_dev, const void *target_dev, void *grad_dev, fl
 int th_adam_step(void *param_dev, void *grad_dev, float *exp_avg_dev, float *exp_avg_sq_dev, int64_t n_elems,
                  float lr, float beta1, float beta2, float eps, int step, float grad_scale, int zero_grad,
                  int dtype, int *skipped_dev, void *stream);
+
+/* th_adam_step for up to 16 tensors of one dtype in one launch; arrays of n_tensors entries (host). */
+int th_adam_steps(int n_tensors, void *const *param_dev, void *const *grad_dev, float *const *exp_avg_dev,
+                  float *const *exp_avg_sq_dev, const int64_t *n_elems, const float *grad_scale, const int *zero_grad, float lr,
+                  float beta1, float beta2, float eps, int step, int dtype, int *skipped_dev, void *stream);
+
+/* dst = src converted, up to 16 tensors in one launch; one of the two dtypes is TH_F32, the other a 16-bit one. */
+int th_cast(int n_tensors, const void *const *src_dev, void *const *dst_dev, const int64_t *n_elems, int src_dtype, int dst_dtype,
+            void *stream);
 
 /* dst[i] = src[i] * scale rounded to `dtype`: turns the fp32 sums th_mlp_bwd leaves in its workspace
  * (laid out [w_in | w_hid | w_out | b_in | b_hid | b_out]) into a normalised 16-bit gradient buffer. */

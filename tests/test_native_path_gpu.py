@@ -9,6 +9,7 @@ from triton_helpers_b200.layers.hash_encoding import HashEncoding, hash_encoding
 from triton_helpers_b200.layers.hash_encoding.helpers import level_geometry
 from triton_helpers_b200.layers.neural_field import hash_encoded_mlp
 from triton_helpers_b200.layers.reversible_mlp import ReversibleMLP
+from triton_helpers_b200.training import NeuralFieldTrainer
 
 pytestmark = pytest.mark.gpu
 
@@ -49,7 +50,8 @@ def test_hash_encoding(shape, dtype, own_primes):
 
 
 @pytest.mark.parametrize("rows,bias,depth,activation,dtype", [(1, True, 1, "relu", torch.float16), (300, True, 3, "silu", torch.bfloat16),
-                                                              (129, False, 2, "none", torch.float16)])  # fmt: skip
+                                                              (129, False, 2, "none", torch.float16), (1, True, 1, "relu", torch.float32),
+                                                              (300, True, 3, "silu", torch.float32)])  # fmt: skip
 def test_fused_mlp(rows, bias, depth, activation, dtype):
     layer = FullyFusedMLP(16, 32, 8, depth, activation, bias=bias).cuda().to(dtype)
     x = torch.randn(1, rows, 16, device="cuda").to(dtype).requires_grad_(True)
@@ -110,3 +112,31 @@ def test_what_the_native_path_leaves_to_python():
     y = fully_fused_mlp(x, *args)
     y.sum().backward()
     assert layer.w_in.grad is not None and x.grad is None  # w_in.grad: from the first pass above
+
+
+@pytest.mark.parametrize("n,dtype,bias,depth", [(1, torch.float16, False, 1), (1000, torch.bfloat16, True, 3), (2**19 + 3, torch.float16, False, 2),
+                                                (1, torch.float32, True, 1), (5003, torch.float32, False, 3)])  # fmt: skip
+def test_training_step(n, dtype, bias, depth):
+    # the last 16-bit case runs over spatially ordered points
+    def train(deferred):
+        torch.manual_seed(0)
+        encoding, mlp = HashEncoding(2**12, 8, 3, 2, 16, 256), FullyFusedMLP(16, 32, 8, depth, bias=bias)
+        with torch.no_grad():
+            encoding.embeddings.mul_(0.1)
+        trainer = NeuralFieldTrainer(encoding.cuda().to(dtype), mlp.cuda().to(dtype), lr=1e-3, fused=False)
+        g = torch.Generator(device="cuda").manual_seed(3)
+        x, t = torch.rand(n, 3, device="cuda", generator=g), torch.rand(n, 8, device="cuda", generator=g).to(dtype)
+        _lib.native().defer(deferred)
+        try:
+            losses = [float(trainer.step(x, t)) for _ in range(3)]
+        finally:
+            _lib.native().defer(False)
+        assert trainer.skipped_elements() == 0
+        return losses, [p.detach().double() for p in trainer.parameters()], trainer._state is not None
+
+    (loss_n, params_n, state_n), (loss_p, params_p, _) = train(False), train(True)
+    assert state_n, "the native step keeps buffers"
+    for a, b in zip(loss_n, loss_p):
+        assert abs(a - b) <= 2e-3 * abs(b)
+    for a, b in zip(params_n, params_p):  # Adam's first steps are lr * sign: entries whose gradient nearly cancels may differ
+        assert float((a - b).norm() / b.norm()) <= 2e-3

@@ -26,6 +26,7 @@ TH_ERR_UNSUPPORTED = -2  # include/th_b200.h
 
 _I32P = ctypes.POINTER(c_int32)
 _I64P = ctypes.POINTER(c_int64)
+_PTRP = ctypes.POINTER(c_void_p)
 
 # name -> (restype, argtypes); every symbol include/th_b200.h declares
 SIGNATURES = {
@@ -45,6 +46,16 @@ SIGNATURES = {
         c_int,
         [c_void_p, c_int64, c_int64, c_int, c_void_p, c_void_p, c_int64, c_int, c_int, _I32P, _I64P, _I64P,
          c_float, c_void_p],
+    ),
+    "th_hash_fwd_cast": (
+        c_int,
+        [c_void_p, c_int64, c_int64, c_int, c_void_p, c_void_p, c_int, c_int64, c_int64, c_int, c_int, c_int,
+         _I32P, _I64P, _I64P, _I64P, c_float, c_void_p],
+    ),
+    "th_hash_bwd_cast": (
+        c_int,
+        [c_void_p, c_int64, c_int64, c_int, c_void_p, c_int, c_int64, c_void_p, c_int64, c_int, c_int, c_int,
+         _I32P, _I64P, _I64P, _I64P, c_float, c_void_p],
     ),
     "th_hash_order_pays": (c_int, [c_int64, c_int, c_int, c_int]),
     "th_hash_order_scratch_bytes": (c_int64, [c_int64, c_int]),
@@ -87,6 +98,11 @@ SIGNATURES = {
         [c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_void_p,
          c_int64, c_void_p, c_int64, c_void_p, c_float, c_int64, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
     ),
+    "th_mlp_fwd_mse_ordered": (
+        c_int,
+        [c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int, c_void_p,
+         c_void_p, c_int64, c_void_p, c_float, c_float, c_int64, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
+    ),
     "th_mlp_workspace_bytes": (c_int64, [c_int, c_int, c_int, c_int]),
     "th_mlp_tc_status": (c_int, []),
     "th_mlp_tma_available": (c_int, []),
@@ -120,6 +136,12 @@ SIGNATURES = {
         [c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_float, c_float, c_float, c_float, c_int, c_float, c_int,
          c_int, c_void_p, c_void_p],
     ),
+    "th_adam_steps": (
+        c_int,
+        [c_int, _PTRP, _PTRP, _PTRP, _PTRP, _I64P, ctypes.POINTER(c_float), ctypes.POINTER(c_int), c_float, c_float, c_float,
+         c_float, c_int, c_int, c_void_p, c_void_p],
+    ),
+    "th_cast": (c_int, [c_int, _PTRP, _PTRP, _I64P, c_int, c_int, c_void_p]),
     "th_scale_cast": (c_int, [c_void_p, c_void_p, c_int64, c_float, c_int, c_void_p]),
     "th_launch_count": (ctypes.c_longlong, []),
 }  # fmt: skip
@@ -134,7 +156,8 @@ class KernelTimer:
     """
 
     LAUNCHING = ("th_field_fwd", "th_field_bwd", "th_hash_fwd", "th_hash_bwd", "th_hash_order", "th_hash_fwd_ordered", "th_hash_bwd_ordered", "th_mlp_fwd", "th_mlp_fwd_mse", "th_mlp_bwd", "th_rev_fwd", "th_rev_bwd",
-                 "th_mse_grad", "th_adam_step", "th_scale_cast")  # fmt: skip
+                 "th_hash_fwd_cast", "th_hash_bwd_cast", "th_mlp_fwd_mse_ordered", "th_mse_grad", "th_adam_step", "th_adam_steps", "th_cast",
+                 "th_scale_cast")  # fmt: skip
 
     def __init__(self):
         self.records = []

@@ -410,6 +410,7 @@ int launch_mlp_bwd(const MlpShape &s, const MlpParams &p, const void *x, int64_t
             gx ? pairs_ok(gx, gx_stride, s.d_in) : 0);
         if (int rc = launch_status("mlp_bwd_kernel launch")) return rc;
     }
+    if (!dw_in && !dw_hid && !dw_out && !db_in && !db_hid && !db_out) return TH_OK;  // the caller takes the float32 sums
     mlp_grad_convert_kernel<T><<<(W.total + 255) / 256, 256, 0, stream>>>(
         s, workspace, static_cast<T *>(dw_in), static_cast<T *>(dw_hid), static_cast<T *>(dw_out),
         static_cast<T *>(db_in), static_cast<T *>(db_hid), static_cast<T *>(db_out));
@@ -451,27 +452,50 @@ extern "C" int th_mlp_fwd(const void *x_dev, int64_t x_stride, const void *w_in_
     }
 }
 
-extern "C" int th_mlp_fwd_mse(const void *x_dev, int64_t x_stride, const void *w_in_dev, const void *b_in_dev,
+static int fwd_mse(const void *x_dev, int64_t x_stride, const void *w_in_dev, const void *b_in_dev,
                               const void *w_hid_dev, const void *b_hid_dev, const void *w_out_dev, const void *b_out_dev,
                               void *out_dev, int64_t out_stride, const void *target_dev, int64_t target_stride,
                               void *grad_dev, int64_t grad_stride, float *loss_sum_dev, float grad_scale, int64_t rows,
-                              int d_in, int d_hidden, int d_out, int depth, int activation, int dtype, void *stream) {
+                              int d_in, int d_hidden, int d_out, int depth, int activation, int dtype, int target_dtype, const void *order_dev,
+                              float loss_scale, void *stream) {
     if (rows < 0) return fail(TH_ERR_BAD_ARG, "negative row count");
     const bool has_bias = b_in_dev || b_hid_dev || b_out_dev;
     MlpShape s;
     if (int rc = make_shape(s, d_in, d_hidden, d_out, depth, activation, has_bias)) return rc;
     MlpParams p{w_in_dev, w_hid_dev, w_out_dev, b_in_dev, b_hid_dev, b_out_dev};
     if (int rc = check_params(s, p, has_bias)) return rc;
+    if (target_dtype != dtype && target_dtype != TH_F32) return fail(TH_ERR_BAD_ARG, "targets are float32 or of the network's dtype");
+    if (order_dev && !aligned_to(order_dev, 16)) return fail(TH_ERR_ALIGNMENT, "the order must be 16-byte aligned");
     if (rows == 0) return TH_OK;
     if (!x_dev || !target_dev || !grad_dev) return fail(TH_ERR_BAD_ARG, "null input, target or gradient");
     if (x_stride < d_in || target_stride < d_out || grad_stride < d_out || (out_dev && out_stride < d_out))
         return fail(TH_ERR_BAD_ARG, "row stride smaller than the row");
-    const MseArgs mse{target_dev, target_stride, grad_dev, grad_stride, loss_sum_dev, grad_scale};
+    const MseArgs mse{target_dev, target_stride, grad_dev, grad_stride, loss_sum_dev, grad_scale, static_cast<const float4 *>(order_dev), loss_scale,
+                      target_dtype == TH_F32 ? 1 : 0};
     const int rc = mlp_fwd_mse_tc(s, p, x_dev, x_stride, out_dev, out_stride, mse, rows, dtype, static_cast<cudaStream_t>(stream));
     if (rc == kTcNotApplicable)
         return fail(TH_ERR_UNSUPPORTED, "fused forward + MSE needs float16 / bfloat16 rows of whole 16-byte chunks "
                                         "(d_in, d_out multiples of 8, aligned) and a network the multi-slot kernel holds");
     return rc;
+}
+
+extern "C" int th_mlp_fwd_mse(const void *x_dev, int64_t x_stride, const void *w_in_dev, const void *b_in_dev,
+                              const void *w_hid_dev, const void *b_hid_dev, const void *w_out_dev, const void *b_out_dev,
+                              void *out_dev, int64_t out_stride, const void *target_dev, int64_t target_stride,
+                              void *grad_dev, int64_t grad_stride, float *loss_sum_dev, float grad_scale, int64_t rows,
+                              int d_in, int d_hidden, int d_out, int depth, int activation, int dtype, void *stream) {
+    return fwd_mse(x_dev, x_stride, w_in_dev, b_in_dev, w_hid_dev, b_hid_dev, w_out_dev, b_out_dev, out_dev, out_stride, target_dev, target_stride,
+                   grad_dev, grad_stride, loss_sum_dev, grad_scale, rows, d_in, d_hidden, d_out, depth, activation, dtype, dtype, nullptr, 1.f, stream);
+}
+
+extern "C" int th_mlp_fwd_mse_ordered(const void *x_dev, int64_t x_stride, const void *w_in_dev, const void *b_in_dev,
+                                      const void *w_hid_dev, const void *b_hid_dev, const void *w_out_dev, const void *b_out_dev,
+                                      const void *target_dev, int64_t target_stride, int target_dtype, const void *order_dev, void *grad_dev,
+                                      int64_t grad_stride, float *loss_sum_dev, float loss_scale, float grad_scale, int64_t rows, int d_in,
+                                      int d_hidden, int d_out, int depth, int activation, int dtype, void *stream) {
+    return fwd_mse(x_dev, x_stride, w_in_dev, b_in_dev, w_hid_dev, b_hid_dev, w_out_dev, b_out_dev, nullptr, d_out, target_dev, target_stride,
+                   grad_dev, grad_stride, loss_sum_dev, grad_scale, rows, d_in, d_hidden, d_out, depth, activation, dtype, target_dtype, order_dev,
+                   loss_scale, stream);
 }
 
 extern "C" int th_mlp_bwd(const void *x_dev, int64_t x_stride, const void *w_in_dev, const void *b_in_dev,

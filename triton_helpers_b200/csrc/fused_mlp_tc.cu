@@ -344,14 +344,20 @@ mlp_fwd_pipe_kernel(const MlpShape s, const MlpParams p, const __grid_constant__
                     if constexpr (MSE) {
                         // d_out is a multiple of 8 and all rows are 16-byte aligned here (checked by the launcher)
                         const long long r = live ? row0 + row : 0;
-                        const T *target_row = static_cast<const T *>(mse.target) + r * mse.target_stride;
+                        const long long tr = (mse.order && live) ? static_cast<long long>(__float_as_uint(mse.order[r].w)) : r;
+                        const T *target_row = static_cast<const T *>(mse.target) + tr * mse.target_stride;
+                        const float *target_row_f32 = static_cast<const float *>(mse.target) + tr * mse.target_stride;
                         T *grad_row = static_cast<T *>(mse.grad) + r * mse.grad_stride;
                         T *out_row = y ? y + r * y_stride : nullptr;
                         drain_row<T, TH_ACT_NONE, BIAS>(taddr, out_pad, layer_bias, [&](int chunk, uint4 packed) {
                             if (live && 8 * chunk < s.d_out) {
                                 if (out_row) __stcs(reinterpret_cast<uint4 *>(out_row + 8 * chunk), packed);
-                                const uint4 t = __ldcs(reinterpret_cast<const uint4 *>(target_row + 8 * chunk));
-                                __stcs(reinterpret_cast<uint4 *>(grad_row + 8 * chunk), mse_chunk<T>(packed, t, mse.grad_scale, loss));
+                                uint4 g;
+                                if (mse.target_f32)
+                                    g = mse_chunk_f32<T>(packed, target_row_f32 + 8 * chunk, mse.grad_scale, loss);
+                                else
+                                    g = mse_chunk<T>(packed, __ldcs(reinterpret_cast<const uint4 *>(target_row + 8 * chunk)), mse.grad_scale, loss);
+                                __stcs(reinterpret_cast<uint4 *>(grad_row + 8 * chunk), g);
                             }
                         });
                     } else {
@@ -370,7 +376,7 @@ mlp_fwd_pipe_kernel(const MlpShape s, const MlpParams p, const __grid_constant__
     if constexpr (MSE) {
         // one atomic per warp for the whole kernel
         for (int off = 16; off > 0; off >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, off);
-        if ((threadIdx.x & 31) == 0 && mse.loss_sum) atomicAdd(mse.loss_sum, loss);
+        if ((threadIdx.x & 31) == 0 && mse.loss_sum) atomicAdd(mse.loss_sum, loss * mse.loss_scale);
     }
 
     // ---- teardown ----
@@ -1471,7 +1477,9 @@ int mlp_fwd_mse_tc(const MlpShape &s, const MlpParams &p, const void *x, int64_t
     if (tc_disabled() || rows <= 0) return kTcNotApplicable;
     if (s.h != 16 && s.h != 32 && s.h != 64) return kTcNotApplicable;
     // whole 16-byte chunks of every row: prediction (if kept), target and gradient
-    if (s.d_out % 8 != 0 || !rows_vector_ok(mse.target, mse.target_stride, s.d_out) ||
+    const bool target_ok = mse.target_f32 ? aligned_to(mse.target, 16) && mse.target_stride % 4 == 0
+                                          : rows_vector_ok(mse.target, mse.target_stride, s.d_out);
+    if (s.d_out % 8 != 0 || !target_ok ||
         !rows_vector_ok(mse.grad, mse.grad_stride, s.d_out) || (y && !rows_vector_ok(y, y_stride, s.d_out)))
         return kTcNotApplicable;
     switch (dtype) {

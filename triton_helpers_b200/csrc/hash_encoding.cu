@@ -34,10 +34,11 @@ namespace {
 // ---- forward --------------------------------------------------------------------------------
 
 // ORDERED: the points come from a spatially ordered batch; output rows are the caller's (`keep_order` 0) or in order too.
-template <typename T, int D, int F, int LG, bool ORDERED>
+// TO: type of the outputs, the table's own or a 16-bit one that the float32 result is rounded to (what a cast after it would do).
+template <typename T, typename TO, int D, int F, int LG, bool ORDERED>
 __global__ void __launch_bounds__(kThreads)
 hash_fwd_kernel(const __grid_constant__ LevelParams P, const CoordView cv, const float4 *__restrict__ order, int keep_order,
-                const T *__restrict__ table, T *__restrict__ out, long long out_stride, long long n_points, int level_begin,
+                const T *__restrict__ table, TO *__restrict__ out, long long out_stride, long long n_points, int level_begin,
                 int level_end, int vector_ok) {
     constexpr int kPoints = kThreads / 2;
     constexpr int kSide = 1 << (D - 1);   // corners per lane
@@ -65,7 +66,7 @@ hash_fwd_kernel(const __grid_constant__ LevelParams P, const CoordView cv, const
         for (int d = 0; d < D; ++d) x[d] = 0.f;
     }
     const int side = threadIdx.x & 1;
-    T *out_row = out + (live ? i : 0) * out_stride;
+    TO *out_row = out + (live ? i : 0) * out_stride;
 
     // gridDim.y CTAs share a point tile and take every gridDim.y-th level group each
     for (int lg = level_begin + LG * blockIdx.y; lg < level_end; lg += LG * gridDim.y) {
@@ -104,12 +105,12 @@ hash_fwd_kernel(const __grid_constant__ LevelParams P, const CoordView cv, const
                 float part[kFirst];
 #pragma unroll
                 for (int k = 0; k < kFirst; ++k) part[k] = acc[k];
-                store_elems<T, kFirst>(out_row + lg * F, part, vector_ok);
+                store_elems<TO, kFirst>(out_row + lg * F, part, vector_ok);
             } else if constexpr (kCount - kFirst > 0) {
                 float part[kCount - kFirst];
 #pragma unroll
                 for (int k = 0; k < kCount - kFirst; ++k) part[k] = acc[kFirst + k];
-                store_elems<T, kCount - kFirst>(out_row + lg * F + kFirst, part, vector_ok);
+                store_elems<TO, kCount - kFirst>(out_row + lg * F + kFirst, part, vector_ok);
             }
         }
     }
@@ -117,9 +118,10 @@ hash_fwd_kernel(const __grid_constant__ LevelParams P, const CoordView cv, const
 
 // ---- backward -------------------------------------------------------------------------------
 
-template <typename T, int D, int F, int LG>
+// TG: type of grad_out, the table gradient's own or a 16-bit one
+template <typename T, typename TG, int D, int F, int LG>
 __global__ void __launch_bounds__(kThreads)
-hash_bwd_kernel(const __grid_constant__ LevelParams P, const CoordView cv, const T *__restrict__ grad_out,
+hash_bwd_kernel(const __grid_constant__ LevelParams P, const CoordView cv, const TG *__restrict__ grad_out,
                 long long go_stride, T *__restrict__ grad_table, long long n_points, int level_begin,
                 int level_end, int vector_ok, int skip_below) {
     // levels below `skip_below` were accumulated by hash_bwd_coarse_kernel and are passed over here
@@ -140,14 +142,14 @@ hash_bwd_kernel(const __grid_constant__ LevelParams P, const CoordView cv, const
     }
     const int side = threadIdx.x & 1;
     const long long i = static_cast<long long>(blockIdx.x) * kPoints + (threadIdx.x >> 1);
-    const T *go_row = grad_out + (live ? i : 0) * go_stride;
+    const TG *go_row = grad_out + (live ? i : 0) * go_stride;
     const unsigned lane = threadIdx.x & 31u;
 
     // gridDim.y CTAs share a point tile and take every gridDim.y-th level group each
     for (int lg = level_begin + LG * blockIdx.y; lg < level_end; lg += LG * gridDim.y) {
         float go[LG * F];
         if (live) {
-            load_elems_checked<T, LG * F>(go_row + lg * F, go, vector_ok);  // both lanes of a pair: one broadcast load
+            load_elems_checked<TG, LG * F>(go_row + lg * F, go, vector_ok);  // both lanes of a pair: one broadcast load
         } else {
 #pragma unroll
             for (int k = 0; k < LG * F; ++k) go[k] = 0.f;
@@ -237,9 +239,9 @@ hash_bwd_kernel(const __grid_constant__ LevelParams P, const CoordView cv, const
 constexpr int kCoarseThreads = 1024;
 constexpr int kCoarseSmemBytes = 200 * 1024;
 
-template <typename T, int D, int F>
+template <typename T, typename TG, int D, int F>
 __global__ void __launch_bounds__(kCoarseThreads, 1)
-hash_bwd_coarse_kernel(const __grid_constant__ LevelParams P, const CoordView cv, const T *__restrict__ grad_out,
+hash_bwd_coarse_kernel(const __grid_constant__ LevelParams P, const CoordView cv, const TG *__restrict__ grad_out,
                        long long go_stride, T *__restrict__ grad_table, long long n_points, int level_begin,
                        int level_end, long long points_per_cta) {
     extern __shared__ __align__(16) unsigned char coarse_smem[];
@@ -276,7 +278,7 @@ hash_bwd_coarse_kernel(const __grid_constant__ LevelParams P, const CoordView cv
             corner_weights<D>(t, w);
             corner_indices<D>(cell, P, level, idx);
 #pragma unroll
-            for (int f = 0; f < F; ++f) go[f] = live ? to_float<T>(grad_out[i * go_stride + level * F + f]) : 0.f;
+            for (int f = 0; f < F; ++f) go[f] = live ? to_float<TG>(grad_out[i * go_stride + level * F + f]) : 0.f;
             T *base = acc + (P.offset[level] - first_row) * F;
 
             // lanes that meet in one cell (clustered inputs) are summed in registers first and one of
@@ -406,27 +408,36 @@ dim3 point_level_grid(int64_t n, int l0, int l1, int levels_per_group) {
     return dim3(static_cast<unsigned>(tiles), static_cast<unsigned>(split), 1);
 }
 
-template <typename T, int D, int F>
+template <typename T, typename TO, int D, int F, int LG>
+void start_fwd(dim3 grid, cudaStream_t stream, const LevelParams &P, const CoordView &cv, const float4 *order, int keep_order, const T *table,
+               TO *out, int64_t out_stride, int64_t n, int a, int b, int vec) {
+    if constexpr (std::is_same<T, TO>::value) {
+        if (order) {
+            hash_fwd_kernel<T, TO, D, F, LG, true><<<grid, kThreads, 0, stream>>>(P, cv, order, keep_order, table, out, out_stride, n, a, b, vec);
+            return;
+        }
+    }
+    hash_fwd_kernel<T, TO, D, F, LG, false><<<grid, kThreads, 0, stream>>>(P, cv, nullptr, 0, table, out, out_stride, n, a, b, vec);
+}
+
+template <typename T, typename TO, int D, int F>
 int launch_fwd(const LevelParams &P, const CoordView &cv, const float4 *order, int keep_order, const void *table, void *out, int64_t out_stride,
                int64_t n, int l0, int l1, cudaStream_t stream) {
-    const int vec = aligned_to(out, 16) && (out_stride * sizeof(T)) % 16 == 0;
+    const int vec = aligned_to(out, 16) && (out_stride * sizeof(TO)) % 16 == 0;
     const T *tb = static_cast<const T *>(table);
-    T *o = static_cast<T *>(out);
+    TO *o = static_cast<TO *>(out);
     // Ordered points write their rows in random order: passes that fill whole sectors of a row (2^22 clustered points, rows
     // of 4 x 16 float32, one 64 MB level per pass 2.70 ms, two 1.51 ms).
-    const int least = order && F * sizeof(T) < 32 ? static_cast<int>(32 / (F * sizeof(T))) : 1;
+    const int least = order && F * sizeof(TO) < 32 ? static_cast<int>(32 / (F * sizeof(TO))) : 1;
     const LevelPasses passes = plan_level_passes(P, n, l0, l1, F * sizeof(T), least);
     for (int p = 0; p < passes.count; ++p) {
         const int a = passes.begin[p], b = passes.end[p];
         const int lg = pick_level_group(a, b, F);
         const dim3 grid = point_level_grid(n, a, b, lg);
         switch (lg) {
-            case 4: order ? hash_fwd_kernel<T, D, F, 4, true><<<grid, kThreads, 0, stream>>>(P, cv, order, keep_order, tb, o, out_stride, n, a, b, vec)
-                          : hash_fwd_kernel<T, D, F, 4, false><<<grid, kThreads, 0, stream>>>(P, cv, order, 0, tb, o, out_stride, n, a, b, vec); break;
-            case 2: order ? hash_fwd_kernel<T, D, F, 2, true><<<grid, kThreads, 0, stream>>>(P, cv, order, keep_order, tb, o, out_stride, n, a, b, vec)
-                          : hash_fwd_kernel<T, D, F, 2, false><<<grid, kThreads, 0, stream>>>(P, cv, order, 0, tb, o, out_stride, n, a, b, vec); break;
-            default: order ? hash_fwd_kernel<T, D, F, 1, true><<<grid, kThreads, 0, stream>>>(P, cv, order, keep_order, tb, o, out_stride, n, a, b, vec)
-                          : hash_fwd_kernel<T, D, F, 1, false><<<grid, kThreads, 0, stream>>>(P, cv, order, 0, tb, o, out_stride, n, a, b, vec); break;
+            case 4: start_fwd<T, TO, D, F, 4>(grid, stream, P, cv, order, keep_order, tb, o, out_stride, n, a, b, vec); break;
+            case 2: start_fwd<T, TO, D, F, 2>(grid, stream, P, cv, order, keep_order, tb, o, out_stride, n, a, b, vec); break;
+            default: start_fwd<T, TO, D, F, 1>(grid, stream, P, cv, order, keep_order, tb, o, out_stride, n, a, b, vec); break;
         }
         if (int rc = launch_status("hash_fwd_kernel launch")) return rc;
     }
@@ -454,10 +465,10 @@ int coarse_level_end(const LevelParams &P, int64_t n, int l0, int l1, int dims) 
     return end;
 }
 
-template <typename T, int D, int F>
+template <typename T, typename TG, int D, int F>
 int launch_bwd(const LevelParams &P, const CoordView &cv, const void *go, int64_t go_stride, void *grad_table,
                int64_t n, int l0, int l1, cudaStream_t stream) {
-    const T *g = static_cast<const T *>(go);
+    const TG *g = static_cast<const TG *>(go);
     T *gt = static_cast<T *>(grad_table);
     // 1. coarse levels in shared memory
     const int coarse_end = coarse_level_end<T, F>(P, n, l0, l1, D);
@@ -465,7 +476,7 @@ int launch_bwd(const LevelParams &P, const CoordView &cv, const void *go, int64_
         size_t bytes = 0;
         for (int l = l0; l < coarse_end; ++l) bytes += static_cast<size_t>(P.rows[l]) * F * sizeof(T);
         bytes = (bytes + 15) & ~static_cast<size_t>(15);
-        auto kernel = hash_bwd_coarse_kernel<T, D, F>;
+        auto kernel = hash_bwd_coarse_kernel<T, TG, D, F>;
         if (int rc = cuda_status(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)),
                                  "cudaFuncSetAttribute(hash_bwd_coarse_kernel)")) return rc;
         const int ctas = sm_count();
@@ -475,7 +486,7 @@ int launch_bwd(const LevelParams &P, const CoordView &cv, const void *go, int64_
         if (coarse_end == l1) return TH_OK;
     }
     // 2. everything else with global reductions, in passes that keep the rows being updated in L2
-    const int vec = aligned_to(go, 16) && (go_stride * sizeof(T)) % 16 == 0;
+    const int vec = aligned_to(go, 16) && (go_stride * sizeof(TG)) % 16 == 0;
     const LevelPasses passes = plan_level_passes(P, n, l0, l1, F * sizeof(T));
     for (int p = 0; p < passes.count; ++p) {
         const int a = passes.begin[p], b = passes.end[p];
@@ -483,9 +494,9 @@ int launch_bwd(const LevelParams &P, const CoordView &cv, const void *go, int64_
         const int lg = pick_level_group(a, b, F);
         const dim3 grid = point_level_grid(n, a, b, lg);
         switch (lg) {
-            case 4: hash_bwd_kernel<T, D, F, 4><<<grid, kThreads, 0, stream>>>(P, cv, g, go_stride, gt, n, a, b, vec, coarse_end); break;
-            case 2: hash_bwd_kernel<T, D, F, 2><<<grid, kThreads, 0, stream>>>(P, cv, g, go_stride, gt, n, a, b, vec, coarse_end); break;
-            default: hash_bwd_kernel<T, D, F, 1><<<grid, kThreads, 0, stream>>>(P, cv, g, go_stride, gt, n, a, b, vec, coarse_end); break;
+            case 4: hash_bwd_kernel<T, TG, D, F, 4><<<grid, kThreads, 0, stream>>>(P, cv, g, go_stride, gt, n, a, b, vec, coarse_end); break;
+            case 2: hash_bwd_kernel<T, TG, D, F, 2><<<grid, kThreads, 0, stream>>>(P, cv, g, go_stride, gt, n, a, b, vec, coarse_end); break;
+            default: hash_bwd_kernel<T, TG, D, F, 1><<<grid, kThreads, 0, stream>>>(P, cv, g, go_stride, gt, n, a, b, vec, coarse_end); break;
         }
         if (int rc = launch_status("hash_bwd_kernel launch")) return rc;
     }
@@ -522,7 +533,7 @@ extern "C" int th_hash_fwd(const void *coords_dev, int64_t coord_stride_n, int64
     if (!aligned_to(table_dev, row_bytes < 16 ? row_bytes : 16)) return fail(TH_ERR_ALIGNMENT, "table rows must be aligned to min(row bytes, 16)");
     if (out_stride_n < static_cast<int64_t>(n_levels) * n_feats) return fail(TH_ERR_BAD_ARG, "out_stride_n smaller than n_levels * n_feats");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-#define TH_CALL_FWD(T, D, F) launch_fwd<T, D, F>(P, cv, nullptr, 0, table_dev, out_dev, out_stride_n, n_points, level_begin, level_end, s)
+#define TH_CALL_FWD(T, D, F) launch_fwd<T, T, D, F>(P, cv, nullptr, 0, table_dev, out_dev, out_stride_n, n_points, level_begin, level_end, s)
     TH_DISPATCH(TH_CALL_FWD)
 #undef TH_CALL_FWD
 }
@@ -545,7 +556,7 @@ extern "C" int th_hash_bwd(const void *coords_dev, int64_t coord_stride_n, int64
     if (!aligned_to(grad_table_dev, row_bytes < 16 ? row_bytes : 16)) return fail(TH_ERR_ALIGNMENT, "table rows must be aligned to min(row bytes, 16)");
     if (go_stride_n < static_cast<int64_t>(n_levels) * n_feats) return fail(TH_ERR_BAD_ARG, "go_stride_n smaller than n_levels * n_feats");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-#define TH_CALL_BWD(T, D, F) launch_bwd<T, D, F>(P, cv, grad_out_dev, go_stride_n, grad_table_dev, n_points, level_begin, level_end, s)
+#define TH_CALL_BWD(T, D, F) launch_bwd<T, T, D, F>(P, cv, grad_out_dev, go_stride_n, grad_table_dev, n_points, level_begin, level_end, s)
     TH_DISPATCH(TH_CALL_BWD)
 #undef TH_CALL_BWD
 }
@@ -568,9 +579,64 @@ extern "C" int th_hash_fwd_ordered(const void *order_dev, int keep_order, const 
     const CoordView cv{};
     const float4 *order = static_cast<const float4 *>(order_dev);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-#define TH_CALL_FWD(T, D, F) launch_fwd<T, D, F>(P, cv, order, keep_order, table_dev, out_dev, out_stride_n, n_points, level_begin, level_end, s)
+#define TH_CALL_FWD(T, D, F) launch_fwd<T, T, D, F>(P, cv, order, keep_order, table_dev, out_dev, out_stride_n, n_points, level_begin, level_end, s)
     TH_DISPATCH(TH_CALL_FWD)
 #undef TH_CALL_FWD
+}
+
+// float32 tables next to 16-bit activations (a float32 model whose MLP runs with 16-bit operands): two or three dimensions,
+// two or four features.
+#define TH_DISPATCH_CAST(G, CALL)                                                                          \
+    switch (n_dims * 8 + n_feats) {                                                                        \
+        case 18: return CALL(G, 2, 2);                                                                     \
+        case 20: return CALL(G, 2, 4);                                                                     \
+        case 26: return CALL(G, 3, 2);                                                                     \
+        case 28: return CALL(G, 3, 4);                                                                     \
+        default: return fail(TH_ERR_UNSUPPORTED, "mixed types: %d dimensions, %d features", n_dims, n_feats); \
+    }
+
+extern "C" int th_hash_fwd_cast(const void *coords_dev, int64_t coord_stride_n, int64_t coord_stride_d, int coord_dtype, const float *table_dev,
+                                void *out_dev, int out_dtype, int64_t out_stride_n, int64_t n_points, int n_dims, int n_feats, int n_levels,
+                                const int32_t *level_res_host, const int64_t *level_rows_host, const int64_t *level_offset_host,
+                                const int64_t *primes_host, float scale, void *stream) {
+    if (n_points < 0) return fail(TH_ERR_BAD_ARG, "negative n_points");
+    LevelParams P;
+    CoordView cv;
+    if (int rc = fill_params(P, n_dims, n_levels, level_res_host, level_rows_host, level_offset_host, primes_host, scale)) return rc;
+    if (!level_offset_host) return fail(TH_ERR_BAD_ARG, "null level offsets");
+    if (n_points == 0) return TH_OK;
+    if (int rc = make_coord_view(cv, coords_dev, coord_stride_n, coord_stride_d, coord_dtype, n_dims)) return rc;
+    if (!table_dev || !out_dev) return fail(TH_ERR_BAD_ARG, "null table or output");
+    if (!aligned_to(table_dev, 16)) return fail(TH_ERR_ALIGNMENT, "the table must be 16-byte aligned");
+    if (out_stride_n < static_cast<int64_t>(n_levels) * n_feats) return fail(TH_ERR_BAD_ARG, "out_stride_n smaller than n_levels * n_feats");
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+#define TH_CALL_FWD(G, D, F) launch_fwd<float, G, D, F>(P, cv, nullptr, 0, table_dev, out_dev, out_stride_n, n_points, 0, n_levels, s)
+    if (out_dtype == TH_F16) TH_DISPATCH_CAST(__half, TH_CALL_FWD)
+    if (out_dtype == TH_BF16) TH_DISPATCH_CAST(__nv_bfloat16, TH_CALL_FWD)
+#undef TH_CALL_FWD
+    return fail(TH_ERR_BAD_ARG, "output dtype %d is not a 16-bit type", out_dtype);
+}
+
+extern "C" int th_hash_bwd_cast(const void *coords_dev, int64_t coord_stride_n, int64_t coord_stride_d, int coord_dtype, const void *grad_out_dev,
+                                int go_dtype, int64_t go_stride_n, float *grad_table_dev, int64_t n_points, int n_dims, int n_feats, int n_levels,
+                                const int32_t *level_res_host, const int64_t *level_rows_host, const int64_t *level_offset_host,
+                                const int64_t *primes_host, float scale, void *stream) {
+    if (n_points < 0) return fail(TH_ERR_BAD_ARG, "negative n_points");
+    LevelParams P;
+    CoordView cv;
+    if (int rc = fill_params(P, n_dims, n_levels, level_res_host, level_rows_host, level_offset_host, primes_host, scale)) return rc;
+    if (!level_offset_host) return fail(TH_ERR_BAD_ARG, "null level offsets");
+    if (n_points == 0) return TH_OK;
+    if (int rc = make_coord_view(cv, coords_dev, coord_stride_n, coord_stride_d, coord_dtype, n_dims)) return rc;
+    if (!grad_out_dev || !grad_table_dev) return fail(TH_ERR_BAD_ARG, "null gradient pointer");
+    if (!aligned_to(grad_table_dev, 16)) return fail(TH_ERR_ALIGNMENT, "the table gradient must be 16-byte aligned");
+    if (go_stride_n < static_cast<int64_t>(n_levels) * n_feats) return fail(TH_ERR_BAD_ARG, "go_stride_n smaller than n_levels * n_feats");
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+#define TH_CALL_BWD(G, D, F) launch_bwd<float, G, D, F>(P, cv, grad_out_dev, go_stride_n, grad_table_dev, n_points, 0, n_levels, s)
+    if (go_dtype == TH_F16) TH_DISPATCH_CAST(__half, TH_CALL_BWD)
+    if (go_dtype == TH_BF16) TH_DISPATCH_CAST(__nv_bfloat16, TH_CALL_BWD)
+#undef TH_CALL_BWD
+    return fail(TH_ERR_BAD_ARG, "gradient dtype %d is not a 16-bit type", go_dtype);
 }
 
 namespace th {

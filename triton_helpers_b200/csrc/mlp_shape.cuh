@@ -63,6 +63,9 @@ struct MseArgs {
     long long grad_stride;
     float *loss_sum;
     float grad_scale;
+    const float4 *order;  // not null: row r is point r of a spatially ordered batch, its target is row order[r].w
+    float loss_scale;     // multiplies the squared errors that go to *loss_sum
+    int target_f32;       // the targets are float32: the difference is formed with the unrounded target
 };
 int mlp_fwd_mse_tc(const MlpShape &s, const MlpParams &p, const void *x, int64_t x_stride, void *y, int64_t y_stride,
                    const MseArgs &mse, int64_t rows, int dtype, cudaStream_t stream);

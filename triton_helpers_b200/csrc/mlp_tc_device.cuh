@@ -181,6 +181,23 @@ __device__ __forceinline__ uint4 mse_chunk(uint4 pred, uint4 target, float grad_
     return make_uint4(gw[0], gw[1], gw[2], gw[3]);
 }
 
+// The same with the target in float32 (eight values at `target`)
+template <typename T>
+__device__ __forceinline__ uint4 mse_chunk_f32(uint4 pred, const float *target, float grad_scale, float &loss) {
+    const uint32_t pw[4] = {pred.x, pred.y, pred.z, pred.w};
+    const float4 lo = __ldcs(reinterpret_cast<const float4 *>(target)), hi = __ldcs(reinterpret_cast<const float4 *>(target) + 1);
+    const float t[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+    uint32_t gw[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float2 a = unpack_pair<T>(pw[k]);
+        const float d0 = a.x - t[2 * k], d1 = a.y - t[2 * k + 1];
+        loss += d0 * d0 + d1 * d1;
+        gw[k] = pack_pair<T>(d0 * grad_scale, d1 * grad_scale);
+    }
+    return make_uint4(gw[0], gw[1], gw[2], gw[3]);
+}
+
 // ---- epilogues: backward -----------------------------------------------------------------------
 
 // Epilogue of a dgrad: dz of the layer below = dy * act'(that layer's parked output), rounded.

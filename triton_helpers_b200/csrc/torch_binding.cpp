@@ -26,6 +26,7 @@
 
 #include <atomic>
 #include <cstring>
+#include <strings.h>
 #include <memory>
 #include <mutex>
 #include <unordered_map>
@@ -508,6 +509,108 @@ struct MlpNode : public Node {
     }
 };
 
+// float32 networks: every tensor is rounded to a 16-bit operand type, all of them in one launch and into one buffer; the
+// results are cast back.  The backward pass keeps that buffer, not the float32 tensors, and hands out the float32 sums
+// of the weight gradients as they are.
+struct Float32Pack {
+    Tensor buffer;          // 16-bit operands: x, w_in, b_in, w_out, b_out, w_hid, b_hid (where present)
+    void *part[7] = {};
+
+    static at::ScalarType operands() {
+        static const at::ScalarType type = [] {
+            const char *v = getenv("TH_MLP_F32_OPERANDS");
+            if (!v || !strcasecmp(v, "fp16") || !strcasecmp(v, "float16")) return at::kHalf;
+            if (!strcasecmp(v, "bf16") || !strcasecmp(v, "bfloat16")) return at::kBFloat16;
+            return at::kFloat;  // not a valid choice: Python says so
+        }();
+        return type;
+    }
+
+    void fill(const std::vector<Tensor> &tensors, void *stream) {
+        int64_t total = 0, sizes[8];
+        const void *src[8];
+        void *dst[8];
+        int n = 0;
+        for (const Tensor &t : tensors) total += t.defined() ? (t.numel() + 15) / 16 * 16 : 0;
+        buffer = empty_like_shape({total}, operands(), tensors[0].device());
+        char *at = static_cast<char *>(ptr(buffer));
+        for (size_t k = 0; k < tensors.size(); ++k) {
+            part[k] = nullptr;
+            if (!tensors[k].defined()) continue;
+            part[k] = dst[n] = at;
+            src[n] = ptr(tensors[k]);
+            sizes[n++] = tensors[k].numel();
+            at += (tensors[k].numel() + 15) / 16 * 16 * 2;
+        }
+        check(th_cast(n, src, dst, sizes, TH_F32, dtype_code(operands()), stream), "th_cast");
+    }
+};
+
+void cast_one(const Tensor &from, const Tensor &to, void *stream) {
+    const void *src = ptr(from);
+    void *dst = ptr(to);
+    const int64_t n = from.numel();
+    check(th_cast(1, &src, &dst, &n, dtype_code(from.scalar_type()), dtype_code(to.scalar_type()), stream), "th_cast");
+}
+
+struct Float32MlpNode : public Node {
+    MlpCall call;
+    Float32Pack pack;
+    std::vector<int64_t> shapes[6];  // of w_in, b_in, w_out, b_out, w_hid, b_hid
+    bool has_bias = false, released = false;
+
+    std::string name() const override { return "FullyFusedMLPBackward"; }
+    void release_variables() override {
+        pack.buffer.reset();
+        released = true;
+    }
+    variable_list apply(variable_list &&grads) override {
+        variable_list out(7);
+        TORCH_CHECK(!released, torch::autograd::ERR_BACKWARD_TWICE);
+        if (!grads[0].defined()) return out;
+        at::NoGradGuard no_grad;
+        const c10::Device device = pack.buffer.device();
+        const at::ScalarType half = pack.buffer.scalar_type();
+        c10::cuda::CUDAGuard guard(device);
+        void *stream = current_stream();
+        const Tensor given = grads[0].contiguous();
+        Tensor go = given;
+        if (given.scalar_type() == at::kFloat) {
+            go = empty_like_shape(given.sizes(), half, device);
+            cast_one(given, go, stream);
+        } else if (given.scalar_type() != half) {
+            go = given.to(half);
+        }
+        const bool wants_dx = task_should_compute_output(0);
+        const Tensor dx = wants_dx ? empty_like_shape({call.batch, call.length, call.d_in}, half, device) : Tensor();
+        const int64_t bytes = th_mlp_workspace_bytes(call.d_in, call.hidden, call.d_out, call.depth);
+        const Tensor sums = empty_like_shape({bytes / 4}, at::kFloat, device);
+        check(th_mlp_bwd(pack.part[0], call.d_in, pack.part[1], pack.part[2], pack.part[5], pack.part[6], pack.part[3], pack.part[4], ptr(go), call.d_out,
+                         ptr(dx), call.d_in, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, ptr(sums), bytes, call.rows(), call.d_in, call.hidden,
+                         call.d_out, call.depth, call.act, dtype_code(half), 0, stream),
+              "th_mlp_bwd");
+        if (wants_dx) {
+            out[0] = empty_like_shape(dx.sizes(), at::kFloat, device);
+            cast_one(dx, out[0], stream);
+        }
+        const int64_t h = call.hidden, n_in = h * call.d_in, n_hid = (call.depth - 1) * h * h, n_out = h * call.d_out;
+        int64_t at = 0;
+        auto slice = [&](int k, int64_t n) {  // the sums' layout: w_in, w_hid, w_out, b_in, b_hid, b_out
+            out[1 + k] = sums.narrow(0, at, n).view(shapes[k]);
+            at += n;
+        };
+        slice(0, n_in);
+        if (n_hid) slice(4, n_hid);
+        slice(2, n_out);
+        if (has_bias) {
+            slice(1, h);
+            if (n_hid) slice(5, (call.depth - 1) * h);
+            slice(3, call.d_out);
+        }
+        return out;
+    }
+};
+
 // A parameter of the layer: plain, contiguous, same dtype and device as the input.
 bool parameter_like(const Tensor &t, const Tensor &x, c10::IntArrayRef sizes) {
     return plain(t) && t.is_contiguous() && t.scalar_type() == x.scalar_type() && t.device() == x.device() && t.sizes() == sizes;
@@ -516,7 +619,7 @@ bool parameter_like(const Tensor &t, const Tensor &x, c10::IntArrayRef sizes) {
 bool mlp_call(MlpCall &c, const Tensor &x, MlpTensors &p, PyObject *activation) {
     if (!plain(x) || x.dim() != 3 || !plain(p.w_in) || p.w_in.dim() != 2 || !plain(p.w_out) || p.w_out.dim() != 2) return false;
     c.dtype = dtype_code(x.scalar_type());
-    if (c.dtype != TH_F16 && c.dtype != TH_BF16) return false;
+    if (c.dtype < 0 || (c.dtype == TH_F32 && Float32Pack::operands() == at::kFloat)) return false;
     const int64_t hidden = p.w_in.size(0), d_in = p.w_in.size(1), d_out = p.w_out.size(0);
     if (d_in < 1 || d_in > 64 || d_out < 1 || d_out > 64 || (hidden != 16 && hidden != 32 && hidden != 64)) return false;
     if (x.size(2) != d_in) return false;
@@ -546,6 +649,36 @@ bool mlp_call(MlpCall &c, const Tensor &x, MlpTensors &p, PyObject *activation) 
     return true;
 }
 
+Tensor mlp_float32(const MlpCall &call, const Tensor &x, const MlpTensors &p, bool grad) {
+    NoGil release;
+    Tensor out;
+    std::shared_ptr<Float32MlpNode> node;
+    if (grad) {
+        node = make_node<Float32MlpNode>(torch::autograd::collect_next_edges(x, p.w_in, p.b_in, p.w_out, p.b_out, p.w_hid, p.b_hid));
+        node->call = call;
+        node->has_bias = p.b_in.defined();
+        const Tensor *params[6] = {&p.w_in, &p.b_in, &p.w_out, &p.b_out, &p.w_hid, &p.b_hid};
+        for (int k = 0; k < 6; ++k)
+            if (params[k]->defined()) node->shapes[k] = params[k]->sizes().vec();
+    }
+    {
+        at::AutoDispatchBelowADInplaceOrView below;
+        c10::cuda::CUDAGuard guard(x.device());
+        void *stream = current_stream();
+        Float32Pack pack;
+        pack.fill({x.contiguous(), p.w_in, p.b_in, p.w_out, p.b_out, p.w_hid, p.b_hid}, stream);
+        const Tensor half = empty_like_shape({call.batch, call.length, call.d_out}, pack.buffer.scalar_type(), x.device());
+        check(th_mlp_fwd(pack.part[0], call.d_in, pack.part[1], pack.part[2], pack.part[5], pack.part[6], pack.part[3], pack.part[4], ptr(half), call.d_out,
+                         call.rows(), call.d_in, call.hidden, call.d_out, call.depth, call.act, dtype_code(half.scalar_type()), 0, stream),
+              "th_mlp_fwd");
+        out = empty_like_shape(half.sizes(), at::kFloat, x.device());
+        cast_one(half, out, stream);
+        if (grad) node->pack = std::move(pack);
+    }
+    if (grad) torch::autograd::set_history(out, node);
+    return out;
+}
+
 // fully_fused_mlp(x, w_in, b_in, w_out, b_out, w_hid, b_hid, activation)
 PyObject *py_fully_fused_mlp(PyObject *, PyObject *const *args, Py_ssize_t n_args) {
     HANDLE_TH_ERRORS
@@ -556,10 +689,12 @@ PyObject *py_fully_fused_mlp(PyObject *, PyObject *const *args, Py_ssize_t n_arg
         TH_NOT_MINE;
     MlpCall call;
     if (!mlp_call(call, x, p, args[7])) TH_NOT_MINE;
+    const bool grad = torch::autograd::compute_requires_grad(x, p.w_in, p.b_in, p.w_out, p.b_out, p.w_hid, p.b_hid);
+    if (call.dtype == TH_F32 && grad && call.depth >= 4) TH_NOT_MINE;  // its backward pass is refused, by the Python path
+    if (call.dtype == TH_F32) return THPVariable_Wrap(mlp_float32(call, x, p, grad));
     Tensor out;
     {
         NoGil release;
-        const bool grad = torch::autograd::compute_requires_grad(x, p.w_in, p.b_in, p.w_out, p.b_out, p.w_hid, p.b_hid);
         std::shared_ptr<MlpNode> node;
         if (grad) {
             node = make_node<MlpNode>(torch::autograd::collect_next_edges(x, p.w_in, p.b_in, p.w_out, p.b_out, p.w_hid, p.b_hid));
@@ -812,6 +947,200 @@ PyObject *py_hash_encoded_mlp(PyObject *, PyObject *const *args, Py_ssize_t n_ar
     END_HANDLE_TH_ERRORS
 }
 
+// ---- training step ------------------------------------------------------------------------------------------------
+
+bool take_list(PyObject *o, std::vector<Tensor> &out) {
+    if (!PyTuple_Check(o) && !PyList_Check(o)) return false;
+    const Py_ssize_t n = PySequence_Fast_GET_SIZE(o);
+    out.resize(n);
+    for (Py_ssize_t k = 0; k < n; ++k)
+        if (!take(PySequence_Fast_GET_ITEM(o, k), out[k])) return false;
+    return true;
+}
+
+// adam_steps(params, grads, exp_avgs, exp_avg_sqs, grad_scales, zero_grad, lr, beta1, beta2, eps, step, skipped): sequences of
+// one length (tensors of one dtype on one device); the update of all of them in one launch (16 tensors each)
+PyObject *py_adam_steps(PyObject *, PyObject *const *args, Py_ssize_t n_args) {
+    HANDLE_TH_ERRORS
+    std::vector<Tensor> params, grads, m, v;
+    double lr, beta1, beta2, eps;
+    int64_t step;
+    Tensor skipped;
+    if (n_args != 12 || g_deferred.load(std::memory_order_relaxed) || !take_list(args[0], params) || !take_list(args[1], grads) || !take_list(args[2], m) ||
+        !take_list(args[3], v) || !take(args[6], lr) || !take(args[7], beta1) || !take(args[8], beta2) || !take(args[9], eps) || !take(args[10], step) ||
+        !take(args[11], skipped))
+        TH_NOT_MINE;
+    const size_t n = params.size();
+    if (n == 0 || grads.size() != n || m.size() != n || v.size() != n || !PyTuple_Check(args[4]) || !PyTuple_Check(args[5]) ||
+        PyTuple_GET_SIZE(args[4]) != static_cast<Py_ssize_t>(n) || PyTuple_GET_SIZE(args[5]) != static_cast<Py_ssize_t>(n))
+        TH_NOT_MINE;
+    const at::ScalarType type = params[0].scalar_type();
+    std::vector<float> scales(n);
+    std::vector<int> zero(n);
+    auto aligned = [](const Tensor &t) { return reinterpret_cast<uintptr_t>(ptr(t)) % 32 == 0; };
+    if (skipped.defined() && (!plain(skipped) || skipped.scalar_type() != at::kInt)) TH_NOT_MINE;
+    for (size_t k = 0; k < n; ++k) {
+        double scale;
+        if (!take(PyTuple_GET_ITEM(args[4], k), scale)) TH_NOT_MINE;
+        scales[k] = static_cast<float>(scale);
+        zero[k] = PyObject_IsTrue(PyTuple_GET_ITEM(args[5], k)) == 1;
+        for (const Tensor *t : {&params[k], &grads[k], &m[k], &v[k]})
+            if (!plain(*t) || !t->is_contiguous() || t->device() != params[0].device() || t->numel() != params[k].numel() || !aligned(*t)) TH_NOT_MINE;
+        if (params[k].scalar_type() != type || grads[k].scalar_type() != type || m[k].scalar_type() != at::kFloat || v[k].scalar_type() != at::kFloat)
+            TH_NOT_MINE;
+    }
+    if (dtype_code(type) < 0) TH_NOT_MINE;
+    {
+        NoGil release;
+        c10::cuda::CUDAGuard guard(params[0].device());
+        void *stream = current_stream();
+        for (size_t from = 0; from < n; from += 16) {
+            const int count = static_cast<int>(n - from < 16 ? n - from : 16);
+            void *pp[16], *gp[16];
+            float *mp[16], *vp[16];
+            int64_t sizes[16];
+            for (int k = 0; k < count; ++k) {
+                pp[k] = ptr(params[from + k]);
+                gp[k] = ptr(grads[from + k]);
+                mp[k] = m[from + k].data_ptr<float>();
+                vp[k] = v[from + k].data_ptr<float>();
+                sizes[k] = params[from + k].numel();
+            }
+            check(th_adam_steps(count, pp, gp, mp, vp, sizes, scales.data() + from, zero.data() + from, static_cast<float>(lr), static_cast<float>(beta1),
+                                static_cast<float>(beta2), static_cast<float>(eps), static_cast<int>(step), dtype_code(type),
+                                skipped.defined() ? skipped.data_ptr<int>() : nullptr, stream),
+                  "th_adam_steps");
+        }
+    }
+    // in-place updates that autograd has to know of
+    for (const Tensor &t : params) t.unsafeGetTensorImpl()->bump_version();
+    Py_RETURN_TRUE;
+    END_HANDLE_TH_ERRORS
+}
+
+// train_gradients(coords, targets, table, table_grad, (w_in, b_in, w_hid, b_hid, w_out, b_out), sums, feats, grad_pred, grad_feats,
+//                 mlp_grad, pi, max_entries_per_level, min_res, max_res, levels, activation, grad_scale, cast_scale)
+//
+// Forward, squared-error loss and backward of the encoding followed by the MLP, on the caller's buffers: table_grad (adds into it),
+// sums (float32 sums of the MLP's gradients, laid out as th_mlp_bwd's workspace), feats / grad_pred / grad_feats (16-bit rows, scratch).
+// 16-bit tables: sums * cast_scale are rounded into mlp_grad.  float32 tables: the MLP runs on 16-bit copies of its parameters,
+// mlp_grad is None.  Large batches are ordered in space first; nothing in them is kept in the caller's row order.
+// Returns the mean squared error (one float32 element); NotImplemented before anything has been launched that changes table_grad.
+PyObject *py_train_gradients(PyObject *, PyObject *const *args, Py_ssize_t n_args) {
+    HANDLE_TH_ERRORS
+    if (n_args != 18 || !usual_mode()) TH_NOT_MINE;
+    Tensor coords, targets, table, table_grad, sums, feats, grad_pred, grad_feats, mlp_grad;
+    std::vector<Tensor> w;
+    double grad_scale, cast_scale;
+    if (!take(args[0], coords) || !take(args[1], targets) || !take(args[2], table) || !take(args[3], table_grad) || !take_list(args[4], w) || w.size() != 6 ||
+        !take(args[5], sums) || !take(args[6], feats) || !take(args[7], grad_pred) || !take(args[8], grad_feats) || !take(args[9], mlp_grad) ||
+        !take(args[16], grad_scale) || !take(args[17], cast_scale))
+        TH_NOT_MINE;
+    EncodeCall call;
+    static PyObject *one = PyFloat_FromDouble(1.0);
+    if (coords.dim() != 2 || !encode_call(call, coords, table, args[10], args + 11, args[14], one)) TH_NOT_MINE;
+    const int act = activation_code(args[15]);
+    const at::ScalarType type = table.scalar_type();
+    const bool f32 = type == at::kFloat;
+    if (act < 0 || !plain(w[0]) || w[0].dim() != 2 || !plain(w[4]) || w[4].dim() != 2) TH_NOT_MINE;
+    const int64_t hidden = w[0].size(0), d_in = w[0].size(1), d_out = w[4].size(0), n = call.n;
+    const bool bias = w[1].defined();
+    int64_t depth = 1;
+    if (w[2].defined()) {
+        if (w[2].dim() != 2 || hidden < 1 || w[2].numel() == 0) TH_NOT_MINE;
+        depth += w[2].size(0) / hidden;
+        if (!parameter_like(w[2], table, {(depth - 1) * hidden, hidden})) TH_NOT_MINE;
+    }
+    if ((hidden != 16 && hidden != 32 && hidden != 64) || d_in > 64 || d_out > 64 || d_out % 8 || d_in != call.feats * call.geo->levels || n < 1) TH_NOT_MINE;
+    if (!parameter_like(w[0], table, {hidden, d_in}) || !parameter_like(w[4], table, {d_out, hidden}) || w[5].defined() != bias ||
+        w[3].defined() != (bias && depth > 1))
+        TH_NOT_MINE;
+    if (bias && (!parameter_like(w[1], table, {hidden}) || !parameter_like(w[5], table, {d_out}) ||
+                 (depth > 1 && !parameter_like(w[3], table, {depth - 1, hidden}))))
+        TH_NOT_MINE;
+    const at::ScalarType half = f32 ? Float32Pack::operands() : type;
+    if (half == at::kFloat) TH_NOT_MINE;
+    const int64_t bytes = th_mlp_workspace_bytes(static_cast<int>(d_in), static_cast<int>(hidden), static_cast<int>(d_out), static_cast<int>(depth));
+    auto buffer = [&](const Tensor &t, at::ScalarType st, int64_t numel) {
+        return plain(t) && t.is_contiguous() && t.scalar_type() == st && t.numel() == numel && t.device() == table.device();
+    };
+    if (!buffer(table_grad, type, table.numel()) || !buffer(sums, at::kFloat, bytes / 4) || !buffer(feats, half, n * d_in) ||
+        !buffer(grad_pred, half, n * d_out) || !buffer(grad_feats, half, n * d_in) || (!f32 && !buffer(mlp_grad, type, bytes / 4)))
+        TH_NOT_MINE;
+    if (!plain(targets) || targets.device() != table.device() || targets.dim() != 2 || targets.size(0) != n || targets.size(1) != d_out ||
+        dtype_code(targets.scalar_type()) < 0 || targets.requires_grad())
+        TH_NOT_MINE;
+    const bool order_pays = th_hash_order_pays(n, static_cast<int>(call.dims), static_cast<int>(call.feats * table.element_size()), 1);
+    if (f32 && (order_pays || depth >= 4 || call.dims < 2 || (call.feats != 2 && call.feats != 4))) TH_NOT_MINE;
+    Tensor loss;
+    {
+        NoGil release;
+        at::NoGradGuard no_grad;
+        c10::cuda::CUDAGuard guard(table.device());
+        void *stream = current_stream();
+        const Geometry &g = *call.geo;
+        const int D = static_cast<int>(call.dims), F = static_cast<int>(call.feats), L = g.levels;
+        const int code = dtype_code(half);
+        const int ih = static_cast<int>(hidden), ii = static_cast<int>(d_in), io = static_cast<int>(d_out), id = static_cast<int>(depth);
+        Tensor t = targets;
+        if (!f32 && t.scalar_type() != type) t = t.to(type);
+        if (f32 && t.scalar_type() != at::kFloat) t = t.to(at::kFloat);
+        if (t.stride(1) != 1 || t.stride(0) < d_out || t.stride(0) % 8 || reinterpret_cast<uintptr_t>(ptr(t)) % 16) t = t.clone(at::MemoryFormat::Contiguous);
+        loss = at::zeros({1}, sums.options());
+        const CoordArgs x = coord_args(coords, call.dims);
+        const int xcode = dtype_code(x.keep.scalar_type());
+        Tensor order;
+        const void *p[6];
+        for (int k = 0; k < 6; ++k) p[k] = ptr(w[k]);
+        Float32Pack pack;
+        if (f32) {
+            pack.fill(w, stream);
+            for (int k = 0; k < 6; ++k) p[k] = pack.part[k];
+            check(th_hash_fwd_cast(ptr(x.keep), x.stride_n, x.stride_d, xcode, table.data_ptr<float>(), ptr(feats), code, d_in, n, D, F, L, g.res, g.rows,
+                                   g.offsets, call.primes.v, 1.f, stream),
+                  "th_hash_fwd_cast");
+        } else if (order_pays) {
+            order = point_order(call, x, stream);
+            check(th_hash_fwd_ordered(ptr(order), 1, ptr(table), code, ptr(feats), d_in, n, D, F, L, g.res, g.rows, g.offsets, call.primes.v, 0, L, stream),
+                  "th_hash_fwd_ordered");
+        } else {
+            check(th_hash_fwd(ptr(x.keep), x.stride_n, x.stride_d, xcode, ptr(table), code, ptr(feats), d_in, n, D, F, L, g.res, g.rows, g.offsets,
+                              call.primes.v, 1.f, 0, L, stream),
+                  "th_hash_fwd");
+        }
+        const int rc = th_mlp_fwd_mse_ordered(ptr(feats), d_in, p[0], p[1], p[2], p[3], p[4], p[5], ptr(t), t.stride(0), dtype_code(t.scalar_type()),
+                                              ptr(order), ptr(grad_pred), d_out, loss.data_ptr<float>(), static_cast<float>(1.0 / (static_cast<double>(n) * d_out)),
+                                              static_cast<float>(grad_scale), n, ii, ih, io, id, act, code, stream);
+        if (rc == TH_ERR_UNSUPPORTED) {
+            loss.reset();  // the caller takes another way; only feats was written
+        } else {
+            check(rc, "th_mlp_fwd_mse_ordered");
+            check(th_mlp_bwd(ptr(feats), d_in, p[0], p[1], p[2], p[3], p[4], p[5], ptr(grad_pred), d_out, ptr(grad_feats), d_in, nullptr, nullptr, nullptr,
+                             nullptr, nullptr, nullptr, ptr(sums), bytes, n, ii, ih, io, id, act, code, 0, stream),
+                  "th_mlp_bwd");
+            if (f32) {
+                check(th_hash_bwd_cast(ptr(x.keep), x.stride_n, x.stride_d, xcode, ptr(grad_feats), code, d_in, table_grad.data_ptr<float>(), n, D, F, L, g.res,
+                                       g.rows, g.offsets, call.primes.v, 1.f, stream),
+                      "th_hash_bwd_cast");
+            } else {
+                check(th_scale_cast(sums.data_ptr<float>(), ptr(mlp_grad), mlp_grad.numel(), static_cast<float>(cast_scale), code, stream), "th_scale_cast");
+                if (order.defined()) {
+                    check(th_hash_bwd_ordered(ptr(order), 1, ptr(grad_feats), d_in, ptr(table_grad), code, n, D, F, L, g.res, g.rows, g.offsets, call.primes.v,
+                                              0, L, stream),
+                          "th_hash_bwd_ordered");
+                } else {
+                    check(th_hash_bwd(ptr(x.keep), x.stride_n, x.stride_d, xcode, ptr(grad_feats), d_in, ptr(table_grad), code, n, D, F, L, g.res, g.rows,
+                                      g.offsets, call.primes.v, 1.f, 0, L, stream),
+                          "th_hash_bwd");
+                }
+            }
+        }
+    }
+    if (!loss.defined()) TH_NOT_MINE;
+    return THPVariable_Wrap(std::move(loss));
+    END_HANDLE_TH_ERRORS
+}
+
 // ---- module -------------------------------------------------------------------------------------------------
 
 // configure(level_geometry, host_primes): the package's Python helpers this module asks for geometry and primes
@@ -835,7 +1164,8 @@ PyObject *py_defer(PyObject *, PyObject *flag) {
 
 #define TH_FAST(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_##name)), METH_FASTCALL, nullptr}
 PyMethodDef g_methods[] = {
-    TH_FAST(hash_encoding), TH_FAST(fully_fused_mlp), TH_FAST(reversible_mlp), TH_FAST(hash_encoded_mlp), TH_FAST(configure),
+    TH_FAST(hash_encoding), TH_FAST(fully_fused_mlp), TH_FAST(reversible_mlp), TH_FAST(hash_encoded_mlp), TH_FAST(adam_steps),
+    TH_FAST(train_gradients), TH_FAST(configure),
     {"defer", py_defer, METH_O, nullptr},
     {nullptr, nullptr, 0, nullptr},
 };

@@ -1,4 +1,4 @@
-r"""Adam for 16-bit parameters with fp32 moments, one CUDA kernel per parameter tensor.
+r"""Adam for 16-bit parameters with fp32 moments, all tensors of a dtype in one CUDA kernel.
 
 ``torch.optim.Adam`` keeps its moments in the parameter dtype; with float16 hash tables the
 second moment underflows (``g*g < 6e-8`` for ``|g| < 2.4e-4``) and the update divides by
@@ -50,6 +50,14 @@ def adam_update(
         )  # fmt: skip
 
 
+def adam_updates(params, grads, exp_avgs, exp_avg_sqs, grad_scales, zero_grads, step, lr, betas, eps, skipped) -> None:
+    r"""``adam_update`` of several tensors of one dtype and device: one launch where the native path takes them."""
+    done = _lib.native().adam_steps(params, grads, exp_avgs, exp_avg_sqs, tuple(grad_scales), tuple(zero_grads), lr, betas[0], betas[1], eps, step, skipped)
+    if done is NotImplemented:
+        for p, g, m, v, scale, zero in zip(params, grads, exp_avgs, exp_avg_sqs, grad_scales, zero_grads):
+            adam_update(p, g, m, v, step, lr, betas, eps, scale, zero, skipped)
+
+
 class FusedAdam(torch.optim.Optimizer):
 
     def __init__(self, params: Iterable[Tensor], lr: float = 1e-3, betas=(0.9, 0.999), eps: float = 1e-8):
@@ -76,16 +84,21 @@ class FusedAdam(torch.optim.Optimizer):
         gradient buffers (kept allocated) as part of the update kernel.
         """
         for group in self.param_groups:
-            for p in group["params"]:
-                if p.grad is None:
-                    continue
-                state = self.state[p]
-                if not state:
-                    state["step"] = 0
-                    state["exp_avg"] = torch.zeros(p.shape, dtype=torch.float32, device=p.device)
-                    state["exp_avg_sq"] = torch.zeros(p.shape, dtype=torch.float32, device=p.device)
-                state["step"] += 1
-                adam_update(
-                    p, p.grad, state["exp_avg"], state["exp_avg_sq"], state["step"], group["lr"], group["betas"],
-                    group["eps"], grad_scale, zero_grad, self._skip_counter(p.device),
-                )  # fmt: skip
+            live = [p for p in group["params"] if p.grad is not None]
+            self.update(group, live, [p.grad for p in live], [grad_scale] * len(live), [zero_grad] * len(live))
+
+    @torch.no_grad()
+    def update(self, group, params, grads, grad_scales, zero_grads) -> None:
+        r"""``step`` on explicit gradients of some of ``group``'s parameters, each with its own scale and zero flag."""
+        batches: Dict[tuple, list] = {}  # tensors of one dtype, device and step go together
+        for p, g, scale, zero in zip(params, grads, grad_scales, zero_grads):
+            state = self.state[p]
+            if not state:
+                state["step"] = 0
+                state["exp_avg"] = torch.zeros(p.shape, dtype=torch.float32, device=p.device)
+                state["exp_avg_sq"] = torch.zeros(p.shape, dtype=torch.float32, device=p.device)
+            state["step"] += 1
+            batches.setdefault((p.dtype, p.device, state["step"]), []).append((p, g, state["exp_avg"], state["exp_avg_sq"], scale, zero))
+        for (_, device, step), batch in batches.items():
+            columns = [list(c) for c in zip(*batch)]
+            adam_updates(*columns, step, group["lr"], group["betas"], group["eps"], self._skip_counter(device))

@@ -35,10 +35,11 @@ from torch import Tensor
 
 from . import _lib
 from .layers.fully_fused_mlp import FullyFusedMLP
+from .layers.fully_fused_mlp.kernel import _f32_operand_dtype
 from .layers.hash_encoding import HashEncoding
 from .layers.hash_encoding.kernel import _Launch
 from .layers.neural_field.kernel import FieldUnsupported, field_backward, field_forward
-from .optim import FusedAdam, adam_update
+from .optim import FusedAdam, adam_updates
 from .parallel import PendingReduce, allreduce_gradients, gradient_scales, level_passes
 
 
@@ -164,6 +165,9 @@ class NeuralFieldTrainer(nn.Module):
 
     def _step_autograd(self, coords: Tensor, targets: Tensor) -> Tensor:
         world = self.world_size()
+        loss = self._step_float32(coords, targets) if world == 1 else None
+        if loss is not None:
+            return loss
         pred = self.mlp(self.encoding(coords).unsqueeze(0)).squeeze(0)
         grad_out, loss_sum = mse_grad(pred, targets.to(pred.dtype), self.grad_out_scale)
         pred.backward(grad_out)
@@ -174,9 +178,42 @@ class NeuralFieldTrainer(nn.Module):
             p.grad = None
         return loss_sum / pred.numel()
 
+    def _step_float32(self, coords: Tensor, targets: Tensor) -> Optional[Tensor]:
+        r"""The same step without an autograd graph: forward and backward in one native call on kept buffers, Adam in one
+        launch.  ``None`` where the graph has to be built: hooks, frozen parameters, subclasses of the layers, or a call
+        the native path does not take."""
+        enc, mlp = self.encoding, self.mlp
+        if type(enc) is not HashEncoding or type(mlp) is not FullyFusedMLP or len(self.optimizer.param_groups) != 1 or coords.ndim != 2:
+            return None
+        if _hooked(enc) or _hooked(mlp):
+            return None
+        params = [p for p in (enc.embeddings, mlp.w_in, mlp.b_in, mlp.w_hid, mlp.b_hid, mlp.w_out, mlp.b_out) if p is not None]
+        if not all(p.requires_grad and p._backward_hooks is None and p.grad is None for p in params):
+            return None
+        st = self._state
+        if st is None or st.table is not enc.embeddings or st.device != enc.embeddings.device:
+            st = self._state = _Float32State(enc, mlp)
+        st.resize(coords.shape[0])
+        scale = float(self.grad_out_scale)
+        loss = _lib.native().train_gradients(
+            coords, targets, enc.embeddings, st.table_grad, (mlp.w_in, mlp.b_in, mlp.w_hid, mlp.b_hid, mlp.w_out, mlp.b_out),
+            st.sums, st.feats, st.grad_pred, st.grad_feats, None, enc.pi, enc.max_entries_per_level, enc.min_res, enc.max_res,
+            enc.num_levels, mlp.activation, scale, 1.0,
+        )  # fmt: skip
+        if loss is NotImplemented:
+            return None
+        grads = [st.table_grad] + [g.view_as(p) for p, g in zip(params[1:], st.mlp_grads)]
+        # d(mean over the batch)/d pred = 2 (pred - target) / (N * C); Adam clears the table gradient as it consumes it
+        adam_scale = 2.0 / (coords.shape[0] * st.d_out * scale)
+        self.optimizer.update(self.optimizer.param_groups[0], params, grads, [adam_scale] * len(params), [True] + [False] * (len(params) - 1))
+        return loss
+
     # ---- direct mode (one 16-bit dtype) ------------------------------------------------------------
 
     def _step_direct(self, coords: Tensor, targets: Tensor) -> Tensor:
+        loss = self._step_native(coords, targets)
+        if loss is not None:
+            return loss
         st = self._prepare(coords)
         enc, mlp, lib = self.encoding, self.mlp, _lib.lib()
         device, dtype = st.device, st.dtype
@@ -256,10 +293,37 @@ class NeuralFieldTrainer(nn.Module):
                     last = st.flat_grad.numel() if i == 0 else (launch.geo.offsets[end - 1] + launch.geo.rows[end - 1]) * st.n_feats
                     pending.start([st.flat_grad[first:last]])  # one collective per range; the first carries the MLP gradients
             pending.finish()
-        adam_update(enc.embeddings.data.view(-1), st.table_grad.view(-1), st.table_m, st.table_v, self._steps, self.lr, self.betas,
-                    self.eps, table_adam_scale, True, st.skipped)  # fmt: skip
-        adam_update(st.mlp_flat, st.mlp_grad, st.mlp_m, st.mlp_v, self._steps, self.lr, self.betas, self.eps, mlp_adam_scale, False, st.skipped)
+        self._adam_direct(st, table_adam_scale, mlp_adam_scale)
         return st.loss_sum / (n * st.d_out)
+
+    def _adam_direct(self, st: "_DirectState", table_scale: float, mlp_scale: float) -> None:
+        adam_updates(
+            (self.encoding.embeddings.data.view(-1), st.mlp_flat), (st.table_grad_flat, st.mlp_grad), (st.table_m, st.mlp_m), (st.table_v, st.mlp_v),
+            (table_scale, mlp_scale), (True, False), self._steps, self.lr, self.betas, self.eps, st.skipped,
+        )  # fmt: skip
+
+    def _step_native(self, coords: Tensor, targets: Tensor) -> Optional[Tensor]:
+        r"""The direct step with its forward and backward in one native call; ``None`` where the Python sequence has to run
+        (fused kernels or level passes asked for, calls the native path does not take)."""
+        if self.fused not in (None, False) or self.backward_passes:
+            return None
+        st = self._prepare(coords)
+        enc = self.encoding
+        world, scale = self.world_size(), float(self.grad_out_scale)
+        cast_scale, table_adam_scale, mlp_adam_scale = gradient_scales(coords.shape[0], world, st.d_out, scale)
+        loss = _lib.native().train_gradients(
+            coords, targets, enc.embeddings.data, st.table_grad, (st.w_in, st.b_in, st.w_hid, st.b_hid, st.w_out, st.b_out),
+            st.workspace, st.feats, st.grad_pred, st.grad_feats, st.mlp_grad, enc.pi, enc.max_entries_per_level, enc.min_res, enc.max_res,
+            enc.num_levels, self.mlp.activation, scale, cast_scale,
+        )  # fmt: skip
+        if loss is NotImplemented:
+            return None
+        if world > 1:
+            pending = PendingReduce(self.group, bucket_bytes=0)
+            pending.start([st.flat_grad])
+            pending.finish()
+        self._adam_direct(st, table_adam_scale, mlp_adam_scale)
+        return loss
 
     def _fusion_plan(self, st: "_DirectState") -> Tuple[bool, bool]:
         r"""(fused forward?, fused backward?) for this step; see ``fused`` in the class docstring."""
@@ -282,6 +346,41 @@ class NeuralFieldTrainer(nn.Module):
         assert coords.ndim == 2 and 1 <= coords.shape[1] <= 3, "coordinates must be (N, D) with D in 1..3"
         st.resize(coords.shape[0])
         return st
+
+
+def _hooked(module: nn.Module) -> bool:
+    return bool(module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or module._backward_pre_hooks)
+
+
+class _Float32State:
+    r"""Buffers the float32 step keeps: the table's gradient (zero between steps), the float32 sums of the MLP's gradients,
+    16-bit rows."""
+
+    def __init__(self, enc: HashEncoding, mlp: FullyFusedMLP):
+        self.table = enc.embeddings
+        self.device = self.table.device
+        self.d_hidden, self.d_feat = mlp.w_in.shape
+        self.d_out = mlp.w_out.shape[0]
+        depth = 1 if mlp.w_hid is None else mlp.w_hid.shape[0] // self.d_hidden + 1
+        self.table_grad = torch.zeros_like(self.table)
+        self.sums = torch.zeros(_lib.lib().th_mlp_workspace_bytes(self.d_feat, self.d_hidden, self.d_out, depth) // 4, device=self.device)
+        # slices of the sums in the order w_in, b_in, w_hid, b_hid, w_out, b_out of the parameters that exist
+        h, offset, place = self.d_hidden, 0, {}
+        sizes = (("w_in", h * self.d_feat), ("w_hid", (depth - 1) * h * h), ("w_out", self.d_out * h), ("b_in", h), ("b_hid", (depth - 1) * h), ("b_out", self.d_out))
+        for name, size in sizes:
+            place[name] = self.sums[offset : offset + size]
+            offset += size
+        self.mlp_grads = [place[name] for name in ("w_in", "b_in", "w_hid", "b_hid", "w_out", "b_out") if getattr(mlp, name) is not None]
+        self.rows = -1
+
+    def resize(self, n: int) -> None:
+        if n == self.rows:
+            return
+        kw = dict(dtype=_f32_operand_dtype(), device=self.device)
+        self.feats = torch.empty(n, self.d_feat, **kw)
+        self.grad_feats = torch.empty(n, self.d_feat, **kw)
+        self.grad_pred = torch.empty(n, self.d_out, **kw)
+        self.rows = n
 
 
 class _DirectState:
@@ -310,7 +409,8 @@ class _DirectState:
         table_elems = table.numel()
         tail = (table_elems + 15) // 16 * 16  # 32-byte aligned start of the MLP part
         self.flat_grad = torch.zeros(tail + total, dtype=self.dtype, device=self.device)
-        self.table_grad = self.flat_grad[:table_elems].view_as(table)
+        self.table_grad_flat = self.flat_grad[:table_elems]
+        self.table_grad = self.table_grad_flat.view_as(table)
         self.mlp_grad = self.flat_grad[tail:]
         offset = 0
         for name, p in ordered:
