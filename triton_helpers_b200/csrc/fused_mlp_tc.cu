@@ -303,9 +303,22 @@ mlp_fwd_pipe_kernel(const MlpShape s, const MlpParams p, const __grid_constant__
             if (k + S < n_mine && !*reinterpret_cast<volatile int *>(&abort_flag)) fetch_input(b ^ 1, k + S);
             pipe_wait(smem_addr(&bars.in_full[slot][b]), static_cast<uint32_t>((q >> 1) & 1), &abort_flag);
         }
+        // MSE over ordered rows: where this row's target is, and (below) a prefetch of it, so that the random access is over
+        // when the output layer's epilogue needs it (2^21 rows: 0.138 -> 0.10 ms)
+        long long target_at = 0;
+        if constexpr (MSE) {
+            const long long r = row0 + row < n_rows ? row0 + row : 0;
+            target_at = mse.order ? static_cast<long long>(__float_as_uint(__ldg(&mse.order[r].w))) : r;
+        }
         for (int l = 0; l <= s.depth; ++l) {
             const int in_pad = l == 0 ? s.ki : s.h;
             const int out_pad = l == s.depth ? s.no : s.h;
+            if constexpr (MSE) {
+                if (l == 1 && mse.order) {
+                    const char *at = static_cast<const char *>(mse.target) + target_at * mse.target_stride * (mse.target_f32 ? 4 : 2);
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"(at));
+                }
+            }
             // Only the issuer warp polls the mbarrier; the slot's other warps park at the named barrier,
             // which costs no issue slots.  A wait that gives up raises the abort flag, and everybody
             // reads it after the barrier: work stops, the barrier sequence goes on.
@@ -344,9 +357,8 @@ mlp_fwd_pipe_kernel(const MlpShape s, const MlpParams p, const __grid_constant__
                     if constexpr (MSE) {
                         // d_out is a multiple of 8 and all rows are 16-byte aligned here (checked by the launcher)
                         const long long r = live ? row0 + row : 0;
-                        const long long tr = (mse.order && live) ? static_cast<long long>(__float_as_uint(mse.order[r].w)) : r;
-                        const T *target_row = static_cast<const T *>(mse.target) + tr * mse.target_stride;
-                        const float *target_row_f32 = static_cast<const float *>(mse.target) + tr * mse.target_stride;
+                        const T *target_row = static_cast<const T *>(mse.target) + target_at * mse.target_stride;
+                        const float *target_row_f32 = static_cast<const float *>(mse.target) + target_at * mse.target_stride;
                         T *grad_row = static_cast<T *>(mse.grad) + r * mse.grad_stride;
                         T *out_row = y ? y + r * y_stride : nullptr;
                         drain_row<T, TH_ACT_NONE, BIAS>(taddr, out_pad, layer_bias, [&](int chunk, uint4 packed) {

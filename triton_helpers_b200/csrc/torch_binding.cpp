@@ -836,18 +836,25 @@ PyObject *py_reversible_mlp(PyObject *, PyObject *const *args, Py_ssize_t n_args
     END_HANDLE_TH_ERRORS
 }
 
-// ---- hash encoding + MLP in one kernel per direction --------------------------------------------------------
+// ---- hash encoding + MLP --------------------------------------------------------------------------------------
+//
+// Up to eight hidden layers the encoding's kernels and the MLP's run one after the other: each of them fills an SM by
+// itself (the gathers and reductions want all its warps, the MLP its shared memory), large batches can be ordered in
+// space, and together they are faster than the kernels that fuse the two (B200, 200 003 points in two dimensions,
+// forward + backward, 192 -> 150 us; 2^21 points in three, forward 0.72 -> 0.47 ms), which deeper networks still take.
 
 struct FieldNode : public Node {
     EncodeCall call;
     MlpCall mlp;
     SavedVariable coords, table, w_in, w_out, w_hid;
-    Tensor feats;
+    Tensor feats, order;
+    bool separate = true;
 
     std::string name() const override { return "HashEncodedMLPBackward"; }
     void release_variables() override {
         for (SavedVariable *v : {&coords, &table, &w_in, &w_out, &w_hid}) v->reset_data();
         feats.reset();
+        order.reset();
     }
     variable_list apply(variable_list &&grads) override {
         variable_list out(4);
@@ -863,6 +870,23 @@ struct FieldNode : public Node {
         de.zero_();
         const Geometry &geo = *call.geo;
         const int feat = static_cast<int>(call.feats), dims = static_cast<int>(call.dims);
+        if (separate) {
+            const int64_t bytes = th_mlp_workspace_bytes(mlp.d_in, mlp.hidden, mlp.d_out, mlp.depth);
+            const Tensor sums = empty_like_shape({bytes}, at::kByte, t.device()), grad_feats = empty_same(feats);
+            out[1] = empty_same(wi);
+            out[2] = empty_same(wo);
+            if (wh.defined()) out[3] = empty_same(wh);
+            void *stream = current_stream();
+            check(th_mlp_bwd(ptr(feats), mlp.d_in, ptr(wi), nullptr, ptr(wh), nullptr, ptr(wo), nullptr, ptr(g.keep), g.stride, ptr(grad_feats), mlp.d_in,
+                             ptr(out[1]), nullptr, ptr(out[3]), nullptr, ptr(out[2]), nullptr, ptr(sums), bytes, call.n, mlp.d_in, mlp.hidden, mlp.d_out,
+                             mlp.depth, mlp.act, mlp.dtype, 0, stream),
+                  "th_mlp_bwd");
+            Rows rows;
+            rows_of(grad_feats, mlp.d_in, rows);
+            hash_backward(call, coord_args(x, call.dims), order, rows, de, stream);
+            out[0] = std::move(de);
+            return out;
+        }
         const int64_t bytes = th_field_workspace_bytes(geo.levels, feat, mlp.hidden, mlp.d_out, mlp.depth);
         const Tensor sums = empty_like_shape({bytes / 4}, at::kFloat, t.device());
         const CoordArgs c = coord_args(x, call.dims);
@@ -910,6 +934,11 @@ PyObject *py_hash_encoded_mlp(PyObject *, PyObject *const *args, Py_ssize_t n_ar
     mlp.hidden = static_cast<int>(hidden);
     mlp.d_out = static_cast<int>(d_out);
     mlp.depth = static_cast<int>(depth);
+    // what the fused kernels cover: anything else is Python's FieldUnsupported
+    static const bool legacy = getenv("TH_MLP_LEGACY") && getenv("TH_MLP_LEGACY")[0] == '1';
+    const bool separate = !legacy && depth <= 8 && (call.dims == 2 || call.dims == 3) && (call.feats == 2 || call.feats == 4) &&
+                          d_in % 16 == 0 && d_in <= 64 && (mlp.act == TH_ACT_RELU || mlp.act == TH_ACT_NONE) &&
+                          (hidden == 16 || hidden == 32 || hidden == 64) && d_out >= 1 && d_out <= 64;
     Tensor out;
     {
         NoGil release;
@@ -919,6 +948,7 @@ PyObject *py_hash_encoded_mlp(PyObject *, PyObject *const *args, Py_ssize_t n_ar
             node = make_node<FieldNode>(torch::autograd::collect_next_edges(table, p.w_in, p.w_out, p.w_hid));
             node->call = call;
             node->mlp = mlp;
+            node->separate = separate;
             node->coords = SavedVariable(coords, false);
             node->table = SavedVariable(table, false);
             node->w_in = SavedVariable(p.w_in, false);
@@ -930,12 +960,25 @@ PyObject *py_hash_encoded_mlp(PyObject *, PyObject *const *args, Py_ssize_t n_ar
             c10::cuda::CUDAGuard guard(table.device());
             const Geometry &geo = *call.geo;
             const CoordArgs c = coord_args(coords, call.dims);
-            Tensor feats = grad ? empty_like_shape({call.n, d_in}, table.scalar_type(), table.device()) : Tensor();
+            Tensor feats = grad || separate ? empty_like_shape({call.n, d_in}, table.scalar_type(), table.device()) : Tensor();
             out = empty_like_shape(with_last(coords, d_out), table.scalar_type(), table.device());
-            const int rc = th_field_fwd(ptr(c.keep), c.stride_n, c.stride_d, dtype_code(c.keep.scalar_type()), ptr(table), static_cast<int>(call.dims),
+            int rc = 0;
+            if (separate) {
+                void *stream = current_stream();
+                Tensor order;
+                if (th_hash_order_pays(call.n, static_cast<int>(call.dims), static_cast<int>(call.feats * table.element_size()), grad))
+                    order = point_order(call, c, stream);
+                hash_forward(call, c, order, table, feats, stream);
+                check(th_mlp_fwd(ptr(feats), d_in, ptr(p.w_in), nullptr, ptr(p.w_hid), nullptr, ptr(p.w_out), nullptr, ptr(out), d_out, call.n, mlp.d_in,
+                                 mlp.hidden, mlp.d_out, mlp.depth, mlp.act, mlp.dtype, 0, stream),
+                      "th_mlp_fwd");
+                if (grad) node->order = std::move(order);
+            } else {
+                rc = th_field_fwd(ptr(c.keep), c.stride_n, c.stride_d, dtype_code(c.keep.scalar_type()), ptr(table), static_cast<int>(call.dims),
                                         static_cast<int>(call.feats), geo.levels, geo.res, geo.rows, geo.offsets, call.primes.v, call.scale, ptr(p.w_in),
                                         nullptr, ptr(p.w_hid), nullptr, ptr(p.w_out), nullptr, mlp.hidden, mlp.d_out, mlp.depth, mlp.act, ptr(feats), d_in,
                                         ptr(out), d_out, nullptr, d_out, nullptr, d_out, nullptr, 1.f, call.n, mlp.dtype, current_stream());
+            }
             if (rc == TH_ERR_UNSUPPORTED) out.reset();  // nothing was launched: Python raises FieldUnsupported
             else check(rc, "th_field_fwd");
             if (grad) node->feats = std::move(feats);
