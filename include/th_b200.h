@@ -22,8 +22,8 @@
  *   - environment switches, read once per process, for A/B runs and for testing the
  *     fall-back kernels: TH_MLP_LEGACY=1 sends the fused and the reversible MLP to their
  *     mma.sync kernels, TH_MLP_NO_TMA=1 stages weights with plain loads, TH_MLP_NO_PIPE=1
- *     disables the multi-tile tcgen05 MLP kernels, TH_MLP_NO_SLOTS=1 only the backward's
- *     shared-accumulator variant of them, TH_MLP_SLOTS=n caps the forward's row tiles in
+ *     disables the multi-tile tcgen05 forward MLP kernel, TH_MLP_NO_SLOTS=1 keeps the backward
+ *     at one row tile in flight per CTA, TH_MLP_SLOTS=n caps the forward's row tiles in
  *     flight per CTA, TH_MLP_NO_TMEM_A=1 keeps the forward kernels' hidden activations in
  *     shared-memory operand tiles instead of tensor memory.
  *

@@ -41,13 +41,19 @@ def ordered_and_unordered(n, d, feats, dtype, cap, max_res, points, keep_order, 
     return de, de_o
 
 
+def same_rows(de, de_o):
+    r"""Entries that are zero on one side only are sums that cancel to a rounding error in another order."""
+    apart = (de != 0) != (de_o != 0)
+    return not apart.any() or float((de - de_o)[apart].abs().max()) <= 1e-6 * float(de.abs().max())
+
+
 @pytest.mark.parametrize("points", ["uniform", "clustered", "one cell"])
 @pytest.mark.parametrize("n", [1, 1023, 1024, 1025, 20001])
 def test_ordered_matches_unordered(n, points):
     # one point, the edges of a tile of 1024, several tiles; cells of one point and cells of a whole tile
     de, de_o = ordered_and_unordered(n, 3, 2, torch.float32, 2**14, 512, points, keep_order=0)
     assert float((de - de_o).abs().max() / de.abs().max()) <= 2e-5
-    assert torch.equal(de != 0, de_o != 0)
+    assert same_rows(de, de_o)
 
 
 @pytest.mark.parametrize("d,feats,dtype", [(1, 1, torch.float32), (2, 2, torch.float16), (2, 8, torch.float32), (3, 4, torch.float32),
@@ -63,4 +69,4 @@ def test_several_passes_over_a_large_table():
     # 16 levels of up to 16 MB: more than one pass of levels, each of them sorting some tiles
     de, de_o = ordered_and_unordered(2**17 + 77, 3, 4, torch.float32, 2**20, 4096, "clustered", keep_order=0)
     assert float((de - de_o).abs().max() / de.abs().max()) <= 2e-5
-    assert torch.equal(de != 0, de_o != 0)
+    assert same_rows(de, de_o)

@@ -1,0 +1,556 @@
+// Fused MLP backward with several row tiles in flight per SM, for every activation, with and without biases.
+//
+// The backward of a 128-row tile is a chain of 2 depth + 1 short steps (recompute and park every layer's input, then
+// layer by layer backwards), each a round trip "operands written -> barrier -> issue -> commit -> mbarrier -> tcgen05.ld ->
+// convert -> st.shared" of about a microsecond of which the MMAs are a tenth.  Throughput is row tiles in flight over
+// chain length.  ONE CTA per SM runs S independent SLOTS of 128 W threads plus one WGRAD warp:
+//   * warp 0 of a slot issues the slot's recompute and dgrad MMAs into the slot's own accumulator columns, so that chain
+//     never leaves the slot; the W warpgroups of a slot share a tile's columns (thread = tile row = TMEM lane, column half);
+//   * the wgrad warp issues the weight- and bias-gradient MMAs of every slot.  MMAs of one thread execute in order, so all
+//     slots accumulate into ONE shared set of TMEM columns instead of one set per tile in flight;
+//   * dz of layer l - 1 is written in place over the parked input of layer l once both MMAs that read it have finished;
+//   * when features and output gradient are at most 32 wide, the output-gradient rows of a slot live in the logical chunks
+//     4..7 of its feature tile (which uses chunks 0..3): depth + 1 tiles per slot.  The output layer's wgrad then reads the
+//     whole feature tile as its A operand, and the real gradient rows sit at rows 32.. of that layer's accumulator (rows
+//     0..31 are products nobody reads).
+// Bias gradient of a layer = column sums of dz = dz^T . ONES, a small MMA (N = 8) next to the weight gradient's.  SiLU' and
+// ReLU^2' want the pre-activation: the step that needs it issues that layer's forward GEMM again into a second accumulator
+// and rounds z to the storage dtype, as the forward pass did.
+//
+// Per slot three mbarriers: `ready` (one arrival: the operands of the slot's next backward step are in place), `acc` (the
+// slot's own MMAs of the step are done), `wdone` (the step's wgrad is done).  The wgrad warp polls all `ready` barriers at
+// once, one lane per slot, without blocking.  Every wait is bounded by the global timer and watches the CTA's abort flag;
+// after an abort everybody keeps the same barrier sequence without doing work.
+#include "mlp_tc_device.cuh"
+
+#include <cstddef>
+
+namespace th {
+namespace {
+
+constexpr int kSlotsMax = 4;
+constexpr int kStepsMax = 24;  // 2 depth + 1
+
+struct SlotPlan {
+    int packed;          // the output gradient shares the feature tile
+    int tiles_per_slot;
+    int ones;            // byte offset of the tile of ones (biases)
+    int weights;         // byte offset of the weight tiles and biases
+    int tables;          // byte offset of the barriers and step table
+    int total;           // dynamic shared memory
+    int acc_cols;        // accumulator columns of a slot
+    int tmem_cols;
+    TcPlan w;            // weight and bias offsets relative to `weights`
+};
+
+// What the issuing warps need for one step of a tile, worked out once per CTA: both issue paths are on the critical chain of
+// every tile, and each address or descriptor computed there is paid 2 depth + 1 times per tile.
+struct __align__(16) SlotStep {
+    uint32_t a_off;    // the slot's own GEMM: A operand, relative to the slot's first tile
+    uint32_t b_addr;   //   B operand (a weight tile)
+    uint32_t idesc;    //   instruction descriptor; 0 = the step has no GEMM of its own
+    uint32_t k_steps;  //   bits 0..7: K steps of 16; bit 8: B is read MN-major
+    uint32_t wa_off;   // weight gradient: A operand (dz, MN-major), relative to the slot's first tile
+    uint32_t wb_off;   //   B operand (the layer's input, MN-major)
+    uint32_t widesc;   //   instruction descriptor
+    uint32_t dw_col;   //   bits 0..15: accumulator column; bits 16..31: the bias gradient's
+    uint32_t za_off;   // pre-activation of the layer below: A operand
+    uint32_t zb_addr;  //   B operand
+    uint32_t z_k;      //   K steps; 0 = none
+    uint32_t unused;
+};
+
+struct SlotTables {
+    unsigned long long weights_bar;
+    unsigned long long ready[kSlotsMax], acc[kSlotsMax], wdone[kSlotsMax];
+    uint32_t tmem_holder;
+    int abort_flag;
+    SlotStep steps[kStepsMax];
+};
+
+__host__ __device__ constexpr bool needs_preact(int act) { return act == TH_ACT_SILU || act == TH_ACT_RELU2; }
+
+SlotPlan slot_plan(const MlpShape &s, int slots) {
+    SlotPlan b{};
+    b.packed = (s.ki <= 32 && s.no <= 32) ? 1 : 0;
+    b.tiles_per_slot = s.depth + 1 + (b.packed ? 0 : 1);
+    int off = slots * b.tiles_per_slot * kTileBytes;
+    b.ones = off;
+    if (s.has_bias) off += kTileBytes;
+    b.weights = off;
+    b.w = tc_plan(s, false, 0);
+    off += s.has_bias ? b.w.total : b.w.bias_offset;  // the biases are the plan's last part
+    b.tables = off;
+    b.total = off + static_cast<int>(offsetof(SlotTables, steps)) + (2 * s.depth + 1) * static_cast<int>(sizeof(SlotStep));
+    b.acc_cols = kAccCols * (needs_preact(s.act) ? 2 : 1);
+    const int cols = slots * b.acc_cols + s.ki + s.depth * s.h + (s.has_bias ? 8 * (s.depth + 1) : 0);
+    int alloc = 32;
+    while (alloc < cols) alloc <<= 1;
+    b.tmem_cols = alloc;
+    return b;
+}
+
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
+    uint32_t done;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
+                 : "=r"(done)
+                 : "r"(bar), "r"(parity)
+                 : "memory");
+    return done != 0;
+}
+
+__device__ __forceinline__ void mbar_init(const void *bar) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(1u) : "memory");
+}
+
+// This thread's columns of a row of `pad` accumulator columns (all of them, or one half of them), 8 at a time:
+// fn(chunk of the row, eight values)
+template <int W, typename Fn>
+__device__ __forceinline__ void for_row_pieces(uint32_t taddr, int pad, int half, Fn fn) {
+    if constexpr (W == 2) {
+        const int n = pad / 2, first = half * (n / 8);
+        if (n == 32) {
+            for_each_piece_n<32>(taddr + half * n, [&](int u, const uint32_t(&piece)[8]) { fn(first + u, piece); });
+        } else {
+#pragma unroll 1
+            for (int v = 0; v < n / 8; ++v) for_each_piece_n<8>(taddr + half * n + 8 * v, [&](int, const uint32_t(&piece)[8]) { fn(first + v, piece); });
+        }
+    } else {
+        int first = 0;
+#pragma unroll 1
+        for (; first + 32 <= pad; first += 32)
+            for_each_piece_n<32>(taddr + first, [&](int u, const uint32_t(&piece)[8]) { fn(first / 8 + u, piece); });
+        if (first < pad) for_each_piece_n<16>(taddr + first, [&](int u, const uint32_t(&piece)[8]) { fn(first / 8 + u, piece); });
+    }
+}
+
+template <typename T, int ACT, bool BIAS, int S, int W>
+__global__ void __launch_bounds__(128 * S * W + 32, 1)
+slots_mlp_bwd_tc_kernel(const MlpShape s, const MlpParams p, const __grid_constant__ WeightMaps maps, const int use_tma,
+                        const __grid_constant__ SlotPlan P, const T *__restrict__ x, long long x_stride, const T *__restrict__ go,
+                        long long go_stride, T *__restrict__ gx, long long gx_stride, float *__restrict__ workspace, long long n_rows, int x_vec,
+                        int go_vec, int gx_vec) {
+    constexpr bool kPreact = needs_preact(ACT);
+    constexpr int kSlotThreads = 128 * W;
+    constexpr int bf16 = std::is_same<T, __half>::value ? 0 : 1;
+    extern __shared__ __align__(1024) unsigned char smem_slots[];
+    unsigned char *smem = smem_slots;
+    SlotTables &tb = *reinterpret_cast<SlotTables *>(smem + P.tables);
+    const int d = s.depth, n_steps = 2 * d + 1;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const bool is_wgrad_warp = warp == 4 * S * W;
+    unsigned char *wsmem = smem + P.weights;
+    volatile int *abort_now = &tb.abort_flag;
+
+    // ---- set-up ----
+    if (threadIdx.x == 0) {
+        tb.abort_flag = (smem_addr(smem) & 1023u) ? 1 : 0;  // operand tiles need their alignment
+        if (tb.abort_flag) g_tc_status = 1;
+        for (int i = 0; i < S; ++i) {
+            mbar_init(&tb.ready[i]);
+            mbar_init(&tb.acc[i]);
+            mbar_init(&tb.wdone[i]);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    // operand tiles start out as zeros: columns a layer does not use are still read as MMA rows
+    for (int e = threadIdx.x; e < P.ones / 16; e += blockDim.x) reinterpret_cast<uint4 *>(smem)[e] = make_uint4(0, 0, 0, 0);
+    if constexpr (BIAS) {
+        // 128 rows x 8 columns of ones (logical chunk 0 of every row)
+        const uint32_t one2 = pack_pair<T>(1.f, 1.f);
+        for (int e = threadIdx.x; e < kTileBytes / 16; e += blockDim.x) {
+            const int r = e >> 3, c = (e & 7) ^ (r & 7);
+            reinterpret_cast<uint4 *>(smem + P.ones)[e] = c == 0 ? make_uint4(one2, one2, one2, one2) : make_uint4(0, 0, 0, 0);
+        }
+        stage_biases<T>(wsmem, P.w, s, p);
+    }
+    fence_async_smem();
+    bool weights_ok = true;
+    if (use_tma) {
+        weights_ok = tma_stage_weights(wsmem, P.w, s, maps, &tb.weights_bar);  // contains the barrier that publishes the inits
+    } else {
+        stage_all_weights<T>(wsmem, P.w, s, p);
+        fence_async_smem();
+        __syncthreads();
+    }
+    if (is_wgrad_warp) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&tb.tmem_holder)),
+                     "r"(static_cast<uint32_t>(P.tmem_cols))
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if (!weights_ok) {
+        tb.abort_flag = 1;
+        g_tc_status = 1;
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tb.tmem_holder;
+
+    const long long n_tiles = (n_rows + kTileRows - 1) / kTileRows;
+    const long long first_tile = blockIdx.x, tile_stride = gridDim.x;
+    const long long n_mine = first_tile < n_tiles ? (n_tiles - first_tile + tile_stride - 1) / tile_stride : 0;
+    const uint32_t smem_base = smem_addr(smem);
+    const uint32_t slot_bytes = static_cast<uint32_t>(P.tiles_per_slot) * kTileBytes;
+    auto dw_col = [&](int l) { return S * P.acc_cols + (l == 0 ? 0 : s.ki + (l - 1) * s.h); };
+    auto db_col = [&](int l) { return S * P.acc_cols + s.ki + d * s.h + 8 * l; };
+    // the output gradient of a slot: its own tile, or logical chunks 4.. of the slot's feature tile
+    const uint32_t go_off = P.packed ? 64u : static_cast<uint32_t>(d + 1) * kTileBytes;
+    if (static_cast<int>(threadIdx.x) < n_steps) {  // steps 0 .. d - 1 recompute, step j >= d is the backward step of layer 2 d - j
+        const int j = threadIdx.x;
+        SlotStep st{};
+        if (j < d) {
+            st.a_off = static_cast<uint32_t>(j) * kTileBytes;
+            st.b_addr = smem_addr(weight_tile(wsmem, P.w, s, j));
+            st.idesc = instr_desc(128, s.h, bf16, 0, 0);
+            st.k_steps = static_cast<uint32_t>((j == 0 ? s.ki : s.h) / 16);
+        } else {
+            const int l = 2 * d - j;
+            const int in_pad = l == 0 ? s.ki : s.h, out_pad = l == d ? s.no : s.h;
+            const uint32_t dz = l == d ? go_off : static_cast<uint32_t>(l + 1) * kTileBytes;
+            if (l > 0 || gx != nullptr) {
+                st.a_off = dz;
+                st.b_addr = smem_addr(weight_tile(wsmem, P.w, s, l));
+                st.idesc = instr_desc(128, in_pad, bf16, 0, 1);
+                st.k_steps = static_cast<uint32_t>(out_pad / 16) | 256u;
+            }
+            st.wa_off = (l == d && P.packed) ? 0u : dz;  // packed output gradient: the whole feature tile is the A operand
+            st.wb_off = static_cast<uint32_t>(l) * kTileBytes;
+            st.widesc = instr_desc(64, in_pad, bf16, 1, 1);
+            st.dw_col = static_cast<uint32_t>(dw_col(l)) | (static_cast<uint32_t>(db_col(l)) << 16);
+            if (kPreact && l > 0) {
+                st.za_off = static_cast<uint32_t>(l - 1) * kTileBytes;
+                st.zb_addr = smem_addr(weight_tile(wsmem, P.w, s, l - 1));
+                st.z_k = static_cast<uint32_t>((l == 1 ? s.ki : s.h) / 16);
+            }
+        }
+        tb.steps[j] = st;
+    }
+    __syncthreads();
+
+    if (is_wgrad_warp) {
+        // ================= weight gradients of every slot =================
+        // lane i < S keeps slot i's state: its next backward step, the tiles it still has, the parity to wait for
+        int my_step = d;
+        long long my_tiles = lane < S && lane < n_mine ? (n_mine - lane + S - 1) / S : 0;
+        uint32_t my_parity = 0, started = 0;
+        const uint32_t my_bar = smem_addr(&tb.ready[lane < S ? lane : 0]);
+        unsigned long long deadline = 0;
+        unsigned idle = 0;
+        const bool leader = elect_one();  // the same lane every time: MMAs of one thread execute in order
+        while (__any_sync(0xffffffffu, my_tiles > 0)) {
+            uint32_t mask = __ballot_sync(0xffffffffu, my_tiles > 0 && mbar_test(my_bar, my_parity));
+            if (mask == 0) {
+                if ((++idle & 63u) == 0) {
+                    if (*abort_now) break;
+                    const unsigned long long now = global_ns();
+                    if (deadline == 0) deadline = now + kPipeWaitNs;
+                    else if (now > deadline) {
+                        *abort_now = 1;
+                        g_tc_status = 1;
+                        break;
+                    }
+                }
+                continue;
+            }
+            idle = 0;
+            deadline = 0;
+            const bool mine = (mask >> lane) & 1u;
+            tc_fence_after();
+            while (mask) {
+                const int i = __ffs(mask) - 1;
+                mask &= mask - 1;
+                const int j = __shfl_sync(0xffffffffu, my_step, i);
+                const uint4 w = *reinterpret_cast<const uint4 *>(&tb.steps[j].wa_off);
+                const uint32_t tile0 = smem_base + static_cast<uint32_t>(i) * slot_bytes;
+                const bool more = (started >> (j - d)) & 1u;
+                issue_gemm(leader, tmem + (w.w & 0xffffu), tile0 + w.x, 2048, tile0 + w.y, 2048, kTileRows / 16, w.z, more);
+                if constexpr (BIAS)
+                    issue_gemm(leader, tmem + (w.w >> 16), tile0 + w.x, 2048, smem_base + P.ones, 2048, kTileRows / 16, instr_desc(64, 8, bf16, 1, 1), more);
+                started |= 1u << (j - d);
+                if (leader) mma_commit(smem_addr(&tb.wdone[i]));
+            }
+            __syncwarp();
+            if (mine) {
+                my_parity ^= 1u;
+                if (++my_step == n_steps) {
+                    my_step = d;
+                    --my_tiles;
+                }
+            }
+        }
+    } else {
+        // ================= slots: loads, own MMAs, epilogues =================
+        const int slot = warp / (4 * W), wq = warp & 3;
+        const int tid = threadIdx.x - slot * kSlotThreads;
+        const int row = tid & 127, half = W == 2 ? tid >> 7 : 0;
+        const uint32_t acc = tmem + slot * P.acc_cols;
+        const uint32_t taddr = acc + (static_cast<uint32_t>(32 * wq) << 16);
+        const uint32_t acc_bar = smem_addr(&tb.acc[slot]), ready_bar = smem_addr(&tb.ready[slot]), wdone_bar = smem_addr(&tb.wdone[slot]);
+        const uint32_t tile0 = smem_base + static_cast<uint32_t>(slot) * slot_bytes;
+        auto act_addr = [&](int l) { return tile0 + static_cast<uint32_t>(l) * kTileBytes; };
+        const float *bias = reinterpret_cast<const float *>(wsmem + P.w.bias_offset);
+        const uint32_t row_off = row * 128, row_swizzle = (row & 7) << 4;
+        const bool issuer = tid < 32;
+        const bool leader = issuer && elect_one();
+        uint32_t acc_phase = 0, wdone_phase = 0;
+        auto slot_sync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(slot + 1), "n"(kSlotThreads) : "memory"); };
+        auto copy_rows = [&](const T *src, long long stride, long long row0, int cols, int chunks, uint32_t tile, int chunk0, int vec) {
+            if (vec) {
+#pragma unroll 2
+                for (int id = tid; id < kTileRows * chunks; id += kSlotThreads) {
+                    const int r = id / chunks, c = id - r * chunks;
+                    const long long grow = row0 + r;
+                    const bool inside = grow < n_rows && 8 * c < cols;
+                    const T *from = inside ? src + grow * stride + 8 * c : src;
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(tile + r * 128 + (((chunk0 + c) ^ (r & 7)) << 4)), "l"(from),
+                                 "r"(inside ? 16 : 0)
+                                 : "memory");
+                }
+            } else {
+#pragma unroll 1
+                for (int id = tid; id < kTileRows * chunks; id += kSlotThreads) {
+                    const int r = id / chunks, c = id - r * chunks;
+                    const long long grow = row0 + r;
+                    const bool inside = grow < n_rows && 8 * c < cols;
+                    const unsigned short *from = reinterpret_cast<const unsigned short *>(inside ? src + grow * stride + 8 * c : src);
+                    st_shared_16(tile + r * 128 + (((chunk0 + c) ^ (r & 7)) << 4), inside ? gather8(from, 8 * c, cols) : make_uint4(0, 0, 0, 0));
+                }
+            }
+        };
+        // operands written -> the slot's warp 0 issues the step's own MMAs (and hands the wgrad to the wgrad warp)
+        auto start_step = [&](int j) {
+            fence_async_smem();
+            tc_fence_before();
+            slot_sync();
+            if (issuer && !*abort_now) {
+                tc_fence_after();
+                if (j >= d && leader) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(ready_bar) : "memory");
+                const SlotStep &st = tb.steps[j];
+                const uint4 own = *reinterpret_cast<const uint4 *>(&st.a_off);
+                if (own.z != 0) {
+                    issue_gemm(leader, acc, tile0 + own.x, 32, own.y, (own.w & 256u) ? 2048 : 32, static_cast<int>(own.w & 255u), own.z, false);
+                    if constexpr (kPreact) {
+                        if (st.z_k)
+                            issue_gemm(leader, acc + kAccCols, tile0 + st.za_off, 32, st.zb_addr, 32, static_cast<int>(st.z_k), instr_desc(128, s.h, bf16, 0, 0), false);
+                    }
+                    if (leader) mma_commit(acc_bar);
+                }
+                __syncwarp();
+            }
+        };
+        auto finish_step = [&](bool own, bool wgrad) {
+            // every warp polls: parking three of four warps at a barrier behind the polling one measured 2-6 % slower
+            if (own) pipe_wait(acc_bar, acc_phase, &tb.abort_flag);
+            if (wgrad) pipe_wait(wdone_bar, wdone_phase, &tb.abort_flag);
+            __syncwarp();
+            if (own) acc_phase ^= 1u;
+            if (wgrad) wdone_phase ^= 1u;
+            tc_fence_after();
+            return !*abort_now;
+        };
+        for (long long k = slot; k < n_mine; k += S) {
+            const long long row0 = (first_tile + k * tile_stride) * kTileRows;
+            if (!*abort_now) {
+                copy_rows(x, x_stride, row0, s.d_in, s.ki / 8, tile0, 0, x_vec);
+                copy_rows(go, go_stride, row0, s.d_out, s.no / 8, P.packed ? tile0 : act_addr(d + 1), P.packed ? 4 : 0, go_vec);
+                asm volatile("cp.async.commit_group;" ::: "memory");
+                async_tile_wait();
+            }
+            for (int l = 0; l < d; ++l) {  // recomputed activation of layer l -> input tile of layer l + 1
+                start_step(l);
+                if (finish_step(true, false)) {
+                    const uint32_t dst = act_addr(l + 1) + row_off;
+                    const float *layer_bias = bias + l * kMaxDim;
+                    for_row_pieces<W>(taddr, s.h, half, [&](int chunk, const uint32_t(&piece)[8]) {
+                        st_shared_16(dst + ((chunk << 4) ^ row_swizzle), finish8<T, ACT, BIAS>(piece, layer_bias + 8 * chunk));
+                    });
+                }
+            }
+            for (int l = d; l >= 0; --l) {
+                const int in_pad = l == 0 ? s.ki : s.h;
+                start_step(2 * d - l);
+                const bool ok = finish_step(l > 0 || gx != nullptr, true);
+                if (l > 0 && ok) {  // dz of the layer below = dy * act', in place over that layer's parked output
+                    const uint32_t parked = act_addr(l) + row_off;
+                    if constexpr (kPreact) {
+                        const float *layer_bias = bias + (l - 1) * kMaxDim;
+#pragma unroll 1
+                        for (int u = 0; u < in_pad / (8 * W); ++u) {
+                            const int chunk = half * (in_pad / 16) + u;
+                            uint32_t dy[8], zz[8];
+                            tmem_ld8(taddr + 8 * chunk, dy);
+                            tmem_ld8(taddr + kAccCols + 8 * chunk, zz);
+                            tmem_ld_wait();
+                            float g[8];
+#pragma unroll
+                            for (int e = 0; e < 8; ++e) {
+                                float z = __uint_as_float(zz[e]);
+                                if constexpr (BIAS) z += layer_bias[8 * chunk + e];
+                                z = to_float<T>(from_float<T>(z));  // the forward pass stored z rounded
+                                g[e] = activate_grad(ACT, z, __uint_as_float(dy[e]));
+                            }
+                            st_shared_16(parked + ((chunk << 4) ^ row_swizzle),
+                                         make_uint4(pack_pair<T>(g[0], g[1]), pack_pair<T>(g[2], g[3]), pack_pair<T>(g[4], g[5]), pack_pair<T>(g[6], g[7])));
+                        }
+                    } else {
+                        for_row_pieces<W>(taddr, in_pad, half, [&](int chunk, const uint32_t(&piece)[8]) {
+                            const uint32_t off = (chunk << 4) ^ row_swizzle;
+                            uint4 gq = finish8<T, TH_ACT_NONE, false>(piece, nullptr);
+                            if constexpr (ACT == TH_ACT_RELU) {
+                                const uint4 a = ld_shared_16(parked + off);
+                                gq.x = keep_where_positive<T>(gq.x, a.x);
+                                gq.y = keep_where_positive<T>(gq.y, a.y);
+                                gq.z = keep_where_positive<T>(gq.z, a.z);
+                                gq.w = keep_where_positive<T>(gq.w, a.w);
+                            }
+                            st_shared_16(parked + off, gq);
+                        });
+                    }
+                } else if (ok && gx != nullptr) {
+                    const bool live = row0 + row < n_rows;
+                    T *row_ptr = gx + (live ? row0 + row : 0) * gx_stride;
+                    for_row_pieces<W>(taddr, in_pad, half, [&](int chunk, const uint32_t(&piece)[8]) {
+                        if (live) store_chunk_to_global<T>(row_ptr, chunk, s.d_in, finish8<T, TH_ACT_NONE, false>(piece, nullptr), gx_vec);
+                    });
+                    tc_fence_before();
+                }
+            }
+        }
+    }
+
+    // ---- flush the weight gradients (M = 64 layout: lanes 0..15 of warp quarter q hold rows 16 q ..); a warpgroup per layer ----
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (!tb.abort_flag && n_mine > 0 && !is_wgrad_warp) {
+        const MlpGradWorkspace G = grad_workspace_layout(s, workspace);
+        const int wq = warp & 3;
+        const uint32_t lane_base = static_cast<uint32_t>(32 * wq) << 16;
+        for (int l = warp >> 2; l <= d; l += S * W) {
+            const int in_pad = l == 0 ? s.ki : s.h;
+            const int in_dim = l == 0 ? s.d_in : s.d_hid, out_dim = l == d ? s.d_out : s.d_hid;
+            float *dst = G.base + (l == 0 ? G.w_in : (l == d ? G.w_out : G.w_hid + (l - 1) * s.d_hid * s.d_hid));
+            const int o = 16 * wq + lane - ((l == d && P.packed) ? 32 : 0);  // output row this lane holds
+            const bool quads = in_dim % 4 == 0 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0;
+            for (int first = 0; first < in_pad; first += 16) {
+                uint32_t raw[32];
+                tmem_ld16(tmem + lane_base + dw_col(l) + first, raw);
+                tmem_ld_wait();
+                if (lane < 16 && o >= 0 && o < out_dim) {
+#pragma unroll
+                    for (int c = 0; c < 16; c += 4) {
+                        if (quads) {
+                            if (first + c < in_dim)
+                                asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + o * in_dim + first + c), "f"(__uint_as_float(raw[c])),
+                                             "f"(__uint_as_float(raw[c + 1])), "f"(__uint_as_float(raw[c + 2])), "f"(__uint_as_float(raw[c + 3]))
+                                             : "memory");
+                        } else {
+#pragma unroll
+                            for (int e = 0; e < 4; ++e)
+                                if (first + c + e < in_dim) atomicAdd(dst + o * in_dim + first + c + e, __uint_as_float(raw[c + e]));
+                        }
+                    }
+                }
+            }
+            if constexpr (BIAS) {
+                float *bdst = G.base + (l == 0 ? G.b_in : (l == d ? G.b_out : G.b_hid + (l - 1) * s.d_hid));
+                uint32_t raw[8];
+                tmem_ld8(tmem + lane_base + db_col(l), raw);
+                tmem_ld_wait();
+                if (lane < 16 && o >= 0 && o < out_dim) atomicAdd(bdst + o, __uint_as_float(raw[0]));
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (is_wgrad_warp)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(static_cast<uint32_t>(P.tmem_cols)) : "memory");
+}
+
+bool one_slot_only() {
+    static const bool off = [] {
+        const char *v = getenv("TH_MLP_NO_SLOTS");
+        return v && v[0] == '1';
+    }();
+    return off;
+}
+
+// S slots of W warpgroups, if that fits one SM.  Measured (ms, B200), the most slots that fit are the fastest, two warpgroups
+// per slot when there are threads left: 2^21 rows 32-64-64-16 4 x 1 0.234, 3 x 2 0.269; 2^20 rows 32-4x64-16 2 x 2 0.277, 1 x 2 0.45;
+// with biases 32-64-64-16 3 x 2 0.158, 2 x 2 0.20; 300 007 rows 32-3x64-3 SiLU with biases 2 x 2 0.218, 1 x 2 0.40.  The kernels this
+// one replaced (four one-warpgroup slots with a polling warp each; one tile per CTA for biases and SiLU): 0.271, 0.333, 0.340 and
+// 0.412.  Tried: dz in a tile of its own so that the chain waits for a weight gradient one step late, next rows fetched ahead into
+// it (0.290 at 32-4x64-16 against 0.284, and a slot less where it costs one); loops over 32 columns left rolled because
+// unrolled ones overflow the instruction cache (2^21 rows: 0.280 against 0.234).
+template <typename T, int ACT, bool BIAS, int S, int W>
+int launch_slots(const MlpShape &s, const MlpParams &p, const void *x, int64_t x_stride, const void *go, int64_t go_stride,
+                 void *gx, int64_t gx_stride, float *workspace, int64_t rows, cudaStream_t stream) {
+    const SlotPlan P = slot_plan(s, S);
+    if (P.total > kSmemBudget || P.tmem_cols > 512 || 2 * s.depth + 1 > kStepsMax) return kTcNotApplicable;
+    int smem = P.total;
+    if (smem < kSmemBudget / 2 + 1024) smem = kSmemBudget / 2 + 1024;  // one CTA per SM
+    WeightMaps maps;
+    const int use_tma = make_weight_maps(maps, s, p);
+    auto kernel = slots_mlp_bwd_tc_kernel<T, ACT, BIAS, S, W>;
+    if (int rc = cuda_status(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
+                             "cudaFuncSetAttribute(slots_mlp_bwd_tc_kernel)")) return rc;
+    const long long tiles = (rows + kTileRows - 1) / kTileRows;
+    const long long cap = sm_count();
+    kernel<<<static_cast<unsigned>(tiles < cap ? tiles : cap), 128 * S * W + 32, smem, stream>>>(
+        s, p, maps, use_tma, P, static_cast<const T *>(x), x_stride, static_cast<const T *>(go), go_stride, static_cast<T *>(gx), gx_stride,
+        workspace, rows, rows_vector_ok(x, x_stride, s.d_in), rows_vector_ok(go, go_stride, s.d_out), gx ? rows_vector_ok(gx, gx_stride, s.d_in) : 0);
+    return launch_status("slots_mlp_bwd_tc_kernel launch");
+}
+
+template <typename T, int ACT, bool BIAS>
+int launch_any_slots(const MlpShape &s, const MlpParams &p, const void *x, int64_t x_stride, const void *go, int64_t go_stride, void *gx,
+                     int64_t gx_stride, float *workspace, int64_t rows, cudaStream_t stream) {
+#define TH_SLOTS(S, W)                                                                                                          \
+    if (const int rc = launch_slots<T, ACT, BIAS, S, W>(s, p, x, x_stride, go, go_stride, gx, gx_stride, workspace, rows, stream); \
+        rc != kTcNotApplicable)                                                                                                 \
+        return rc;
+    if (!one_slot_only()) {
+        TH_SLOTS(4, 1)
+        TH_SLOTS(3, 2)
+        TH_SLOTS(2, 2)
+    }
+    TH_SLOTS(1, 2)
+#undef TH_SLOTS
+    return kTcNotApplicable;
+}
+
+template <typename T>
+int launch_slots_act(const MlpShape &s, const MlpParams &p, const void *x, int64_t x_stride, const void *go, int64_t go_stride, void *gx,
+                     int64_t gx_stride, float *workspace, int64_t rows, cudaStream_t stream) {
+#define TH_SLOTS_ACT(A)                                                                                                      \
+    (s.has_bias ? launch_any_slots<T, A, true>(s, p, x, x_stride, go, go_stride, gx, gx_stride, workspace, rows, stream)     \
+                : launch_any_slots<T, A, false>(s, p, x, x_stride, go, go_stride, gx, gx_stride, workspace, rows, stream))
+    switch (s.act) {
+        case TH_ACT_RELU: return TH_SLOTS_ACT(TH_ACT_RELU);
+        case TH_ACT_SILU: return TH_SLOTS_ACT(TH_ACT_SILU);
+        case TH_ACT_RELU2: return TH_SLOTS_ACT(TH_ACT_RELU2);
+        default: return TH_SLOTS_ACT(TH_ACT_NONE);
+    }
+#undef TH_SLOTS_ACT
+}
+
+}  // namespace
+
+int mlp_bwd_slots(const MlpShape &s, const MlpParams &p, const void *x, int64_t x_stride, const void *go, int64_t go_stride, void *gx,
+                  int64_t gx_stride, float *workspace, int64_t rows, int dtype, cudaStream_t stream) {
+    switch (dtype) {
+        case TH_F16: return launch_slots_act<__half>(s, p, x, x_stride, go, go_stride, gx, gx_stride, workspace, rows, stream);
+        case TH_BF16: return launch_slots_act<__nv_bfloat16>(s, p, x, x_stride, go, go_stride, gx, gx_stride, workspace, rows, stream);
+        default: return kTcNotApplicable;
+    }
+}
+
+int mlp_bwd_slots_status() {
+    int status = 0;
+    if (cudaMemcpyFromSymbol(&status, g_tc_status, sizeof(int)) != cudaSuccess) return -1;
+    return status;
+}
+
+}  // namespace th

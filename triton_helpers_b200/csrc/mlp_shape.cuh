@@ -76,4 +76,9 @@ int mlp_bwd_tc(const MlpShape &s, const MlpParams &p, const void *x, int64_t x_s
                int64_t go_stride, void *gx, int64_t gx_stride, float *workspace, int64_t rows, int dtype,
                cudaStream_t stream);
 
+// The backward with several row tiles in flight per SM (fused_mlp_bwd.cu), tried first by mlp_bwd_tc.
+int mlp_bwd_slots(const MlpShape &s, const MlpParams &p, const void *x, int64_t x_stride, const void *go, int64_t go_stride,
+                  void *gx, int64_t gx_stride, float *workspace, int64_t rows, int dtype, cudaStream_t stream);
+int mlp_bwd_slots_status();  // its copy of the status word
+
 }  // namespace th

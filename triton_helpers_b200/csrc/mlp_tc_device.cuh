@@ -17,6 +17,41 @@ namespace {
 
 constexpr int kAccCols = 64;  // TMEM columns of the forward / dgrad accumulator
 
+// ---- bounded waits ----
+
+// Bounded by wall-clock time (the nanosecond global timer, looked at every 64 polls): two seconds are
+// orders of magnitude above any wait of a healthy run, also under a profiler's replay.
+constexpr unsigned long long kPipeWaitNs = 2000000000ull;
+
+__device__ __forceinline__ unsigned long long global_ns() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    return t;
+}
+
+__device__ __forceinline__ bool pipe_wait(uint32_t bar, uint32_t parity, int *abort_flag) {
+    if (*reinterpret_cast<volatile int *>(abort_flag)) return false;
+    unsigned long long deadline = 0;
+    for (unsigned poll = 0;; ++poll) {
+        uint32_t done;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
+            : "=r"(done)
+            : "r"(bar), "r"(parity)
+            : "memory");
+        if (done) return true;
+        if ((poll & 63u) == 63u) {
+            if (*reinterpret_cast<volatile int *>(abort_flag)) return false;
+            const unsigned long long now = global_ns();
+            if (deadline == 0) deadline = now + kPipeWaitNs;
+            else if (now > deadline) break;
+        }
+    }
+    *reinterpret_cast<volatile int *>(abort_flag) = 1;
+    g_tc_status = 1;
+    return false;
+}
+
 // ---- shared-memory plan ------------------------------------------------------------------------
 
 struct TcPlan {
@@ -157,6 +192,7 @@ __device__ __forceinline__ void drain_row(uint32_t taddr, int out_pad, const flo
         for (int u = 0; u < 2; ++u) sink(u, finish8<T, ACT, BIAS>(raw + 8 * u, bias + 8 * u));
         return;
     }
+#pragma unroll 1
     for (int first = 0; first < out_pad; first += 32) {
         tmem_ld32(taddr + first, raw);
         tmem_ld_wait();
