@@ -109,12 +109,7 @@ template <int W, typename Fn>
 __device__ __forceinline__ void for_row_pieces(uint32_t taddr, int pad, int half, Fn fn) {
     if constexpr (W == 2) {
         const int n = pad / 2, first = half * (n / 8);
-        if (n == 32) {
-            for_each_piece_n<32>(taddr + half * n, [&](int u, const uint32_t(&piece)[8]) { fn(first + u, piece); });
-        } else {
-#pragma unroll 1
-            for (int v = 0; v < n / 8; ++v) for_each_piece_n<8>(taddr + half * n + 8 * v, [&](int, const uint32_t(&piece)[8]) { fn(first + v, piece); });
-        }
+        for_each_piece(taddr + half * n, n, [&](int u, const uint32_t(&piece)[8]) { fn(first + u, piece); });
     } else {
         int first = 0;
 #pragma unroll 1

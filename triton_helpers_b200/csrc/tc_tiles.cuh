@@ -285,10 +285,14 @@ __device__ __forceinline__ void for_each_piece_n(uint32_t taddr, Fn fn) {
 // two threads share a row)
 template <typename Fn>
 __device__ __forceinline__ void for_each_piece(uint32_t taddr, int n, Fn fn) {
-    if (n == 32) for_each_piece_n<32>(taddr, fn);
-    else if (n == 24) for_each_piece_n<24>(taddr, fn);
-    else if (n == 16) for_each_piece_n<16>(taddr, fn);
-    else for_each_piece_n<8>(taddr, fn);
+    // two forms only, the second rolled: every call is inlined several times in kernels that live on their instruction cache
+    // (reversible forward, 2^20 rows: 0.655 -> 0.631 ms)
+    if (n == 32) {
+        for_each_piece_n<32>(taddr, fn);
+    } else {
+#pragma unroll 1
+        for (int u = 0; u < n / 8; ++u) for_each_piece_n<8>(taddr + 8 * u, [&](int, const uint32_t(&piece)[8]) { fn(u, piece); });
+    }
 }
 
 // 8 fp32 accumulator columns (+ bias) -> activation -> one 16-byte chunk; the ReLU-without-bias case
