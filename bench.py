@@ -264,6 +264,11 @@ class TrainStep:
             "th_mse_grad": ("hbm", 3 * S * 16 * n),
             "th_scale_cast": ("hbm", 6 * 7168),
             "th_adam_step": ("hbm", (3 * S + 16) * self.table_elems),
+            "th_adam_steps": ("hbm", (3 * S + 16) * self.table_elems),
+            "th_hash_order": ("hbm", (2 * 12 + 2 * 4 + 16) * n),
+            "th_hash_fwd_ordered": ("hbm", enc),
+            "th_hash_bwd_ordered": ("hbm", enc),
+            "th_mlp_fwd_mse_ordered": ("tensor", mlp_flops * n),
         }
 
 
@@ -312,7 +317,8 @@ class HashOnly:
 
     def work(self):
         b = hash_bytes_per_point(16, self.c["feats"], 4) * self.units
-        return {"th_hash_fwd": ("hbm", b), "th_hash_bwd": ("hbm", b)}
+        return {"th_hash_fwd": ("hbm", b), "th_hash_bwd": ("hbm", b), "th_hash_fwd_ordered": ("hbm", b), "th_hash_bwd_ordered": ("hbm", b),
+                "th_hash_order": ("hbm", (2 * 12 + 2 * 4 + 16) * self.units)}  # fmt: skip
 
 
 

@@ -838,7 +838,7 @@ PyObject *py_reversible_mlp(PyObject *, PyObject *const *args, Py_ssize_t n_args
 
 // ---- hash encoding + MLP --------------------------------------------------------------------------------------
 //
-// Up to eight hidden layers the encoding's kernels and the MLP's run one after the other: each of them fills an SM by
+// Up to six layers before the output (what the MLP backward holds at any width) the encoding's kernels and the MLP's run one after the other: each of them fills an SM by
 // itself (the gathers and reductions want all its warps, the MLP its shared memory), large batches can be ordered in
 // space, and together they are faster than the kernels that fuse the two (B200, 200 003 points in two dimensions,
 // forward + backward, 192 -> 150 us; 2^21 points in three, forward 0.72 -> 0.47 ms), which deeper networks still take.
@@ -936,7 +936,7 @@ PyObject *py_hash_encoded_mlp(PyObject *, PyObject *const *args, Py_ssize_t n_ar
     mlp.depth = static_cast<int>(depth);
     // what the fused kernels cover: anything else is Python's FieldUnsupported
     static const bool legacy = getenv("TH_MLP_LEGACY") && getenv("TH_MLP_LEGACY")[0] == '1';
-    const bool separate = !legacy && depth <= 8 && (call.dims == 2 || call.dims == 3) && (call.feats == 2 || call.feats == 4) &&
+    const bool separate = !legacy && depth <= 6 && (call.dims == 2 || call.dims == 3) && (call.feats == 2 || call.feats == 4) &&
                           d_in % 16 == 0 && d_in <= 64 && (mlp.act == TH_ACT_RELU || mlp.act == TH_ACT_NONE) &&
                           (hidden == 16 || hidden == 32 || hidden == 64) && d_out >= 1 && d_out <= 64;
     Tensor out;

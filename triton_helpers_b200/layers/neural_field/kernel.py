@@ -1,10 +1,12 @@
-r"""Hash encoding and fused MLP in one kernel per direction (``th_field_fwd`` / ``th_field_bwd``).
+r"""Hash encoding and fused MLP as one operator, with kernels that fuse the two (``th_field_fwd`` / ``th_field_bwd``).
 
 triton_helpers has no such operator: it launches ``hash_encoding`` and ``fully_fused_mlp`` one after the
 other and notes that the encoding is meant to feed a fully fused MLP with its ``L * F`` columns staying on
 chip (``triton_helpers/layers/hash_encoding/kernel.py:241-243``).  ``hash_encoded_mlp(coords, embeddings,
 w_in, w_out, w_hid, ...)`` computes ``fully_fused_mlp(hash_encoding(coords, embeddings, ...), w_in, None,
-w_out, None, w_hid, None, activation)`` - same arguments, same values, same gradients - without the
+w_out, None, w_hid, None, activation)`` - same arguments, same values, same gradients.  Networks of up to six
+layers before the output run the encoding's and the MLP's own kernels back to back from one native call, which is
+faster than the fused kernels; ``field_forward`` / ``field_backward`` and deeper networks use those, without the
 encoding making a round trip through memory between the two.
 
 Covered by the fused kernels: one 16-bit dtype for table and weights, 2 or 3 coordinate dimensions, 2 or 4

@@ -7,9 +7,9 @@ the drop-in ``HashEncoding`` and ``FullyFusedMLP`` modules.
 Two ways through the step:
 
 * **direct** (table and MLP share one 16-bit dtype): the trainer calls the C ABI itself on buffers it
-  keeps from step to step - by default the fused pair ``th_field_fwd`` (encoding + MLP + loss) and
-  ``th_field_bwd`` (MLP backward + encoding backward), else ``th_hash_fwd``, ``th_mlp_fwd_mse``,
-  ``th_mlp_bwd``, ``th_hash_bwd``; then ``th_scale_cast`` and ``th_adam_step``.  All gradients live in ONE flat 16-bit
+  keeps from step to step - ``th_hash_fwd``, ``th_mlp_fwd_mse``, ``th_mlp_bwd``, ``th_hash_bwd`` (their ordered forms for
+  large batches) from one native call, or on request the fused pair ``th_field_fwd`` (encoding + MLP + loss) and
+  ``th_field_bwd`` (MLP backward + encoding backward); then ``th_scale_cast`` and ``th_adam_steps``.  All gradients live in ONE flat 16-bit
   buffer ``[table gradient | MLP gradients]`` so that a step costs one all-reduce:
 
   - the table part holds ``grad_out_scale * sum over the local batch`` (the encoding backward adds
@@ -19,7 +19,8 @@ Two ways through the step:
     rounded.  A sum over 2^21 rows reaches 1e4..1e5 and four ranks of that exceed float16's 65504;
     means stay below one at any batch size and world size.
 
-* **autograd** (float32 parameters): forward and backward through the layers' autograd functions,
+* **float32 parameters**: on one rank the same sequence in one native call, the MLP on 16-bit copies of its
+  parameters; otherwise forward and backward through the layers' autograd functions and
   ``parallel.allreduce_gradients`` on the float32 gradients.
 
 With more than one process the point batch is split across ranks (every rank passes the same
@@ -89,11 +90,10 @@ class NeuralFieldTrainer(nn.Module):
             global batch of the first step.
         group: process group for data parallelism (``None``: the default group, if initialised).
         fused: direct mode only; which steps run in the kernels that fuse the encoding with the MLP.
-            ``None`` (default): the backward pass when the fused kernel covers the configuration (measured
-            at benchmark configuration 3 on a B200: fused backward 1.04 ms against 0.36 + 0.78 ms for MLP
-            backward + encoding backward; fused forward 0.71 ms against 0.55 + 0.12 ms, so the forward stays
-            separate); ``"backward"``: the same, but raise if it is not covered; ``True``: forward and
-            backward fused, raise if not covered; ``False``: always the separate operators.
+            ``None`` (default) or ``False``: none, the separate operators, over spatially ordered points where
+            that pays (benchmark configuration 3 on a B200: 1.48 ms per step; with the fused backward 1.73 ms);
+            ``"backward"``: the backward pass, raise if it is not covered; ``True``: forward and backward, raise
+            if not covered.
         backward_passes: ``None`` (default): one encoding backward, then one gradient sum over the
             ranks.  An integer n (direct mode): the encoding backward runs in n level ranges, finest
             first; the gradient rows of a finished range are summed over the ranks (NCCL,
@@ -244,7 +244,25 @@ class NeuralFieldTrainer(nn.Module):
                         raise
                     self._no_fused_forward = True  # nothing was launched: the separate operators from now on
                     fuse_fwd = False
-            if not fuse_fwd:
+            # ---- or, for large batches, in spatial order from the features to the table gradient ----
+            order = None
+            if not (fuse_fwd or fuse_bwd or self.backward_passes):
+                order = launch.order(st.n_feats * st.flat_grad.element_size(), True)
+            if order is not None:
+                _lib.check(
+                    lib.th_hash_fwd_ordered(order.data_ptr(), 1, enc.embeddings.data_ptr(), code, st.feats.data_ptr(), st.d_feat, *geometry[:-1],
+                                            0, enc.num_levels, stream),
+                    "th_hash_fwd_ordered",
+                )  # fmt: skip
+                rc = lib.th_mlp_fwd_mse_ordered(
+                    st.feats.data_ptr(), st.d_feat, *mlp_ptrs, targets.data_ptr(), targets.stride(0), code, order.data_ptr(),
+                    st.grad_pred.data_ptr(), st.d_out, st.loss_sum.data_ptr(), 1.0, scale, n, *dims, act, code, stream,
+                )  # fmt: skip
+                if rc == _lib.TH_ERR_UNSUPPORTED:
+                    order = None
+                else:
+                    _lib.check(rc, "th_mlp_fwd_mse_ordered")
+            if not fuse_fwd and order is None:
                 _lib.check(
                     lib.th_hash_fwd(*launch.coord_args, enc.embeddings.data_ptr(), code, st.feats.data_ptr(), st.d_feat,
                                     *geometry, 0, enc.num_levels, stream),
@@ -280,6 +298,13 @@ class NeuralFieldTrainer(nn.Module):
             _lib.check(lib.th_scale_cast(st.workspace.data_ptr(), st.mlp_grad.data_ptr(), st.mlp_grad.numel(), cast_scale, code, stream), "th_scale_cast")
             pending = PendingReduce(self.group, bucket_bytes=0)
             if fuse_bwd:
+                pending.start([st.flat_grad])
+            elif order is not None:
+                _lib.check(
+                    lib.th_hash_bwd_ordered(order.data_ptr(), 1, st.grad_feats.data_ptr(), st.d_feat, st.table_grad.data_ptr(), code,
+                                            *geometry[:-1], 0, enc.num_levels, stream),
+                    "th_hash_bwd_ordered",
+                )  # fmt: skip
                 pending.start([st.flat_grad])
             else:
                 passes = [(0, enc.num_levels)] if not self.backward_passes else level_passes(launch.geo.rows, self.backward_passes)
@@ -328,10 +353,10 @@ class NeuralFieldTrainer(nn.Module):
     def _fusion_plan(self, st: "_DirectState") -> Tuple[bool, bool]:
         r"""(fused forward?, fused backward?) for this step; see ``fused`` in the class docstring."""
         mode = self.fused
-        if mode is False:
+        if not mode:
             return False, False
         want_fwd = mode is True
-        want_bwd = mode in (None, True, "backward")
+        want_bwd = mode in (True, "backward")
         if st.b_in is not None or self.backward_passes:
             # the fused backward is built for bias-free networks; level-range passes need the separate encoding backward
             if mode in (True, "backward"):
