@@ -431,7 +431,7 @@ int launch_rev_bwd(const RevShape &s, const RevParams &p, const void *y, int64_t
     const size_t bytes = sizeof(float) * rev_cta_floats(s) * grid;
     if (int rc = cuda_status(cudaMemsetAsync(workspace, 0, bytes, stream), "cudaMemsetAsync(workspace)")) return rc;
     // tensor-core kernels first (they also reduce and write the gradients); mma.sync kernels otherwise
-    const int tc = rows > 0 ? rev_bwd_tc(s, p, y, y_stride, go, go_stride, gx, gx_stride, x_rec, xr_stride, dw, workspace, grid,
+    const int tc = rows > 0 ? rev_bwd_tc(s, p, y, y_stride, go, go_stride, gx, gx_stride, x_rec, xr_stride, dw, db, workspace, grid,
                                          rows, std::is_same<T, __half>::value ? TH_F16 : TH_BF16, stream)
                             : kRevTcNotApplicable;
     if (tc != kRevTcNotApplicable) return tc;

@@ -23,8 +23,10 @@
 // kernel sums the copies.  The backward pass needs all 512 TMEM columns, so one CTA per SM; the
 // forward pass needs 192 (256 allocated), two CTAs per SM.
 //
-// Covered here: float16 / bfloat16, 16-byte-aligned rows; backward: ReLU or no activation, no
-// biases.  Everything else stays on the mma.sync kernels.
+// Bias gradients are column sums of DY and DZ, summed over each warp's rows with shuffles in the epilogues: tensor memory
+// has no columns left for the MMA with ones that the fused MLP uses.
+//
+// Covered here: float16 / bfloat16, 16-byte-aligned rows.  Everything else stays on the mma.sync kernels.
 #include "rev_shape.cuh"
 #include "tc_tiles.cuh"
 
@@ -145,9 +147,9 @@ __device__ __forceinline__ void tile_row_to_tmem(unsigned char *tile, const Seat
     }
 }
 
-// This thread's pieces of an fp32 TMEM accumulator -> (optional bias, written back) -> rounded into an
-// operand tile and / or a global row.
-template <typename T, bool BIAS>
+// This thread's pieces of an fp32 TMEM accumulator -> (optional bias, added or - when a branch is undone - taken off, written
+// back) -> rounded into an operand tile and / or a global row.
+template <typename T, bool BIAS, bool UNDO = false>
 __device__ __forceinline__ void stream_epilogue(uint32_t taddr, const Seat &seat, int width, const float *bias,
                                                 unsigned char *tile, T *global_row, bool live) {
     const int n = width / kGroups, first = seat.group * (n / 8);  // this thread's columns / first 8-column piece
@@ -158,7 +160,10 @@ __device__ __forceinline__ void stream_epilogue(uint32_t taddr, const Seat &seat
         for (int k = 0; k < 8; ++k) v[k] = piece[k];
         if constexpr (BIAS) {
 #pragma unroll
-            for (int k = 0; k < 8; ++k) v[k] = __float_as_uint(__uint_as_float(v[k]) + bias[8 * (first + u) + k]);
+            for (int k = 0; k < 8; ++k) {
+                const float b = bias[8 * (first + u) + k];
+                v[k] = __float_as_uint(__uint_as_float(v[k]) + (UNDO ? -b : b));
+            }
             tmem_st8(taddr + 8 * (first + u), v);
         }
         const uint4 packed = finish8<T, TH_ACT_NONE, false>(v, nullptr);
@@ -396,7 +401,34 @@ __device__ __forceinline__ void flush_dw_quadrant(uint32_t tmem, int q, uint32_t
     }
 }
 
-template <typename T, int ACT>
+// Adds the sums of eight columns over the warp's 32 rows to dst[0 .. 7]: a reduce-scatter over five shuffle levels, then one
+// 32-byte reduction.
+template <typename T>
+__device__ __forceinline__ void add_column_sums(uint4 packed, float *dst) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t w[4] = {packed.x, packed.y, packed.z, packed.w};
+    float v[8];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float2 f = unpack_pair<T>(w[k]);
+        v[2 * k] = f.x;
+        v[2 * k + 1] = f.y;
+    }
+#pragma unroll
+    for (int keep = 4; keep > 0; keep /= 2) {
+        const bool high = lane & (4 * keep);
+#pragma unroll
+        for (int k = 0; k < keep; ++k) {
+            const float other = __shfl_xor_sync(0xffffffffu, high ? v[k] : v[k + keep], 4 * keep);
+            v[k] = (high ? v[k + keep] : v[k]) + other;
+        }
+    }
+    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
+    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+    if ((lane & 3) == 0) atomicAdd(dst + (lane >> 2), v[0]);
+}
+
+template <typename T, int ACT, bool BIAS>
 __global__ void __launch_bounds__(kTcThreads + kRevFlushThreads, 1)
 rev_bwd_tc_kernel(const RevShape s, const RevParams p, const __grid_constant__ RevWeightMaps maps, const int use_tma,
                   const T *__restrict__ y, long long y_stride,
@@ -512,6 +544,8 @@ rev_bwd_tc_kernel(const RevShape s, const RevParams p, const __grid_constant__ R
                     else prefetch_weights<T>(smem, P, s, p, k > 0 ? k - 1 : s.blocks - 1, stage ^ 1);
                 }
                 const unsigned char *w = smem + P.ring + stage * kStageBytes;
+                const float *block_bias = reinterpret_cast<const float *>(smem + P.bias) + stage * 4 * kMaxDim;
+                float *bias_sums = cta_acc + static_cast<size_t>(s.blocks) * 4 * kMatFloats + static_cast<size_t>(k) * 4 * kMaxDim;
 #pragma unroll 1
                 for (int pass = 0; pass < 2; ++pass, ++n) {
                     // pass 0 undoes y2 = x2 + G(y1): input stream S1, output stream S2, gradient flows D2 -> D1
@@ -538,21 +572,45 @@ rev_bwd_tc_kernel(const RevShape s, const RevParams p, const __grid_constant__ R
                         const int nn = s.hid / kGroups, first = seat.group * (nn / 8);
                         const uint32_t row_off = seat.row * 128, row_swizzle = (seat.row & 7) << 4;
                         const uint32_t h_row = smem_addr(h_tile) + row_off, dz_row = smem_addr(dz_tile) + row_off;
+                        const float *bias1 = block_bias + m1 * kMaxDim;
                         for_each_piece(taddr + kZ + seat.group * nn, nn, [&](int u, const uint32_t(&piece)[8]) {
-                            st_shared_16(h_row + (((first + u) << 4) ^ row_swizzle), finish8<T, ACT, false>(piece, nullptr));
+                            st_shared_16(h_row + (((first + u) << 4) ^ row_swizzle), finish8<T, ACT, BIAS>(piece, bias1 + 8 * (first + u)));
                         });
-                        for_each_piece(taddr + kDH + seat.group * nn, nn, [&](int u, const uint32_t(&piece)[8]) {
-                            const uint32_t off = ((first + u) << 4) ^ row_swizzle;
-                            uint4 g = finish8<T, TH_ACT_NONE, false>(piece, nullptr);
-                            if constexpr (ACT == TH_ACT_RELU) {
-                                const uint4 h = ld_shared_16(h_row + off);  // this thread's own store above
-                                g.x = keep_where_positive<T>(g.x, h.x);
-                                g.y = keep_where_positive<T>(g.y, h.y);
-                                g.z = keep_where_positive<T>(g.z, h.z);
-                                g.w = keep_where_positive<T>(g.w, h.w);
+                        auto store_dz = [&](int u, uint4 g) {
+                            st_shared_16(dz_row + (((first + u) << 4) ^ row_swizzle), g);
+                            if constexpr (BIAS) add_column_sums<T>(g, bias_sums + m1 * kMaxDim + 8 * (first + u));
+                        };
+                        if constexpr (ACT == TH_ACT_SILU || ACT == TH_ACT_RELU2) {
+                            // the derivative is taken at the pre-activation rounded to the storage type
+#pragma unroll 1
+                            for (int u = 0; u < nn / 8; ++u) {
+                                uint32_t dh[8], zz[8];
+                                tmem_ld8(taddr + kDH + seat.group * nn + 8 * u, dh);
+                                tmem_ld8(taddr + kZ + seat.group * nn + 8 * u, zz);
+                                tmem_ld_wait();
+                                float g[8];
+#pragma unroll
+                                for (int e = 0; e < 8; ++e) {
+                                    float z = __uint_as_float(zz[e]);
+                                    if constexpr (BIAS) z += bias1[8 * (first + u) + e];
+                                    z = to_float<T>(from_float<T>(z));
+                                    g[e] = activate_grad(ACT, z, __uint_as_float(dh[e]));
+                                }
+                                store_dz(u, make_uint4(pack_pair<T>(g[0], g[1]), pack_pair<T>(g[2], g[3]), pack_pair<T>(g[4], g[5]), pack_pair<T>(g[6], g[7])));
                             }
-                            st_shared_16(dz_row + off, g);
-                        });
+                        } else {
+                            for_each_piece(taddr + kDH + seat.group * nn, nn, [&](int u, const uint32_t(&piece)[8]) {
+                                uint4 g = finish8<T, TH_ACT_NONE, false>(piece, nullptr);
+                                if constexpr (ACT == TH_ACT_RELU) {
+                                    const uint4 h = ld_shared_16(h_row + (((first + u) << 4) ^ row_swizzle));  // this thread's own store above
+                                    g.x = keep_where_positive<T>(g.x, h.x);
+                                    g.y = keep_where_positive<T>(g.y, h.y);
+                                    g.z = keep_where_positive<T>(g.z, h.z);
+                                    g.w = keep_where_positive<T>(g.w, h.w);
+                                }
+                                store_dz(u, g);
+                            });
+                        }
                     }
                     main_publish();
                     // step B: undo the branch and push the gradient through (waited for below); then both weight
@@ -573,9 +631,16 @@ rev_bwd_tc_kernel(const RevShape s, const RevParams p, const __grid_constant__ R
                         }
                         __syncwarp();
                     }
+                    if constexpr (BIAS) {  // under those MMAs: the second layer's bias gradient, column sums of DY
+                        const int nh = s.half / kGroups, first_h = seat.group * (nh / 8);
+                        const uint32_t dy_row = dy_cur + seat.row * 128, swizzle = (seat.row & 7) << 4;
+#pragma unroll 1
+                        for (int u = 0; u < nh / 8; ++u)
+                            add_column_sums<T>(ld_shared_16(dy_row + (((first_h + u) << 4) ^ swizzle)), bias_sums + m2 * kMaxDim + 8 * (first_h + u));
+                    }
                     main_wait_mma(bar, phase, &abort_flag);
                     // next pass: its input is the stream just reconstructed, its output gradient the one just updated
-                    stream_epilogue<T, false>(taddr + out_col, seat, s.half, nullptr, u_next, nullptr, false);
+                    stream_epilogue<T, BIAS, true>(taddr + out_col, seat, s.half, block_bias + m2 * kMaxDim, u_next, nullptr, false);
                     stream_epilogue<T, false>(taddr + in_d_col, seat, s.half, nullptr, dy_next, nullptr, false);
                     if (pass == 1) {  // next block's weights have landed
                         if (!use_tma) async_tile_wait();
@@ -605,24 +670,36 @@ rev_bwd_tc_kernel(const RevShape s, const RevParams p, const __grid_constant__ R
     cta_teardown(tmem, P.tmem_cols);
 }
 
-// Sum the per-CTA accumulators ([cta][block][matrix][64][64]) into the gradient tensors.
+// Sum the per-CTA accumulators ([cta][block][matrix][64][64], then [block][4][64] bias sums) into the gradient tensors.
 template <typename T>
-__global__ void rev_grad_reduce_tc_kernel(const RevShape s, const float *__restrict__ workspace, int n_ctas, T *dw_f1,
-                                          T *dw_f2, T *dw_g1, T *dw_g2) {
+__global__ void rev_grad_reduce_tc_kernel(const RevShape s, const float *__restrict__ workspace, int n_ctas, T *dw_f1, T *dw_f2, T *dw_g1,
+                                          T *dw_g2, T *db_f1, T *db_f2, T *db_g1, T *db_g2) {
     const size_t per_cta = rev_cta_floats(s);
     const size_t mat_total = static_cast<size_t>(s.blocks) * 4 * kMatFloats;
+    const size_t total = s.has_bias ? per_cta : mat_total;
     T *dw[4] = {dw_f1, dw_f2, dw_g1, dw_g2};
-    for (size_t e = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; e < mat_total;
+    T *db[4] = {db_f1, db_f2, db_g1, db_g2};
+    for (size_t e = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; e < total;
          e += static_cast<size_t>(gridDim.x) * blockDim.x) {
-        const int k = static_cast<int>(e / (4 * kMatFloats));
-        const int m = static_cast<int>((e / kMatFloats) % 4);
-        const int row = static_cast<int>((e % kMatFloats) / 64), col = static_cast<int>(e % 64);
-        const int out_dim = (m & 1) ? s.half : s.hid, in_dim = (m & 1) ? s.hid : s.half;
-        if (row >= out_dim || col >= in_dim || !dw[m]) continue;
-        const size_t at = (e / kMatFloats) * kMatFloats + dw_private_index(row, col);
+        size_t at = e;
+        T *dst;
+        if (e < mat_total) {
+            const int k = static_cast<int>(e / (4 * kMatFloats));
+            const int m = static_cast<int>((e / kMatFloats) % 4);
+            const int row = static_cast<int>((e % kMatFloats) / 64), col = static_cast<int>(e % 64);
+            const int out_dim = (m & 1) ? s.half : s.hid, in_dim = (m & 1) ? s.hid : s.half;
+            if (row >= out_dim || col >= in_dim || !dw[m]) continue;
+            at = (e / kMatFloats) * kMatFloats + dw_private_index(row, col);
+            dst = dw[m] + (static_cast<size_t>(k) * out_dim + row) * in_dim + col;
+        } else {
+            const int b = static_cast<int>(e - mat_total), k = b / 256, m = (b / 64) % 4, c = b % 64;
+            const int width = (m & 1) ? s.half : s.hid;
+            if (c >= width || !db[m]) continue;
+            dst = db[m] + static_cast<size_t>(k) * width + c;
+        }
         float sum = 0.f;
         for (int c = 0; c < n_ctas; ++c) sum += workspace[c * per_cta + at];
-        dw[m][(static_cast<size_t>(k) * out_dim + row) * in_dim + col] = from_float<T>(sum);
+        *dst = from_float<T>(sum);
     }
 }
 
@@ -714,13 +791,13 @@ int launch_rev_fwd(const RevShape &s, const RevParams &p, const void *x, int64_t
                       : launch_rev_fwd_act<T, false>(s, p, x, x_stride, y, y_stride, rows, stream);
 }
 
-template <typename T, int ACT>
+template <typename T, int ACT, bool BIAS>
 int launch_rev_bwd_t(const RevShape &s, const RevParams &p, const void *y, int64_t y_stride, const void *go,
                      int64_t go_stride, void *gx, int64_t gx_stride, void *x_rec, int64_t xr_stride, void *const dw[4],
-                     float *workspace, int n_ctas, int64_t rows, cudaStream_t stream) {
+                     void *const db[4], float *workspace, int n_ctas, int64_t rows, cudaStream_t stream) {
     const RevTcPlan P = rev_tc_plan(true);
     const int smem = smem_request(P, 1);  // all 512 TMEM columns: one CTA per SM
-    auto kernel = rev_bwd_tc_kernel<T, ACT>;
+    auto kernel = rev_bwd_tc_kernel<T, ACT, BIAS>;
     if (int rc = cuda_status(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
                              "cudaFuncSetAttribute(rev_bwd_tc_kernel)")) return rc;
     RevWeightMaps maps;
@@ -729,10 +806,9 @@ int launch_rev_bwd_t(const RevShape &s, const RevParams &p, const void *y, int64
                                                 static_cast<const T *>(go), go_stride, static_cast<T *>(gx), gx_stride,
                                                 static_cast<T *>(x_rec), xr_stride, workspace, rows);
     if (int rc = launch_status("rev_bwd_tc_kernel launch")) return rc;
-    const size_t mat_total = static_cast<size_t>(s.blocks) * 4 * kMatFloats;
-    rev_grad_reduce_tc_kernel<T><<<static_cast<unsigned>((mat_total + 255) / 256), 256, 0, stream>>>(
+    rev_grad_reduce_tc_kernel<T><<<static_cast<unsigned>((rev_cta_floats(s) + 255) / 256), 256, 0, stream>>>(
         s, workspace, n_ctas, static_cast<T *>(dw[0]), static_cast<T *>(dw[1]), static_cast<T *>(dw[2]),
-        static_cast<T *>(dw[3]));
+        static_cast<T *>(dw[3]), static_cast<T *>(db[0]), static_cast<T *>(db[1]), static_cast<T *>(db[2]), static_cast<T *>(db[3]));
     return launch_status("rev_grad_reduce_tc_kernel launch");
 }
 
@@ -750,23 +826,28 @@ int rev_fwd_tc(const RevShape &s, const RevParams &p, const void *x, int64_t x_s
 }
 
 int rev_bwd_tc(const RevShape &s, const RevParams &p, const void *y, int64_t y_stride, const void *go, int64_t go_stride,
-               void *gx, int64_t gx_stride, void *x_rec, int64_t xr_stride, void *const dw[4], float *workspace,
+               void *gx, int64_t gx_stride, void *x_rec, int64_t xr_stride, void *const dw[4], void *const db[4], float *workspace,
                int n_ctas, int64_t rows, int dtype, cudaStream_t stream) {
     if (rev_tc_disabled() || rows <= 0) return kRevTcNotApplicable;
-    if (s.has_bias || (s.act != TH_ACT_RELU && s.act != TH_ACT_NONE)) return kRevTcNotApplicable;
     if (!rows16_ok(y, y_stride) || !rows16_ok(go, go_stride) || (gx && !rows16_ok(gx, gx_stride)) ||
         (x_rec && !rows16_ok(x_rec, xr_stride)))
         return kRevTcNotApplicable;
-#define TH_REV_BWD(T)                                                                                                        \
-    (s.act == TH_ACT_RELU ? launch_rev_bwd_t<T, TH_ACT_RELU>(s, p, y, y_stride, go, go_stride, gx, gx_stride, x_rec,         \
-                                                            xr_stride, dw, workspace, n_ctas, rows, stream)                 \
-                          : launch_rev_bwd_t<T, TH_ACT_NONE>(s, p, y, y_stride, go, go_stride, gx, gx_stride, x_rec,         \
-                                                            xr_stride, dw, workspace, n_ctas, rows, stream))
-    switch (dtype) {
-        case TH_F16: return TH_REV_BWD(__half);
-        case TH_BF16: return TH_REV_BWD(__nv_bfloat16);
-        default: return kRevTcNotApplicable;
+#define TH_REV_BWD(T, A)                                                                                                              \
+    (s.has_bias ? launch_rev_bwd_t<T, A, true>(s, p, y, y_stride, go, go_stride, gx, gx_stride, x_rec, xr_stride, dw, db, workspace,  \
+                                               n_ctas, rows, stream)                                                                  \
+                : launch_rev_bwd_t<T, A, false>(s, p, y, y_stride, go, go_stride, gx, gx_stride, x_rec, xr_stride, dw, db, workspace, \
+                                                n_ctas, rows, stream))
+#define TH_REV_BWD_ACT(T)                                          \
+    switch (s.act) {                                               \
+        case TH_ACT_RELU: return TH_REV_BWD(T, TH_ACT_RELU);       \
+        case TH_ACT_SILU: return TH_REV_BWD(T, TH_ACT_SILU);       \
+        case TH_ACT_RELU2: return TH_REV_BWD(T, TH_ACT_RELU2);     \
+        default: return TH_REV_BWD(T, TH_ACT_NONE);                \
     }
+    if (dtype == TH_F16) { TH_REV_BWD_ACT(__half) }
+    if (dtype == TH_BF16) { TH_REV_BWD_ACT(__nv_bfloat16) }
+    return kRevTcNotApplicable;
+#undef TH_REV_BWD_ACT
 #undef TH_REV_BWD
 }
 
