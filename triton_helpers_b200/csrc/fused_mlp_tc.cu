@@ -173,16 +173,17 @@ template <typename T, int ACT, bool BIAS, int S, bool MSE, bool TA>
 __global__ void __launch_bounds__(128 * S, 1)
 mlp_fwd_pipe_kernel(const MlpShape s, const MlpParams p, const __grid_constant__ WeightMaps maps,
                     const __grid_constant__ CUtensorMap x_map, T *__restrict__ y, long long y_stride, long long n_rows,
-                    int y_vec, const int buffers, const MseArgs mse) {
+                    int y_vec, const MseArgs mse) {
     extern __shared__ unsigned char smem_raw[];
     unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     __shared__ uint32_t tmem_holder;
     __shared__ int abort_flag;
     __shared__ __align__(8) unsigned long long wbar;
     __shared__ __align__(8) SlotBarriers bars;
-    // buffers = 1 (TA only): the input tile is free as soon as the first layer has read it, and the next one is fetched into it
-    // under the others
-    const TcPlan P = tc_plan(s, false, buffers * S);
+    // TA: the input tile is free as soon as the first layer has read it, and the next one is fetched into it under the others:
+    // one tile per slot, so that deep networks keep five slots too (2^18 rows, ten 64-wide layers: four slots 0.058 ms, five 0.051)
+    constexpr int kBuffers = TA ? 1 : 2;
+    const TcPlan P = tc_plan(s, false, kBuffers * S);
     constexpr int bf16 = std::is_same<T, __half>::value ? 0 : 1;
     constexpr uint32_t kTmemCols = S * (kAccCols + (TA ? 32 : 0)) <= 256 ? 256 : 512;
     const int warp = threadIdx.x >> 5;
@@ -243,7 +244,7 @@ mlp_fwd_pipe_kernel(const MlpShape s, const MlpParams p, const __grid_constant__
     const uint32_t act_tmem = tmem + S * kAccCols + slot * 32;  // TA: the slot's hidden activations, 16-bit pairs
     const uint32_t act_taddr = act_tmem + (static_cast<uint32_t>(32 * (warp & 3)) << 16);
     const uint32_t acc_bar = smem_addr(&bars.acc_full[slot]);
-    unsigned char *inputs = smem + buffers * slot * kTileBytes;
+    unsigned char *buffers = smem + kBuffers * slot * kTileBytes;
     uint32_t acc_phase = 0;  // tracked by the issuer warp
     float loss = 0.f;        // MSE: this thread's share of sum (prediction - target)^2
 
@@ -252,22 +253,22 @@ mlp_fwd_pipe_kernel(const MlpShape s, const MlpParams p, const __grid_constant__
             const uint32_t bar = smem_addr(&bars.in_full[slot][b]);
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(static_cast<uint32_t>(kTileBytes))
                          : "memory");
-            tma_load_2d(inputs + b * kTileBytes, &x_map, 0, static_cast<int>((first_tile + k * gridDim.x) * kTileRows), bar);
+            tma_load_2d(buffers + b * kTileBytes, &x_map, 0, static_cast<int>((first_tile + k * gridDim.x) * kTileRows), bar);
         }
         __syncwarp();
     };
     if (issuer && slot < n_mine && !abort_flag) fetch_input(0, slot);
 
     for (long long k = slot, q = 0; k < n_mine; k += S, ++q) {
-        const int b = buffers == 1 ? 0 : static_cast<int>(q & 1);
+        const int b = TA ? 0 : static_cast<int>(q & 1);
         const long long row0 = (first_tile + k * gridDim.x) * kTileRows;
-        unsigned char *tile = inputs + b * kTileBytes;
+        unsigned char *tile = buffers + b * kTileBytes;
         const uint32_t tile_addr = smem_addr(tile);
         const uint32_t row_addr = tile_addr + row * 128, row_swizzle = (row & 7) << 4;  // chunk c of the row: row_addr + ((c << 4) ^ row_swizzle)
         if (issuer) {
             // the other buffer's last reader was the previous tile of this slot: finished
-            if (buffers == 2 && k + S < n_mine && !*reinterpret_cast<volatile int *>(&abort_flag)) fetch_input(b ^ 1, k + S);
-            pipe_wait(smem_addr(&bars.in_full[slot][b]), static_cast<uint32_t>((buffers == 1 ? q : q >> 1) & 1), &abort_flag);
+            if (!TA && k + S < n_mine && !*reinterpret_cast<volatile int *>(&abort_flag)) fetch_input(b ^ 1, k + S);
+            pipe_wait(smem_addr(&bars.in_full[slot][b]), static_cast<uint32_t>((TA ? q : q >> 1) & 1), &abort_flag);
         }
         // MSE over ordered rows: where this row's target is, and (below) a prefetch of it, so that the random access is over
         // when the output layer's epilogue needs it (2^21 rows: 0.138 -> 0.10 ms)
@@ -302,7 +303,7 @@ mlp_fwd_pipe_kernel(const MlpShape s, const MlpParams p, const __grid_constant__
                     __syncwarp();
                     pipe_wait(acc_bar, acc_phase, &abort_flag);
                     acc_phase ^= 1u;
-                    if (buffers == 1 && l == 0 && k + S < n_mine && !*reinterpret_cast<volatile int *>(&abort_flag)) fetch_input(0, k + S);
+                    if (TA && l == 0 && k + S < n_mine && !*reinterpret_cast<volatile int *>(&abort_flag)) fetch_input(0, k + S);
                 }
             }
             slot_barrier(slot);
@@ -383,8 +384,8 @@ bool tmem_a_enabled() {
 
 template <typename T, int ACT, bool BIAS, int S, bool MSE, bool TA>
 int launch_fwd_pipe(const MlpShape &s, const MlpParams &p, const void *x, int64_t x_stride, void *y, int64_t y_stride,
-                    int64_t rows, cudaStream_t stream, const MseArgs &mse, int buffers) {
-    const TcPlan P = tc_plan(s, false, buffers * S);
+                    int64_t rows, cudaStream_t stream, const MseArgs &mse = MseArgs{}) {
+    const TcPlan P = tc_plan(s, false, (TA ? 1 : 2) * S);
     const int smem = P.total + 1024;
     if (smem > kSmemBudget || pipe_disabled()) return kTcNotApplicable;
     if (rows >= (1ll << 31) - kTileRows) return kTcNotApplicable;  // TMA coordinates are 32-bit
@@ -399,7 +400,7 @@ int launch_fwd_pipe(const MlpShape &s, const MlpParams &p, const void *x, int64_
     const long long tiles = (rows + kTileRows - 1) / kTileRows;
     const long long cap = sm_count();
     kernel<<<static_cast<unsigned>(tiles < cap ? tiles : cap), 128 * S, smem, stream>>>(
-        s, p, maps, x_map, static_cast<T *>(y), y_stride, rows, y ? rows_vector_ok(y, y_stride, s.d_out) : 0, buffers, mse);
+        s, p, maps, x_map, static_cast<T *>(y), y_stride, rows, y ? rows_vector_ok(y, y_stride, s.d_out) : 0, mse);
     return launch_status("mlp_fwd_pipe_kernel launch");
 }
 
@@ -418,16 +419,13 @@ int launch_fwd_slots(const MlpShape &s, const MlpParams &p, const void *x, int64
     }();
     int rc = kTcNotApplicable;
     if (tmem_a_enabled()) {
-        // five slots, if need be with one input tile each (ten 64-wide layers, 2^18 rows: four slots 0.058 ms, five 0.050; where
-        // two tiles fit they are 3 % faster)
-        if (cap >= 5) rc = launch_fwd_pipe<T, ACT, BIAS, 5, MSE, true>(s, p, x, x_stride, y, y_stride, rows, stream, mse, 2);
-        if (rc == kTcNotApplicable && cap >= 5) rc = launch_fwd_pipe<T, ACT, BIAS, 5, MSE, true>(s, p, x, x_stride, y, y_stride, rows, stream, mse, 1);
-        if (rc == kTcNotApplicable && cap >= 4) rc = launch_fwd_pipe<T, ACT, BIAS, 4, MSE, true>(s, p, x, x_stride, y, y_stride, rows, stream, mse, 1);
-        if (rc == kTcNotApplicable && cap >= 3) rc = launch_fwd_pipe<T, ACT, BIAS, 3, MSE, true>(s, p, x, x_stride, y, y_stride, rows, stream, mse, 1);
+        if (cap >= 5) rc = launch_fwd_pipe<T, ACT, BIAS, 5, MSE, true>(s, p, x, x_stride, y, y_stride, rows, stream, mse);
+        if (rc == kTcNotApplicable && cap >= 4) rc = launch_fwd_pipe<T, ACT, BIAS, 4, MSE, true>(s, p, x, x_stride, y, y_stride, rows, stream, mse);
+        if (rc == kTcNotApplicable && cap >= 3) rc = launch_fwd_pipe<T, ACT, BIAS, 3, MSE, true>(s, p, x, x_stride, y, y_stride, rows, stream, mse);
         return rc;
     }
-    if (cap >= 4) rc = launch_fwd_pipe<T, ACT, BIAS, 4, MSE, false>(s, p, x, x_stride, y, y_stride, rows, stream, mse, 2);
-    if (rc == kTcNotApplicable && cap >= 3) rc = launch_fwd_pipe<T, ACT, BIAS, 3, MSE, false>(s, p, x, x_stride, y, y_stride, rows, stream, mse, 2);
+    if (cap >= 4) rc = launch_fwd_pipe<T, ACT, BIAS, 4, MSE, false>(s, p, x, x_stride, y, y_stride, rows, stream, mse);
+    if (rc == kTcNotApplicable && cap >= 3) rc = launch_fwd_pipe<T, ACT, BIAS, 3, MSE, false>(s, p, x, x_stride, y, y_stride, rows, stream, mse);
     return rc;
 }
 

@@ -23,8 +23,8 @@
 // kernel sums the copies.  The backward pass needs all 512 TMEM columns, so one CTA per SM; the
 // forward pass needs 192 (256 allocated), two CTAs per SM.
 //
-// Bias gradients are column sums of DY and DZ, summed over each warp's rows with shuffles in the epilogues: tensor memory
-// has no columns left for the MMA with ones that the fused MLP uses.
+// Bias gradients are column sums of the DY and DZ tiles, formed by the flush warps while the chain goes on (in the chain's
+// epilogues they cost 2 us a pass): tensor memory has no columns left for the MMA with ones that the fused MLP uses.
 //
 // Covered here: float16 / bfloat16, 16-byte-aligned rows.  Everything else stays on the mma.sync kernels.
 #include "rev_shape.cuh"
@@ -147,9 +147,9 @@ __device__ __forceinline__ void tile_row_to_tmem(unsigned char *tile, const Seat
     }
 }
 
-// This thread's pieces of an fp32 TMEM accumulator -> (optional bias, added or - when a branch is undone - taken off, written
-// back) -> rounded into an operand tile and / or a global row.
-template <typename T, bool BIAS, bool UNDO = false>
+// This thread's pieces of an fp32 TMEM accumulator -> (optional bias, written back) -> rounded into an
+// operand tile and / or a global row.
+template <typename T, bool BIAS>
 __device__ __forceinline__ void stream_epilogue(uint32_t taddr, const Seat &seat, int width, const float *bias,
                                                 unsigned char *tile, T *global_row, bool live) {
     const int n = width / kGroups, first = seat.group * (n / 8);  // this thread's columns / first 8-column piece
@@ -160,10 +160,7 @@ __device__ __forceinline__ void stream_epilogue(uint32_t taddr, const Seat &seat
         for (int k = 0; k < 8; ++k) v[k] = piece[k];
         if constexpr (BIAS) {
 #pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                const float b = bias[8 * (first + u) + k];
-                v[k] = __float_as_uint(__uint_as_float(v[k]) + (UNDO ? -b : b));
-            }
+            for (int k = 0; k < 8; ++k) v[k] = __float_as_uint(__uint_as_float(v[k]) + bias[8 * (first + u) + k]);
             tmem_st8(taddr + 8 * (first + u), v);
         }
         const uint4 packed = finish8<T, TH_ACT_NONE, false>(v, nullptr);
@@ -401,31 +398,34 @@ __device__ __forceinline__ void flush_dw_quadrant(uint32_t tmem, int q, uint32_t
     }
 }
 
-// Adds the sums of eight columns over the warp's 32 rows to dst[0 .. 7]: a reduce-scatter over five shuffle levels, then one
-// 32-byte reduction.
+// Column sums of a 128 x 64 operand tile by the 128 flush threads, added to dst: a thread sums eight rows of one 16-byte chunk,
+// the four threads of a warp with the same chunk meet in two shuffles.
 template <typename T>
-__device__ __forceinline__ void add_column_sums(uint4 packed, float *dst) {
-    const int lane = threadIdx.x & 31;
-    const uint32_t w[4] = {packed.x, packed.y, packed.z, packed.w};
-    float v[8];
+__device__ __forceinline__ void add_tile_column_sums(uint32_t tile, int width, float *dst) {
+    const int t = threadIdx.x & 127, chunk = t & 7, row0 = (t >> 3) * 8;
+    float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const float2 f = unpack_pair<T>(w[k]);
-        v[2 * k] = f.x;
-        v[2 * k + 1] = f.y;
-    }
+    for (int r = 0; r < 8; ++r) {
+        const uint4 q = ld_shared_16(tile + (row0 + r) * 128 + ((chunk ^ r) << 4));
+        const uint32_t w[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
-    for (int keep = 4; keep > 0; keep /= 2) {
-        const bool high = lane & (4 * keep);
-#pragma unroll
-        for (int k = 0; k < keep; ++k) {
-            const float other = __shfl_xor_sync(0xffffffffu, high ? v[k] : v[k + keep], 4 * keep);
-            v[k] = (high ? v[k + keep] : v[k]) + other;
+        for (int k = 0; k < 4; ++k) {
+            const float2 f = unpack_pair<T>(w[k]);
+            v[2 * k] += f.x;
+            v[2 * k + 1] += f.y;
         }
     }
-    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
-    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
-    if ((lane & 3) == 0) atomicAdd(dst + (lane >> 2), v[0]);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        v[k] += __shfl_xor_sync(0xffffffffu, v[k], 8);
+        v[k] += __shfl_xor_sync(0xffffffffu, v[k], 16);
+    }
+    if ((t & 31) < 8 && 8 * chunk < width) {
+#pragma unroll
+        for (int k = 0; k < 8; k += 4)
+            asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + 8 * chunk + k), "f"(v[k]), "f"(v[k + 1]), "f"(v[k + 2]), "f"(v[k + 3])
+                         : "memory");
+    }
 }
 
 template <typename T, int ACT, bool BIAS>
@@ -449,12 +449,15 @@ rev_bwd_tc_kernel(const RevShape s, const RevParams p, const __grid_constant__ R
     __shared__ __align__(8) unsigned long long ring_bars[2];
     // wgrad_bar: the weight-gradient MMAs of a pass are done (one commit per pass); flushed_bar: the flush warps
     // have read them out (one arrival per flush warp), so the next pass may overwrite the accumulators
-    __shared__ __align__(8) unsigned long long wgrad_bar, flushed_bar;
+    // BIAS - operands_bar: dz of a pass is in place (one arrival); summed_bar: the flush warps have summed its columns and dy's
+    __shared__ __align__(8) unsigned long long wgrad_bar, flushed_bar, operands_bar, summed_bar;
     if (threadIdx.x == 0) {
         abort_flag = 0;
         asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&ring_bars[0])), "r"(1u) : "memory");
         asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&ring_bars[1])), "r"(1u) : "memory");
         asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&wgrad_bar)), "r"(1u) : "memory");
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&operands_bar)), "r"(1u) : "memory");
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&summed_bar)), "r"(static_cast<uint32_t>(kRevFlushThreads / 32)) : "memory");
         asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&flushed_bar)), "r"(static_cast<uint32_t>(kRevFlushThreads / 32)) : "memory");
     }
     for (int e = threadIdx.x; e < P.tiles * kTileBytes / 16; e += blockDim.x) reinterpret_cast<uint4 *>(smem)[e] = make_uint4(0, 0, 0, 0);
@@ -463,6 +466,7 @@ rev_bwd_tc_kernel(const RevShape s, const RevParams p, const __grid_constant__ R
     const uint32_t tmem = cta_setup(&tmem_holder, &mbar, P.tmem_cols);  // publishes the barrier inits
     float *cta_acc = workspace + static_cast<size_t>(blockIdx.x) * rev_cta_floats(s);
     const uint32_t wgrad_addr = smem_addr(&wgrad_bar), flushed_addr = smem_addr(&flushed_bar);
+    const uint32_t operands_addr = smem_addr(&operands_bar), summed_addr = smem_addr(&summed_bar);
 
     if (is_flush) {
         // ================= weight gradients out of TMEM, one pass behind the main threads =================
@@ -473,6 +477,15 @@ rev_bwd_tc_kernel(const RevShape s, const RevParams p, const __grid_constant__ R
             for (int k = s.blocks - 1; alive && k >= 0; --k) {
                 float *block_acc = cta_acc + static_cast<size_t>(k) * 4 * kMatFloats;
                 for (int pass = 0; pass < 2; ++pass, ++n) {
+                    if constexpr (BIAS) {
+                        alive = __all_sync(0xffffffffu, rev_wait(operands_addr, n & 1u, &abort_flag));
+                        if (!alive) break;
+                        float *sums = cta_acc + static_cast<size_t>(s.blocks) * 4 * kMatFloats + (static_cast<size_t>(k) * 4 + (pass == 0 ? 2 : 0)) * kMaxDim;
+                        add_tile_column_sums<T>(smem_addr(dz_tile), s.hid, sums);
+                        add_tile_column_sums<T>(smem_addr(dy_tiles + (n & 1u) * kTileBytes), s.half, sums + kMaxDim);
+                        __syncwarp();
+                        if ((threadIdx.x & 31) == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(summed_addr) : "memory");
+                    }
                     alive = __all_sync(0xffffffffu, rev_wait(wgrad_addr, n & 1u, &abort_flag));
                     if (!alive) break;
                     tc_fence_after();
@@ -511,7 +524,10 @@ rev_bwd_tc_kernel(const RevShape s, const RevParams p, const __grid_constant__ R
             unsigned char *u_in = u_tiles + (n & 1u) * kTileBytes, *dy_in = dy_tiles + (n & 1u) * kTileBytes;
             // the scratch tiles below were operands of the previous tile's last weight-gradient MMAs
             if (n > 0) {
-                if (threadIdx.x < 32) rev_wait(wgrad_addr, (n - 1) & 1u, &abort_flag);
+                if (threadIdx.x < 32) {
+                    rev_wait(wgrad_addr, (n - 1) & 1u, &abort_flag);
+                    if (BIAS) rev_wait(summed_addr, (n - 1) & 1u, &abort_flag);
+                }
                 main_sync();
             }
             // y1 -> U (input of the last G), y2 -> scratch, go1 -> scratch, go2 -> DY (gradient of G's output)
@@ -545,7 +561,6 @@ rev_bwd_tc_kernel(const RevShape s, const RevParams p, const __grid_constant__ R
                 }
                 const unsigned char *w = smem + P.ring + stage * kStageBytes;
                 const float *block_bias = reinterpret_cast<const float *>(smem + P.bias) + stage * 4 * kMaxDim;
-                float *bias_sums = cta_acc + static_cast<size_t>(s.blocks) * 4 * kMatFloats + static_cast<size_t>(k) * 4 * kMaxDim;
 #pragma unroll 1
                 for (int pass = 0; pass < 2; ++pass, ++n) {
                     // pass 0 undoes y2 = x2 + G(y1): input stream S1, output stream S2, gradient flows D2 -> D1
@@ -566,6 +581,20 @@ rev_bwd_tc_kernel(const RevShape s, const RevParams p, const __grid_constant__ R
                         if (leader) mma_commit(bar);
                         __syncwarp();
                     }
+                    if constexpr (BIAS) {
+                        // under those MMAs: the branch's second bias comes off the stream that step B takes the rest from; and the
+                        // flush warps must have summed the previous pass's dz before it is overwritten below
+                        const int nh = s.half / kGroups, first_h = seat.group * (nh / 8);
+                        const float *bias2 = block_bias + m2 * kMaxDim;
+                        for_each_piece(taddr + out_col + seat.group * nh, nh, [&](int u, const uint32_t(&piece)[8]) {
+                            uint32_t v[8];
+#pragma unroll
+                            for (int e = 0; e < 8; ++e) v[e] = __float_as_uint(__uint_as_float(piece[e]) - bias2[8 * (first_h + u) + e]);
+                            tmem_st8(taddr + out_col + seat.group * nh + 8 * u, v);
+                        });
+                        tmem_st_wait();
+                        if (threadIdx.x < 32 && n > 0) rev_wait(summed_addr, (n - 1) & 1u, &abort_flag);
+                    }
                     main_wait_mma(bar, phase, &abort_flag);
                     {
                         // h = act(z) first (also the ReLU mask), then dz = dh where h > 0
@@ -578,7 +607,6 @@ rev_bwd_tc_kernel(const RevShape s, const RevParams p, const __grid_constant__ R
                         });
                         auto store_dz = [&](int u, uint4 g) {
                             st_shared_16(dz_row + (((first + u) << 4) ^ row_swizzle), g);
-                            if constexpr (BIAS) add_column_sums<T>(g, bias_sums + m1 * kMaxDim + 8 * (first + u));
                         };
                         if constexpr (ACT == TH_ACT_SILU || ACT == TH_ACT_RELU2) {
                             // the derivative is taken at the pre-activation rounded to the storage type
@@ -613,6 +641,7 @@ rev_bwd_tc_kernel(const RevShape s, const RevParams p, const __grid_constant__ R
                         }
                     }
                     main_publish();
+                    if (BIAS && threadIdx.x == 64) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(operands_addr) : "memory");
                     // step B: undo the branch and push the gradient through (waited for below); then both weight
                     // gradients, committed on their own for the flush warps
                     if (threadIdx.x < 32) {
@@ -631,16 +660,9 @@ rev_bwd_tc_kernel(const RevShape s, const RevParams p, const __grid_constant__ R
                         }
                         __syncwarp();
                     }
-                    if constexpr (BIAS) {  // under those MMAs: the second layer's bias gradient, column sums of DY
-                        const int nh = s.half / kGroups, first_h = seat.group * (nh / 8);
-                        const uint32_t dy_row = dy_cur + seat.row * 128, swizzle = (seat.row & 7) << 4;
-#pragma unroll 1
-                        for (int u = 0; u < nh / 8; ++u)
-                            add_column_sums<T>(ld_shared_16(dy_row + (((first_h + u) << 4) ^ swizzle)), bias_sums + m2 * kMaxDim + 8 * (first_h + u));
-                    }
                     main_wait_mma(bar, phase, &abort_flag);
                     // next pass: its input is the stream just reconstructed, its output gradient the one just updated
-                    stream_epilogue<T, BIAS, true>(taddr + out_col, seat, s.half, block_bias + m2 * kMaxDim, u_next, nullptr, false);
+                    stream_epilogue<T, false>(taddr + out_col, seat, s.half, nullptr, u_next, nullptr, false);
                     stream_epilogue<T, false>(taddr + in_d_col, seat, s.half, nullptr, dy_next, nullptr, false);
                     if (pass == 1) {  // next block's weights have landed
                         if (!use_tma) async_tile_wait();
