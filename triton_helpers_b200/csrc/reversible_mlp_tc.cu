@@ -26,6 +26,9 @@
 // Bias gradients are column sums of the DY and DZ tiles, formed by the flush warps while the chain goes on (in the chain's
 // epilogues they cost 2 us a pass): tensor memory has no columns left for the MMA with ones that the fused MLP uses.
 //
+// Measured with biases and SiLU, 2^17 rows, six blocks of 64 -> 64 -> 64: 0.431 ms (mma.sync 0.70); without biases, ReLU,
+// 2^20 rows, eight blocks: 2.22 ms.
+//
 // Covered here: float16 / bfloat16, 16-byte-aligned rows.  Everything else stays on the mma.sync kernels.
 #include "rev_shape.cuh"
 #include "tc_tiles.cuh"
@@ -851,6 +854,10 @@ int rev_bwd_tc(const RevShape &s, const RevParams &p, const void *y, int64_t y_s
                void *gx, int64_t gx_stride, void *x_rec, int64_t xr_stride, void *const dw[4], void *const db[4], float *workspace,
                int n_ctas, int64_t rows, int dtype, cudaStream_t stream) {
     if (rev_tc_disabled() || rows <= 0) return kRevTcNotApplicable;
+    // Biased batches that do not fill one tile stay with the mma.sync kernel: its streams are rounded to nearest in registers once
+    // per branch, the tensor core's accumulation into tensor memory switches twice as many ReLUs that sit within a rounding of
+    // zero (1.1 against 0.6 % of the rows of eight float16 blocks), and there is no throughput to gain from a handful of rows.
+    if (s.has_bias && rows < kTileRows) return kRevTcNotApplicable;
     if (!rows16_ok(y, y_stride) || !rows16_ok(go, go_stride) || (gx && !rows16_ok(gx, gx_stride)) ||
         (x_rec && !rows16_ok(x_rec, xr_stride)))
         return kRevTcNotApplicable;
