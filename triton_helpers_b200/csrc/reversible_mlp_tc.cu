@@ -452,7 +452,8 @@ rev_bwd_tc_kernel(const RevShape s, const RevParams p, const __grid_constant__ R
     __shared__ __align__(8) unsigned long long ring_bars[2];
     // wgrad_bar: the weight-gradient MMAs of a pass are done (one commit per pass); flushed_bar: the flush warps
     // have read them out (one arrival per flush warp), so the next pass may overwrite the accumulators
-    // BIAS - operands_bar: dz of a pass is in place (one arrival); summed_bar: the flush warps have summed its columns and dy's
+    // operands_bar: h and dz of a pass are in place and the chain's MMAs on them issued (one arrival)
+    // BIAS - summed_bar: the flush warps have summed the columns of dz and dy
     __shared__ __align__(8) unsigned long long wgrad_bar, flushed_bar, operands_bar, summed_bar;
     if (threadIdx.x == 0) {
         abort_flag = 0;
@@ -474,18 +475,33 @@ rev_bwd_tc_kernel(const RevShape s, const RevParams p, const __grid_constant__ R
     if (is_flush) {
         // ================= weight gradients out of TMEM, one pass behind the main threads =================
         const int q = (threadIdx.x >> 5) & 3;
+        const uint32_t id_dw2 = instr_desc(64, s.hid, bf16, 1, 1), id_dw1 = instr_desc(64, s.half, bf16, 1, 1);  // both operands MN-major, M = 64
         uint32_t n = 0;  // passes flushed so far
         bool alive = true;
         for (long long tile = blockIdx.x; alive && tile < n_tiles; tile += gridDim.x) {
             for (int k = s.blocks - 1; alive && k >= 0; --k) {
                 float *block_acc = cta_acc + static_cast<size_t>(k) * 4 * kMatFloats;
                 for (int pass = 0; pass < 2; ++pass, ++n) {
-                    if constexpr (BIAS) {
+                    const uint32_t dy_cur = smem_addr(dy_tiles + (n & 1u) * kTileBytes);
+                    if (BIAS || q == 0) {
                         alive = __all_sync(0xffffffffu, rev_wait(operands_addr, n & 1u, &abort_flag));
+                        // the accumulators hold the previous pass's sums until all four flush warps have read them
+                        if (q == 0 && alive && n > 0) alive = __all_sync(0xffffffffu, rev_wait(flushed_addr, (n - 1) & 1u, &abort_flag));
                         if (!alive) break;
+                    }
+                    if (q == 0) {
+                        const bool leader = elect_one();
+                        tc_fence_after();
+                        const uint32_t u_cur = smem_addr(u_tiles + (n & 1u) * kTileBytes);
+                        issue_gemm(leader, tmem + kDW2, dy_cur, 2048, smem_addr(h_tile), 2048, kTileRows / 16, id_dw2, false);
+                        issue_gemm(leader, tmem + kDW1, smem_addr(dz_tile), 2048, u_cur, 2048, kTileRows / 16, id_dw1, false);
+                        if (leader) mma_commit(wgrad_addr);
+                        __syncwarp();
+                    }
+                    if constexpr (BIAS) {
                         float *sums = cta_acc + static_cast<size_t>(s.blocks) * 4 * kMatFloats + (static_cast<size_t>(k) * 4 + (pass == 0 ? 2 : 0)) * kMaxDim;
                         add_tile_column_sums<T>(smem_addr(dz_tile), s.hid, sums);
-                        add_tile_column_sums<T>(smem_addr(dy_tiles + (n & 1u) * kTileBytes), s.half, sums + kMaxDim);
+                        add_tile_column_sums<T>(dy_cur, s.half, sums + kMaxDim);
                         __syncwarp();
                         if ((threadIdx.x & 31) == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(summed_addr) : "memory");
                     }
@@ -513,12 +529,11 @@ rev_bwd_tc_kernel(const RevShape s, const RevParams p, const __grid_constant__ R
         uint32_t phase = 0;
         int step = 0;
         uint32_t n = 0;  // passes started so far; pass n reads U / DY copy n & 1 and writes copy (n + 1) & 1
-        // instruction descriptors: forward-type, dgrad (B MN-major), reconstruction (A negated), wgrad (both MN-major, M = 64)
+        // instruction descriptors: forward-type, dgrad (B MN-major), reconstruction (A negated)
         const uint32_t id_z = instr_desc(128, s.hid, bf16, 0, 0);
         const uint32_t id_dh = instr_desc(128, s.hid, bf16, 0, 1);
         const uint32_t id_undo = instr_desc(128, s.half, bf16, 0, 0) | (1u << 13);
         const uint32_t id_din = instr_desc(128, s.half, bf16, 0, 1);
-        const uint32_t id_dw2 = instr_desc(64, s.hid, bf16, 1, 1), id_dw1 = instr_desc(64, s.half, bf16, 1, 1);
         volatile int *abort_now = &abort_flag;
 
         for (long long tile = blockIdx.x; tile < n_tiles && !*abort_now; tile += gridDim.x) {
@@ -573,9 +588,7 @@ rev_bwd_tc_kernel(const RevShape s, const RevParams p, const __grid_constant__ R
                     const uint32_t out_col = pass == 0 ? kS2 : kS1, in_d_col = pass == 0 ? kD1 : kD2;
                     const uint32_t u_cur = smem_addr(u_tiles + (n & 1u) * kTileBytes), dy_cur = smem_addr(dy_tiles + (n & 1u) * kTileBytes);
                     unsigned char *u_next = u_tiles + ((n + 1) & 1u) * kTileBytes, *dy_next = dy_tiles + ((n + 1) & 1u) * kTileBytes;
-                    // step A: z = U . W1^T and dh = DY . W2 together.  This commit also covers the previous pass's
-                    // weight-gradient MMAs (a commit tracks everything its thread issued before), which read the
-                    // h and dz tiles the epilogue below overwrites.
+                    // step A: z = U . W1^T and dh = DY . W2 together
                     if (threadIdx.x < 32) {
                         const bool leader = elect_one();
                         tc_fence_after();
@@ -598,6 +611,8 @@ rev_bwd_tc_kernel(const RevShape s, const RevParams p, const __grid_constant__ R
                         tmem_st_wait();
                         if (threadIdx.x < 32 && n > 0) rev_wait(summed_addr, (n - 1) & 1u, &abort_flag);
                     }
+                    // the previous pass's weight-gradient MMAs read the h and dz tiles the epilogue below overwrites
+                    if (threadIdx.x < 32 && n > 0) rev_wait(wgrad_addr, (n - 1) & 1u, &abort_flag);
                     main_wait_mma(bar, phase, &abort_flag);
                     {
                         // h = act(z) first (also the ReLU mask), then dz = dh where h > 0
@@ -644,23 +659,16 @@ rev_bwd_tc_kernel(const RevShape s, const RevParams p, const __grid_constant__ R
                         }
                     }
                     main_publish();
-                    if (BIAS && threadIdx.x == 64) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(operands_addr) : "memory");
-                    // step B: undo the branch and push the gradient through (waited for below); then both weight
-                    // gradients, committed on their own for the flush warps
+                    // step B: undo the branch and push the gradient through.  Then the flush warps may issue the two weight gradients:
+                    // MMAs execute in the order of issue and an issuing thread is held while the queue is full, so sixteen more
+                    // of them here would keep the chain waiting until most of them have run.
                     if (threadIdx.x < 32) {
                         const bool leader = elect_one();
                         tc_fence_after();
                         issue_gemm(leader, tmem + out_col, smem_addr(h_tile), 32, w2, 32, s.hid / 16, id_undo, true);
                         issue_gemm(leader, tmem + in_d_col, smem_addr(dz_tile), 32, w1, 2048, s.hid / 16, id_din, true);
                         if (leader) mma_commit(bar);
-                        // the accumulators still hold the previous pass's sums until the flush warps have read them
-                        const bool free_dw = n == 0 || __all_sync(0xffffffffu, rev_wait(flushed_addr, (n - 1) & 1u, &abort_flag));
-                        if (free_dw) {
-                            tc_fence_after();
-                            issue_gemm(leader, tmem + kDW2, dy_cur, 2048, smem_addr(h_tile), 2048, kTileRows / 16, id_dw2, false);
-                            issue_gemm(leader, tmem + kDW1, smem_addr(dz_tile), 2048, u_cur, 2048, kTileRows / 16, id_dw1, false);
-                            if (leader) mma_commit(wgrad_addr);
-                        }
+                        if (leader) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(operands_addr) : "memory");
                         __syncwarp();
                     }
                     main_wait_mma(bar, phase, &abort_flag);
