@@ -49,7 +49,7 @@ constexpr int kFwdAU = 192, kFwdAH = 224;        // forward: 16-bit A operands (
 constexpr int kD1 = 128, kD2 = 192, kZ = 256, kDH = 320, kDW1 = 384, kDW2 = 448;  // backward
 
 struct RevTcPlan {
-    int tiles;     // operand tiles before the weight ring (2 forward, 6 backward)
+    int tiles;     // operand tiles before the weight ring (2 forward, 8 backward)
     int ring;      // byte offset of the ring (2 stages)
     int bias;      // fp32 [2 stages][4][64]
     int total;
@@ -58,7 +58,7 @@ struct RevTcPlan {
 
 __host__ __device__ inline RevTcPlan rev_tc_plan(bool backward) {
     RevTcPlan p{};
-    p.tiles = backward ? 6 : 2;
+    p.tiles = backward ? 8 : 2;
     p.ring = p.tiles * kTileBytes;
     p.bias = p.ring + 2 * kStageBytes;
     p.total = p.bias + 2 * 4 * kMaxDim * 4;
@@ -103,6 +103,11 @@ __device__ void prefetch_weights(unsigned char *smem, const RevTcPlan &P, const 
 // ~1 800 cycles per block).  Biases, when present, still come with plain loads.
 struct RevWeightMaps {
     CUtensorMap m[4];  // w_f1, w_f2, w_g1, w_g2: [blocks * rows][cols], 16-bit
+};
+
+// The row tiles of the backward pass, a column half of y or of the output gradient each: [rows][half], box = 128 rows
+struct RevRowMaps {
+    CUtensorMap y1, y2, go1, go2;
 };
 
 template <typename T>
@@ -433,7 +438,8 @@ __device__ __forceinline__ void add_tile_column_sums(uint32_t tile, int width, f
 
 template <typename T, int ACT, bool BIAS>
 __global__ void __launch_bounds__(kTcThreads + kRevFlushThreads, 1)
-rev_bwd_tc_kernel(const RevShape s, const RevParams p, const __grid_constant__ RevWeightMaps maps, const int use_tma,
+rev_bwd_tc_kernel(const RevShape s, const RevParams p, const __grid_constant__ RevWeightMaps maps,
+                  const __grid_constant__ RevRowMaps row_maps, const int use_tma,
                   const T *__restrict__ y, long long y_stride,
                   const T *__restrict__ go, long long go_stride, T *__restrict__ gx, long long gx_stride,
                   T *__restrict__ x_rec, long long xr_stride, float *__restrict__ workspace, long long n_rows) {
@@ -447,6 +453,7 @@ rev_bwd_tc_kernel(const RevShape s, const RevParams p, const __grid_constant__ R
     // U (the branch's input, 16-bit) and DY (the gradient of its output) alternate between two tiles each: the
     // epilogue of a pass writes the next pass's copies while this pass's weight-gradient MMAs still read theirs
     unsigned char *u_tiles = smem, *h_tile = smem + 2 * kTileBytes, *dy_tiles = smem + 3 * kTileBytes, *dz_tile = smem + 5 * kTileBytes;
+    unsigned char *y2_tile = smem + 6 * kTileBytes, *go1_tile = smem + 7 * kTileBytes;  // the next row tile's, on their way to tensor memory
     const bool is_flush = threadIdx.x >= kTcThreads;
 
     __shared__ __align__(8) unsigned long long ring_bars[2];
@@ -454,13 +461,15 @@ rev_bwd_tc_kernel(const RevShape s, const RevParams p, const __grid_constant__ R
     // have read them out (one arrival per flush warp), so the next pass may overwrite the accumulators
     // operands_bar: h and dz of a pass are in place and the chain's MMAs on them issued (one arrival)
     // BIAS - summed_bar: the flush warps have summed the columns of dz and dy
-    __shared__ __align__(8) unsigned long long wgrad_bar, flushed_bar, operands_bar, summed_bar;
+    // rows_bar: the four TMA boxes of a row tile have landed
+    __shared__ __align__(8) unsigned long long wgrad_bar, flushed_bar, operands_bar, summed_bar, rows_bar;
     if (threadIdx.x == 0) {
         abort_flag = 0;
         asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&ring_bars[0])), "r"(1u) : "memory");
         asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&ring_bars[1])), "r"(1u) : "memory");
         asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&wgrad_bar)), "r"(1u) : "memory");
         asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&operands_bar)), "r"(1u) : "memory");
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&rows_bar)), "r"(1u) : "memory");
         asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&summed_bar)), "r"(static_cast<uint32_t>(kRevFlushThreads / 32)) : "memory");
         asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&flushed_bar)), "r"(static_cast<uint32_t>(kRevFlushThreads / 32)) : "memory");
     }
@@ -536,36 +545,44 @@ rev_bwd_tc_kernel(const RevShape s, const RevParams p, const __grid_constant__ R
         const uint32_t id_din = instr_desc(128, s.half, bf16, 0, 1);
         volatile int *abort_now = &abort_flag;
 
+        // A row tile: y1 -> U (input of the last G), go2 -> DY (gradient of G's output), the other halves -> scratch.  Fetched
+        // during the last pass of the tile before, whose epilogue leaves its U / DY copies free.
+        const uint32_t rows_addr = smem_addr(&rows_bar);
+        auto fetch_rows = [&](long long row0, uint32_t copy) {
+            unsigned char *u_in = u_tiles + copy * kTileBytes, *dy_in = dy_tiles + copy * kTileBytes;
+            if (use_tma) {
+                if (threadIdx.x == 64) {
+                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(rows_addr), "r"(4u * kTileBytes) : "memory");
+                    const int at = static_cast<int>(row0);
+                    tma_load_2d(u_in, &row_maps.y1, 0, at, rows_addr);
+                    tma_load_2d(dy_in, &row_maps.go2, 0, at, rows_addr);
+                    tma_load_2d(y2_tile, &row_maps.y2, 0, at, rows_addr);
+                    tma_load_2d(go1_tile, &row_maps.go1, 0, at, rows_addr);
+                }
+            } else {
+                async_tile_load<T>(u_in, y, y_stride, row0, n_rows, s.half, s.half);
+                async_tile_load<T>(y2_tile, y + s.half, y_stride, row0, n_rows, s.half, s.half);
+                async_tile_load<T>(go1_tile, go, go_stride, row0, n_rows, s.half, s.half);
+                async_tile_load<T>(dy_in, go + s.half, go_stride, row0, n_rows, s.half, s.half);
+            }
+        };
+        uint32_t rows_phase = 0;
+        if (static_cast<long long>(blockIdx.x) < n_tiles) fetch_rows(static_cast<long long>(blockIdx.x) * kTileRows, 0);
+
         for (long long tile = blockIdx.x; tile < n_tiles && !*abort_now; tile += gridDim.x) {
             const long long row0 = tile * kTileRows;
             const bool live = row0 + seat.row < n_rows;
             unsigned char *u_in = u_tiles + (n & 1u) * kTileBytes, *dy_in = dy_tiles + (n & 1u) * kTileBytes;
-            // the scratch tiles below were operands of the previous tile's last weight-gradient MMAs
-            if (n > 0) {
-                if (threadIdx.x < 32) {
-                    rev_wait(wgrad_addr, (n - 1) & 1u, &abort_flag);
-                    if (BIAS) rev_wait(summed_addr, (n - 1) & 1u, &abort_flag);
-                }
+            if (use_tma) {
+                rev_wait(rows_addr, rows_phase, &abort_flag);
+                rows_phase ^= 1;
+            } else {
+                async_tile_wait();
                 main_sync();
             }
-            // y1 -> U (input of the last G), y2 -> scratch, go1 -> scratch, go2 -> DY (gradient of G's output)
-            async_tile_load<T>(u_in, y, y_stride, row0, n_rows, s.half, s.half);
-            async_tile_load<T>(h_tile, y + s.half, y_stride, row0, n_rows, s.half, s.half);
-            async_tile_load<T>(dz_tile, go, go_stride, row0, n_rows, s.half, s.half);
-            async_tile_load<T>(dy_in, go + s.half, go_stride, row0, n_rows, s.half, s.half);
-            {  // the next tile's rows into L2 meanwhile (2^20 rows: 2.26 -> 2.22 ms): one column half of the threads y, the other go
-                const long long next = row0 + static_cast<long long>(gridDim.x) * kTileRows + seat.row;
-                if (next < n_rows) {
-                    const char *at = reinterpret_cast<const char *>(seat.group == 0 ? y + next * y_stride : go + next * go_stride);
-                    asm volatile("prefetch.global.L2 [%0];" ::"l"(at));
-                    if (s.half > 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(at + 128));
-                }
-            }
-            async_tile_wait();
-            main_sync();
             tile_row_to_tmem<T>(u_in, seat, s.half, taddr + kS1);
-            tile_row_to_tmem<T>(h_tile, seat, s.half, taddr + kS2);
-            tile_row_to_tmem<T>(dz_tile, seat, s.half, taddr + kD1);
+            tile_row_to_tmem<T>(y2_tile, seat, s.half, taddr + kS2);
+            tile_row_to_tmem<T>(go1_tile, seat, s.half, taddr + kD1);
             tile_row_to_tmem<T>(dy_in, seat, s.half, taddr + kD2);
             tmem_st_wait();
             main_publish();
@@ -614,6 +631,8 @@ rev_bwd_tc_kernel(const RevShape s, const RevParams p, const __grid_constant__ R
                     // the previous pass's weight-gradient MMAs read the h and dz tiles the epilogue below overwrites
                     if (threadIdx.x < 32 && n > 0) rev_wait(wgrad_addr, (n - 1) & 1u, &abort_flag);
                     main_wait_mma(bar, phase, &abort_flag);
+                    const bool last = k == 0 && pass == 1;
+                    if (last && tile + gridDim.x < n_tiles) fetch_rows(row0 + static_cast<long long>(gridDim.x) * kTileRows, (n + 1) & 1u);
                     {
                         // h = act(z) first (also the ReLU mask), then dz = dh where h > 0
                         const int nn = s.hid / kGroups, first = seat.group * (nn / 8);
@@ -673,8 +692,10 @@ rev_bwd_tc_kernel(const RevShape s, const RevParams p, const __grid_constant__ R
                     }
                     main_wait_mma(bar, phase, &abort_flag);
                     // next pass: its input is the stream just reconstructed, its output gradient the one just updated
-                    stream_epilogue<T, false>(taddr + out_col, seat, s.half, nullptr, u_next, nullptr, false);
-                    stream_epilogue<T, false>(taddr + in_d_col, seat, s.half, nullptr, dy_next, nullptr, false);
+                    if (!last) {
+                        stream_epilogue<T, false>(taddr + out_col, seat, s.half, nullptr, u_next, nullptr, false);
+                        stream_epilogue<T, false>(taddr + in_d_col, seat, s.half, nullptr, dy_next, nullptr, false);
+                    }
                     if (pass == 1) {  // next block's weights have landed
                         if (!use_tma) async_tile_wait();
                         else if (more) ring_wait(ring_bars, step + 1, &abort_flag);
@@ -694,8 +715,6 @@ rev_bwd_tc_kernel(const RevShape s, const RevParams p, const __grid_constant__ R
                         stream_epilogue<T, false>(taddr + col, seat, s.half, nullptr, nullptr,
                                                   base + (live ? row0 + seat.row : 0) * stride + (q & 1) * s.half, live);
                 }
-                tc_fence_before();
-                main_sync();
             }
         }
     }
@@ -834,8 +853,14 @@ int launch_rev_bwd_t(const RevShape &s, const RevParams &p, const void *y, int64
     if (int rc = cuda_status(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
                              "cudaFuncSetAttribute(rev_bwd_tc_kernel)")) return rc;
     RevWeightMaps maps;
-    const int use_tma = make_rev_maps(maps, s, p);
-    kernel<<<n_ctas, kTcThreads + kRevFlushThreads, smem, stream>>>(s, p, maps, use_tma, static_cast<const T *>(y), y_stride,
+    RevRowMaps row_maps;
+    memset(&row_maps, 0, sizeof(row_maps));
+    const T *y_rows = static_cast<const T *>(y), *go_rows = static_cast<const T *>(go);
+    const int use_tma = rows < (1ll << 31) - kTileRows && make_rev_maps(maps, s, p) && make_map(&row_maps.y1, y_rows, rows, s.half, kTileRows, y_stride) &&
+                        make_map(&row_maps.y2, y_rows + s.half, rows, s.half, kTileRows, y_stride) &&
+                        make_map(&row_maps.go1, go_rows, rows, s.half, kTileRows, go_stride) &&
+                        make_map(&row_maps.go2, go_rows + s.half, rows, s.half, kTileRows, go_stride);
+    kernel<<<n_ctas, kTcThreads + kRevFlushThreads, smem, stream>>>(s, p, maps, row_maps, use_tma, static_cast<const T *>(y), y_stride,
                                                 static_cast<const T *>(go), go_stride, static_cast<T *>(gx), gx_stride,
                                                 static_cast<T *>(x_rec), xr_stride, workspace, rows);
     if (int rc = launch_status("rev_bwd_tc_kernel launch")) return rc;
