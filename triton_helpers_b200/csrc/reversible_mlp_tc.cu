@@ -67,8 +67,9 @@ __host__ __device__ inline RevTcPlan rev_tc_plan(bool backward) {
 }
 
 // Queue block k's four weight matrices into ring stage `stage` (cp.async, operand-tile layout).
+// A call, not inlined: the kernels live on their instruction cache and almost never come here.
 template <typename T>
-__device__ void prefetch_weights(unsigned char *smem, const RevTcPlan &P, const RevShape &s, const RevParams &p, int k,
+__device__ __noinline__ void prefetch_weights(unsigned char *smem, const RevTcPlan &P, const RevShape &s, const RevParams &p, int k,
                                  int stage) {
     const T *src[4] = {static_cast<const T *>(p.w_f1), static_cast<const T *>(p.w_f2), static_cast<const T *>(p.w_g1),
                        static_cast<const T *>(p.w_g2)};
@@ -110,8 +111,8 @@ struct RevRowMaps {
     CUtensorMap y1, y2, go1, go2;
 };
 
-template <typename T>
-__device__ void prefetch_weights_tma(unsigned char *smem, const RevTcPlan &P, const RevShape &s, const RevParams &p,
+template <typename T, bool BIAS>
+__device__ __forceinline__ void prefetch_weights_tma(unsigned char *smem, const RevTcPlan &P, const RevShape &s, const RevParams &p,
                                      const RevWeightMaps &maps, unsigned long long *ring_bars, int k, int stage) {
     if (threadIdx.x == 64) {  // not warp 0, which is about to issue MMAs
         const uint32_t bar = smem_addr(&ring_bars[stage]);
@@ -123,7 +124,7 @@ __device__ void prefetch_weights_tma(unsigned char *smem, const RevTcPlan &P, co
             tma_load_2d(smem + P.ring + stage * kStageBytes + m * kWTileBytes, &maps.m[m], 0, k * rows, bar);
         }
     }
-    if (s.has_bias) {
+    if constexpr (BIAS) {
         float *bias = reinterpret_cast<float *>(smem + P.bias) + stage * 4 * kMaxDim;
         const T *bsrc[4] = {static_cast<const T *>(p.b_f1), static_cast<const T *>(p.b_f2), static_cast<const T *>(p.b_g1),
                             static_cast<const T *>(p.b_g2)};
@@ -240,7 +241,7 @@ rev_fwd_tc_kernel(const RevShape s, const RevParams p, const __grid_constant__ R
     if (!use_tma && static_cast<long long>(blockIdx.x) < n_tiles) prefetch_weights<T>(smem, P, s, p, 0, 0);
     const uint32_t tmem = cta_setup(&tmem_holder, &mbar, P.tmem_cols);  // publishes the barrier inits
     if (use_tma && static_cast<long long>(blockIdx.x) < n_tiles) {
-        prefetch_weights_tma<T>(smem, P, s, p, maps, ring_bars, 0, 0);
+        prefetch_weights_tma<T, BIAS>(smem, P, s, p, maps, ring_bars, 0, 0);
         ring_wait(ring_bars, 0, &abort_flag);
     }
     const uint32_t bar = smem_addr(&mbar);
@@ -274,7 +275,7 @@ rev_fwd_tc_kernel(const RevShape s, const RevParams p, const __grid_constant__ R
             // the other stage was last read by the previous block, whose GEMMs have all completed
             const bool more = k + 1 < s.blocks || tile + gridDim.x < n_tiles;
             if (more) {
-                if (use_tma) prefetch_weights_tma<T>(smem, P, s, p, maps, ring_bars, (k + 1) % s.blocks, stage ^ 1);
+                if (use_tma) prefetch_weights_tma<T, BIAS>(smem, P, s, p, maps, ring_bars, (k + 1) % s.blocks, stage ^ 1);
                 else prefetch_weights<T>(smem, P, s, p, (k + 1) % s.blocks, stage ^ 1);
             }
             const unsigned char *w = smem + P.ring + stage * kStageBytes;
@@ -529,7 +530,7 @@ rev_bwd_tc_kernel(const RevShape s, const RevParams p, const __grid_constant__ R
     } else {
         // ================= the chain =================
         if (use_tma && static_cast<long long>(blockIdx.x) < n_tiles) {
-            prefetch_weights_tma<T>(smem, P, s, p, maps, ring_bars, s.blocks - 1, 0);
+            prefetch_weights_tma<T, BIAS>(smem, P, s, p, maps, ring_bars, s.blocks - 1, 0);
             ring_wait(ring_bars, 0, &abort_flag);
         }
         const uint32_t bar = smem_addr(&mbar);
@@ -591,7 +592,7 @@ rev_bwd_tc_kernel(const RevShape s, const RevParams p, const __grid_constant__ R
                 const int stage = step & 1;
                 const bool more = k > 0 || tile + gridDim.x < n_tiles;
                 if (more) {
-                    if (use_tma) prefetch_weights_tma<T>(smem, P, s, p, maps, ring_bars, k > 0 ? k - 1 : s.blocks - 1, stage ^ 1);
+                    if (use_tma) prefetch_weights_tma<T, BIAS>(smem, P, s, p, maps, ring_bars, k > 0 ? k - 1 : s.blocks - 1, stage ^ 1);
                     else prefetch_weights<T>(smem, P, s, p, k > 0 ? k - 1 : s.blocks - 1, stage ^ 1);
                 }
                 const unsigned char *w = smem + P.ring + stage * kStageBytes;

