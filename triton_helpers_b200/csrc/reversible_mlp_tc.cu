@@ -106,6 +106,13 @@ struct RevWeightMaps {
     CUtensorMap m[4];  // w_f1, w_f2, w_g1, w_g2: [blocks * rows][cols], 16-bit
 };
 
+// FULL: both widths are 64 at compile time.  The kernels then hold one form of every epilogue and of every GEMM's issue.
+template <bool FULL>
+__device__ __forceinline__ RevShape known_widths(RevShape s) {
+    if constexpr (FULL) s.half = s.hid = 64;
+    return s;
+}
+
 // The row tiles of the backward pass, a column half of y or of the output gradient each: [rows][half], box = 128 rows
 struct RevRowMaps {
     CUtensorMap y1, y2, go1, go2;
@@ -437,13 +444,14 @@ __device__ __forceinline__ void add_tile_column_sums(uint32_t tile, int width, f
     }
 }
 
-template <typename T, int ACT, bool BIAS>
+template <typename T, int ACT, bool BIAS, bool FULL>
 __global__ void __launch_bounds__(kTcThreads + kRevFlushThreads, 1)
-rev_bwd_tc_kernel(const RevShape s, const RevParams p, const __grid_constant__ RevWeightMaps maps,
+rev_bwd_tc_kernel(const RevShape shape, const RevParams p, const __grid_constant__ RevWeightMaps maps,
                   const __grid_constant__ RevRowMaps row_maps, const int use_tma,
                   const T *__restrict__ y, long long y_stride,
                   const T *__restrict__ go, long long go_stride, T *__restrict__ gx, long long gx_stride,
                   T *__restrict__ x_rec, long long xr_stride, float *__restrict__ workspace, long long n_rows) {
+    const RevShape s = known_widths<FULL>(shape);
     extern __shared__ unsigned char smem_raw[];
     unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     __shared__ uint32_t tmem_holder;
@@ -476,7 +484,7 @@ rev_bwd_tc_kernel(const RevShape s, const RevParams p, const __grid_constant__ R
     }
     for (int e = threadIdx.x; e < P.tiles * kTileBytes / 16; e += blockDim.x) reinterpret_cast<uint4 *>(smem)[e] = make_uint4(0, 0, 0, 0);
     const long long n_tiles = (n_rows + kTileRows - 1) / kTileRows;
-    if (!is_flush && !use_tma && static_cast<long long>(blockIdx.x) < n_tiles) prefetch_weights<T>(smem, P, s, p, s.blocks - 1, 0);
+    if (!is_flush && !use_tma && static_cast<long long>(blockIdx.x) < n_tiles) prefetch_weights<T>(smem, P, shape, p, s.blocks - 1, 0);
     const uint32_t tmem = cta_setup(&tmem_holder, &mbar, P.tmem_cols);  // publishes the barrier inits
     float *cta_acc = workspace + static_cast<size_t>(blockIdx.x) * rev_cta_floats(s);
     const uint32_t wgrad_addr = smem_addr(&wgrad_bar), flushed_addr = smem_addr(&flushed_bar);
@@ -593,7 +601,7 @@ rev_bwd_tc_kernel(const RevShape s, const RevParams p, const __grid_constant__ R
                 const bool more = k > 0 || tile + gridDim.x < n_tiles;
                 if (more) {
                     if (use_tma) prefetch_weights_tma<T, BIAS>(smem, P, s, p, maps, ring_bars, k > 0 ? k - 1 : s.blocks - 1, stage ^ 1);
-                    else prefetch_weights<T>(smem, P, s, p, k > 0 ? k - 1 : s.blocks - 1, stage ^ 1);
+                    else prefetch_weights<T>(smem, P, shape, p, k > 0 ? k - 1 : s.blocks - 1, stage ^ 1);
                 }
                 const unsigned char *w = smem + P.ring + stage * kStageBytes;
                 const float *block_bias = reinterpret_cast<const float *>(smem + P.bias) + stage * 4 * kMaxDim;
@@ -850,7 +858,7 @@ int launch_rev_bwd_t(const RevShape &s, const RevParams &p, const void *y, int64
                      void *const db[4], float *workspace, int n_ctas, int64_t rows, cudaStream_t stream) {
     const RevTcPlan P = rev_tc_plan(true);
     const int smem = smem_request(P, 1);  // all 512 TMEM columns: one CTA per SM
-    auto kernel = rev_bwd_tc_kernel<T, ACT, BIAS>;
+    auto kernel = s.half == 64 && s.hid == 64 ? rev_bwd_tc_kernel<T, ACT, BIAS, true> : rev_bwd_tc_kernel<T, ACT, BIAS, false>;
     if (int rc = cuda_status(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
                              "cudaFuncSetAttribute(rev_bwd_tc_kernel)")) return rc;
     RevWeightMaps maps;
