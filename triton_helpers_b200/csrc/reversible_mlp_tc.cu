@@ -225,10 +225,11 @@ __device__ __forceinline__ void publish_tiles() {
 
 // TA: the two A operands of a branch (the 16-bit copy of its input stream, its hidden activation) live in tensor
 // memory and never touch shared memory; the operand tiles only stage the rows as they arrive.
-template <typename T, int ACT, bool BIAS, bool TA>
+template <typename T, int ACT, bool BIAS, bool TA, bool FULL>
 __global__ void __launch_bounds__(kTcThreads, 2)
-rev_fwd_tc_kernel(const RevShape s, const RevParams p, const __grid_constant__ RevWeightMaps maps, const int use_tma,
+rev_fwd_tc_kernel(const RevShape shape, const RevParams p, const __grid_constant__ RevWeightMaps maps, const int use_tma,
                   const T *__restrict__ x, long long x_stride, T *__restrict__ y, long long y_stride, long long n_rows) {
+    const RevShape s = known_widths<FULL>(shape);
     extern __shared__ unsigned char smem_raw[];
     unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     __shared__ uint32_t tmem_holder;
@@ -245,7 +246,7 @@ rev_fwd_tc_kernel(const RevShape s, const RevParams p, const __grid_constant__ R
         asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&ring_bars[1])), "r"(1u) : "memory");
     }
     const long long n_tiles = (n_rows + kTileRows - 1) / kTileRows;
-    if (!use_tma && static_cast<long long>(blockIdx.x) < n_tiles) prefetch_weights<T>(smem, P, s, p, 0, 0);
+    if (!use_tma && static_cast<long long>(blockIdx.x) < n_tiles) prefetch_weights<T>(smem, P, shape, p, 0, 0);
     const uint32_t tmem = cta_setup(&tmem_holder, &mbar, P.tmem_cols);  // publishes the barrier inits
     if (use_tma && static_cast<long long>(blockIdx.x) < n_tiles) {
         prefetch_weights_tma<T, BIAS>(smem, P, s, p, maps, ring_bars, 0, 0);
@@ -283,7 +284,7 @@ rev_fwd_tc_kernel(const RevShape s, const RevParams p, const __grid_constant__ R
             const bool more = k + 1 < s.blocks || tile + gridDim.x < n_tiles;
             if (more) {
                 if (use_tma) prefetch_weights_tma<T, BIAS>(smem, P, s, p, maps, ring_bars, (k + 1) % s.blocks, stage ^ 1);
-                else prefetch_weights<T>(smem, P, s, p, (k + 1) % s.blocks, stage ^ 1);
+                else prefetch_weights<T>(smem, P, shape, p, (k + 1) % s.blocks, stage ^ 1);
             }
             const unsigned char *w = smem + P.ring + stage * kStageBytes;
             const float *bias = reinterpret_cast<const float *>(smem + P.bias) + stage * 4 * kMaxDim;
@@ -815,7 +816,7 @@ int launch_rev_fwd_ta(const RevShape &s, const RevParams &p, const void *x, int6
     const RevTcPlan P = rev_tc_plan(false);
     const int ctas = 2;  // 256 of the 512 TMEM columns each
     const int smem = smem_request(P, ctas);
-    auto kernel = rev_fwd_tc_kernel<T, ACT, BIAS, TA>;
+    auto kernel = s.half == 64 && s.hid == 64 ? rev_fwd_tc_kernel<T, ACT, BIAS, TA, true> : rev_fwd_tc_kernel<T, ACT, BIAS, TA, false>;
     if (int rc = cuda_status(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
                              "cudaFuncSetAttribute(rev_fwd_tc_kernel)")) return rc;
     const long long tiles = (rows + kTileRows - 1) / kTileRows;

@@ -495,12 +495,22 @@ __device__ __forceinline__ void mma_f16_ta(uint32_t tmem_d, uint32_t tmem_a, uin
         : "memory");
 }
 
+template <int N>
+__device__ __forceinline__ void issue_steps_ta(uint32_t tmem_d, uint32_t tmem_a, uint32_t b_low, uint32_t b_step, uint32_t idesc, uint32_t acc) {
+#pragma unroll
+    for (int k = 0; k < N; ++k) mma_f16_ta(tmem_d, tmem_a + 8 * k, smem_desc(b_low + k * b_step), idesc, k > 0 ? 1u : acc);
+}
+
 __device__ __forceinline__ void issue_gemm_ta(bool leader, uint32_t tmem_d, uint32_t tmem_a, uint32_t b_addr, uint32_t b_step, int k_steps,
                                               uint32_t idesc, bool accumulate) {
-    uint32_t b_low = desc_low(b_addr);
-    for (int k = 0; k < k_steps; ++k) {
-        if (leader) mma_f16_ta(tmem_d, tmem_a + 8 * k, smem_desc(b_low), idesc, (accumulate || k > 0) ? 1u : 0u);
-        b_low += b_step >> 4;
+    const uint32_t b_low = desc_low(b_addr), acc = accumulate ? 1u : 0u;
+    b_step >>= 4;
+    if (leader) {
+        if (k_steps == 4) {
+            issue_steps_ta<4>(tmem_d, tmem_a, b_low, b_step, idesc, acc);
+        } else {
+            for (int k = 0; k < k_steps; ++k) issue_steps_ta<1>(tmem_d, tmem_a + 8 * k, b_low + k * b_step, 0, idesc, k > 0 ? 1u : acc);
+        }
     }
 }
 
