@@ -17,6 +17,8 @@ def ordered_and_unordered(n, d, feats, dtype, cap, max_res, points, keep_order, 
     elif points == "clustered":
         x = (torch.rand(4, d, device="cuda", generator=g)[torch.randint(0, 4, (n,), device="cuda", generator=g)] * 0.8 + 0.1
              + 0.01 * torch.randn(n, d, device="cuda", generator=g)).clamp_(0, 1)  # fmt: skip
+    elif points != "uniform":  # a cube of this width above the unit range, next to points inside it
+        x = torch.where(torch.rand(n, 1, device="cuda", generator=g) < 0.8, 1.2 + points * x, x)
     geo = level_geometry(levels, cap, d, 16, max_res)
     table = torch.randn(geo.total_rows, feats, device="cuda", generator=g).to(dtype)
     go = torch.randn(n, levels * feats, device="cuda", generator=g).to(dtype)
@@ -68,5 +70,13 @@ def test_ordered_shapes(d, feats, dtype, keep_order):
 def test_several_passes_over_a_large_table():
     # 16 levels of up to 16 MB: more than one pass of levels, each of them sorting some tiles
     de, de_o = ordered_and_unordered(2**17 + 77, 3, 4, torch.float32, 2**20, 4096, "clustered", keep_order=0)
+    assert float((de - de_o).abs().max() / de.abs().max()) <= 2e-5
+    assert same_rows(de, de_o)
+
+
+@pytest.mark.parametrize("d,max_res,width", [(3, 1000, 0.005), (2, 60000, 2.5e-4)])
+def test_cells_above_the_unit_range_keep_their_rows(d, max_res, width):
+    # many points per cell, on grids whose cells fit the packed key only inside the unit range
+    de, de_o = ordered_and_unordered(6000, d, 2, torch.float32, 2**14, max_res, width, keep_order=0)
     assert float((de - de_o).abs().max() / de.abs().max()) <= 2e-5
     assert same_rows(de, de_o)

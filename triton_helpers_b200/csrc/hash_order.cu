@@ -170,7 +170,9 @@ int launch_order(const CoordView &cv, float scale, int64_t n, float4 *order, uin
 
 constexpr int kTileBins = 2048;
 
-// A cell's coordinates in one word, exact on grids up to kMaxSortedRes; finer levels are not sorted.
+// A cell's coordinates in one word, exact for cells up to kMask: grids up to kMaxSortedRes with coordinates in the unit range.
+// Finer levels are not sorted, nor is a tile whose points could reach past cell kMask (coordinates above the range are accepted
+// and hashed as they are: a clamped cell would send their gradients to other rows than their values come from).
 template <int D>
 struct CellKey {
     static constexpr int kBits = 32 / D;  // 32, 16, 10
@@ -182,6 +184,11 @@ struct CellKey {
 #pragma unroll
         for (int d = 0; d < D; ++d) key |= (D == 1 ? cell[d] : min(cell[d], kMask)) << (d * kBits % 32);
         return key;
+    }
+    // Whether the cells of points up to `top` fit their fields on every grid that is sorted: locate()'s product, which grows with
+    // the coordinate and the grid.
+    static __device__ __forceinline__ bool fits(float top) {
+        return D == 1 || !(__fmul_rn(top, static_cast<float>(kMaxSortedRes)) >= static_cast<float>(kMask) + 1.f);
     }
     static __device__ __forceinline__ void unpack(uint32_t key, uint32_t (&cell)[D]) {
 #pragma unroll
@@ -235,7 +242,8 @@ hash_bwd_tile_kernel(const __grid_constant__ LevelParams P, const __grid_constan
                 if (keep_order) row[j] = static_cast<uint32_t>(first + id);
             }
         }
-        // the tile's bounding box: a level on which it has far more cells than the tile has points is not worth a look
+        // the tile's bounding box: a level on which it has far more cells than the tile has points is not worth a look (infinite, and no
+        // level is, where a cell would not fit its key)
         float extent[D];
 #pragma unroll
         for (int d = 0; d < D; ++d) {
@@ -266,7 +274,7 @@ hash_bwd_tile_kernel(const __grid_constant__ LevelParams P, const __grid_constan
                 low = fminf(low, warp_low[w][d]);
                 high = fmaxf(high, warp_high[w][d]);
             }
-            extent[d] = high - low;
+            extent[d] = Key::fits(high) ? high - low : __int_as_float(0x7f800000);
         }
         for (; level < level_end && P.res[level] <= Key::kMaxSortedRes; ++level) {
             const uint32_t res = P.res[level];
