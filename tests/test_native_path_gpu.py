@@ -2,6 +2,7 @@ r"""The operators' native host path (``_native``) against their Python autograd 
 gradients, same errors, and the calls it leaves to Python."""
 import pytest
 import torch
+import torch.autograd.forward_ad as forward_ad
 
 from triton_helpers_b200 import _lib
 from triton_helpers_b200.layers.fully_fused_mlp import FullyFusedMLP, fully_fused_mlp
@@ -112,6 +113,35 @@ def test_what_the_native_path_leaves_to_python():
     y = fully_fused_mlp(x, *args)
     y.sum().backward()
     assert layer.w_in.grad is not None and x.grad is None  # w_in.grad: from the first pass above
+
+
+def operator(name):
+    r"""A call of one tensor, that tensor, and a parameter the call differentiates."""
+    torch.manual_seed(0)
+    if name == "encoding":
+        layer = HashEncoding(2**12, 8, 3, 2, 16, 128).cuda()
+        return layer, torch.rand(40, 3, device="cuda"), layer.embeddings
+    if name in ("mlp", "mlp float32"):
+        layer = FullyFusedMLP(16, 32, 8, 2).cuda()
+        layer = layer if name == "mlp float32" else layer.half()
+        return layer, torch.randn(1, 40, 16, device="cuda").to(layer.w_in.dtype), layer.w_in
+    if name == "reversible":
+        layer = ReversibleMLP(64, 2, 32).cuda().half()
+        return layer, torch.randn(40, 64, device="cuda").half(), layer.w_f1
+    table = (torch.randn(level_geometry(16, 2**12, 3, 16, 128).total_rows, 2, device="cuda") * 0.1).half()
+    mlp = FullyFusedMLP(32, 64, 16, 2, bias=False).cuda().half()
+    call = lambda x: hash_encoded_mlp(x, table, mlp.w_in, mlp.w_out, mlp.w_hid, None, 2**12, 16, 128, 16)  # noqa: E731
+    return call, torch.rand(40, 3, device="cuda"), mlp.w_in
+
+
+OPERATORS = ["encoding", "mlp", "mlp float32", "reversible", "field"]
+
+
+@pytest.mark.parametrize("name", OPERATORS)
+def test_forward_mode_is_refused(name):
+    call, x, _ = operator(name)
+    with forward_ad.dual_level(), pytest.raises(NotImplementedError, match="jvp"):
+        call(forward_ad.make_dual(x, torch.ones_like(x)))
 
 
 @pytest.mark.parametrize("n,dtype,bias,depth", [(1, torch.float16, False, 1), (1000, torch.bfloat16, True, 3), (2**19 + 3, torch.float16, False, 2),

@@ -45,13 +45,14 @@ using torch::autograd::variable_list;
 
 std::atomic<bool> g_deferred{false};  // event timing of every launch is on: leave the calls to Python
 
-// A CUDA tensor nothing else has a say in: no Python or functorch dispatch, no lazy conjugation or negation.
+// A CUDA tensor nothing else has a say in: no Python or functorch dispatch, no lazy conjugation or negation, no forward-mode
+// tangent (the operators have no forward-mode derivative; the Python functions raise the error for it).
 bool plain(const Tensor &t) {
     using c10::DispatchKey;
     static const c10::DispatchKeySet others({DispatchKey::Python, DispatchKey::PythonTLSSnapshot, DispatchKey::FuncTorchBatched,
                                              DispatchKey::FuncTorchGradWrapper, DispatchKey::Batched, DispatchKey::Functionalize,
                                              DispatchKey::Conjugate, DispatchKey::Negative, DispatchKey::ZeroTensor, DispatchKey::NestedTensor});
-    return t.defined() && t.is_cuda() && !t.key_set().has_any(others) && t.layout() == at::kStrided;
+    return t.defined() && t.is_cuda() && !t.key_set().has_any(others) && t.layout() == at::kStrided && !t._fw_grad(0).defined();
 }
 
 bool usual_mode() {
