@@ -144,6 +144,14 @@ def test_forward_mode_is_refused(name):
         call(forward_ad.make_dual(x, torch.ones_like(x)))
 
 
+@pytest.mark.parametrize("name", OPERATORS[:4])  # the fifth closes over its tensors, which a trace cannot hold
+def test_a_trace_follows_its_input(name):
+    layer, x, _ = operator(name)
+    with torch.no_grad():
+        traced = torch.jit.trace(layer, x, check_trace=False)
+        assert torch.equal(traced(x * 0.5), layer(x * 0.5))
+
+
 @pytest.mark.parametrize("n,dtype,bias,depth", [(1, torch.float16, False, 1), (1000, torch.bfloat16, True, 3), (2**19 + 3, torch.float16, False, 2),
                                                 (1, torch.float32, True, 1), (5003, torch.float32, False, 3)])  # fmt: skip
 def test_training_step(n, dtype, bias, depth):

@@ -56,10 +56,11 @@ bool plain(const Tensor &t) {
 }
 
 bool usual_mode() {
-    // a dispatch or function mode, or a functorch level, shows up in the thread's included keys
+    // a dispatch or function mode, a functorch level or a torch.jit trace (which records the Python functions) shows up in the
+    // thread's included keys
     using c10::DispatchKey;
     static const c10::DispatchKeySet modes({DispatchKey::Python, DispatchKey::PythonTLSSnapshot, DispatchKey::FuncTorchDynamicLayerFrontMode,
-                                            DispatchKey::FuncTorchDynamicLayerBackMode, DispatchKey::Functionalize});
+                                            DispatchKey::FuncTorchDynamicLayerBackMode, DispatchKey::Functionalize, DispatchKey::Tracer});
     return !g_deferred.load(std::memory_order_relaxed) && !at::autocast::is_autocast_enabled(at::kCUDA) &&
            !c10::impl::tls_local_dispatch_key_set().included_.has_any(modes);
 }
