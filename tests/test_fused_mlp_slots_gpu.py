@@ -6,6 +6,7 @@ import torch
 from test_fused_mlp_gpu import NAMES, make_params, nerr, rows_outside, run_both
 
 from triton_helpers_b200 import _lib
+from triton_helpers_b200.layers.fully_fused_mlp import fully_fused_mlp
 
 pytestmark = pytest.mark.gpu
 
@@ -40,3 +41,25 @@ def test_backward_at_the_edges_of_the_slot_plan(rows, d_in, d_hid, d_out, depth,
         else:
             assert nerr(gg, w) <= (tight if name == "y" else 5 * tight), f"{name}: {nerr(gg, w)}"
     assert _lib.lib().th_mlp_tc_status() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_silu_of_every_16_bit_value(dtype):
+    # identity weights: hidden = silu(z), and the input's gradient is silu'(z).  Half a unit of the last place for the rounding to
+    # 16 bits, and what __expf is off by in float32: 2 + 1.17 |z| units, |z| <= 104 before the result is 0 -> 1.5e-5, 0.03 units in float16.
+    z = torch.arange(65536, dtype=torch.int32).to(torch.int16).view(dtype)
+    z = z[torch.isfinite(z.float())].cuda()
+    x = torch.zeros(1, z.numel(), 16, device="cuda", dtype=dtype)
+    x[0, :, 0] = z
+    x.requires_grad_(True)
+    eye = torch.eye(16, device="cuda", dtype=dtype)
+    y = fully_fused_mlp(x, eye, None, eye, None, None, None, "silu")
+    go = torch.zeros_like(x)
+    go[..., 0] = 1
+    (dx,) = torch.autograd.grad(y, x, go)
+    zd = z.double()
+    s = torch.sigmoid(zd)
+    info = torch.finfo(dtype)
+    for got, want in ((y[0, :, 0], zd * s), (dx[0, :, 0], s * (1 + zd * (1 - s)))):
+        unit = info.eps * 2.0 ** torch.floor(torch.log2(want.abs().clamp_min(info.tiny)))
+        assert float(((got.detach().double() - want).abs() / unit).max()) <= 0.53

@@ -88,9 +88,18 @@ __device__ __forceinline__ float round_to(float v) { return to_float<T>(from_flo
 
 // ---- activations (triton_helpers/ops.py:38-66) ----------------------------------------------
 
-// The fast reciprocal (two units in the last place of float32, like __expf) in place of the IEEE division: the result is rounded
-// to 16 bits, and the division was most of a SiLU epilogue.
-__device__ __forceinline__ float sigmoidf(float z) { return __fdividef(1.f, 1.f + __expf(-z)); }
+// exp(-|z|) is at most one, so the reciprocal's argument is in [1, 2] whatever z is: the approximate one (one unit in the last
+// place of float32) needs no range handling there, and a negative z keeps its tail down to the subnormals (1 / (1 + exp(-z)) ends
+// where exp overflows, and __fdividef is 0 from 2^126 on).  Values that are not the correctly rounded 16-bit ones, over all
+// 16-bit z against float64: silu float16 3, bfloat16 1, its derivative 7 and 2; with an IEEE division 1, 17, 7, 18; with
+// __fdividef of 1 + exp(-z) 1, 20, 8, 21.  A division was most of a SiLU epilogue (300 007 rows 32-3x64-3 with biases, forward:
+// division 78 us, this 48, __fdividef 44; a Newton step after the reciprocal, 49, corrects one more value of the derivative).
+__device__ __forceinline__ float sigmoidf(float z) {
+    const float t = __expf(-fabsf(z));
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.f + t));
+    return z < 0.f ? t * r : r;
+}
 
 __device__ __forceinline__ float activate(int act, float z) {
     switch (act) {
