@@ -152,6 +152,23 @@ def test_a_trace_follows_its_input(name):
         assert torch.equal(traced(x * 0.5), layer(x * 0.5))
 
 
+def test_a_saved_tensor_hook_may_change_the_layout():
+    # rows of a wider array come back from the host packed
+    layer, _, leaf = operator("mlp")
+    x = torch.randn(1, 40, 32, device="cuda").half()[..., :16]
+    assert _lib.native().fully_fused_mlp(x, *(getattr(layer, n) for n in ("w_in", "b_in", "w_out", "b_out", "w_hid", "b_hid")), "relu") is not NotImplemented
+    go = torch.randn(1, 40, 8, device="cuda").half()
+    (want,) = torch.autograd.grad(layer(x), leaf, go)
+    with torch.autograd.graph.save_on_cpu():
+        y = layer(x)
+    (got,) = torch.autograd.grad(y, leaf, go)
+    assert torch.equal(got, want)
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t, lambda t: t[..., :8]):
+        y = layer(x)
+    with pytest.raises(RuntimeError, match="saved-tensor hook"):
+        torch.autograd.grad(y, leaf, go)
+
+
 @pytest.mark.parametrize("n,dtype,bias,depth", [(1, torch.float16, False, 1), (1000, torch.bfloat16, True, 3), (2**19 + 3, torch.float16, False, 2),
                                                 (1, torch.float32, True, 1), (5003, torch.float32, False, 3)])  # fmt: skip
 def test_training_step(n, dtype, bias, depth):

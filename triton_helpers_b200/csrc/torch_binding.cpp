@@ -159,6 +159,21 @@ Rows rows_or_copy(const Tensor &t, int64_t width) {
     return r;
 }
 
+// A tensor that a node kept, checked to be what it was: a saved-tensor hook may hand back another one, with another layout, so
+// no stride or pointer is remembered from the forward pass.
+const Tensor &same(const Tensor &t, at::ScalarType type, int64_t numel) {
+    TORCH_CHECK(t.defined() && t.is_cuda() && t.scalar_type() == type && t.numel() == numel,
+                "a saved-tensor hook returned a tensor of another device, type or size than the one it was given");
+    return t;
+}
+
+Tensor restored(const Tensor &t, at::ScalarType type, int64_t numel) { return same(t, type, numel).contiguous(); }
+
+// Three-dimensional rows evenly strided over both leading dimensions, unit stride inside a row
+bool even_rows(const Tensor &x) {
+    return x.stride(2) == 1 && (x.size(0) <= 1 || x.stride(0) == x.size(1) * x.stride(1)) && x.stride(1) >= x.size(2);
+}
+
 template <typename N>
 std::shared_ptr<N> make_node(torch::autograd::edge_list &&edges) {
     auto node = std::shared_ptr<N>(new N(), torch::autograd::deleteNode);
@@ -285,7 +300,8 @@ bool primes_of(PyObject *o, const Tensor &pi, int64_t dims, Primes &out) {
 struct EncodeCall {
     std::shared_ptr<const Geometry> geo;
     Primes primes;
-    int64_t dims = 0, feats = 0, n = 0;
+    int64_t dims = 0, feats = 0, n = 0, table_elems = 0;
+    at::ScalarType table_type = at::kFloat;
     float scale = 1.f;
 };
 
@@ -360,6 +376,8 @@ struct HashEncodingNode : public Node {
         const Tensor x = coords.unpack(), t = table.unpack();
         at::NoGradGuard no_grad;
         c10::cuda::CUDAGuard guard(t.device());
+        same(x, x.scalar_type(), call.n * call.dims);
+        same(t, call.table_type, call.table_elems);
         Tensor go = grads[0];
         if (go.scalar_type() != t.scalar_type()) go = go.to(t.scalar_type());
         const Rows rows = rows_or_copy(go, call.feats * call.geo->levels);
@@ -386,6 +404,8 @@ bool encode_call(EncodeCall &c, const Tensor &coords, const Tensor &table, PyObj
     c.feats = table.size(1);
     if (c.dims < 1 || c.dims > TH_MAX_DIMS || (c.feats != 1 && c.feats != 2 && c.feats != 4 && c.feats != 8)) return false;
     c.n = coords.numel() / c.dims;
+    c.table_elems = table.numel();
+    c.table_type = table.scalar_type();
     c.scale = static_cast<float>(scale);
     if (pi_object != Py_None) {
         if (!THPVariable_Check(pi_object)) return false;
@@ -471,17 +491,30 @@ struct MlpNode : public Node {
         variable_list out(7);
         if (!grads[0].defined()) return out;
         const bool hidden = call.depth > 1;
-        const Tensor xs = x.unpack();
-        MlpTensors p;
-        p.w_in = w_in.unpack();
-        p.w_out = w_out.unpack();
-        if (hidden) p.w_hid = w_hid.unpack();
+        const int64_t h = call.hidden, deep = call.depth - 1;
+        Tensor xs = x.unpack();
+        MlpTensors k;
+        k.w_in = w_in.unpack();
+        k.w_out = w_out.unpack();
+        if (hidden) k.w_hid = w_hid.unpack();
         if (has_bias) {
-            p.b_in = b_in.unpack();
-            p.b_out = b_out.unpack();
-            if (hidden) p.b_hid = b_hid.unpack();
+            k.b_in = b_in.unpack();
+            k.b_out = b_out.unpack();
+            if (hidden) k.b_hid = b_hid.unpack();
         }
         at::NoGradGuard no_grad;
+        const at::ScalarType type = call.dtype == TH_F16 ? at::kHalf : at::kBFloat16;
+        same(xs, type, call.rows() * call.d_in);
+        if (xs.dim() != 3 || xs.size(2) != call.d_in || !even_rows(xs)) xs = xs.contiguous().view({call.batch, call.length, call.d_in});
+        MlpTensors p;
+        p.w_in = restored(k.w_in, type, h * call.d_in);
+        p.w_out = restored(k.w_out, type, call.d_out * h);
+        if (hidden) p.w_hid = restored(k.w_hid, type, deep * h * h);
+        if (has_bias) {
+            p.b_in = restored(k.b_in, type, h);
+            p.b_out = restored(k.b_out, type, call.d_out);
+            if (hidden) p.b_hid = restored(k.b_hid, type, deep * h);
+        }
         c10::cuda::CUDAGuard guard(xs.device());
         Tensor go = grads[0];
         if (go.scalar_type() != xs.scalar_type()) go = go.to(xs.scalar_type());
@@ -496,7 +529,7 @@ struct MlpNode : public Node {
         d.b_hid = empty_same(p.b_hid);
         const int64_t bytes = th_mlp_workspace_bytes(call.d_in, call.hidden, call.d_out, call.depth);
         const Tensor workspace = empty_like_shape({bytes}, at::kByte, xs.device());
-        check(th_mlp_bwd(ptr(xs), call.x_stride, ptr(p.w_in), ptr(p.b_in), ptr(p.w_hid), ptr(p.b_hid), ptr(p.w_out), ptr(p.b_out), ptr(g.keep), g.stride,
+        check(th_mlp_bwd(ptr(xs), xs.stride(1), ptr(p.w_in), ptr(p.b_in), ptr(p.w_hid), ptr(p.b_hid), ptr(p.w_out), ptr(p.b_out), ptr(g.keep), g.stride,
                          ptr(dx), call.d_in, ptr(d.w_in), ptr(d.b_in), ptr(d.w_hid), ptr(d.b_hid), ptr(d.w_out), ptr(d.b_out), ptr(workspace), bytes,
                          call.rows(), call.d_in, call.hidden, call.d_out, call.depth, call.act, call.dtype, 0, current_stream()),
               "th_mlp_bwd");
@@ -641,8 +674,7 @@ bool mlp_call(MlpCall &c, const Tensor &x, MlpTensors &p, PyObject *activation) 
     if (bias && (!parameter_like(p.b_in, x, {hidden}) || !parameter_like(p.b_out, x, {d_out}) ||
                  (depth > 1 && !parameter_like(p.b_hid, x, {depth - 1, hidden}))))
         return false;
-    // rows evenly strided over both leading dimensions
-    if (x.stride(2) != 1 || (c.batch > 1 && x.stride(0) != c.length * x.stride(1)) || x.stride(1) < d_in) return false;
+    if (!even_rows(x)) return false;
     c.x_stride = x.stride(1);
     c.d_in = static_cast<int>(d_in);
     c.hidden = static_cast<int>(hidden);
@@ -745,13 +777,19 @@ struct ReversibleNode : public Node {
     variable_list apply(variable_list &&grads) override {
         variable_list out(9);
         if (!grads[0].defined()) return out;
-        const Tensor ys = y.unpack(shared_from_this());
+        Tensor ys = y.unpack(shared_from_this());
         Tensor ws[4], bs[4], dw[4], db[4];
         for (int i = 0; i < 4; ++i) {
             ws[i] = w[i].unpack();
             if (has_bias) bs[i] = b[i].unpack();
         }
         at::NoGradGuard no_grad;
+        const at::ScalarType type = call.dtype == TH_F16 ? at::kHalf : at::kBFloat16;
+        ys = restored(ys, type, call.rows * call.d_model);
+        for (int i = 0; i < 4; ++i) {
+            ws[i] = restored(ws[i], type, static_cast<int64_t>(call.blocks) * call.hidden * (call.d_model / 2));
+            if (has_bias) bs[i] = restored(bs[i], type, static_cast<int64_t>(call.blocks) * (i % 2 ? call.d_model / 2 : call.hidden));
+        }
         c10::cuda::CUDAGuard guard(ys.device());
         Tensor go = grads[0];
         if (go.scalar_type() != ys.scalar_type()) go = go.to(ys.scalar_type());
@@ -861,10 +899,16 @@ struct FieldNode : public Node {
     variable_list apply(variable_list &&grads) override {
         variable_list out(4);
         if (!grads[0].defined()) return out;
-        const Tensor x = coords.unpack(), t = table.unpack(), wi = w_in.unpack(), wo = w_out.unpack();
-        const Tensor wh = mlp.depth > 1 ? w_hid.unpack() : Tensor();
+        const Tensor x = coords.unpack(), t = table.unpack();
+        Tensor wi = w_in.unpack(), wo = w_out.unpack(), wh = mlp.depth > 1 ? w_hid.unpack() : Tensor();
         at::NoGradGuard no_grad;
         c10::cuda::CUDAGuard guard(t.device());
+        same(x, x.scalar_type(), call.n * call.dims);
+        same(t, call.table_type, call.table_elems);
+        const int64_t width = mlp.hidden;
+        wi = restored(wi, call.table_type, width * mlp.d_in);
+        wo = restored(wo, call.table_type, mlp.d_out * width);
+        if (mlp.depth > 1) wh = restored(wh, call.table_type, (mlp.depth - 1) * width * width);
         Tensor go = grads[0];
         if (go.scalar_type() != t.scalar_type()) go = go.to(t.scalar_type());
         const Rows g = rows_or_copy(go, mlp.d_out);
