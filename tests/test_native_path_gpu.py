@@ -169,6 +169,33 @@ def test_a_saved_tensor_hook_may_change_the_layout():
         torch.autograd.grad(y, leaf, go)
 
 
+@pytest.mark.parametrize("name,kept", zip(OPERATORS, [40 * 3 * 4, 40 * 16 * 2, None, 40 * 64 * 2, 40 * 32 * 2]))
+def test_saved_tensors_go_through_their_hooks(name, kept):
+    # the bytes of the rows an operator keeps (a float32 network: one buffer of all its 16-bit operands) reach the hook
+    call, x, leaf = operator(name)
+    kept = kept or sum((t.numel() + 15) // 16 * 16 * 2 for t in (x, *call.parameters()))
+    packed = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: packed.append(t.numel() * t.element_size()) or t.cpu(), lambda t: t.cuda()):
+        y = call(x)
+    assert kept in packed, packed
+    go = torch.randn_like(y)
+    (got,) = torch.autograd.grad(y, leaf, go)
+    (want,) = torch.autograd.grad(call(x), leaf, go)
+    assert float((got - want).norm() / want.norm()) <= 1e-2  # float16 sums in no fixed order
+
+
+@pytest.mark.parametrize("deferred", [False, True])
+def test_a_saved_order_goes_through_its_hooks(deferred):
+    layer, x, packed = HashEncoding(2**12, 16, 3, 2, 16, 128).cuda(), torch.rand(2**21, 3, device="cuda"), []
+    _lib.native().defer(deferred)
+    try:
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: packed.append(t.numel() * t.element_size()) or t, lambda t: t):
+            layer(x)
+    finally:
+        _lib.native().defer(False)
+    assert 16 * 2**21 in packed
+
+
 @pytest.mark.parametrize("n,dtype,bias,depth", [(1, torch.float16, False, 1), (1000, torch.bfloat16, True, 3), (2**19 + 3, torch.float16, False, 2),
                                                 (1, torch.float32, True, 1), (5003, torch.float32, False, 3)])  # fmt: skip
 def test_training_step(n, dtype, bias, depth):

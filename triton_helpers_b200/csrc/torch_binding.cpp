@@ -361,12 +361,12 @@ void hash_backward(const EncodeCall &c, const CoordArgs &x, const Tensor &order,
 
 struct HashEncodingNode : public Node {
     EncodeCall call;
-    SavedVariable coords, table;
-    Tensor order;
+    SavedVariable coords, table, order;  // order: default-constructed where the batch was not ordered
+    bool ordered = false;
 
     std::string name() const override { return "HashEncodingBackward"; }
     void release_variables() override {
-        order.reset();
+        order.reset_data();
         coords.reset_data();
         table.reset_data();
     }
@@ -374,16 +374,18 @@ struct HashEncodingNode : public Node {
         variable_list out(1);
         if (!grads[0].defined()) return out;
         const Tensor x = coords.unpack(), t = table.unpack();
+        Tensor o = ordered ? order.unpack() : Tensor();
         at::NoGradGuard no_grad;
         c10::cuda::CUDAGuard guard(t.device());
         same(x, x.scalar_type(), call.n * call.dims);
         same(t, call.table_type, call.table_elems);
+        if (ordered) o = restored(o, at::kFloat, call.n * 4);
         Tensor go = grads[0];
         if (go.scalar_type() != t.scalar_type()) go = go.to(t.scalar_type());
         const Rows rows = rows_or_copy(go, call.feats * call.geo->levels);
         Tensor de = empty_like_shape(t.sizes(), t.scalar_type(), t.device());
         de.zero_();
-        hash_backward(call, coord_args(x, call.dims), order, rows, de, current_stream());
+        hash_backward(call, coord_args(x, call.dims), o, rows, de, current_stream());
         out[0] = std::move(de);
         return out;
     }
@@ -431,7 +433,7 @@ PyObject *py_hash_encoding(PyObject *, PyObject *const *args, Py_ssize_t n_args)
     const Tensor coords = THPVariable_Unpack(args[0]), table = THPVariable_Unpack(args[1]);
     EncodeCall call;
     if (!encode_call(call, coords, table, args[3], args + 4, args[7], args[10])) TH_NOT_MINE;
-    Tensor out;
+    Tensor out, order;
     {
         NoGil release;
         const bool grad = torch::autograd::compute_requires_grad(table);
@@ -448,11 +450,14 @@ PyObject *py_hash_encoding(PyObject *, PyObject *const *args, Py_ssize_t n_args)
             out = empty_like_shape(with_last(coords, call.feats * call.geo->levels), table.scalar_type(), table.device());
             const CoordArgs x = coord_args(coords, call.dims);
             void *stream = current_stream();
-            Tensor order = th_hash_order_pays(call.n, static_cast<int>(call.dims), static_cast<int>(call.feats * table.element_size()), grad) ? point_order(call, x, stream) : Tensor();
+            if (th_hash_order_pays(call.n, static_cast<int>(call.dims), static_cast<int>(call.feats * table.element_size()), grad)) order = point_order(call, x, stream);
             hash_forward(call, x, order, table, out, stream);
-            if (grad) node->order = std::move(order);
         }
-        if (grad) torch::autograd::set_history(out, node);
+        if (grad) {
+            node->ordered = order.defined();
+            if (node->ordered) node->order = SavedVariable(order, false);
+            torch::autograd::set_history(out, node);
+        }
     }
     return THPVariable_Wrap(std::move(out));
     END_HANDLE_TH_ERRORS
@@ -545,11 +550,14 @@ struct MlpNode : public Node {
 };
 
 // float32 networks: every tensor is rounded to a 16-bit operand type, all of them in one launch and into one buffer; the
-// results are cast back.  The backward pass keeps that buffer, not the float32 tensors, and hands out the float32 sums
-// of the weight gradients as they are.
+// results are cast back.  The backward pass keeps that buffer (as a saved tensor), not the float32 tensors, and hands out the
+// float32 sums of the weight gradients as they are.
 struct Float32Pack {
     Tensor buffer;          // 16-bit operands: x, w_in, b_in, w_out, b_out, w_hid, b_hid (where present)
-    void *part[7] = {};
+    int64_t offset[7] = {-1, -1, -1, -1, -1, -1, -1};  // in elements; -1: absent
+
+    void *part(int k, const Tensor &in) const { return offset[k] < 0 ? nullptr : static_cast<char *>(ptr(in)) + 2 * offset[k]; }
+    void *part(int k) const { return part(k, buffer); }
 
     static at::ScalarType operands() {
         static const at::ScalarType type = [] {
@@ -568,14 +576,14 @@ struct Float32Pack {
         int n = 0;
         for (const Tensor &t : tensors) total += t.defined() ? (t.numel() + 15) / 16 * 16 : 0;
         buffer = empty_like_shape({total}, operands(), tensors[0].device());
-        char *at = static_cast<char *>(ptr(buffer));
+        int64_t at = 0;
         for (size_t k = 0; k < tensors.size(); ++k) {
-            part[k] = nullptr;
             if (!tensors[k].defined()) continue;
-            part[k] = dst[n] = at;
+            offset[k] = at;
+            dst[n] = part(static_cast<int>(k));
             src[n] = ptr(tensors[k]);
             sizes[n++] = tensors[k].numel();
-            at += (tensors[k].numel() + 15) / 16 * 16 * 2;
+            at += (tensors[k].numel() + 15) / 16 * 16;
         }
         check(th_cast(n, src, dst, sizes, TH_F32, dtype_code(operands()), stream), "th_cast");
     }
@@ -590,23 +598,24 @@ void cast_one(const Tensor &from, const Tensor &to, void *stream) {
 
 struct Float32MlpNode : public Node {
     MlpCall call;
-    Float32Pack pack;
+    Float32Pack pack;      // offsets; its buffer is in `saved`
+    SavedVariable saved;
+    int64_t saved_elems = 0;
     std::vector<int64_t> shapes[6];  // of w_in, b_in, w_out, b_out, w_hid, b_hid
-    bool has_bias = false, released = false;
+    bool has_bias = false;
 
     std::string name() const override { return "FullyFusedMLPBackward"; }
-    void release_variables() override {
-        pack.buffer.reset();
-        released = true;
-    }
+    void release_variables() override { saved.reset_data(); }
     variable_list apply(variable_list &&grads) override {
         variable_list out(7);
-        TORCH_CHECK(!released, torch::autograd::ERR_BACKWARD_TWICE);
         if (!grads[0].defined()) return out;
+        Tensor buffer = saved.unpack();
         at::NoGradGuard no_grad;
-        const c10::Device device = pack.buffer.device();
-        const at::ScalarType half = pack.buffer.scalar_type();
+        buffer = restored(buffer, Float32Pack::operands(), saved_elems);
+        const c10::Device device = buffer.device();
+        const at::ScalarType half = buffer.scalar_type();
         c10::cuda::CUDAGuard guard(device);
+        auto part = [&](int k) { return pack.part(k, buffer); };
         void *stream = current_stream();
         const Tensor given = grads[0].contiguous();
         Tensor go = given;
@@ -620,7 +629,7 @@ struct Float32MlpNode : public Node {
         const Tensor dx = wants_dx ? empty_like_shape({call.batch, call.length, call.d_in}, half, device) : Tensor();
         const int64_t bytes = th_mlp_workspace_bytes(call.d_in, call.hidden, call.d_out, call.depth);
         const Tensor sums = empty_like_shape({bytes / 4}, at::kFloat, device);
-        check(th_mlp_bwd(pack.part[0], call.d_in, pack.part[1], pack.part[2], pack.part[5], pack.part[6], pack.part[3], pack.part[4], ptr(go), call.d_out,
+        check(th_mlp_bwd(part(0), call.d_in, part(1), part(2), part(5), part(6), part(3), part(4), ptr(go), call.d_out,
                          ptr(dx), call.d_in, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, ptr(sums), bytes, call.rows(), call.d_in, call.hidden,
                          call.d_out, call.depth, call.act, dtype_code(half), 0, stream),
               "th_mlp_bwd");
@@ -686,6 +695,7 @@ bool mlp_call(MlpCall &c, const Tensor &x, MlpTensors &p, PyObject *activation) 
 Tensor mlp_float32(const MlpCall &call, const Tensor &x, const MlpTensors &p, bool grad) {
     NoGil release;
     Tensor out;
+    Float32Pack pack;
     std::shared_ptr<Float32MlpNode> node;
     if (grad) {
         node = make_node<Float32MlpNode>(torch::autograd::collect_next_edges(x, p.w_in, p.b_in, p.w_out, p.b_out, p.w_hid, p.b_hid));
@@ -699,17 +709,20 @@ Tensor mlp_float32(const MlpCall &call, const Tensor &x, const MlpTensors &p, bo
         at::AutoDispatchBelowADInplaceOrView below;
         c10::cuda::CUDAGuard guard(x.device());
         void *stream = current_stream();
-        Float32Pack pack;
         pack.fill({x.contiguous(), p.w_in, p.b_in, p.w_out, p.b_out, p.w_hid, p.b_hid}, stream);
         const Tensor half = empty_like_shape({call.batch, call.length, call.d_out}, pack.buffer.scalar_type(), x.device());
-        check(th_mlp_fwd(pack.part[0], call.d_in, pack.part[1], pack.part[2], pack.part[5], pack.part[6], pack.part[3], pack.part[4], ptr(half), call.d_out,
+        check(th_mlp_fwd(pack.part(0), call.d_in, pack.part(1), pack.part(2), pack.part(5), pack.part(6), pack.part(3), pack.part(4), ptr(half), call.d_out,
                          call.rows(), call.d_in, call.hidden, call.d_out, call.depth, call.act, dtype_code(half.scalar_type()), 0, stream),
               "th_mlp_fwd");
         out = empty_like_shape(half.sizes(), at::kFloat, x.device());
         cast_one(half, out, stream);
-        if (grad) node->pack = std::move(pack);
     }
-    if (grad) torch::autograd::set_history(out, node);
+    if (grad) {
+        node->saved_elems = pack.buffer.numel();
+        node->saved = SavedVariable(std::move(pack.buffer), false);
+        node->pack = pack;
+        torch::autograd::set_history(out, node);
+    }
     return out;
 }
 
@@ -886,21 +899,19 @@ PyObject *py_reversible_mlp(PyObject *, PyObject *const *args, Py_ssize_t n_args
 struct FieldNode : public Node {
     EncodeCall call;
     MlpCall mlp;
-    SavedVariable coords, table, w_in, w_out, w_hid;
-    Tensor feats, order;
-    bool separate = true;
+    SavedVariable coords, table, w_in, w_out, w_hid, feats, order;  // order: default-constructed where the batch was not ordered
+    bool separate = true, ordered = false;
 
     std::string name() const override { return "HashEncodedMLPBackward"; }
     void release_variables() override {
-        for (SavedVariable *v : {&coords, &table, &w_in, &w_out, &w_hid}) v->reset_data();
-        feats.reset();
-        order.reset();
+        for (SavedVariable *v : {&coords, &table, &w_in, &w_out, &w_hid, &feats, &order}) v->reset_data();
     }
     variable_list apply(variable_list &&grads) override {
         variable_list out(4);
         if (!grads[0].defined()) return out;
         const Tensor x = coords.unpack(), t = table.unpack();
         Tensor wi = w_in.unpack(), wo = w_out.unpack(), wh = mlp.depth > 1 ? w_hid.unpack() : Tensor();
+        Tensor rows_in = feats.unpack(), o = ordered ? order.unpack() : Tensor();
         at::NoGradGuard no_grad;
         c10::cuda::CUDAGuard guard(t.device());
         same(x, x.scalar_type(), call.n * call.dims);
@@ -909,6 +920,8 @@ struct FieldNode : public Node {
         wi = restored(wi, call.table_type, width * mlp.d_in);
         wo = restored(wo, call.table_type, mlp.d_out * width);
         if (mlp.depth > 1) wh = restored(wh, call.table_type, (mlp.depth - 1) * width * width);
+        rows_in = restored(rows_in, call.table_type, call.n * mlp.d_in);
+        if (ordered) o = restored(o, at::kFloat, call.n * 4);
         Tensor go = grads[0];
         if (go.scalar_type() != t.scalar_type()) go = go.to(t.scalar_type());
         const Rows g = rows_or_copy(go, mlp.d_out);
@@ -918,18 +931,18 @@ struct FieldNode : public Node {
         const int feat = static_cast<int>(call.feats), dims = static_cast<int>(call.dims);
         if (separate) {
             const int64_t bytes = th_mlp_workspace_bytes(mlp.d_in, mlp.hidden, mlp.d_out, mlp.depth);
-            const Tensor sums = empty_like_shape({bytes}, at::kByte, t.device()), grad_feats = empty_same(feats);
+            const Tensor sums = empty_like_shape({bytes}, at::kByte, t.device()), grad_feats = empty_same(rows_in);
             out[1] = empty_same(wi);
             out[2] = empty_same(wo);
             if (wh.defined()) out[3] = empty_same(wh);
             void *stream = current_stream();
-            check(th_mlp_bwd(ptr(feats), mlp.d_in, ptr(wi), nullptr, ptr(wh), nullptr, ptr(wo), nullptr, ptr(g.keep), g.stride, ptr(grad_feats), mlp.d_in,
+            check(th_mlp_bwd(ptr(rows_in), mlp.d_in, ptr(wi), nullptr, ptr(wh), nullptr, ptr(wo), nullptr, ptr(g.keep), g.stride, ptr(grad_feats), mlp.d_in,
                              ptr(out[1]), nullptr, ptr(out[3]), nullptr, ptr(out[2]), nullptr, ptr(sums), bytes, call.n, mlp.d_in, mlp.hidden, mlp.d_out,
                              mlp.depth, mlp.act, mlp.dtype, 0, stream),
                   "th_mlp_bwd");
             Rows rows;
             rows_of(grad_feats, mlp.d_in, rows);
-            hash_backward(call, coord_args(x, call.dims), order, rows, de, stream);
+            hash_backward(call, coord_args(x, call.dims), o, rows, de, stream);
             out[0] = std::move(de);
             return out;
         }
@@ -938,7 +951,7 @@ struct FieldNode : public Node {
         const CoordArgs c = coord_args(x, call.dims);
         void *stream = current_stream();
         check(th_field_bwd(ptr(c.keep), c.stride_n, c.stride_d, dtype_code(c.keep.scalar_type()), dims, feat, geo.levels, geo.res, geo.rows, geo.offsets,
-                           call.primes.v, call.scale, ptr(wi), ptr(wh), ptr(wo), mlp.hidden, mlp.d_out, mlp.depth, mlp.act, ptr(feats), mlp.d_in,
+                           call.primes.v, call.scale, ptr(wi), ptr(wh), ptr(wo), mlp.hidden, mlp.d_out, mlp.depth, mlp.act, ptr(rows_in), mlp.d_in,
                            ptr(g.keep), g.stride, ptr(de), nullptr, mlp.d_in, ptr(sums), bytes, call.n, dtype_code(t.scalar_type()), stream),
               "th_field_bwd");
         // float32 sums -> gradients in the parameter dtype: one rounding of the whole block, handed out as slices of it
@@ -985,7 +998,7 @@ PyObject *py_hash_encoded_mlp(PyObject *, PyObject *const *args, Py_ssize_t n_ar
     const bool separate = !legacy && depth <= 6 && (call.dims == 2 || call.dims == 3) && (call.feats == 2 || call.feats == 4) &&
                           d_in % 16 == 0 && d_in <= 64 && (mlp.act == TH_ACT_RELU || mlp.act == TH_ACT_NONE) &&
                           (hidden == 16 || hidden == 32 || hidden == 64) && d_out >= 1 && d_out <= 64;
-    Tensor out;
+    Tensor out, feats, order;
     {
         NoGil release;
         const bool grad = torch::autograd::compute_requires_grad(table, p.w_in, p.w_out, p.w_hid);
@@ -1006,19 +1019,17 @@ PyObject *py_hash_encoded_mlp(PyObject *, PyObject *const *args, Py_ssize_t n_ar
             c10::cuda::CUDAGuard guard(table.device());
             const Geometry &geo = *call.geo;
             const CoordArgs c = coord_args(coords, call.dims);
-            Tensor feats = grad || separate ? empty_like_shape({call.n, d_in}, table.scalar_type(), table.device()) : Tensor();
+            if (grad || separate) feats = empty_like_shape({call.n, d_in}, table.scalar_type(), table.device());
             out = empty_like_shape(with_last(coords, d_out), table.scalar_type(), table.device());
             int rc = 0;
             if (separate) {
                 void *stream = current_stream();
-                Tensor order;
                 if (th_hash_order_pays(call.n, static_cast<int>(call.dims), static_cast<int>(call.feats * table.element_size()), grad))
                     order = point_order(call, c, stream);
                 hash_forward(call, c, order, table, feats, stream);
                 check(th_mlp_fwd(ptr(feats), d_in, ptr(p.w_in), nullptr, ptr(p.w_hid), nullptr, ptr(p.w_out), nullptr, ptr(out), d_out, call.n, mlp.d_in,
                                  mlp.hidden, mlp.d_out, mlp.depth, mlp.act, mlp.dtype, 0, stream),
                       "th_mlp_fwd");
-                if (grad) node->order = std::move(order);
             } else {
                 rc = th_field_fwd(ptr(c.keep), c.stride_n, c.stride_d, dtype_code(c.keep.scalar_type()), ptr(table), static_cast<int>(call.dims),
                                         static_cast<int>(call.feats), geo.levels, geo.res, geo.rows, geo.offsets, call.primes.v, call.scale, ptr(p.w_in),
@@ -1027,9 +1038,13 @@ PyObject *py_hash_encoded_mlp(PyObject *, PyObject *const *args, Py_ssize_t n_ar
             }
             if (rc == TH_ERR_UNSUPPORTED) out.reset();  // nothing was launched: Python raises FieldUnsupported
             else check(rc, "th_field_fwd");
-            if (grad) node->feats = std::move(feats);
         }
-        if (grad && out.defined()) torch::autograd::set_history(out, node);
+        if (grad && out.defined()) {
+            node->feats = SavedVariable(std::move(feats), false);
+            node->ordered = order.defined();
+            if (node->ordered) node->order = SavedVariable(std::move(order), false);
+            torch::autograd::set_history(out, node);
+        }
     }
     if (!out.defined()) TH_NOT_MINE;
     return THPVariable_Wrap(std::move(out));
@@ -1184,7 +1199,7 @@ PyObject *py_train_gradients(PyObject *, PyObject *const *args, Py_ssize_t n_arg
         Float32Pack pack;
         if (f32) {
             pack.fill(w, stream);
-            for (int k = 0; k < 6; ++k) p[k] = pack.part[k];
+            for (int k = 0; k < 6; ++k) p[k] = pack.part(k);
             check(th_hash_fwd_cast(ptr(x.keep), x.stride_n, x.stride_d, xcode, table.data_ptr<float>(), ptr(feats), code, d_in, n, D, F, L, g.res, g.rows,
                                    g.offsets, call.primes.v, 1.f, stream),
                   "th_hash_fwd_cast");

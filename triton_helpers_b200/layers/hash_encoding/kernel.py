@@ -283,9 +283,8 @@ class HashEncoding(torch.autograd.Function):
         if features is not None:
             o[..., D_embed * levels :] = features
 
-        ctx.save_for_backward(coords, embeddings, pi)
+        ctx.save_for_backward(coords, embeddings, pi, order if any(ctx.needs_input_grad) else None)
         ctx.prime_values = launch.prime_values  # the backward pass needs no second look at `pi`
-        ctx.order = order if any(ctx.needs_input_grad) else None
         ctx.max_entries_per_level = max_entries_per_level
         ctx.min_res = min_res
         ctx.max_res = max_res
@@ -298,7 +297,7 @@ class HashEncoding(torch.autograd.Function):
     @torch.amp.custom_bwd(device_type="cuda")
     @torch.no_grad()
     def backward(ctx, do: Tensor):
-        coords, embeddings, pi = ctx.saved_tensors
+        coords, embeddings, _, order = ctx.saved_tensors
         D_in = coords.shape[-1]
         D_embed = embeddings.shape[-1]
         levels = ctx.levels
@@ -309,7 +308,7 @@ class HashEncoding(torch.autograd.Function):
         de = torch.zeros(embeddings.shape, dtype=embeddings.dtype, device=embeddings.device)
         step = ctx.bwd_divider if ctx.bwd_divider is not None else levels
         for begin in range(0, levels, step):
-            _launch_backward(launch, do, de, D_in, D_embed, levels, begin, begin + step, ctx.order)
+            _launch_backward(launch, do, de, D_in, D_embed, levels, begin, begin + step, order)
         return None, de, None, None, None, None, None, None, None, None, None
 
     @staticmethod
