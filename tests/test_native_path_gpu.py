@@ -9,6 +9,7 @@ from triton_helpers_b200.layers.fully_fused_mlp import FullyFusedMLP, fully_fuse
 from triton_helpers_b200.layers.hash_encoding import HashEncoding, hash_encoding
 from triton_helpers_b200.layers.hash_encoding.helpers import level_geometry
 from triton_helpers_b200.layers.neural_field import hash_encoded_mlp
+from triton_helpers_b200.layers.neural_field.kernel import FieldUnsupported
 from triton_helpers_b200.layers.reversible_mlp import ReversibleMLP
 from triton_helpers_b200.training import NeuralFieldTrainer
 
@@ -194,6 +195,14 @@ def test_a_saved_order_goes_through_its_hooks(deferred):
     finally:
         _lib.native().defer(False)
     assert 16 * 2**21 in packed
+
+
+def test_a_network_too_deep_for_the_fused_backward_says_so():
+    table = (torch.randn(level_geometry(16, 2**12, 3, 16, 128).total_rows, 2, device="cuda") * 0.1).half().requires_grad_(True)
+    mlp = FullyFusedMLP(32, 64, 16, 8, bias=False).cuda().half()
+    y = hash_encoded_mlp(torch.rand(40, 3, device="cuda"), table, mlp.w_in, mlp.w_out, mlp.w_hid, None, 2**12, 16, 128, 16)
+    with pytest.raises(FieldUnsupported):
+        y.sum().backward()
 
 
 @pytest.mark.parametrize("n,dtype,bias,depth", [(1, torch.float16, False, 1), (1000, torch.bfloat16, True, 3), (2**19 + 3, torch.float16, False, 2),

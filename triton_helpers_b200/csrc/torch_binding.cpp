@@ -900,7 +900,7 @@ struct FieldNode : public Node {
     EncodeCall call;
     MlpCall mlp;
     SavedVariable coords, table, w_in, w_out, w_hid, feats, order;  // order: default-constructed where the batch was not ordered
-    bool separate = true, ordered = false;
+    bool ordered = false;
 
     std::string name() const override { return "HashEncodedMLPBackward"; }
     void release_variables() override {
@@ -927,41 +927,20 @@ struct FieldNode : public Node {
         const Rows g = rows_or_copy(go, mlp.d_out);
         Tensor de = empty_like_shape(t.sizes(), t.scalar_type(), t.device());
         de.zero_();
-        const Geometry &geo = *call.geo;
-        const int feat = static_cast<int>(call.feats), dims = static_cast<int>(call.dims);
-        if (separate) {
-            const int64_t bytes = th_mlp_workspace_bytes(mlp.d_in, mlp.hidden, mlp.d_out, mlp.depth);
-            const Tensor sums = empty_like_shape({bytes}, at::kByte, t.device()), grad_feats = empty_same(rows_in);
-            out[1] = empty_same(wi);
-            out[2] = empty_same(wo);
-            if (wh.defined()) out[3] = empty_same(wh);
-            void *stream = current_stream();
-            check(th_mlp_bwd(ptr(rows_in), mlp.d_in, ptr(wi), nullptr, ptr(wh), nullptr, ptr(wo), nullptr, ptr(g.keep), g.stride, ptr(grad_feats), mlp.d_in,
-                             ptr(out[1]), nullptr, ptr(out[3]), nullptr, ptr(out[2]), nullptr, ptr(sums), bytes, call.n, mlp.d_in, mlp.hidden, mlp.d_out,
-                             mlp.depth, mlp.act, mlp.dtype, 0, stream),
-                  "th_mlp_bwd");
-            Rows rows;
-            rows_of(grad_feats, mlp.d_in, rows);
-            hash_backward(call, coord_args(x, call.dims), o, rows, de, stream);
-            out[0] = std::move(de);
-            return out;
-        }
-        const int64_t bytes = th_field_workspace_bytes(geo.levels, feat, mlp.hidden, mlp.d_out, mlp.depth);
-        const Tensor sums = empty_like_shape({bytes / 4}, at::kFloat, t.device());
-        const CoordArgs c = coord_args(x, call.dims);
+        const int64_t bytes = th_mlp_workspace_bytes(mlp.d_in, mlp.hidden, mlp.d_out, mlp.depth);
+        const Tensor sums = empty_like_shape({bytes}, at::kByte, t.device()), grad_feats = empty_same(rows_in);
+        out[1] = empty_same(wi);
+        out[2] = empty_same(wo);
+        if (wh.defined()) out[3] = empty_same(wh);
         void *stream = current_stream();
-        check(th_field_bwd(ptr(c.keep), c.stride_n, c.stride_d, dtype_code(c.keep.scalar_type()), dims, feat, geo.levels, geo.res, geo.rows, geo.offsets,
-                           call.primes.v, call.scale, ptr(wi), ptr(wh), ptr(wo), mlp.hidden, mlp.d_out, mlp.depth, mlp.act, ptr(rows_in), mlp.d_in,
-                           ptr(g.keep), g.stride, ptr(de), nullptr, mlp.d_in, ptr(sums), bytes, call.n, dtype_code(t.scalar_type()), stream),
-              "th_field_bwd");
-        // float32 sums -> gradients in the parameter dtype: one rounding of the whole block, handed out as slices of it
-        const int64_t n_in = wi.numel(), n_hid = wh.defined() ? wh.numel() : 0, n_out = wo.numel();
-        const Tensor rounded = empty_like_shape({n_in + n_hid + n_out}, t.scalar_type(), t.device());
-        check(th_scale_cast(sums.data_ptr<float>(), ptr(rounded), rounded.numel(), 1.f, mlp.dtype, stream), "th_scale_cast");
+        check(th_mlp_bwd(ptr(rows_in), mlp.d_in, ptr(wi), nullptr, ptr(wh), nullptr, ptr(wo), nullptr, ptr(g.keep), g.stride, ptr(grad_feats), mlp.d_in,
+                         ptr(out[1]), nullptr, ptr(out[3]), nullptr, ptr(out[2]), nullptr, ptr(sums), bytes, call.n, mlp.d_in, mlp.hidden, mlp.d_out,
+                         mlp.depth, mlp.act, mlp.dtype, 0, stream),
+              "th_mlp_bwd");
+        Rows rows;
+        rows_of(grad_feats, mlp.d_in, rows);
+        hash_backward(call, coord_args(x, call.dims), o, rows, de, stream);
         out[0] = std::move(de);
-        out[1] = rounded.narrow(0, 0, n_in).view(wi.sizes());
-        out[2] = rounded.narrow(0, n_in + n_hid, n_out).view(wo.sizes());
-        if (n_hid) out[3] = rounded.narrow(0, n_in, n_hid).view(wh.sizes());
         return out;
     }
 };
@@ -998,16 +977,16 @@ PyObject *py_hash_encoded_mlp(PyObject *, PyObject *const *args, Py_ssize_t n_ar
     const bool separate = !legacy && depth <= 6 && (call.dims == 2 || call.dims == 3) && (call.feats == 2 || call.feats == 4) &&
                           d_in % 16 == 0 && d_in <= 64 && (mlp.act == TH_ACT_RELU || mlp.act == TH_ACT_NONE) &&
                           (hidden == 16 || hidden == 32 || hidden == 64) && d_out >= 1 && d_out <= 64;
+    const bool grad = torch::autograd::compute_requires_grad(table, p.w_in, p.w_out, p.w_hid);
+    if (grad && !separate) TH_NOT_MINE;  // the fused backward may turn out not to hold the network: Python's FieldUnsupported again
     Tensor out, feats, order;
     {
         NoGil release;
-        const bool grad = torch::autograd::compute_requires_grad(table, p.w_in, p.w_out, p.w_hid);
         std::shared_ptr<FieldNode> node;
         if (grad) {
             node = make_node<FieldNode>(torch::autograd::collect_next_edges(table, p.w_in, p.w_out, p.w_hid));
             node->call = call;
             node->mlp = mlp;
-            node->separate = separate;
             node->coords = SavedVariable(coords, false);
             node->table = SavedVariable(table, false);
             node->w_in = SavedVariable(p.w_in, false);
@@ -1019,7 +998,7 @@ PyObject *py_hash_encoded_mlp(PyObject *, PyObject *const *args, Py_ssize_t n_ar
             c10::cuda::CUDAGuard guard(table.device());
             const Geometry &geo = *call.geo;
             const CoordArgs c = coord_args(coords, call.dims);
-            if (grad || separate) feats = empty_like_shape({call.n, d_in}, table.scalar_type(), table.device());
+            if (separate) feats = empty_like_shape({call.n, d_in}, table.scalar_type(), table.device());
             out = empty_like_shape(with_last(coords, d_out), table.scalar_type(), table.device());
             int rc = 0;
             if (separate) {
