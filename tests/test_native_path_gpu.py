@@ -205,6 +205,15 @@ def test_a_network_too_deep_for_the_fused_backward_says_so():
         y.sum().backward()
 
 
+def test_a_tensor_subclass_keeps_its_type():
+    class Rows(torch.Tensor):
+        pass
+
+    layer, x, _ = operator("mlp")
+    y = layer(x.as_subclass(Rows))
+    assert type(y) is Rows and torch.equal(y.as_subclass(torch.Tensor), layer(x))
+
+
 @pytest.mark.parametrize("n,dtype,bias,depth", [(1, torch.float16, False, 1), (1000, torch.bfloat16, True, 3), (2**19 + 3, torch.float16, False, 2),
                                                 (1, torch.float32, True, 1), (5003, torch.float32, False, 3)])  # fmt: skip
 def test_training_step(n, dtype, bias, depth):

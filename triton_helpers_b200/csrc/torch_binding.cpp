@@ -65,10 +65,11 @@ bool usual_mode() {
            !c10::impl::tls_local_dispatch_key_set().included_.has_any(modes);
 }
 
-// One optional tensor argument; false when it is neither None nor a tensor.
+// One optional tensor argument; false when it is neither None nor a tensor (or Parameter) itself: a subclass keeps its type through
+// the Python functions.
 bool take(PyObject *o, Tensor &t) {
     if (o == Py_None) return true;
-    if (!THPVariable_Check(o)) return false;
+    if (!THPVariable_CheckExact(o)) return false;
     t = THPVariable_Unpack(o);
     return true;
 }
@@ -410,7 +411,7 @@ bool encode_call(EncodeCall &c, const Tensor &coords, const Tensor &table, PyObj
     c.table_type = table.scalar_type();
     c.scale = static_cast<float>(scale);
     if (pi_object != Py_None) {
-        if (!THPVariable_Check(pi_object)) return false;
+        if (!THPVariable_CheckExact(pi_object)) return false;
         const Tensor &pi = THPVariable_Unpack(pi_object);
         if (!plain(pi) || pi.device() != coords.device() || !primes_of(pi_object, pi, c.dims, c.primes)) return false;
     }
@@ -427,7 +428,7 @@ std::vector<int64_t> with_last(const Tensor &t, int64_t last) {
 // hash_encoding(coord, embeddings, features, pi, max_entries_per_level, min_res, max_res, levels, divider, bwd_divider, scale)
 PyObject *py_hash_encoding(PyObject *, PyObject *const *args, Py_ssize_t n_args) {
     HANDLE_TH_ERRORS
-    if (n_args != 11 || !usual_mode() || !THPVariable_Check(args[0]) || !THPVariable_Check(args[1]) || args[2] != Py_None ||
+    if (n_args != 11 || !usual_mode() || !THPVariable_CheckExact(args[0]) || !THPVariable_CheckExact(args[1]) || args[2] != Py_None ||
         args[8] != Py_None || args[9] != Py_None)
         TH_NOT_MINE;
     const Tensor coords = THPVariable_Unpack(args[0]), table = THPVariable_Unpack(args[1]);
@@ -948,7 +949,7 @@ struct FieldNode : public Node {
 // hash_encoded_mlp(coord, embeddings, w_in, w_out, w_hid, pi, max_entries_per_level, min_res, max_res, levels, activation, scale)
 PyObject *py_hash_encoded_mlp(PyObject *, PyObject *const *args, Py_ssize_t n_args) {
     HANDLE_TH_ERRORS
-    if (n_args != 12 || !usual_mode() || !THPVariable_Check(args[0]) || !THPVariable_Check(args[1])) TH_NOT_MINE;
+    if (n_args != 12 || !usual_mode() || !THPVariable_CheckExact(args[0]) || !THPVariable_CheckExact(args[1])) TH_NOT_MINE;
     const Tensor coords = THPVariable_Unpack(args[0]), table = THPVariable_Unpack(args[1]);
     MlpTensors p;
     EncodeCall call;
