@@ -1,5 +1,7 @@
 r"""The operators' native host path (``_native``) against their Python autograd functions: same outputs, same
 gradients, same errors, and the calls it leaves to Python."""
+import warnings
+
 import pytest
 import torch
 import torch.autograd.forward_ad as forward_ad
@@ -240,3 +242,69 @@ def test_training_step(n, dtype, bias, depth):
         assert abs(a - b) <= 2e-3 * abs(b)
     for a, b in zip(params_n, params_p):  # Adam's first steps are lr * sign: entries whose gradient nearly cancels may differ
         assert float((a - b).norm() / b.norm()) <= 2e-3
+
+
+def float32_trainer(d_out=8, feats=2, levels=8, d=3, depth=2, bias=True):
+    torch.manual_seed(0)
+    encoding, mlp = HashEncoding(2**12, levels, d, feats, 16, 256), FullyFusedMLP(levels * feats, 32, d_out, depth, bias=bias)
+    with torch.no_grad():
+        encoding.embeddings.mul_(0.1)
+    return NeuralFieldTrainer(encoding.cuda(), mlp.cuda(), lr=1e-3)
+
+
+def batch(n=1000, d=3, d_out=8):
+    g = torch.Generator(device="cuda").manual_seed(1)
+    return torch.rand(n, d, device="cuda", generator=g), torch.rand(n, d_out, device="cuda", generator=g)
+
+
+@pytest.mark.parametrize("hook", ["post accumulate", "parameter", "module", "every module", "before the optimizer", "after the optimizer"])
+def test_hooks_run_in_a_float32_step(hook):
+    trainer, seen = float32_trainer(), []
+    call = lambda *args, **kwargs: seen.append(1)  # noqa: E731
+    register = {
+        "post accumulate": trainer.mlp.w_in.register_post_accumulate_grad_hook,
+        "parameter": trainer.mlp.w_in.register_hook,
+        "module": trainer.mlp.register_forward_hook,
+        "every module": torch.nn.modules.module.register_module_forward_hook,
+        "before the optimizer": trainer.optimizer.register_step_pre_hook,
+        "after the optimizer": trainer.optimizer.register_step_post_hook,
+    }[hook]
+    handle = register(call)
+    try:
+        trainer.step(*batch())
+    finally:
+        handle.remove()
+    assert seen
+
+
+def test_a_scheduler_sees_the_float32_steps():
+    trainer = float32_trainer()
+    scheduler = torch.optim.lr_scheduler.StepLR(trainer.optimizer, 1)
+    with warnings.catch_warnings():
+        warnings.simplefilter("error")
+        trainer.step(*batch())
+        scheduler.step()
+
+
+def test_a_gradient_replaced_by_a_hook_leaves_nothing_behind():
+    # the table's gradient is dropped before one step: the next one starts from zero
+    def run(drop):
+        trainer = float32_trainer()
+        table = trainer.encoding.embeddings
+        handle = trainer.optimizer.register_step_pre_hook(lambda *args, **kwargs: setattr(table, "grad", None)) if drop else None
+        before = table.detach().clone()
+        trainer.step(*batch())
+        if drop:
+            handle.remove()
+            assert torch.equal(table, before)
+            return float(trainer._state.table_grad.abs().max())
+        return float((table - before).abs().max())
+
+    assert run(drop=True) == 0 and run(drop=False) > 0
+
+
+def test_anomaly_detection_sees_a_float32_step():
+    x, target = batch()
+    target[0] = float("nan")
+    with pytest.raises(RuntimeError, match="nan"), torch.autograd.detect_anomaly(check_nan=True):
+        float32_trainer().step(x, target)

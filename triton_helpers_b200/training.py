@@ -179,16 +179,16 @@ class NeuralFieldTrainer(nn.Module):
         return loss_sum / pred.numel()
 
     def _step_float32(self, coords: Tensor, targets: Tensor) -> Optional[Tensor]:
-        r"""The same step without an autograd graph: forward and backward in one native call on kept buffers, Adam in one
-        launch.  ``None`` where the graph has to be built: hooks, frozen parameters, subclasses of the layers, or a call
-        the native path does not take."""
+        r"""The same step without an autograd graph: forward and backward in one native call on kept buffers, then the
+        optimizer's own step.  ``None`` where the graph has to be built: hooks of modules or parameters, anomaly detection,
+        frozen parameters, subclasses of the layers, or a call the native path does not take."""
         enc, mlp = self.encoding, self.mlp
         if type(enc) is not HashEncoding or type(mlp) is not FullyFusedMLP or len(self.optimizer.param_groups) != 1 or coords.ndim != 2:
             return None
-        if _hooked(enc) or _hooked(mlp):
+        if _hooked(enc) or _hooked(mlp) or nn.modules.module._has_any_global_hook() or torch.is_anomaly_enabled():
             return None
         params = [p for p in (enc.embeddings, mlp.w_in, mlp.b_in, mlp.w_hid, mlp.b_hid, mlp.w_out, mlp.b_out) if p is not None]
-        if not all(p.requires_grad and p._backward_hooks is None and p.grad is None for p in params):
+        if not all(p.requires_grad and p.grad is None and not p._backward_hooks and not p._post_accumulate_grad_hooks for p in params):
             return None
         st = self._state
         if st is None or st.table is not enc.embeddings or st.device != enc.embeddings.device:
@@ -205,7 +205,18 @@ class NeuralFieldTrainer(nn.Module):
         grads = [st.table_grad] + [g.view_as(p) for p, g in zip(params[1:], st.mlp_grads)]
         # d(mean over the batch)/d pred = 2 (pred - target) / (N * C); Adam clears the table gradient as it consumes it
         adam_scale = 2.0 / (coords.shape[0] * st.d_out * scale)
-        self.optimizer.update(self.optimizer.param_groups[0], params, grads, [adam_scale] * len(params), [True] + [False] * (len(params) - 1))
+        try:
+            for p, g in zip(params, grads):
+                p.grad = g
+            self.optimizer.step(grad_scale=adam_scale, zero_grad=True)  # the public step: its hooks, and schedulers that watch it
+            if enc.embeddings.grad is not st.table_grad:
+                st.table_grad.zero_()  # a hook put another gradient in its place
+        except BaseException:
+            self._state = None  # its table gradient may not be zero
+            raise
+        finally:
+            for p in params:
+                p.grad = None
         return loss
 
     # ---- direct mode (one 16-bit dtype) ------------------------------------------------------------
