@@ -308,3 +308,24 @@ def test_anomaly_detection_sees_a_float32_step():
     target[0] = float("nan")
     with pytest.raises(RuntimeError, match="nan"), torch.autograd.detect_anomaly(check_nan=True):
         float32_trainer().step(x, target)
+
+
+@pytest.mark.parametrize("kw", [dict(d=1), dict(feats=1, levels=16), dict(d_out=3)])
+def test_a_float32_step_keeps_buffers_only_where_it_uses_them(kw):
+    trainer = float32_trainer(**kw)
+    trainer.step(*batch(d=kw.get("d", 3), d_out=kw.get("d_out", 8)))
+    assert trainer._state is None
+
+
+def test_a_replaced_network_is_not_trained_by_the_old_optimizer():
+    # as through the graph: the optimizer holds the first network's parameters
+    trainer, other = float32_trainer(depth=1, bias=False), FullyFusedMLP(16, 32, 8, 1).cuda()
+    trainer.step(*batch())
+    before = [p.detach().clone() for p in other.parameters()]
+    trainer.mlp = other
+    trainer.step(*batch())
+    assert all(torch.equal(a, b) for a, b in zip(before, other.parameters()))
+    # a network of another layout under a new optimizer gets buffers of its own
+    trainer.optimizer = type(trainer.optimizer)(trainer.parameters(), lr=1e-3)
+    trainer.step(*batch())
+    assert not any(torch.equal(a, b) for a, b in zip(before, other.parameters()))

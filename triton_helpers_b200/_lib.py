@@ -226,6 +226,11 @@ def lib() -> _Library:
     return _Library(handle)
 
 
+def timing() -> bool:
+    r"""Whether a ``KernelTimer`` is active."""
+    return _ACTIVE_TIMER is not None
+
+
 @lru_cache(maxsize=1)
 def native():
     r"""The extension module ``triton_helpers_b200._native``.  Its functions take the arguments of the public

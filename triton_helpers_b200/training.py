@@ -190,8 +190,12 @@ class NeuralFieldTrainer(nn.Module):
         params = [p for p in (enc.embeddings, mlp.w_in, mlp.b_in, mlp.w_hid, mlp.b_hid, mlp.w_out, mlp.b_out) if p is not None]
         if not all(p.requires_grad and p.grad is None and not p._backward_hooks and not p._post_accumulate_grad_hooks for p in params):
             return None
+        held = {id(p) for p in self.optimizer.param_groups[0]["params"]}
+        if any(id(p) not in held for p in params) or not _float32_native(enc, mlp, coords):
+            return None
+        layout = _Float32State.layout(enc, mlp)
         st = self._state
-        if st is None or st.table is not enc.embeddings or st.device != enc.embeddings.device:
+        if st is None or st.key != layout:
             st = self._state = _Float32State(enc, mlp)
         st.resize(coords.shape[0])
         scale = float(self.grad_out_scale)
@@ -201,6 +205,7 @@ class NeuralFieldTrainer(nn.Module):
             enc.num_levels, mlp.activation, scale, 1.0,
         )  # fmt: skip
         if loss is NotImplemented:
+            self._state = None
             return None
         grads = [st.table_grad] + [g.view_as(p) for p, g in zip(params[1:], st.mlp_grads)]
         # d(mean over the batch)/d pred = 2 (pred - target) / (N * C); Adam clears the table gradient as it consumes it
@@ -388,17 +393,37 @@ def _hooked(module: nn.Module) -> bool:
     return bool(module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or module._backward_pre_hooks)
 
 
+def _float32_native(enc: HashEncoding, mlp: FullyFusedMLP, coords: Tensor) -> bool:
+    r"""What the native float32 step declines for good, before buffers are made for it: shapes it has no kernels for, batches that
+    are better ordered in space (the layers' own functions do that), modes in which the native path stands back."""
+    n, d = coords.shape
+    feats, hidden, d_out = enc.embeddings.shape[1], mlp.w_in.shape[0], mlp.w_out.shape[0]
+    depth = 1 if mlp.w_hid is None else mlp.w_hid.shape[0] // hidden + 1
+    if not coords.is_cuda or n < 1 or d not in (2, 3) or feats not in (2, 4) or hidden not in (16, 32, 64) or depth >= 4:
+        return False
+    if d_out > 64 or d_out % 8 or enc.num_levels * feats > 64 or torch.is_autocast_enabled("cuda") or _lib.timing():
+        return False
+    return not _lib.lib().th_hash_order_pays(n, d, 4 * feats, 1)
+
+
 class _Float32State:
     r"""Buffers the float32 step keeps: the table's gradient (zero between steps), the float32 sums of the MLP's gradients,
     16-bit rows."""
 
+    @staticmethod
+    def layout(enc: HashEncoding, mlp: FullyFusedMLP) -> tuple:
+        r"""What the buffers depend on."""
+        tensors = (enc.embeddings, mlp.w_in, mlp.b_in, mlp.w_hid, mlp.b_hid, mlp.w_out, mlp.b_out)
+        return (enc.embeddings.device, *(None if t is None else (t.dtype, t.shape) for t in tensors))
+
     def __init__(self, enc: HashEncoding, mlp: FullyFusedMLP):
-        self.table = enc.embeddings
-        self.device = self.table.device
+        self.key = self.layout(enc, mlp)
+        table = enc.embeddings
+        self.device = table.device
         self.d_hidden, self.d_feat = mlp.w_in.shape
         self.d_out = mlp.w_out.shape[0]
         depth = 1 if mlp.w_hid is None else mlp.w_hid.shape[0] // self.d_hidden + 1
-        self.table_grad = torch.zeros_like(self.table)
+        self.table_grad = torch.zeros_like(table)
         self.sums = torch.zeros(_lib.lib().th_mlp_workspace_bytes(self.d_feat, self.d_hidden, self.d_out, depth) // 4, device=self.device)
         # slices of the sums in the order w_in, b_in, w_hid, b_hid, w_out, b_out of the parameters that exist
         h, offset, place = self.d_hidden, 0, {}
