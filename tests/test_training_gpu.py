@@ -280,3 +280,17 @@ def test_no_stream_synchronisation_in_the_encoding_calls():
         out.backward(torch.ones_like(out))
     finally:
         torch.cuda.set_sync_debug_mode("default")
+
+
+@pytest.mark.parametrize("d_out", [1, 3, 4])
+def test_a_large_step_with_few_outputs_encodes_once(d_out):
+    # widths the loss epilogue does not take: nothing is ordered or gathered that is then thrown away
+    torch.manual_seed(0)
+    encoding, mlp = HashEncoding(2**12, 16, 3, 2, 16, 256), FullyFusedMLP(32, 64, d_out, 1)
+    trainer = NeuralFieldTrainer(encoding.cuda().half(), mlp.cuda().half(), lr=1e-3)
+    n = 2**19 + 3
+    x, t = torch.rand(n, 3, device="cuda"), torch.rand(n, d_out, device="cuda").half()
+    with _lib.KernelTimer() as timer:
+        trainer.step(x, t)
+    calls = {name: count for name, (count, _) in timer.summary().items()}
+    assert calls.get("th_hash_fwd", 0) + calls.get("th_hash_fwd_ordered", 0) == 1 and "th_hash_order" not in calls, calls

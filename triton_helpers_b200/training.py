@@ -117,7 +117,7 @@ class NeuralFieldTrainer(nn.Module):
     ):
         super().__init__()
         self.fused = fused
-        self._no_fused_forward = self._no_fused_backward = False
+        self._no_fused_forward = self._no_fused_backward = self._no_ordered = False
         self.encoding = encoding
         self.mlp = mlp
         self.grad_out_scale = grad_out_scale
@@ -261,9 +261,12 @@ class NeuralFieldTrainer(nn.Module):
                     self._no_fused_forward = True  # nothing was launched: the separate operators from now on
                     fuse_fwd = False
             # ---- or, for large batches, in spatial order from the features to the table gradient ----
+            # (the loss epilogue takes whole 16-byte chunks of targets and gradients: decided before anything is ordered)
             order = None
-            if not (fuse_fwd or fuse_bwd or self.backward_passes):
+            if not (fuse_fwd or fuse_bwd or self.backward_passes or self._no_ordered or st.d_out % 8):
                 order = launch.order(st.n_feats * st.flat_grad.element_size(), True)
+            if order is not None and (targets.stride(0) % 8 or targets.data_ptr() % 16):
+                targets = targets.clone(memory_format=torch.contiguous_format)
             if order is not None:
                 _lib.check(
                     lib.th_hash_fwd_ordered(order.data_ptr(), 1, enc.embeddings.data_ptr(), code, st.feats.data_ptr(), st.d_feat, *geometry[:-1],
@@ -275,7 +278,7 @@ class NeuralFieldTrainer(nn.Module):
                     st.grad_pred.data_ptr(), st.d_out, st.loss_sum.data_ptr(), 1.0, scale, n, *dims, act, code, stream,
                 )  # fmt: skip
                 if rc == _lib.TH_ERR_UNSUPPORTED:
-                    order = None
+                    order, self._no_ordered = None, True  # a switch turned its kernel off: the unordered operators from now on
                 else:
                     _lib.check(rc, "th_mlp_fwd_mse_ordered")
             if not fuse_fwd and order is None:
