@@ -123,9 +123,10 @@ int th_hash_bwd(const void *coords_dev, int64_t coord_stride_n, int64_t coord_st
  * gradients differ from th_hash_bwd's in the order of the sums.  order_dev: 16 * n_points bytes; scratch_dev:
  * th_hash_order_scratch_bytes, free once the work queued by th_hash_order is done.  Both 16-byte aligned.
  * th_hash_order_pays: 1 where the ordering is measured to pay for itself, for a forward pass alone (backward = 0) or a
- * forward and a backward pass, with table rows of row_bytes.  No counterpart in the reference.
+ * forward and a backward pass, over n_levels levels of together table_rows rows of n_feats features and row_bytes bytes.
+ * No counterpart in the reference.
  */
-int th_hash_order_pays(int64_t n_points, int n_dims, int row_bytes, int backward);
+int th_hash_order_pays(int64_t n_points, int n_dims, int n_feats, int n_levels, int row_bytes, int64_t table_rows, int backward);
 int64_t th_hash_order_scratch_bytes(int64_t n_points, int n_dims);
 int th_hash_order(const void *coords_dev, int64_t coord_stride_n, int64_t coord_stride_d, int coord_dtype, int64_t n_points,
                   int n_dims, float scale, void *order_dev, void *scratch_dev, int64_t scratch_bytes, void *stream);

@@ -66,6 +66,35 @@ def test_argument_errors_are_reported_without_touching_a_gpu(library):
     assert rc == -1 and b"level range" in library.th_last_error_string()
 
 
+@pytest.mark.parametrize(
+    "n,dims,feats,levels,row_bytes,rows,backward,ordered",
+    [
+        (2**21, 3, 2, 16, 4, 6_000_000, 1, 1),  # a training step on 2^19 rows per level
+        (2**19 - 1, 3, 2, 16, 4, 10_000, 1, 0),
+        (2**19, 3, 2, 16, 4, 6_000_000, 1, 1),
+        (2**19, 3, 2, 16, 4, 20_000_000, 1, 0),  # more than twelve rows a point
+        (2**22, 3, 4, 16, 16, 42_000_000, 1, 1),
+        (2**22, 3, 2, 16, 4, 42_000_000, 1, 0),
+        (2**21, 3, 8, 16, 16, 10_000, 1, 0),
+        (2**21, 3, 1, 16, 2, 10_000, 1, 0),
+        (2**20, 3, 2, 8, 4, 10_000, 1, 1),
+        (2**20 - 1, 3, 2, 8, 4, 10_000, 1, 0),
+        (2**20, 2, 4, 16, 16, 10_000, 1, 1),
+        (2**20 + 1, 2, 4, 16, 16, 10_000, 1, 0),
+        (2**21, 2, 2, 16, 8, 10_000, 1, 0),
+        (2**17, 1, 8, 16, 32, 10_000, 1, 1),
+        (2**19, 1, 4, 16, 16, 10_000, 1, 0),
+        (2**21, 3, 2, 16, 4, 6_000_000, 0, 1),
+        (2**21 - 1, 3, 2, 16, 4, 6_000_000, 0, 0),
+        (2**21, 3, 4, 16, 16, 6_000_000, 0, 0),  # outputs past 256 MB
+        (2**21, 2, 4, 16, 16, 10_000, 0, 0),
+        (2**31, 3, 2, 16, 4, 10_000, 1, 0),
+    ],
+)
+def test_which_batches_are_ordered(library, n, dims, feats, levels, row_bytes, rows, backward, ordered):
+    assert library.th_hash_order_pays(n, dims, feats, levels, row_bytes, rows, backward) == ordered
+
+
 def test_missing_library_fails_loudly(monkeypatch, tmp_path):
     monkeypatch.setattr(_lib, "LIB_PATH", tmp_path / "libth_b200.so")
     _lib.lib.cache_clear()

@@ -216,7 +216,7 @@ def test_a_tensor_subclass_keeps_its_type():
     assert type(y) is Rows and torch.equal(y.as_subclass(torch.Tensor), layer(x))
 
 
-@pytest.mark.parametrize("n,dtype,bias,depth", [(1, torch.float16, False, 1), (1000, torch.bfloat16, True, 3), (2**19 + 3, torch.float16, False, 2),
+@pytest.mark.parametrize("n,dtype,bias,depth", [(1, torch.float16, False, 1), (1000, torch.bfloat16, True, 3), (2**20 + 3, torch.float16, False, 2),
                                                 (1, torch.float32, True, 1), (5003, torch.float32, False, 3)])  # fmt: skip
 def test_training_step(n, dtype, bias, depth):
     # the last 16-bit case runs over spatially ordered points

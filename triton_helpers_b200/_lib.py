@@ -57,7 +57,7 @@ SIGNATURES = {
         [c_void_p, c_int64, c_int64, c_int, c_void_p, c_int, c_int64, c_void_p, c_int64, c_int, c_int, c_int,
          _I32P, _I64P, _I64P, _I64P, c_float, c_void_p],
     ),
-    "th_hash_order_pays": (c_int, [c_int64, c_int, c_int, c_int]),
+    "th_hash_order_pays": (c_int, [c_int64, c_int, c_int, c_int, c_int, c_int64, c_int]),
     "th_hash_order_scratch_bytes": (c_int64, [c_int64, c_int]),
     "th_hash_order": (
         c_int,

@@ -514,17 +514,33 @@ int launch_bwd_ordered(const LevelParams &P, const float4 *order, int keep_order
 
 using namespace th;
 
-// Where the order pays (B200, forward + backward with the sorting, unordered time / ordered time, uniform points):
-//   D = 3, 16 levels: 2^16 0.83-0.91, 2^17 0.83-1.11, 2^18 0.90-1.14, 2^19 0.95-1.18, 2^20 1.01-1.29, 2^21 1.03-1.20; clustered
-//     points, which the host cannot tell, gain more (300 001: 1.40, 2^22: 1.61)
-//   D = 2, rows of 16 bytes: 2^16 0.98, 2^17 1.19-1.47, 2^18 1.17-1.19, 2^20 1.11-1.31; smaller rows: from 2^18 on 0.79-1.07, because
-//     hash_bwd_coarse_kernel holds more of the levels there
-// Forward alone (sorting costs 14 us at 2^18 points, 55 at 2^21): D = 3 2^18 0.77-1.04, 2^19 1.06-1.18, 2^20 1.09-1.48; D = 2 with
-//   16-byte rows 2^18 0.99-1.37, 2^19 1.14-2.26, smaller rows 0.67-1.07 at every size.
-extern "C" int th_hash_order_pays(int64_t n_points, int n_dims, int row_bytes, int backward) {
-    if (n_points >= (1ll << 31)) return 0;
-    if (n_dims >= 3) return n_points >= (1 << 19);
-    return row_bytes >= 16 && n_points >= (backward ? 1 << 17 : 1 << 18);
+// Where the order pays: time with it, sorting included, over time without (B200; 2, 4, 8 or 16 levels, tables of 2^14 .. 2^22 rows per
+// level, finest grids of 512 .. 4096, 1 .. 8 features of 2 or 4 bytes, points uniform or in eight clusters, which the host cannot tell
+// apart).  A form is ordered where none of its points is more than a run's spread above 1:
+//   forward + backward, three dimensions, 16 levels: 2^19 0.40-0.99, 2^20 0.40-0.96, 2^21 0.41-0.97, 2^23 0.78-1.01; eight levels share
+//     the cost of sorting: 2^19 0.40-1.04, 2^20 0.45-1.01, 2^21 0.46-0.94; four: 2^19 0.50-1.35, 2^21 0.42-1.16.  Left out: tables with
+//     more than twelve rows a point (0.42-1.24), past 24 M rows with rows below 16 bytes (2^22 0.98-1.05), past 8 M rows with
+//     eight levels (2^21 up to 1.13), rows of 8 x 16 bit (0.54-1.16) and of one 16-bit element (single-element atomics, 0.25-1.3).
+//   two dimensions, 4 x float32, 16 levels: 2^16 0.99, 2^17 0.63-0.91, 2^19 0.62-0.95, 2^20 0.66-1.00, 2^21 0.78-1.14 (the ordered
+//     forward writes whole rows in random order, and loses once all of them are past twice the L2); eight: 2^17 0.75-0.99, 2^20
+//     0.65-0.93; four: up to 1.14.  8 x float32 in one or two: 16 levels 2^17 0.33-0.86, 2^21 0.62-0.95, four 2^17 0.55-0.98, two up to
+//     1.24.  Narrower rows: two dimensions 0.80-1.35, one 0.74-1.94.
+//   forward alone, three dimensions, 16 levels, up to four features: 2^19 0.65-1.35, 2^20 0.59-1.12, 2^21 0.55-0.94 and 2^22 0.66-0.87
+//     with outputs up to 256 MB (more: up to 1.25) and tables up to 24 M rows (more: 0.73-1.22); eight levels 2^21 0.66-1.54; eight
+//     features 0.81-2.2; two dimensions 0.69-3.9; one 1.16-3.5.
+extern "C" int th_hash_order_pays(int64_t n_points, int n_dims, int n_feats, int n_levels, int row_bytes, int64_t table_rows, int backward) {
+    if (n_points >= (1ll << 31) || row_bytes < 4) return 0;
+    const int64_t outputs = n_points * n_levels * row_bytes;
+    const bool large = table_rows > (24ll << 20);
+    if (!backward) return n_dims >= 3 && n_feats <= 4 && n_levels >= 16 && n_points >= (1 << 21) && outputs <= (1ll << 28) && !large;
+    if (n_feats == 8 && row_bytes < 32) return 0;
+    if (n_dims >= 3) {
+        if (n_points < (1 << 19) || 12 * n_points < table_rows || (large && row_bytes < 16)) return 0;
+        return n_levels >= 16 || (n_levels >= 8 && n_points >= (1 << 20) && outputs <= (1ll << 28) && table_rows <= (8ll << 20));
+    }
+    if (n_points < (1 << 17)) return 0;
+    if (row_bytes >= 32) return n_levels >= 4;
+    return n_dims == 2 && row_bytes == 16 && n_levels >= 8 && outputs <= (1ll << 28);
 }
 
 extern "C" int64_t th_hash_order_scratch_bytes(int64_t n_points, int n_dims) {

@@ -320,6 +320,11 @@ CoordArgs coord_args(const Tensor &coords, int64_t dims) {
     return a;
 }
 
+bool order_pays(const EncodeCall &c, const Tensor &table, bool backward) {
+    return th_hash_order_pays(c.n, static_cast<int>(c.dims), static_cast<int>(c.feats), c.geo->levels, static_cast<int>(c.feats * table.element_size()),
+                              c.geo->total_rows, backward);
+}
+
 // The batch along a space-filling curve, 16 bytes per point
 Tensor point_order(const EncodeCall &c, const CoordArgs &x, void *stream) {
     Tensor order = empty_like_shape({c.n, 4}, at::kFloat, x.keep.device());
@@ -451,7 +456,7 @@ PyObject *py_hash_encoding(PyObject *, PyObject *const *args, Py_ssize_t n_args)
             out = empty_like_shape(with_last(coords, call.feats * call.geo->levels), table.scalar_type(), table.device());
             const CoordArgs x = coord_args(coords, call.dims);
             void *stream = current_stream();
-            if (th_hash_order_pays(call.n, static_cast<int>(call.dims), static_cast<int>(call.feats * table.element_size()), grad)) order = point_order(call, x, stream);
+            if (order_pays(call, table, grad)) order = point_order(call, x, stream);
             hash_forward(call, x, order, table, out, stream);
         }
         if (grad) {
@@ -1004,7 +1009,7 @@ PyObject *py_hash_encoded_mlp(PyObject *, PyObject *const *args, Py_ssize_t n_ar
             int rc = 0;
             if (separate) {
                 void *stream = current_stream();
-                if (th_hash_order_pays(call.n, static_cast<int>(call.dims), static_cast<int>(call.feats * table.element_size()), grad))
+                if (order_pays(call, table, grad))
                     order = point_order(call, c, stream);
                 hash_forward(call, c, order, table, feats, stream);
                 check(th_mlp_fwd(ptr(feats), d_in, ptr(p.w_in), nullptr, ptr(p.w_hid), nullptr, ptr(p.w_out), nullptr, ptr(out), d_out, call.n, mlp.d_in,
@@ -1154,8 +1159,8 @@ PyObject *py_train_gradients(PyObject *, PyObject *const *args, Py_ssize_t n_arg
     if (!plain(targets) || targets.device() != table.device() || targets.dim() != 2 || targets.size(0) != n || targets.size(1) != d_out ||
         dtype_code(targets.scalar_type()) < 0 || targets.requires_grad())
         TH_NOT_MINE;
-    const bool order_pays = th_hash_order_pays(n, static_cast<int>(call.dims), static_cast<int>(call.feats * table.element_size()), 1);
-    if (f32 && (order_pays || depth >= 4 || call.dims < 2 || (call.feats != 2 && call.feats != 4))) TH_NOT_MINE;
+    const bool ordered = order_pays(call, table, true);
+    if (f32 && (ordered || depth >= 4 || call.dims < 2 || (call.feats != 2 && call.feats != 4))) TH_NOT_MINE;
     Tensor loss;
     {
         NoGil release;
@@ -1183,7 +1188,7 @@ PyObject *py_train_gradients(PyObject *, PyObject *const *args, Py_ssize_t n_arg
             check(th_hash_fwd_cast(ptr(x.keep), x.stride_n, x.stride_d, xcode, table.data_ptr<float>(), ptr(feats), code, d_in, n, D, F, L, g.res, g.rows,
                                    g.offsets, call.primes.v, 1.f, stream),
                   "th_hash_fwd_cast");
-        } else if (order_pays) {
+        } else if (ordered) {
             order = point_order(call, x, stream);
             check(th_hash_fwd_ordered(ptr(order), 1, ptr(table), code, ptr(feats), d_in, n, D, F, L, g.res, g.rows, g.offsets, call.primes.v, 0, L, stream),
                   "th_hash_fwd_ordered");

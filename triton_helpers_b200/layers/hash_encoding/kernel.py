@@ -117,11 +117,11 @@ class _Launch:
         )
 
 
-    def order(self, row_bytes: int, backward: bool) -> Optional[Tensor]:
+    def order(self, feats: int, row_bytes: int, backward: bool) -> Optional[Tensor]:
         r"""The batch along a space-filling curve (16 bytes per point) where that pays, else ``None``."""
         D = self.coords2d.shape[1]
         lib = _lib.lib()
-        if not lib.th_hash_order_pays(self.n, D, row_bytes, int(backward)):
+        if not lib.th_hash_order_pays(self.n, D, feats, len(self.geo.rows), row_bytes, self.geo.total_rows, int(backward)):
             return None
         device = self.coords2d.device
         order = torch.empty(self.n, 4, dtype=torch.float32, device=device)
@@ -260,7 +260,7 @@ class HashEncoding(torch.autograd.Function):
         D_out = D_embed * levels + D_feature
         o = embeddings.new_empty(*coords.shape[:-1], D_out)
         step = divider if divider is not None else levels
-        order = launch.order(D_embed * table.element_size(), any(ctx.needs_input_grad)) if divider is None and bwd_divider is None else None
+        order = launch.order(D_embed, D_embed * table.element_size(), any(ctx.needs_input_grad)) if divider is None and bwd_divider is None else None
         with torch.cuda.device(device):
             stream = _lib.stream_ptr(device)
             if order is not None:

@@ -38,6 +38,7 @@ from . import _lib
 from .layers.fully_fused_mlp import FullyFusedMLP
 from .layers.fully_fused_mlp.kernel import _f32_operand_dtype
 from .layers.hash_encoding import HashEncoding
+from .layers.hash_encoding.helpers import level_geometry
 from .layers.hash_encoding.kernel import _Launch
 from .layers.neural_field.kernel import FieldUnsupported, field_backward, field_forward
 from .optim import FusedAdam, adam_updates
@@ -264,7 +265,7 @@ class NeuralFieldTrainer(nn.Module):
             # (the loss epilogue takes whole 16-byte chunks of targets and gradients: decided before anything is ordered)
             order = None
             if not (fuse_fwd or fuse_bwd or self.backward_passes or self._no_ordered or st.d_out % 8):
-                order = launch.order(st.n_feats * st.flat_grad.element_size(), True)
+                order = launch.order(st.n_feats, st.n_feats * st.flat_grad.element_size(), True)
             if order is not None and (targets.stride(0) % 8 or targets.data_ptr() % 16):
                 targets = targets.clone(memory_format=torch.contiguous_format)
             if order is not None:
@@ -406,7 +407,8 @@ def _float32_native(enc: HashEncoding, mlp: FullyFusedMLP, coords: Tensor) -> bo
         return False
     if d_out > 64 or d_out % 8 or enc.num_levels * feats > 64 or torch.is_autocast_enabled("cuda") or _lib.timing():
         return False
-    return not _lib.lib().th_hash_order_pays(n, d, 4 * feats, 1)
+    rows = level_geometry(enc.num_levels, enc.max_entries_per_level, d, enc.min_res, enc.max_res).total_rows
+    return not _lib.lib().th_hash_order_pays(n, d, feats, enc.num_levels, 4 * feats, rows, 1)
 
 
 class _Float32State:
