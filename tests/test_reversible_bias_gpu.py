@@ -39,3 +39,25 @@ def test_biased_and_preactivation_backward(rows, d_model, hidden, blocks, bias, 
         if want is not None:
             assert nerr(have, want) <= 5 * TIGHT[dtype], f"{name}: {nerr(have, want)}"
     assert _lib.lib().th_rev_tc_status() == 0
+
+
+@pytest.mark.parametrize("half", [16, 32, 48, 64])
+@pytest.mark.parametrize("hidden", [16, 32, 48, 64])
+@pytest.mark.parametrize("activation,dtype", [("relu", torch.float16), ("none", torch.bfloat16)])
+def test_every_width(half, hidden, activation, dtype):
+    # the kernels know the half at compile time; a full tile and a ragged one, two blocks
+    rows, blocks = 200, 2
+    weights, biases = make_params(blocks, half, hidden, False, dtype, seed=half + hidden)
+    g = torch.Generator().manual_seed(hidden)
+    x = torch.randn(rows, 2 * half, generator=g).to(dtype)
+    go = torch.randn(rows, 2 * half, generator=g).to(dtype)
+    wc = to_cuda(weights)
+    y = reversible_mlp_forward(x.cuda(), wc, biases, activation)
+    got = reversible_mlp_backward(y, go.cuda(), wc, biases, activation, reconstruct=True)
+    y_r, _, _, _ = oracle.forward_backward_storage_rounded(x, weights, biases, go, activation)
+    _, dx_r, grads_r, xrec_r = oracle.forward_backward_storage_rounded(x, weights, biases, go, activation, y_saved=y.cpu())
+    assert rows_outside(y, y_r, TIGHT[dtype]) <= 1e-2
+    assert rows_outside(got.dx, dx_r, 2 * TIGHT[dtype]) <= 5e-2
+    assert rows_outside(got.x_reconstructed, xrec_r, 2 * TIGHT[dtype]) <= 5e-2
+    for name, want, have in zip(("dw_f1", "dw_f2", "dw_g1", "dw_g2"), grads_r, got[1:5]):
+        assert nerr(have, want) <= 5 * TIGHT[dtype], f"{name}: {nerr(have, want)}"

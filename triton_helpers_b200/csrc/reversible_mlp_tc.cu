@@ -106,10 +106,17 @@ struct RevWeightMaps {
     CUtensorMap m[4];  // w_f1, w_f2, w_g1, w_g2: [blocks * rows][cols], 16-bit
 };
 
-// FULL: both widths are 64 at compile time.  The kernels then hold one form of every epilogue and of every GEMM's issue.
-template <bool FULL>
+// What a kernel knows of the widths at compile time, and the form of its code that goes with it:
+//   <64, 64>  everything: one form of every epilogue and of every GEMM's issue remains (2^20 rows, eight blocks, forward
+//             0.63 -> 0.50 ms, backward 1.97 -> 1.69)
+//   <h, 0>    the half: the hidden layer's epilogue and issue keep a form per width
+//   <0, 0>    nothing: rolled loops
+// 2^17 rows, eight float16 blocks of 32 -> 32 -> 32, ReLU without biases: <0, 0> forward 78, backward 248 us, <32, 0> 62 and 211;
+// 16 -> 16 -> 16: 66 and 240, 57 and 193; 48 -> 48 -> 48: 88 and 307, 71 and 253.
+template <int HALF, int HID>
 __device__ __forceinline__ RevShape known_widths(RevShape s) {
-    if constexpr (FULL) s.half = s.hid = 64;
+    if constexpr (HALF > 0) s.half = HALF;
+    if constexpr (HID > 0) s.hid = HID;
     return s;
 }
 
@@ -165,12 +172,12 @@ __device__ __forceinline__ void tile_row_to_tmem(unsigned char *tile, const Seat
 
 // This thread's pieces of an fp32 TMEM accumulator -> (optional bias, written back) -> rounded into an
 // operand tile and / or a global row.
-template <typename T, bool BIAS>
+template <typename T, bool BIAS, bool ROLLED>
 __device__ __forceinline__ void stream_epilogue(uint32_t taddr, const Seat &seat, int width, const float *bias,
                                                 unsigned char *tile, T *global_row, bool live) {
     const int n = width / kGroups, first = seat.group * (n / 8);  // this thread's columns / first 8-column piece
     const uint32_t row_addr = (tile ? smem_addr(tile) : 0u) + seat.row * 128, row_swizzle = (seat.row & 7) << 4;
-    for_each_piece(taddr + seat.group * n, n, [&](int u, const uint32_t(&piece)[8]) {
+    for_each_piece<ROLLED>(taddr + seat.group * n, n, [&](int u, const uint32_t(&piece)[8]) {
         uint32_t v[8];
 #pragma unroll
         for (int k = 0; k < 8; ++k) v[k] = piece[k];
@@ -187,11 +194,11 @@ __device__ __forceinline__ void stream_epilogue(uint32_t taddr, const Seat &seat
 }
 
 // The same with the rounded copy going to a 16-bit A operand in tensor memory (4 columns per 16-byte chunk).
-template <typename T, bool BIAS>
+template <typename T, bool BIAS, bool ROLLED>
 __device__ __forceinline__ void stream_epilogue_ta(uint32_t taddr, const Seat &seat, int width, const float *bias, uint32_t a_taddr,
                                                    T *global_row, bool live) {
     const int n = width / kGroups, first = seat.group * (n / 8);
-    for_each_piece(taddr + seat.group * n, n, [&](int u, const uint32_t(&piece)[8]) {
+    for_each_piece<ROLLED>(taddr + seat.group * n, n, [&](int u, const uint32_t(&piece)[8]) {
         uint32_t v[8];
 #pragma unroll
         for (int k = 0; k < 8; ++k) v[k] = piece[k];
@@ -225,11 +232,12 @@ __device__ __forceinline__ void publish_tiles() {
 
 // TA: the two A operands of a branch (the 16-bit copy of its input stream, its hidden activation) live in tensor
 // memory and never touch shared memory; the operand tiles only stage the rows as they arrive.
-template <typename T, int ACT, bool BIAS, bool TA, bool FULL>
+template <typename T, int ACT, bool BIAS, bool TA, int HALF, int HID>
 __global__ void __launch_bounds__(kTcThreads, 2)
 rev_fwd_tc_kernel(const RevShape shape, const RevParams p, const __grid_constant__ RevWeightMaps maps, const int use_tma,
                   const T *__restrict__ x, long long x_stride, T *__restrict__ y, long long y_stride, long long n_rows) {
-    const RevShape s = known_widths<FULL>(shape);
+    constexpr bool kRolled = HALF == 0, kLines = HALF > 0 && HID == 0;
+    const RevShape s = known_widths<HALF, HID>(shape);
     extern __shared__ unsigned char smem_raw[];
     unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     __shared__ uint32_t tmem_holder;
@@ -297,15 +305,15 @@ rev_fwd_tc_kernel(const RevShape shape, const RevParams p, const __grid_constant
                 if (threadIdx.x < 32) {
                     leader = elect_one();
                     tc_fence_after();
-                    if constexpr (TA) issue_gemm_ta(leader, tmem + kFwdHid, tmem + kFwdAU, w1, 32, s.half / 16, idesc_hid, false);
-                    else issue_gemm(leader, tmem + kFwdHid, smem_addr(u_tile), 32, w1, 32, s.half / 16, idesc_hid, false);
+                    if constexpr (TA) issue_gemm_ta<kLines>(leader, tmem + kFwdHid, tmem + kFwdAU, w1, 32, s.half / 16, idesc_hid, false);
+                    else issue_gemm<kLines>(leader, tmem + kFwdHid, smem_addr(u_tile), 32, w1, 32, s.half / 16, idesc_hid, false);
                 }
                 commit_and_wait(leader, bar, phase, &abort_flag);
                 {
                     const int n = s.hid / kGroups, first = seat.group * (n / 8);
                     const uint32_t row_addr = smem_addr(h_tile) + seat.row * 128, row_swizzle = (seat.row & 7) << 4;
                     const float *layer_bias = bias + (2 * branch) * kMaxDim;
-                    for_each_piece(taddr + kFwdHid + seat.group * n, n, [&](int u, const uint32_t(&piece)[8]) {
+                    for_each_piece<kRolled>(taddr + kFwdHid + seat.group * n, n, [&](int u, const uint32_t(&piece)[8]) {
                         const uint4 packed = finish8<T, ACT, BIAS>(piece, layer_bias + 8 * (first + u));
                         if constexpr (TA) tmem_st4(taddr + kFwdAH + 4 * (first + u), packed);
                         else st_shared_16(row_addr + (((first + u) << 4) ^ row_swizzle), packed);
@@ -316,17 +324,17 @@ rev_fwd_tc_kernel(const RevShape shape, const RevParams p, const __grid_constant
                 if (threadIdx.x < 32) {
                     leader = elect_one();
                     tc_fence_after();
-                    if constexpr (TA) issue_gemm_ta(leader, tmem + out_col, tmem + kFwdAH, w2, 32, s.hid / 16, idesc_half, true);
-                    else issue_gemm(leader, tmem + out_col, smem_addr(h_tile), 32, w2, 32, s.hid / 16, idesc_half, true);
+                    if constexpr (TA) issue_gemm_ta<kLines>(leader, tmem + out_col, tmem + kFwdAH, w2, 32, s.hid / 16, idesc_half, true);
+                    else issue_gemm<kLines>(leader, tmem + out_col, smem_addr(h_tile), 32, w2, 32, s.hid / 16, idesc_half, true);
                 }
                 commit_and_wait(leader, bar, phase, &abort_flag);
                 // the updated stream: rounded copy for the next branch, and the output after the last block
                 const bool last = k == s.blocks - 1;
                 if constexpr (TA)
-                    stream_epilogue_ta<T, BIAS>(taddr + out_col, seat, s.half, bias + (2 * branch + 1) * kMaxDim, taddr + kFwdAU,
+                    stream_epilogue_ta<T, BIAS, kRolled>(taddr + out_col, seat, s.half, bias + (2 * branch + 1) * kMaxDim, taddr + kFwdAU,
                                                 last ? y_row + branch * s.half : nullptr, live);
                 else
-                    stream_epilogue<T, BIAS>(taddr + out_col, seat, s.half, bias + (2 * branch + 1) * kMaxDim, u_tile,
+                    stream_epilogue<T, BIAS, kRolled>(taddr + out_col, seat, s.half, bias + (2 * branch + 1) * kMaxDim, u_tile,
                                              last ? y_row + branch * s.half : nullptr, live);
                 if (branch == 1) {  // next block's weights have landed
                     if (!use_tma) async_tile_wait();
@@ -445,14 +453,15 @@ __device__ __forceinline__ void add_tile_column_sums(uint32_t tile, int width, f
     }
 }
 
-template <typename T, int ACT, bool BIAS, bool FULL>
+template <typename T, int ACT, bool BIAS, int HALF, int HID>
 __global__ void __launch_bounds__(kTcThreads + kRevFlushThreads, 1)
 rev_bwd_tc_kernel(const RevShape shape, const RevParams p, const __grid_constant__ RevWeightMaps maps,
                   const __grid_constant__ RevRowMaps row_maps, const int use_tma,
                   const T *__restrict__ y, long long y_stride,
                   const T *__restrict__ go, long long go_stride, T *__restrict__ gx, long long gx_stride,
                   T *__restrict__ x_rec, long long xr_stride, float *__restrict__ workspace, long long n_rows) {
-    const RevShape s = known_widths<FULL>(shape);
+    constexpr bool kRolled = HALF == 0, kLines = HALF > 0 && HID == 0;
+    const RevShape s = known_widths<HALF, HID>(shape);
     extern __shared__ unsigned char smem_raw[];
     unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     __shared__ uint32_t tmem_holder;
@@ -512,8 +521,8 @@ rev_bwd_tc_kernel(const RevShape shape, const RevParams p, const __grid_constant
                         const bool leader = elect_one();
                         tc_fence_after();
                         const uint32_t u_cur = smem_addr(u_tiles + (n & 1u) * kTileBytes);
-                        issue_gemm(leader, tmem + kDW2, dy_cur, 2048, smem_addr(h_tile), 2048, kTileRows / 16, id_dw2, false);
-                        issue_gemm(leader, tmem + kDW1, smem_addr(dz_tile), 2048, u_cur, 2048, kTileRows / 16, id_dw1, false);
+                        issue_gemm<kLines>(leader, tmem + kDW2, dy_cur, 2048, smem_addr(h_tile), 2048, kTileRows / 16, id_dw2, false);
+                        issue_gemm<kLines>(leader, tmem + kDW1, smem_addr(dz_tile), 2048, u_cur, 2048, kTileRows / 16, id_dw1, false);
                         if (leader) mma_commit(wgrad_addr);
                         __syncwarp();
                     }
@@ -619,8 +628,8 @@ rev_bwd_tc_kernel(const RevShape shape, const RevParams p, const __grid_constant
                     if (threadIdx.x < 32) {
                         const bool leader = elect_one();
                         tc_fence_after();
-                        issue_gemm(leader, tmem + kZ, u_cur, 32, w1, 32, s.half / 16, id_z, false);
-                        issue_gemm(leader, tmem + kDH, dy_cur, 32, w2, 2048, s.half / 16, id_dh, false);
+                        issue_gemm<kLines>(leader, tmem + kZ, u_cur, 32, w1, 32, s.half / 16, id_z, false);
+                        issue_gemm<kLines>(leader, tmem + kDH, dy_cur, 32, w2, 2048, s.half / 16, id_dh, false);
                         if (leader) mma_commit(bar);
                         __syncwarp();
                     }
@@ -629,7 +638,7 @@ rev_bwd_tc_kernel(const RevShape shape, const RevParams p, const __grid_constant
                         // flush warps must have summed the previous pass's dz before it is overwritten below
                         const int nh = s.half / kGroups, first_h = seat.group * (nh / 8);
                         const float *bias2 = block_bias + m2 * kMaxDim;
-                        for_each_piece(taddr + out_col + seat.group * nh, nh, [&](int u, const uint32_t(&piece)[8]) {
+                        for_each_piece<kRolled>(taddr + out_col + seat.group * nh, nh, [&](int u, const uint32_t(&piece)[8]) {
                             uint32_t v[8];
 #pragma unroll
                             for (int e = 0; e < 8; ++e) v[e] = __float_as_uint(__uint_as_float(piece[e]) - bias2[8 * (first_h + u) + e]);
@@ -649,7 +658,7 @@ rev_bwd_tc_kernel(const RevShape shape, const RevParams p, const __grid_constant
                         const uint32_t row_off = seat.row * 128, row_swizzle = (seat.row & 7) << 4;
                         const uint32_t h_row = smem_addr(h_tile) + row_off, dz_row = smem_addr(dz_tile) + row_off;
                         const float *bias1 = block_bias + m1 * kMaxDim;
-                        for_each_piece(taddr + kZ + seat.group * nn, nn, [&](int u, const uint32_t(&piece)[8]) {
+                        for_each_piece<kRolled>(taddr + kZ + seat.group * nn, nn, [&](int u, const uint32_t(&piece)[8]) {
                             st_shared_16(h_row + (((first + u) << 4) ^ row_swizzle), finish8<T, ACT, BIAS>(piece, bias1 + 8 * (first + u)));
                         });
                         auto store_dz = [&](int u, uint4 g) {
@@ -674,7 +683,7 @@ rev_bwd_tc_kernel(const RevShape shape, const RevParams p, const __grid_constant
                                 store_dz(u, make_uint4(pack_pair<T>(g[0], g[1]), pack_pair<T>(g[2], g[3]), pack_pair<T>(g[4], g[5]), pack_pair<T>(g[6], g[7])));
                             }
                         } else {
-                            for_each_piece(taddr + kDH + seat.group * nn, nn, [&](int u, const uint32_t(&piece)[8]) {
+                            for_each_piece<kRolled>(taddr + kDH + seat.group * nn, nn, [&](int u, const uint32_t(&piece)[8]) {
                                 uint4 g = finish8<T, TH_ACT_NONE, false>(piece, nullptr);
                                 if constexpr (ACT == TH_ACT_RELU) {
                                     const uint4 h = ld_shared_16(h_row + (((first + u) << 4) ^ row_swizzle));  // this thread's own store above
@@ -694,8 +703,8 @@ rev_bwd_tc_kernel(const RevShape shape, const RevParams p, const __grid_constant
                     if (threadIdx.x < 32) {
                         const bool leader = elect_one();
                         tc_fence_after();
-                        issue_gemm(leader, tmem + out_col, smem_addr(h_tile), 32, w2, 32, s.hid / 16, id_undo, true);
-                        issue_gemm(leader, tmem + in_d_col, smem_addr(dz_tile), 32, w1, 2048, s.hid / 16, id_din, true);
+                        issue_gemm<kLines>(leader, tmem + out_col, smem_addr(h_tile), 32, w2, 32, s.hid / 16, id_undo, true);
+                        issue_gemm<kLines>(leader, tmem + in_d_col, smem_addr(dz_tile), 32, w1, 2048, s.hid / 16, id_din, true);
                         if (leader) mma_commit(bar);
                         if (leader) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(operands_addr) : "memory");
                         __syncwarp();
@@ -703,8 +712,8 @@ rev_bwd_tc_kernel(const RevShape shape, const RevParams p, const __grid_constant
                     main_wait_mma(bar, phase, &abort_flag);
                     // next pass: its input is the stream just reconstructed, its output gradient the one just updated
                     if (!last) {
-                        stream_epilogue<T, false>(taddr + out_col, seat, s.half, nullptr, u_next, nullptr, false);
-                        stream_epilogue<T, false>(taddr + in_d_col, seat, s.half, nullptr, dy_next, nullptr, false);
+                        stream_epilogue<T, false, kRolled>(taddr + out_col, seat, s.half, nullptr, u_next, nullptr, false);
+                        stream_epilogue<T, false, kRolled>(taddr + in_d_col, seat, s.half, nullptr, dy_next, nullptr, false);
                     }
                     if (pass == 1) {  // next block's weights have landed
                         if (!use_tma) async_tile_wait();
@@ -722,7 +731,7 @@ rev_bwd_tc_kernel(const RevShape shape, const RevParams p, const __grid_constant
                     const long long stride = q < 2 ? gx_stride : xr_stride;
                     const uint32_t col = q == 0 ? kD1 : (q == 1 ? kD2 : (q == 2 ? kS1 : kS2));
                     if (base != nullptr)
-                        stream_epilogue<T, false>(taddr + col, seat, s.half, nullptr, nullptr,
+                        stream_epilogue<T, false, kRolled>(taddr + col, seat, s.half, nullptr, nullptr,
                                                   base + (live ? row0 + seat.row : 0) * stride + (q & 1) * s.half, live);
                 }
             }
@@ -816,7 +825,14 @@ int launch_rev_fwd_ta(const RevShape &s, const RevParams &p, const void *x, int6
     const RevTcPlan P = rev_tc_plan(false);
     const int ctas = 2;  // 256 of the 512 TMEM columns each
     const int smem = smem_request(P, ctas);
-    auto kernel = s.half == 64 && s.hid == 64 ? rev_fwd_tc_kernel<T, ACT, BIAS, TA, true> : rev_fwd_tc_kernel<T, ACT, BIAS, TA, false>;
+    auto kernel = rev_fwd_tc_kernel<T, ACT, BIAS, TA, 0, 0>;
+    if constexpr (TA) {
+        if (s.half == 64 && s.hid == 64) kernel = rev_fwd_tc_kernel<T, ACT, BIAS, TA, 64, 64>;
+        else if (s.half == 64) kernel = rev_fwd_tc_kernel<T, ACT, BIAS, TA, 64, 0>;
+        else if (s.half == 48) kernel = rev_fwd_tc_kernel<T, ACT, BIAS, TA, 48, 0>;
+        else if (s.half == 32) kernel = rev_fwd_tc_kernel<T, ACT, BIAS, TA, 32, 0>;
+        else kernel = rev_fwd_tc_kernel<T, ACT, BIAS, TA, 16, 0>;
+    }
     if (int rc = cuda_status(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
                              "cudaFuncSetAttribute(rev_fwd_tc_kernel)")) return rc;
     const long long tiles = (rows + kTileRows - 1) / kTileRows;
@@ -859,7 +875,13 @@ int launch_rev_bwd_t(const RevShape &s, const RevParams &p, const void *y, int64
                      void *const db[4], float *workspace, int n_ctas, int64_t rows, cudaStream_t stream) {
     const RevTcPlan P = rev_tc_plan(true);
     const int smem = smem_request(P, 1);  // all 512 TMEM columns: one CTA per SM
-    auto kernel = s.half == 64 && s.hid == 64 ? rev_bwd_tc_kernel<T, ACT, BIAS, true> : rev_bwd_tc_kernel<T, ACT, BIAS, false>;
+    auto kernel = s.half == 64 && s.hid == 64 ? rev_bwd_tc_kernel<T, ACT, BIAS, 64, 64> : rev_bwd_tc_kernel<T, ACT, BIAS, 0, 0>;
+    if constexpr (!BIAS && (ACT == TH_ACT_RELU || ACT == TH_ACT_NONE)) {
+        if (s.half == 64 && s.hid != 64) kernel = rev_bwd_tc_kernel<T, ACT, BIAS, 64, 0>;
+        else if (s.half == 48) kernel = rev_bwd_tc_kernel<T, ACT, BIAS, 48, 0>;
+        else if (s.half == 32) kernel = rev_bwd_tc_kernel<T, ACT, BIAS, 32, 0>;
+        else if (s.half == 16) kernel = rev_bwd_tc_kernel<T, ACT, BIAS, 16, 0>;
+    }
     if (int rc = cuda_status(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
                              "cudaFuncSetAttribute(rev_bwd_tc_kernel)")) return rc;
     RevWeightMaps maps;

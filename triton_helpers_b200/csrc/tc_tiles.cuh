@@ -281,17 +281,23 @@ __device__ __forceinline__ void for_each_piece_n(uint32_t taddr, Fn fn) {
         fn(u, piece);
     }
 }
-// the same for a run-time n in {8, 16, 24, 32} (warp uniform; padded widths are multiples of 16 and
-// two threads share a row)
-template <typename Fn>
+// The same for an n in {8, 16, 24, 32} (warp uniform; padded widths are multiples of 16 and two threads share a row).
+// ROLLED: two forms only, the second rolled: every call is inlined several times in kernels that live on their instruction cache
+// (reversible forward, 2^20 rows, run-time widths: 0.655 -> 0.631 ms).  Otherwise a form for each n, of which one remains
+// where n is known at compile time.
+template <bool ROLLED = true, typename Fn>
 __device__ __forceinline__ void for_each_piece(uint32_t taddr, int n, Fn fn) {
-    // two forms only, the second rolled: every call is inlined several times in kernels that live on their instruction cache
-    // (reversible forward, 2^20 rows: 0.655 -> 0.631 ms)
     if (n == 32) {
         for_each_piece_n<32>(taddr, fn);
-    } else {
+    } else if constexpr (ROLLED) {
 #pragma unroll 1
         for (int u = 0; u < n / 8; ++u) for_each_piece_n<8>(taddr + 8 * u, [&](int, const uint32_t(&piece)[8]) { fn(u, piece); });
+    } else if (n == 24) {
+        for_each_piece_n<24>(taddr, fn);
+    } else if (n == 16) {
+        for_each_piece_n<16>(taddr, fn);
+    } else {
+        for_each_piece_n<8>(taddr, fn);
     }
 }
 
@@ -468,7 +474,8 @@ __device__ __forceinline__ void issue_steps(uint32_t tmem_d, uint32_t a_low, uin
 
 // Issue the K-loop of one GEMM; called by all of warp 0, `leader` marks the elected lane.
 // a_step / b_step: bytes the operand's start address advances per 16-deep K step (32 for a K-major
-// operand, 2048 for an MN-major one).
+// operand, 2048 for an MN-major one).  LINES: one and three steps, and the eight of a weight gradient, in straight lines as well.
+template <bool LINES = false>
 __device__ __forceinline__ void issue_gemm(bool leader, uint32_t tmem_d, uint32_t a_addr, uint32_t a_step, uint32_t b_addr,
                                            uint32_t b_step, int k_steps, uint32_t idesc, bool accumulate) {
     const uint32_t a_low = desc_low(a_addr), b_low = desc_low(b_addr), acc = accumulate ? 1u : 0u;
@@ -479,6 +486,12 @@ __device__ __forceinline__ void issue_gemm(bool leader, uint32_t tmem_d, uint32_
             issue_steps<4>(tmem_d, a_low, a_step, b_low, b_step, idesc, acc);
         } else if (k_steps == 2) {
             issue_steps<2>(tmem_d, a_low, a_step, b_low, b_step, idesc, acc);
+        } else if (LINES && k_steps == 3) {
+            issue_steps<3>(tmem_d, a_low, a_step, b_low, b_step, idesc, acc);
+        } else if (LINES && k_steps == 1) {
+            issue_steps<1>(tmem_d, a_low, a_step, b_low, b_step, idesc, acc);
+        } else if (LINES && k_steps == 8) {
+            issue_steps<8>(tmem_d, a_low, a_step, b_low, b_step, idesc, acc);
         } else {
             for (int k = 0; k < k_steps; ++k) issue_steps<1>(tmem_d, a_low + k * a_step, 0, b_low + k * b_step, 0, idesc, k > 0 ? 1u : acc);
         }
@@ -501,6 +514,7 @@ __device__ __forceinline__ void issue_steps_ta(uint32_t tmem_d, uint32_t tmem_a,
     for (int k = 0; k < N; ++k) mma_f16_ta(tmem_d, tmem_a + 8 * k, smem_desc(b_low + k * b_step), idesc, k > 0 ? 1u : acc);
 }
 
+template <bool LINES = false>
 __device__ __forceinline__ void issue_gemm_ta(bool leader, uint32_t tmem_d, uint32_t tmem_a, uint32_t b_addr, uint32_t b_step, int k_steps,
                                               uint32_t idesc, bool accumulate) {
     const uint32_t b_low = desc_low(b_addr), acc = accumulate ? 1u : 0u;
@@ -508,6 +522,12 @@ __device__ __forceinline__ void issue_gemm_ta(bool leader, uint32_t tmem_d, uint
     if (leader) {
         if (k_steps == 4) {
             issue_steps_ta<4>(tmem_d, tmem_a, b_low, b_step, idesc, acc);
+        } else if (LINES && k_steps == 3) {
+            issue_steps_ta<3>(tmem_d, tmem_a, b_low, b_step, idesc, acc);
+        } else if (LINES && k_steps == 2) {
+            issue_steps_ta<2>(tmem_d, tmem_a, b_low, b_step, idesc, acc);
+        } else if (LINES && k_steps == 1) {
+            issue_steps_ta<1>(tmem_d, tmem_a, b_low, b_step, idesc, acc);
         } else {
             for (int k = 0; k < k_steps; ++k) issue_steps_ta<1>(tmem_d, tmem_a + 8 * k, b_low + k * b_step, 0, idesc, k > 0 ? 1u : acc);
         }
