@@ -329,3 +329,17 @@ def test_a_replaced_network_is_not_trained_by_the_old_optimizer():
     trainer.optimizer = type(trainer.optimizer)(trainer.parameters(), lr=1e-3)
     trainer.step(*batch())
     assert not any(torch.equal(a, b) for a, b in zip(before, other.parameters()))
+
+
+@pytest.mark.parametrize("n,d,hidden,depth,fused", [(2**19 + 3, 2, 32, 1, True), (2**18 + 3, 3, 16, 2, True), (2**19 - 1, 2, 32, 1, False), (2**18 + 3, 3, 32, 2, False)])
+def test_sixty_four_features_and_a_small_network(n, d, hidden, depth, fused):
+    # forward + backward in the fused kernels from this size on; same gradients as the two layers
+    table = (torch.randn(level_geometry(16, 2**12, d, 16, 128).total_rows, 4, device="cuda") * 0.1).half().requires_grad_(True)
+    mlp = FullyFusedMLP(64, hidden, 8, depth, bias=False).cuda().half()
+    x, go = torch.rand(n, d, device="cuda"), torch.randn(n, 8, device="cuda").half() * 1e-3
+    leaves = [table, mlp.w_in, mlp.w_out]
+    y = hash_encoded_mlp(x, table, mlp.w_in, mlp.w_out, mlp.w_hid, None, 2**12, 16, 128, 16)
+    assert isinstance(y.grad_fn, torch.autograd.function.BackwardCFunction) == fused
+    got = [y.detach(), *torch.autograd.grad(y, leaves, go)]
+    z = mlp(hash_encoding(x, table, None, None, 2**12, 16, 128, 16).unsqueeze(0)).squeeze(0)
+    close(got, [z.detach(), *torch.autograd.grad(z, leaves, go)], 1e-2)

@@ -897,10 +897,19 @@ PyObject *py_reversible_mlp(PyObject *, PyObject *const *args, Py_ssize_t n_args
 
 // ---- hash encoding + MLP --------------------------------------------------------------------------------------
 //
-// Up to six layers before the output (what the MLP backward holds at any width) the encoding's kernels and the MLP's run one after the other: each of them fills an SM by
-// itself (the gathers and reductions want all its warps, the MLP its shared memory), large batches can be ordered in
-// space, and together they are faster than the kernels that fuse the two (B200, 200 003 points in two dimensions,
-// forward + backward, 192 -> 150 us; 2^21 points in three, forward 0.72 -> 0.47 ms), which deeper networks still take.
+// Up to six layers before the output (what the MLP backward holds at any width) the encoding's kernels and the MLP's run one after
+// the other: each of them fills an SM by itself (the gathers and reductions want all its warps, the MLP its shared memory),
+// large batches can be ordered in space, and together they are faster than the kernels that fuse the two (B200, 200 003 points in
+// two dimensions, forward + backward, 192 -> 150 us; 2^21 points in three, forward 0.72 -> 0.47 ms).  Deeper networks take the fused
+// kernels: without a gradient from here, with one from Python, whose FieldUnsupported says when the backward does not hold them.
+
+// Unordered batches large enough to hide the host path, with 64 features and next to no network: the separate kernels write and read
+// the features' gradient, 128 bytes a point, for a backward pass that takes no longer fused.  Forward + backward, separate over
+// fused: 64 features, two dimensions, 2^19 .. 2^21 points, one layer 0.95-1.09, two layers of 16 1.02-1.08 (of 32 0.95-1.03,
+// of 64 0.97-1.00), 2^18 0.85-0.97; three dimensions 2^18 0.96-1.05, 2^17 0.68-0.84; 32 features 0.72-1.03.
+bool fused_pays(const EncodeCall &c, const MlpCall &m, bool ordered) {
+    return !ordered && m.d_in == 64 && (m.depth == 1 || (m.depth == 2 && m.hidden == 16)) && c.n >= (c.dims == 2 ? 1 << 19 : 1 << 18);
+}
 
 struct FieldNode : public Node {
     EncodeCall call;
@@ -984,7 +993,7 @@ PyObject *py_hash_encoded_mlp(PyObject *, PyObject *const *args, Py_ssize_t n_ar
                           d_in % 16 == 0 && d_in <= 64 && (mlp.act == TH_ACT_RELU || mlp.act == TH_ACT_NONE) &&
                           (hidden == 16 || hidden == 32 || hidden == 64) && d_out >= 1 && d_out <= 64;
     const bool grad = torch::autograd::compute_requires_grad(table, p.w_in, p.w_out, p.w_hid);
-    if (grad && !separate) TH_NOT_MINE;  // the fused backward may turn out not to hold the network: Python's FieldUnsupported again
+    if (grad && (!separate || fused_pays(call, mlp, order_pays(call, table, true)))) TH_NOT_MINE;
     Tensor out, feats, order;
     {
         NoGil release;
