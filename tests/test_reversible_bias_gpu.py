@@ -7,7 +7,7 @@ from oracle import reversible_mlp as oracle
 from test_reversible_mlp_gpu import TIGHT, make_params, nerr, rows_outside, to_cuda
 
 from triton_helpers_b200 import _lib
-from triton_helpers_b200.layers.reversible_mlp import reversible_mlp_backward, reversible_mlp_forward
+from triton_helpers_b200.layers.reversible_mlp import ReversibleMLP, reversible_mlp_backward, reversible_mlp_forward
 
 pytestmark = pytest.mark.gpu
 
@@ -61,3 +61,48 @@ def test_every_width(half, hidden, activation, dtype):
     assert rows_outside(got.x_reconstructed, xrec_r, 2 * TIGHT[dtype]) <= 5e-2
     for name, want, have in zip(("dw_f1", "dw_f2", "dw_g1", "dw_g2"), grads_r, got[1:5]):
         assert nerr(have, want) <= 5 * TIGHT[dtype], f"{name}: {nerr(have, want)}"
+
+
+def float64_gradients(x, params, go, half, hidden, blocks):
+    r"""Gradients of the biased ReLU stack by autograd in float64: ``[dx, dw_f1, dw_f2, dw_g1, dw_g2, db_f1, db_f2, db_g1, db_g2]``."""
+    x, *params = (t.detach().double().requires_grad_(True) for t in (x, *params))
+    w_f1, w_f2, w_g1, w_g2, b_f1, b_f2, b_g1, b_g2 = params
+
+    def branch(u, w1, b1, w2, b2, k):
+        h = torch.relu(u @ w1[k * hidden : (k + 1) * hidden].t() + b1[k])
+        return h @ w2[k * half : (k + 1) * half].t() + b2[k]
+
+    x1, x2 = x[:, :half], x[:, half:]
+    for k in range(blocks):
+        x1 = x1 + branch(x2, w_f1, b_f1, w_f2, b_f2, k)
+        x2 = x2 + branch(x1, w_g1, b_g1, w_g2, b_g2, k)
+    return torch.autograd.grad(torch.cat([x1, x2], -1), [x, *params], go.double())
+
+
+@pytest.mark.parametrize(
+    "dtype,rows,blocks,dx,dw,db",
+    [
+        # relative errors against float64 of the mma.sync backward, which took biased stacks before: mean of four seeds
+        (torch.float16, 128, 8, 0.00920, 0.01042, 0.01029),
+        (torch.float16, 1000, 10, 0.01274, 0.01361, 0.01398),
+        (torch.float16, 4099, 8, 0.01046, 0.01218, 0.01242),
+        (torch.bfloat16, 128, 10, 0.03707, 0.04045, 0.04113),
+        (torch.bfloat16, 1000, 8, 0.03007, 0.03535, 0.03714),
+        (torch.bfloat16, 4099, 10, 0.03517, 0.03881, 0.04028),
+    ],
+)
+def test_deep_biased_stacks_are_as_exact_as_on_mma_sync(dtype, rows, blocks, dx, dw, db):
+    # what remains is where ReLUs within a rounding of zero switch, which depends on the last bits: over 24 such combinations the ratio
+    # of the two kernels' errors is 0.995 +- 0.006 (float16) and 1.0004 +- 0.002
+    errors = torch.zeros(3, dtype=torch.float64)
+    for seed in range(4):
+        torch.manual_seed(seed)
+        layer = ReversibleMLP(128, blocks, 64, "relu", bias=True).cuda().to(dtype)
+        x = torch.randn(rows, 128, device="cuda").to(dtype).requires_grad_(True)
+        go = torch.randn(rows, 128, device="cuda").to(dtype)
+        params = [getattr(layer, n) for n in ("w_f1", "w_f2", "w_g1", "w_g2", "b_f1", "b_f2", "b_g1", "b_g2")]
+        got = torch.autograd.grad(layer(x), [x, *params], go)
+        want = float64_gradients(x, params, go, 64, 64, blocks)
+        e = torch.tensor([float((g.double() - w).norm() / w.norm()) for g, w in zip(got, want)], dtype=torch.float64)
+        errors += torch.stack([e[0], e[1:5].mean(), e[5:].mean()]) / 4
+    assert (errors <= 1.05 * torch.tensor([dx, dw, db], dtype=torch.float64)).all(), errors
