@@ -458,6 +458,7 @@ slots_mlp_bwd_tc_kernel(const MlpShape s, const MlpParams p, const __grid_consta
             }
         }
     }
+    if (tb.abort_flag && use_tma && threadIdx.x == 0) drain_copies(&tb.weights_bar, 1);
     tc_fence_before();
     __syncthreads();
     if (is_wgrad_warp)

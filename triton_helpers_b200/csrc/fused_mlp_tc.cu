@@ -364,6 +364,10 @@ mlp_fwd_pipe_kernel(const MlpShape shape, const MlpParams p, const __grid_consta
     }
 
     // ---- teardown ----
+    if (abort_flag && (threadIdx.x & 127) == 0) {
+        drain_copies(bars.in_full[slot], 2);
+        if (threadIdx.x == 0) drain_copies(&wbar, 1);
+    }
     tc_fence_before();
     __syncthreads();
     if (warp == 0)

@@ -344,7 +344,10 @@ rev_fwd_tc_kernel(const RevShape shape, const RevParams p, const __grid_constant
             }
         }
     }
-    if (abort_flag) g_tc_status = 1;
+    if (abort_flag) {
+        g_tc_status = 1;
+        if (use_tma && threadIdx.x == 64) drain_copies(ring_bars, 2);
+    }
     cta_teardown(tmem, P.tmem_cols);
 }
 
@@ -737,7 +740,13 @@ rev_bwd_tc_kernel(const RevShape shape, const RevParams p, const __grid_constant
             }
         }
     }
-    if (abort_flag) g_tc_status = 1;
+    if (abort_flag) {
+        g_tc_status = 1;
+        if (use_tma && threadIdx.x == 64) {
+            drain_copies(ring_bars, 2);
+            drain_copies(&rows_bar, 1);
+        }
+    }
     cta_teardown(tmem, P.tmem_cols);
 }
 

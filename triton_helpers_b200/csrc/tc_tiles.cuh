@@ -96,6 +96,22 @@ __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity) {
     return done != 0;
 }
 
+// On the way out after a wait gave up: boxes this CTA asked for may still be on their way into its shared memory, so one thread
+// waits (bounded) for them.  It does not know which phase a barrier is in: one of the two waits ends with the phase that is
+// open, the other one runs out or finds its phase over.
+constexpr int kDrainPolls = 1 << 16;
+__device__ __noinline__ void drain_copies(const unsigned long long *bars, int count) {
+    for (int b = 0; b < 2 * count; ++b) {
+        uint32_t done = 0;
+        for (int poll = 0; poll < kDrainPolls && !done; ++poll)
+            asm volatile(
+                "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
+                : "=r"(done)
+                : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(bars + b / 2))), "r"(static_cast<uint32_t>(b & 1))
+                : "memory");
+    }
+}
+
 // CTA-wide wait for the MMAs committed to `mbar`: only warp 0 polls the mbarrier (bounded); the other
 // warps park at the CTA barrier, which costs no issue slots while they wait.  Returns false (for
 // every thread alike) when the wait ran out; `abort_flag` lives in shared memory.
