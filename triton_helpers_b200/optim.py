@@ -14,6 +14,7 @@ from typing import Dict, Iterable, Optional, Tuple
 
 import torch
 from torch import Tensor
+from torch.optim.optimizer import _global_optimizer_post_hooks, _global_optimizer_pre_hooks
 
 from . import _lib
 
@@ -86,6 +87,11 @@ class FusedAdam(torch.optim.Optimizer):
         for group in self.param_groups:
             live = [p for p in group["params"] if p.grad is not None]
             self.update(group, live, [p.grad for p in live], [grad_scale] * len(live), [zero_grad] * len(live))
+
+    def watched(self) -> bool:
+        r"""Whether something runs with, or counts, calls of ``step``: hooks of this optimizer or of every optimizer, a scheduler."""
+        hooks = (self._optimizer_step_pre_hooks, self._optimizer_step_post_hooks, _global_optimizer_pre_hooks, _global_optimizer_post_hooks)
+        return any(hooks) or "step" in self.__dict__
 
     @torch.no_grad()
     def update(self, group, params, grads, grad_scales, zero_grads) -> None:

@@ -181,7 +181,7 @@ class NeuralFieldTrainer(nn.Module):
 
     def _step_float32(self, coords: Tensor, targets: Tensor) -> Optional[Tensor]:
         r"""The same step without an autograd graph: forward and backward in one native call on kept buffers, then the
-        optimizer's own step.  ``None`` where the graph has to be built: hooks of modules or parameters, anomaly detection,
+        optimizer's step.  ``None`` where the graph has to be built: hooks of modules or parameters, anomaly detection,
         frozen parameters, subclasses of the layers, or a call the native path does not take."""
         enc, mlp = self.encoding, self.mlp
         if type(enc) is not HashEncoding or type(mlp) is not FullyFusedMLP or len(self.optimizer.param_groups) != 1 or coords.ndim != 2:
@@ -212,17 +212,20 @@ class NeuralFieldTrainer(nn.Module):
         # d(mean over the batch)/d pred = 2 (pred - target) / (N * C); Adam clears the table gradient as it consumes it
         adam_scale = 2.0 / (coords.shape[0] * st.d_out * scale)
         try:
-            for p, g in zip(params, grads):
-                p.grad = g
-            self.optimizer.step(grad_scale=adam_scale, zero_grad=True)  # the public step: its hooks, and schedulers that watch it
-            if enc.embeddings.grad is not st.table_grad:
-                st.table_grad.zero_()  # a hook put another gradient in its place
+            if self.optimizer.watched():  # by step hooks or a scheduler: the public step, on the parameters' grad
+                for p, g in zip(params, grads):
+                    p.grad = g
+                self.optimizer.step(grad_scale=adam_scale, zero_grad=True)
+                if enc.embeddings.grad is not st.table_grad:
+                    st.table_grad.zero_()  # a hook put another gradient in its place
+                for p in params:
+                    p.grad = None
+            else:
+                zero = [True] + [False] * (len(params) - 1)
+                self.optimizer.update(self.optimizer.param_groups[0], params, grads, [adam_scale] * len(params), zero)
         except BaseException:
             self._state = None  # its table gradient may not be zero
             raise
-        finally:
-            for p in params:
-                p.grad = None
         return loss
 
     # ---- direct mode (one 16-bit dtype) ------------------------------------------------------------
@@ -407,6 +410,8 @@ def _float32_native(enc: HashEncoding, mlp: FullyFusedMLP, coords: Tensor) -> bo
         return False
     if d_out > 64 or d_out % 8 or enc.num_levels * feats > 64 or torch.is_autocast_enabled("cuda") or _lib.timing():
         return False
+    if n < 2**17:  # no batch below is ordered, whatever its form
+        return True
     rows = level_geometry(enc.num_levels, enc.max_entries_per_level, d, enc.min_res, enc.max_res).total_rows
     return not _lib.lib().th_hash_order_pays(n, d, feats, enc.num_levels, 4 * feats, rows, 1)
 
@@ -418,8 +423,8 @@ class _Float32State:
     @staticmethod
     def layout(enc: HashEncoding, mlp: FullyFusedMLP) -> tuple:
         r"""What the buffers depend on."""
-        tensors = (enc.embeddings, mlp.w_in, mlp.b_in, mlp.w_hid, mlp.b_hid, mlp.w_out, mlp.b_out)
-        return (enc.embeddings.device, *(None if t is None else (t.dtype, t.shape) for t in tensors))
+        table, hidden = enc.embeddings, mlp.w_hid
+        return table.device, table.dtype, table.shape, mlp.w_in.shape, None if hidden is None else hidden.shape, mlp.w_out.shape, mlp.b_in is None
 
     def __init__(self, enc: HashEncoding, mlp: FullyFusedMLP):
         self.key = self.layout(enc, mlp)
