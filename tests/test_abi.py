@@ -66,6 +66,15 @@ def test_argument_errors_are_reported_without_touching_a_gpu(library):
     assert rc == -1 and b"level range" in library.th_last_error_string()
 
 
+def test_fused_forward_refuses_rows_off_their_size(library):
+    # four 16-bit features are one 8-byte load: a table 4 bytes off is refused before anything is launched
+    res, rows, offs = _lib.i32_array([16, 32, 64, 128]), _lib.i64_array([17**3, 2**14, 2**14, 2**14]), _lib.i64_array([0, 4913, 21297, 37681])
+    primes, aligned = _lib.i64_array([1, 2654435761, 805459861]), 1 << 20
+    rc = library.th_field_fwd(aligned, 3, 1, 0, aligned + 4, 3, 4, 4, res, rows, offs, primes, 1.0, aligned, None, None, None, aligned, None, 64, 16, 1, 1,
+                              None, 16, aligned, 16, None, 16, None, 16, None, 1.0, 100, 1, None)  # fmt: skip
+    assert rc == -3 and b"aligned" in library.th_last_error_string()
+
+
 @pytest.mark.parametrize(
     "n,dims,feats,levels,row_bytes,rows,backward,ordered",
     [

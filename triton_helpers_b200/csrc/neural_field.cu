@@ -928,7 +928,7 @@ extern "C" int th_field_fwd(const void *coords_dev, int64_t coord_stride_n, int6
     if (target_dev && (d_out % 8 != 0 || !rows_vector_ok(target_dev, target_stride, d_out) || !rows_vector_ok(grad_dev, grad_stride, d_out) ||
                        (out_dev && !rows_vector_ok(out_dev, out_stride, d_out))))
         return fail(TH_ERR_UNSUPPORTED, "fused loss needs d_out a multiple of 8 and 16-byte aligned prediction / target / gradient rows");
-    if (!aligned_to(table_dev, 4)) return fail(TH_ERR_ALIGNMENT, "table rows must be aligned to their size");
+    if (!aligned_to(table_dev, n_feats * 2)) return fail(TH_ERR_ALIGNMENT, "table rows must be aligned to their size");  // a row is one load
     const MseArgs mse{target_dev, target_stride, grad_dev, grad_stride, loss_sum_dev, grad_scale, nullptr, 1.f, 0};
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     int rc = kTcNotApplicable;
