@@ -84,7 +84,10 @@ def test_fused_forward_refuses_rows_off_their_size(library):
         (2**19, 3, 2, 16, 4, 20_000_000, 1, 0),  # more than twelve rows a point
         (2**22, 3, 4, 16, 16, 42_000_000, 1, 1),
         (2**22, 3, 2, 16, 4, 42_000_000, 1, 0),
-        (2**21, 3, 8, 16, 16, 10_000, 1, 0),
+        (2**21, 3, 8, 16, 16, 6_000_000, 1, 1),
+        (2**21, 3, 8, 16, 16, 20_000_000, 1, 0),
+        (2**20, 2, 8, 16, 16, 10_000, 1, 1),
+        (2**20, 1, 8, 16, 16, 10_000, 1, 0),
         (2**21, 3, 1, 16, 2, 10_000, 1, 0),
         (2**20, 3, 2, 8, 4, 10_000, 1, 1),
         (2**20 - 1, 3, 2, 8, 4, 10_000, 1, 0),
@@ -95,7 +98,9 @@ def test_fused_forward_refuses_rows_off_their_size(library):
         (2**19, 1, 4, 16, 16, 10_000, 1, 0),
         (2**21, 3, 2, 16, 4, 6_000_000, 0, 1),
         (2**21 - 1, 3, 2, 16, 4, 6_000_000, 0, 0),
-        (2**21, 3, 4, 16, 16, 6_000_000, 0, 0),  # outputs past 256 MB
+        (2**20, 3, 4, 16, 16, 6_000_000, 0, 1),
+        (2**20 - 1, 3, 4, 16, 16, 6_000_000, 0, 0),
+        (2**21 + 1, 3, 4, 16, 16, 6_000_000, 0, 0),  # outputs past 512 MB
         (2**21, 2, 4, 16, 16, 10_000, 0, 0),
         (2**31, 3, 2, 16, 4, 10_000, 1, 0),
     ],

@@ -516,26 +516,27 @@ using namespace th;
 
 // Where the order pays: time with it, sorting included, over time without (B200; 2, 4, 8 or 16 levels, tables of 2^14 .. 2^22 rows per
 // level, finest grids of 512 .. 4096, 1 .. 8 features of 2 or 4 bytes, points uniform or in eight clusters, which the host cannot tell
-// apart).  A form is ordered where none of its points is more than a run's spread above 1:
+// apart).  A form is ordered where none of these is more than a few hundredths above 1:
 //   forward + backward, three dimensions, 16 levels: 2^19 0.40-0.99, 2^20 0.40-0.96, 2^21 0.41-0.97, 2^23 0.78-1.01; eight levels share
 //     the cost of sorting: 2^19 0.40-1.04, 2^20 0.45-1.01, 2^21 0.46-0.94; four: 2^19 0.50-1.35, 2^21 0.42-1.16.  Left out: tables with
 //     more than twelve rows a point (0.42-1.24), past 24 M rows with rows below 16 bytes (2^22 0.98-1.05), past 8 M rows with
-//     eight levels (2^21 up to 1.13), rows of 8 x 16 bit (0.54-1.16) and of one 16-bit element (single-element atomics, 0.25-1.3).
+//     eight levels (2^21 up to 1.13) or rows of 8 x 16 bit (up to 1.05; less 0.41-1.00), rows of one 16-bit element (single-element
+//     atomics, 0.25-1.3).
 //   two dimensions, 4 x float32, 16 levels: 2^16 0.99, 2^17 0.63-0.91, 2^19 0.62-0.95, 2^20 0.66-1.00, 2^21 0.78-1.14 (the ordered
 //     forward writes whole rows in random order, and loses once all of them are past twice the L2); eight: 2^17 0.75-0.99, 2^20
-//     0.65-0.93; four: up to 1.14.  8 x float32 in one or two: 16 levels 2^17 0.33-0.86, 2^21 0.62-0.95, four 2^17 0.55-0.98, two up to
-//     1.24.  Narrower rows: two dimensions 0.80-1.35, one 0.74-1.94.
-//   forward alone, three dimensions, 16 levels, up to four features: 2^19 0.65-1.35, 2^20 0.59-1.12, 2^21 0.55-0.94 and 2^22 0.66-0.87
-//     with outputs up to 256 MB (more: up to 1.25) and tables up to 24 M rows (more: 0.73-1.22); eight levels 2^21 0.66-1.54; eight
-//     features 0.81-2.2; two dimensions 0.69-3.9; one 1.16-3.5.
+//     0.65-0.93; four: up to 1.14; 8 x 16 bit 0.56-1.02, 2^21 up to 1.05, one dimension up to 1.16.  8 x float32 in one or two: 16 levels
+//     2^17 0.33-0.86, 2^21 0.62-0.95, four 2^17 0.55-0.98, two up to 1.24.  Narrower rows: two dimensions 0.80-1.35, one 0.74-1.94.
+//   forward alone, three dimensions, 16 levels, up to four features, outputs up to 512 MB (more: up to 1.25), tables up to 24 M rows
+//     (more: 0.73-1.22): rows of 8 and 16 bytes 2^19 0.65-1.15, 2^20 0.59-1.04, 2^21 0.55-1.03; of 4 bytes 2^20 0.62-1.12, 2^21
+//     0.55-0.94, 2^23 0.77-0.91; eight levels 2^21 0.66-1.54; eight features 0.81-2.2; two dimensions 0.69-3.9; one 1.16-3.5.
 extern "C" int th_hash_order_pays(int64_t n_points, int n_dims, int n_feats, int n_levels, int row_bytes, int64_t table_rows, int backward) {
     if (n_points >= (1ll << 31) || row_bytes < 4) return 0;
     const int64_t outputs = n_points * n_levels * row_bytes;
     const bool large = table_rows > (24ll << 20);
-    if (!backward) return n_dims >= 3 && n_feats <= 4 && n_levels >= 16 && n_points >= (1 << 21) && outputs <= (1ll << 28) && !large;
-    if (n_feats == 8 && row_bytes < 32) return 0;
+    if (!backward) return n_dims >= 3 && n_feats <= 4 && n_levels >= 16 && n_points >= (row_bytes >= 8 ? 1 << 20 : 1 << 21) && outputs <= (1ll << 29) && !large;
     if (n_dims >= 3) {
         if (n_points < (1 << 19) || 12 * n_points < table_rows || (large && row_bytes < 16)) return 0;
+        if (n_feats == 8 && row_bytes < 32 && table_rows > (8ll << 20)) return 0;
         return n_levels >= 16 || (n_levels >= 8 && n_points >= (1 << 20) && outputs <= (1ll << 28) && table_rows <= (8ll << 20));
     }
     if (n_points < (1 << 17)) return 0;

@@ -911,6 +911,13 @@ bool fused_pays(const EncodeCall &c, const MlpCall &m, bool ordered) {
     return !ordered && m.d_in == 64 && (m.depth == 1 || (m.depth == 2 && m.hidden == 16)) && c.n >= (c.dims == 2 ? 1 << 19 : 1 << 18);
 }
 
+// Forward alone, three dimensions, 16 levels, 64 -> 16 -> 16, time over the fused kernels' (tables of 2^14 .. 2^21 rows per level): from
+// 2^20 points the order is worth it next to an MLP for 4-byte rows too (uniform points 0.68-0.88, clustered 0.91-1.03; without it
+// 0.90-0.96 and 0.89-1.10).  Unordered batches of 2^19 points with 64 features stay fused (separate: 0.79-1.04 and 1.02-1.14).
+bool field_ordered(const EncodeCall &c, const Tensor &table, bool grad) {
+    return order_pays(c, table, grad) || (!grad && c.geo->levels >= 16 && c.n >= 1 << 20 && order_pays(c, table, true));
+}
+
 struct FieldNode : public Node {
     EncodeCall call;
     MlpCall mlp;
@@ -989,11 +996,13 @@ PyObject *py_hash_encoded_mlp(PyObject *, PyObject *const *args, Py_ssize_t n_ar
     mlp.depth = static_cast<int>(depth);
     // what the fused kernels cover: anything else is Python's FieldUnsupported
     static const bool legacy = getenv("TH_MLP_LEGACY") && getenv("TH_MLP_LEGACY")[0] == '1';
-    const bool separate = !legacy && depth <= 6 && (call.dims == 2 || call.dims == 3) && (call.feats == 2 || call.feats == 4) &&
+    bool separate = !legacy && depth <= 6 && (call.dims == 2 || call.dims == 3) && (call.feats == 2 || call.feats == 4) &&
                           d_in % 16 == 0 && d_in <= 64 && (mlp.act == TH_ACT_RELU || mlp.act == TH_ACT_NONE) &&
                           (hidden == 16 || hidden == 32 || hidden == 64) && d_out >= 1 && d_out <= 64;
     const bool grad = torch::autograd::compute_requires_grad(table, p.w_in, p.w_out, p.w_hid);
-    if (grad && (!separate || fused_pays(call, mlp, order_pays(call, table, true)))) TH_NOT_MINE;
+    const bool ordered = separate && field_ordered(call, table, grad);
+    if (grad && (!separate || fused_pays(call, mlp, ordered))) TH_NOT_MINE;
+    if (!grad && separate && !ordered && d_in == 64 && call.dims == 3 && call.n >= 1 << 19) separate = false;
     Tensor out, feats, order;
     {
         NoGil release;
@@ -1018,8 +1027,7 @@ PyObject *py_hash_encoded_mlp(PyObject *, PyObject *const *args, Py_ssize_t n_ar
             int rc = 0;
             if (separate) {
                 void *stream = current_stream();
-                if (order_pays(call, table, grad))
-                    order = point_order(call, c, stream);
+                if (ordered) order = point_order(call, c, stream);
                 hash_forward(call, c, order, table, feats, stream);
                 check(th_mlp_fwd(ptr(feats), d_in, ptr(p.w_in), nullptr, ptr(p.w_hid), nullptr, ptr(p.w_out), nullptr, ptr(out), d_out, call.n, mlp.d_in,
                                  mlp.hidden, mlp.d_out, mlp.depth, mlp.act, mlp.dtype, 0, stream),
