@@ -168,7 +168,7 @@ const Tensor &same(const Tensor &t, at::ScalarType type, int64_t numel) {
     return t;
 }
 
-Tensor restored(const Tensor &t, at::ScalarType type, int64_t numel) { return same(t, type, numel).contiguous(); }
+Tensor restored(const Tensor &t, at::ScalarType type, int64_t numel) { return same(t, type, numel).is_contiguous() ? t : t.contiguous(); }
 
 // Three-dimensional rows evenly strided over both leading dimensions, unit stride inside a row
 bool even_rows(const Tensor &x) {
