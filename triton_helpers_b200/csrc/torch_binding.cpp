@@ -19,6 +19,7 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/forward_grad.h>
 #include <torch/csrc/autograd/function.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/python_variable.h>
@@ -45,14 +46,13 @@ using torch::autograd::variable_list;
 
 std::atomic<bool> g_deferred{false};  // event timing of every launch is on: leave the calls to Python
 
-// A CUDA tensor nothing else has a say in: no Python or functorch dispatch, no lazy conjugation or negation, no forward-mode
-// tangent (the operators have no forward-mode derivative; the Python functions raise the error for it).
+// A CUDA tensor nothing else has a say in: no Python or functorch dispatch, no lazy conjugation or negation.
 bool plain(const Tensor &t) {
     using c10::DispatchKey;
     static const c10::DispatchKeySet others({DispatchKey::Python, DispatchKey::PythonTLSSnapshot, DispatchKey::FuncTorchBatched,
                                              DispatchKey::FuncTorchGradWrapper, DispatchKey::Batched, DispatchKey::Functionalize,
                                              DispatchKey::Conjugate, DispatchKey::Negative, DispatchKey::ZeroTensor, DispatchKey::NestedTensor});
-    return t.defined() && t.is_cuda() && !t.key_set().has_any(others) && t.layout() == at::kStrided && !t._fw_grad(0).defined();
+    return t.defined() && t.is_cuda() && !t.key_set().has_any(others) && t.layout() == at::kStrided;
 }
 
 bool usual_mode() {
@@ -62,7 +62,9 @@ bool usual_mode() {
     static const c10::DispatchKeySet modes({DispatchKey::Python, DispatchKey::PythonTLSSnapshot, DispatchKey::FuncTorchDynamicLayerFrontMode,
                                             DispatchKey::FuncTorchDynamicLayerBackMode, DispatchKey::Functionalize, DispatchKey::Tracer});
     return !g_deferred.load(std::memory_order_relaxed) && !at::autocast::is_autocast_enabled(at::kCUDA) &&
-           !c10::impl::tls_local_dispatch_key_set().included_.has_any(modes);
+           !c10::impl::tls_local_dispatch_key_set().included_.has_any(modes) &&
+           // inside a forward-mode level tensors may have tangents: the Python functions raise for lack of a derivative
+           !torch::autograd::ForwardADLevel::try_get_by_idx(0);
 }
 
 // One optional tensor argument; false when it is neither None nor a tensor (or Parameter) itself: a subclass keeps its type through
