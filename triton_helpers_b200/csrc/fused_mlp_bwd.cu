@@ -475,7 +475,7 @@ bool one_slot_only() {
 
 // S slots of W warpgroups, if that fits one SM.  Measured (ms, B200), the most slots that fit are the fastest, two warpgroups
 // per slot when there are threads left: 2^21 rows 32-64-64-16 4 x 1 0.234, 3 x 2 0.269; 2^20 rows 32-4x64-16 2 x 2 0.277, 1 x 2 0.45;
-// with biases 32-64-64-16 3 x 2 0.158, 2 x 2 0.20; 300 007 rows 32-3x64-3 SiLU with biases 2 x 2 0.218, 1 x 2 0.40.  The kernels this
+// with biases 32-64-64-16 3 x 2 0.158, 2 x 2 0.20; 300 007 rows 32-3x64-3 SiLU with biases 2 x 2 0.145 (0.218, and 1 x 2 0.40, with a division in the sigmoid).  The kernels this
 // one replaced (four one-warpgroup slots with a polling warp each; one tile per CTA for biases and SiLU): 0.271, 0.333, 0.340 and
 // 0.412.  Tried: dz in a tile of its own so that the chain waits for a weight gradient one step late, next rows fetched ahead into
 // it (0.290 at 32-4x64-16 against 0.284, and a slot less where it costs one); loops over 32 columns left rolled because

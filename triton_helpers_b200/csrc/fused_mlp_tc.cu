@@ -137,8 +137,8 @@ mlp_fwd_tc_kernel(const MlpShape s, const MlpParams p, const __grid_constant__ W
 // The kernel above keeps one row tile per CTA in flight and every thread walks the same chain
 // (issue, wait, epilogue, barrier); only co-resident CTAs overlap, and each of them needs its own
 // copy of the weights.  Here one CTA per SM runs S independent "slots" of 128 threads (4 warps).
-// A slot is what a CTA is above - it owns 64 TMEM columns, two operand tiles and two mbarriers, and
-// walks its row tiles layer by layer - but the slots share the weights, and they never meet at a
+// A slot is what a CTA is above - it owns 64 TMEM columns (96 with its hidden activations there), one operand tile (two
+// where those stay in shared memory) and its mbarriers, and walks its row tiles layer by layer - but the slots share the weights, and they never meet at a
 // CTA-wide barrier after set-up, so one slot's MMAs run under the other slots' epilogues:
 //
 //   warp 0 of the slot  : fetches the slot's next input tile by TMA (a box of 64 columns x 128 rows
@@ -150,7 +150,7 @@ mlp_fwd_tc_kernel(const MlpShape s, const MlpParams p, const __grid_constant__ W
 //                         TMEM lane) into the next layer's operand rows in place, or into output
 //                         rows in global memory, and meet at the slot's named barrier.
 //
-// Tile k of a slot computes in buffer k & 1 while the prefetch of tile k + 1 lands in the other.
+// The prefetch of a slot's next tile lands in its one buffer once the first layer has read it, or (two buffers) in the other.
 // Every mbarrier wait is bounded and watches a shared abort flag; after an abort a slot keeps the
 // SAME sequence of named barriers (doing no work) so nobody is left waiting at one.
 

@@ -24,7 +24,7 @@ constexpr int kScanThreads = 512;
 constexpr int kScanItems = 4;  // counters per thread
 constexpr int kScanTile = kScanThreads * kScanItems;
 
-// Interleaves the low bits of up to three coordinates: bit j of axis d goes to bit j * D + d.
+// Morton (Z-order) code by the usual halving masks: bit j of axis d goes to bit j * D + d.
 template <int D>
 __device__ __forceinline__ uint32_t spread(uint32_t v) {
     if constexpr (D == 1) return v;
@@ -163,10 +163,10 @@ int launch_order(const CoordView &cv, float scale, int64_t n, float4 *order, uin
 // would save requests there.  The choice is the tile's own, so clustered batches keep sorting on levels where uniform
 // ones do not.
 //
-// Bound by instruction issue and shared-memory latency on the sorted levels (24 warps of 80 registers per SM), by the
-// SMs' requests to L2 on the others; CTAs in different phases overlap.  Against hash_bwd_kernel + hash_bwd_coarse_kernel on
-// unordered points: 2^21 uniform points, 16 levels, 2 x float16: 0.70 against 0.77 ms; 2^22 points in 8 clusters, 4 x float32,
-// 681 MB: 2.30 against 4.37 ms; 200 003 points in two dimensions: 0.052 against 0.143 ms.
+// Bound by the SMs' requests to L2 (request path 68 % busy, L2 68 %, a third of the issue slots used: 22 warps per SM that wait for
+// memory most of the time); CTAs that sort and CTAs on the fine levels overlap.  Against hash_bwd_kernel + hash_bwd_coarse_kernel
+// on unordered points: 2^21 uniform points, 16 levels, 2 x float16: 0.65 against 0.77 ms (gradients in order; 0.70 in the caller's);
+// 2^22 points in 8 clusters, 4 x float32, 681 MB: 2.31 against 4.12 ms.
 
 constexpr int kTileBins = 2048;
 

@@ -178,8 +178,8 @@ def hash_encoded_mlp(
     scale: float = 1.0,
 ) -> Tensor:
     r"""``fully_fused_mlp(hash_encoding(coord, embeddings, ...), w_in, None, w_out, None, w_hid, None, activation)``
-    in one kernel per direction.  Arguments are those of the two functions (bias-free network); output
-    ``(..., D_out)``.  Raises ``FieldUnsupported`` for configurations the fused kernels do not cover."""
+    in one call per direction (the separate kernels or the fused ones, whichever is the faster for the shape).  Arguments are
+    those of the two functions (bias-free network); output ``(..., D_out)``.  Raises ``FieldUnsupported`` for configurations the fused kernels do not cover."""
     activation = ensure_str(activation)
     out = _lib.native().hash_encoded_mlp(
         coord, embeddings, w_in, w_out, w_hid, pi, max_entries_per_level, min_res, max_res, levels, activation, scale
