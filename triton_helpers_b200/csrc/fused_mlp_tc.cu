@@ -156,6 +156,35 @@ mlp_fwd_tc_kernel(const MlpShape s, const MlpParams p, const __grid_constant__ W
 
 constexpr int kMaxSlots = 5;
 
+// Wide output rows leave through shared memory: a warp rounds its 32 rows, 32 columns at a time, into 2 KB of staging and one TMA
+// store writes the box.  Written by the threads, a row each, one instruction touches 32 lines for 16 bytes of each (2^18 rows, ten
+// 64-wide layers: 5 000 cycles a tile for the output against 1 500; 0.0387 -> 0.0313 ms).  Rows of up to 32 bytes are whole
+// sectors of neighbouring lines either way, and the staging costs more than it saves (2^20 rows 32-4x64-16: 0.0531 against 0.0517).
+constexpr int kStageCols = 32;
+constexpr int kStageBytes = 32 * kStageCols * 2;
+
+// Shared memory of the multi-slot kernel: the TcPlan's tiles and weights, then the biases and the output staging.
+struct PipePlan {
+    TcPlan w;
+    int bias;      // BIAS_MMA: operand tiles, four layers each; otherwise fp32 [(depth + 1)][64]
+    int staging;   // kStageBytes per warp
+    int total;     // excluding the 1 KB alignment slack
+};
+
+__host__ __device__ inline PipePlan pipe_plan(const MlpShape &s, int tiles, int slots, bool bias_mma, bool staged) {
+    PipePlan p{};
+    p.w = tc_plan(s, false, tiles);
+    p.bias = p.w.bias_offset;
+    p.staging = p.bias;
+    if (s.has_bias) p.staging += bias_mma ? (s.depth / 4 + 1) * 64 * 128 : (s.depth + 1) * kMaxDim * 4;
+    p.staging = (p.staging + 1023) & ~1023;
+    p.total = p.staging + (staged ? slots * 4 * kStageBytes : 0);
+    return p;
+}
+
+// How a kernel's output rows are written: element by element, in 16-byte chunks, or through the staging
+constexpr int kRowsStaged = 2;
+
 struct SlotBarriers {
     unsigned long long in_full[kMaxSlots][2];
     unsigned long long acc_full[kMaxSlots];
@@ -171,11 +200,15 @@ __device__ __forceinline__ void slot_barrier(int slot) {
 // the operand tile in shared memory; the first layer still reads the TMA-fetched input tile.
 // H64: the hidden width (padded) is 64 at compile time: one form of the hidden layers' epilogue and of their GEMMs' issue
 // (2^20 rows 32-4x64-16: 0.058 -> 0.054 ms; 2^21 rows 32-64-64-16: 0.070 -> 0.065).
-template <typename T, int ACT, bool BIAS, int S, bool MSE, bool TA, bool H64>
+// BM: a layer's bias is one more K step of its GEMM, ahead of the others: A is a constant in tensor memory (element 0 of every row
+// is one), B an operand tile whose element 16 (l % 4) of row n is b_l[n].  The elements beside it are zeros, so that no other layer's
+// bias (it may be infinite) is multiplied by anything.  The additions in the epilogue it replaces cost 64 instructions and 16
+// shared loads a row and layer, 600 of 2 900 cycles (2^18 rows, ten 64-wide layers: 0.0434 -> 0.0339 ms).
+template <typename T, int ACT, bool BIAS, int S, bool MSE, bool TA, bool H64, bool BM>
 __global__ void __launch_bounds__(128 * S, 1)
 mlp_fwd_pipe_kernel(const MlpShape shape, const MlpParams p, const __grid_constant__ WeightMaps maps,
-                    const __grid_constant__ CUtensorMap x_map, T *__restrict__ y, long long y_stride, long long n_rows,
-                    int y_vec, const MseArgs mse) {
+                    const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap y_map, T *__restrict__ y,
+                    long long y_stride, long long n_rows, int y_vec, const MseArgs mse) {
     MlpShape s = shape;
     if constexpr (H64) s.h = 64;
     extern __shared__ unsigned char smem_raw[];
@@ -187,10 +220,13 @@ mlp_fwd_pipe_kernel(const MlpShape shape, const MlpParams p, const __grid_consta
     // TA: the input tile is free as soon as the first layer has read it, and the next one is fetched into it under the others:
     // one tile per slot, so that deep networks keep five slots too (2^18 rows, ten 64-wide layers: four slots 0.058 ms, five 0.051)
     constexpr int kBuffers = TA ? 1 : 2;
-    const TcPlan P = tc_plan(s, false, kBuffers * S);
+    constexpr bool kBiasMma = BIAS && BM;  // the epilogues have no bias to add
+    static_assert(!BM || TA, "the bias step takes its A operand from tensor memory");
+    const PipePlan plan = pipe_plan(s, kBuffers * S, S, BM, y_vec == kRowsStaged);
+    const TcPlan &P = plan.w;
     constexpr int bf16 = std::is_same<T, __half>::value ? 0 : 1;
-    constexpr uint32_t kTmemCols = S * (kAccCols + (TA ? 32 : 0)) <= 256 ? 256 : 512;
-    const int warp = threadIdx.x >> 5;
+    constexpr uint32_t kTmemCols = S * (kAccCols + (TA ? 32 : 0)) + (kBiasMma ? 8 : 0) <= 256 ? 256 : 512;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
     // ---- set-up: barriers, biases, weights, TMEM ----
     if (threadIdx.x == 0) {
@@ -201,19 +237,28 @@ mlp_fwd_pipe_kernel(const MlpShape shape, const MlpParams p, const __grid_consta
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&bars.acc_full[i])), "r"(1u) : "memory");
         }
     }
-    {
-        float *bias = reinterpret_cast<float *>(smem + P.bias_offset);
+    if constexpr (kBiasMma) {
+        for (int e = threadIdx.x; e < (s.depth / 4 + 1) * 64 * 8; e += blockDim.x) {
+            const int r = (e >> 3) & 63, c = (e & 7) ^ (r & 7), l = (e >> 9) * 4 + (c >> 1);  // 16-byte chunk c of row r holds K elements 8 c ..
+            unsigned short v = 0;
+            if ((c & 1) == 0 && l <= s.depth && r < (l == s.depth ? s.d_out : s.d_hid)) {
+                const void *b = l == 0 ? p.b_in : (l == s.depth ? p.b_out : p.b_hid);
+                v = static_cast<const unsigned short *>(b)[l == 0 || l == s.depth ? r : (l - 1) * s.d_hid + r];
+            }
+            reinterpret_cast<uint4 *>(smem + plan.bias)[e] = make_uint4(v, 0, 0, 0);
+        }
+        fence_async_smem();
+    } else if constexpr (BIAS) {
+        float *bias = reinterpret_cast<float *>(smem + plan.bias);
         for (int e = threadIdx.x; e < (s.depth + 1) * kMaxDim; e += blockDim.x) {
             const int layer = e / kMaxDim, c = e % kMaxDim;
             float v = 0.f;
-            if (BIAS) {
-                if (layer == 0) {
-                    if (c < s.d_hid) v = to_float<T>(static_cast<const T *>(p.b_in)[c]);
-                } else if (layer < s.depth) {
-                    if (c < s.d_hid) v = to_float<T>(static_cast<const T *>(p.b_hid)[(layer - 1) * s.d_hid + c]);
-                } else if (c < s.d_out) {
-                    v = to_float<T>(static_cast<const T *>(p.b_out)[c]);
-                }
+            if (layer == 0) {
+                if (c < s.d_hid) v = to_float<T>(static_cast<const T *>(p.b_in)[c]);
+            } else if (layer < s.depth) {
+                if (c < s.d_hid) v = to_float<T>(static_cast<const T *>(p.b_hid)[(layer - 1) * s.d_hid + c]);
+            } else if (c < s.d_out) {
+                v = to_float<T>(static_cast<const T *>(p.b_out)[c]);
             }
             bias[e] = v;
         }
@@ -233,7 +278,18 @@ mlp_fwd_pipe_kernel(const MlpShape shape, const MlpParams p, const __grid_consta
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_holder;
-    const float *bias = reinterpret_cast<const float *>(smem + P.bias_offset);
+    const float *bias = reinterpret_cast<const float *>(smem + plan.bias);
+    const uint32_t one_tmem = tmem + S * (kAccCols + 32);
+    if constexpr (kBiasMma) {
+        if (warp < 4) {
+            const uint32_t one[8] = {pack_pair<T>(1.f, 0.f), 0, 0, 0, 0, 0, 0, 0};
+            tmem_st8(one_tmem + (static_cast<uint32_t>(32 * warp) << 16), one);
+            tmem_st_wait();
+        }
+        tc_fence_before();
+        __syncthreads();
+        tc_fence_after();
+    }
 
     const long long n_tiles = (n_rows + kTileRows - 1) / kTileRows;
     const long long first_tile = blockIdx.x;
@@ -242,7 +298,8 @@ mlp_fwd_pipe_kernel(const MlpShape shape, const MlpParams p, const __grid_consta
     // ---- the slot's life; nothing below depends on other slots ----
     const int slot = warp >> 2;
     const bool issuer = (warp & 3) == 0;
-    const int row = 32 * (warp & 3) + (threadIdx.x & 31);
+    const int row = 32 * (warp & 3) + lane;
+    const uint32_t stage = smem_addr(smem + plan.staging) + static_cast<uint32_t>(warp) * kStageBytes;
     const uint32_t acc = tmem + slot * kAccCols;
     const uint32_t taddr = acc + (static_cast<uint32_t>(32 * (warp & 3)) << 16);
     const uint32_t act_tmem = tmem + S * kAccCols + slot * 32;  // TA: the slot's hidden activations, 16-bit pairs
@@ -292,17 +349,20 @@ mlp_fwd_pipe_kernel(const MlpShape shape, const MlpParams p, const __grid_consta
             }
             // Only the issuer warp polls the mbarrier; the slot's other warps park at the named barrier,
             // which costs no issue slots (all four polling: 2^21 rows 0.069 against 0.067 ms).  A wait that gives up raises
-            // the abort flag, and everybody reads it after the barrier: work stops, the barrier sequence goes on.
+            // the abort flag; everybody reads it a step late, where the load costs nothing: work stops, the barrier sequence goes on.
+            const int given_up = *reinterpret_cast<volatile int *>(&abort_flag);
             if (issuer) {
                 if (__all_sync(0xffffffffu, !*reinterpret_cast<volatile int *>(&abort_flag))) {
                     const bool leader = elect_one();
                     tc_fence_after();
+                    const uint32_t idesc = instr_desc(128, out_pad, bf16, 0, 0);
+                    if constexpr (kBiasMma) {
+                        if (leader) mma_f16_ta(acc, one_tmem, smem_desc(desc_low(smem_addr(smem + plan.bias) + (l >> 2) * 64 * 128) + 2 * (l & 3)), idesc, 0);
+                    }
                     if (TA && l > 0)
-                        issue_gemm_ta(leader, acc, act_tmem, smem_addr(weight_tile(smem, P, s, l)), 32, in_pad / 16,
-                                      instr_desc(128, out_pad, bf16, 0, 0), false);
+                        issue_gemm_ta(leader, acc, act_tmem, smem_addr(weight_tile(smem, P, s, l)), 32, in_pad / 16, idesc, kBiasMma);
                     else
-                        issue_gemm(leader, acc, tile_addr, 32, smem_addr(weight_tile(smem, P, s, l)), 32, in_pad / 16,
-                                   instr_desc(128, out_pad, bf16, 0, 0), false);
+                        issue_gemm(leader, acc, tile_addr, 32, smem_addr(weight_tile(smem, P, s, l)), 32, in_pad / 16, idesc, kBiasMma);
                     if (leader) mma_commit(acc_bar);
                     __syncwarp();
                     pipe_wait(acc_bar, acc_phase, &abort_flag);
@@ -311,15 +371,15 @@ mlp_fwd_pipe_kernel(const MlpShape shape, const MlpParams p, const __grid_consta
                 }
             }
             slot_barrier(slot);
-            if (!*reinterpret_cast<volatile int *>(&abort_flag)) {
+            if (!given_up) {
                 tc_fence_after();
                 const float *layer_bias = bias + l * kMaxDim;
                 if (l < s.depth) {
                     if constexpr (TA) {
-                        drain_row<T, ACT, BIAS>(taddr, out_pad, layer_bias, [&](int chunk, uint4 packed) { tmem_st4(act_taddr + 4 * chunk, packed); });
+                        drain_row<T, ACT, BIAS && !BM>(taddr, out_pad, layer_bias, [&](int chunk, uint4 packed) { tmem_st4(act_taddr + 4 * chunk, packed); });
                         tmem_st_wait();
                     } else {
-                        drain_row<T, ACT, BIAS>(taddr, out_pad, layer_bias, [&](int chunk, uint4 packed) {
+                        drain_row<T, ACT, BIAS && !BM>(taddr, out_pad, layer_bias, [&](int chunk, uint4 packed) {
                             st_shared_16(row_addr + ((chunk << 4) ^ row_swizzle), packed);
                         });
                         fence_async_smem();
@@ -333,7 +393,7 @@ mlp_fwd_pipe_kernel(const MlpShape shape, const MlpParams p, const __grid_consta
                         const float *target_row_f32 = static_cast<const float *>(mse.target) + target_at * mse.target_stride;
                         T *grad_row = static_cast<T *>(mse.grad) + r * mse.grad_stride;
                         T *out_row = y ? y + r * y_stride : nullptr;
-                        drain_row<T, TH_ACT_NONE, BIAS>(taddr, out_pad, layer_bias, [&](int chunk, uint4 packed) {
+                        drain_row<T, TH_ACT_NONE, BIAS && !BM>(taddr, out_pad, layer_bias, [&](int chunk, uint4 packed) {
                             if (live && 8 * chunk < s.d_out) {
                                 if (out_row) __stcs(reinterpret_cast<uint4 *>(out_row + 8 * chunk), packed);
                                 uint4 g;
@@ -346,9 +406,27 @@ mlp_fwd_pipe_kernel(const MlpShape shape, const MlpParams p, const __grid_consta
                         });
                     } else {
                         T *out_row = y + (live ? row0 + row : 0) * y_stride;
-                        drain_row<T, TH_ACT_NONE, BIAS>(taddr, out_pad, layer_bias, [&](int chunk, uint4 packed) {
-                            if (live) store_chunk_to_global<T>(out_row, chunk, s.d_out, packed, y_vec);
-                        });
+                        if (y_vec == kRowsStaged) {
+                            const uint32_t stage_row = stage + lane * (kStageCols * 2), stage_swizzle = ((lane >> 1) & 3) << 4;
+#pragma unroll 1
+                            for (int first = 0; first < out_pad; first += kStageCols) {
+                                if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // the box before has been read
+                                __syncwarp();
+                                uint32_t raw[32];
+                                tmem_ld32(taddr + first, raw);  // (columns past out_pad are the slot's own and are not stored)
+                                tmem_ld_wait();
+#pragma unroll
+                                for (int u = 0; u < 4; ++u)
+                                    st_shared_16(stage_row + ((u << 4) ^ stage_swizzle), finish8<T, TH_ACT_NONE, BIAS && !BM>(raw + 8 * u, layer_bias + first + 8 * u));
+                                fence_async_smem();
+                                __syncwarp();
+                                if (lane == 0 && row0 + 32 * (warp & 3) < n_rows) tma_store_2d(&y_map, stage, first, static_cast<int>(row0) + 32 * (warp & 3));
+                            }
+                        } else {
+                            drain_row<T, TH_ACT_NONE, BIAS && !BM>(taddr, out_pad, layer_bias, [&](int chunk, uint4 packed) {
+                                if (live) store_chunk_to_global<T>(out_row, chunk, s.d_out, packed, y_vec);
+                            });
+                        }
                     }
                 }
                 tc_fence_before();
@@ -364,6 +442,7 @@ mlp_fwd_pipe_kernel(const MlpShape shape, const MlpParams p, const __grid_consta
     }
 
     // ---- teardown ----
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     if (abort_flag && (threadIdx.x & 127) == 0) {
         drain_copies(bars.in_full[slot], 2);
         if (threadIdx.x == 0) drain_copies(&wbar, 1);
@@ -372,6 +451,20 @@ mlp_fwd_pipe_kernel(const MlpShape shape, const MlpParams p, const __grid_consta
     __syncthreads();
     if (warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
+}
+
+constexpr int kPipeSmem = kSmemBudget - static_cast<int>(sizeof(SlotBarriers)) - 64;  // dynamic; the rest is the kernel's static shared memory
+
+// One warp's box of an output matrix: 32 rows x 32 columns, 64-byte swizzle (16-byte chunk c of row r at c ^ (r / 2 % 4))
+bool make_store_map(CUtensorMap *map, void *base, long long rows, int cols, long long row_stride) {
+    EncodeTiledFn encode = encode_tiled_fn();
+    if (!encode || cols % 8 != 0 || row_stride % 8 != 0 || !aligned_to(base, 16)) return false;
+    const cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
+    const cuuint64_t strides[1] = {static_cast<cuuint64_t>(row_stride) * 2};
+    const cuuint32_t box[2] = {kStageCols, 32};
+    const cuuint32_t elem[2] = {1, 1};
+    return encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, base, dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
+                  CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 bool pipe_disabled() {
@@ -390,25 +483,29 @@ bool tmem_a_enabled() {
     return on;
 }
 
-template <typename T, int ACT, bool BIAS, int S, bool MSE, bool TA>
+template <typename T, int ACT, bool BIAS, int S, bool MSE, bool TA, bool BM = TA && BIAS>
 int launch_fwd_pipe(const MlpShape &s, const MlpParams &p, const void *x, int64_t x_stride, void *y, int64_t y_stride,
                     int64_t rows, cudaStream_t stream, const MseArgs &mse = MseArgs{}) {
-    const TcPlan P = tc_plan(s, false, (TA ? 1 : 2) * S);
-    const int smem = P.total + 1024;
-    if (smem > kSmemBudget || pipe_disabled()) return kTcNotApplicable;
+    CUtensorMap y_map;
+    memset(&y_map, 0, sizeof(y_map));
+    int y_vec = y ? rows_vector_ok(y, y_stride, s.d_out) : 0;
+    if (!MSE && y_vec && s.no > 16 && pipe_plan(s, (TA ? 1 : 2) * S, S, BM, true).total + 1024 <= kPipeSmem && make_store_map(&y_map, y, rows, s.d_out, y_stride))
+        y_vec = kRowsStaged;
+    const int smem = pipe_plan(s, (TA ? 1 : 2) * S, S, BM, y_vec == kRowsStaged).total + 1024;
+    if (smem > kPipeSmem || pipe_disabled()) return kTcNotApplicable;
     if (rows >= (1ll << 31) - kTileRows) return kTcNotApplicable;  // TMA coordinates are 32-bit
     WeightMaps maps;
     CUtensorMap x_map;
     if (!make_weight_maps(maps, s, p)) return kTcNotApplicable;
     if (!make_map(&x_map, x, rows, s.d_in, kTileRows, x_stride)) return kTcNotApplicable;
     if (S * (kAccCols + (TA ? 32 : 0)) > 512) return kTcNotApplicable;
-    auto kernel = TA && s.h == 64 ? mlp_fwd_pipe_kernel<T, ACT, BIAS, S, MSE, TA, TA> : mlp_fwd_pipe_kernel<T, ACT, BIAS, S, MSE, TA, false>;
+    auto kernel = TA && BM == BIAS && s.h == 64 ? mlp_fwd_pipe_kernel<T, ACT, BIAS, S, MSE, TA, TA && BM == BIAS, BM> : mlp_fwd_pipe_kernel<T, ACT, BIAS, S, MSE, TA, false, BM>;
     if (int rc = cuda_status(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
                              "cudaFuncSetAttribute(mlp_fwd_pipe_kernel)")) return rc;
     const long long tiles = (rows + kTileRows - 1) / kTileRows;
     const long long cap = sm_count();
     kernel<<<static_cast<unsigned>(tiles < cap ? tiles : cap), 128 * S, smem, stream>>>(
-        s, p, maps, x_map, static_cast<T *>(y), y_stride, rows, y ? rows_vector_ok(y, y_stride, s.d_out) : 0, mse);
+        s, p, maps, x_map, y_map, static_cast<T *>(y), y_stride, rows, y_vec, mse);
     return launch_status("mlp_fwd_pipe_kernel launch");
 }
 
@@ -430,6 +527,9 @@ int launch_fwd_slots(const MlpShape &s, const MlpParams &p, const void *x, int64
         if (cap >= 5) rc = launch_fwd_pipe<T, ACT, BIAS, 5, MSE, true>(s, p, x, x_stride, y, y_stride, rows, stream, mse);
         if (rc == kTcNotApplicable && cap >= 4) rc = launch_fwd_pipe<T, ACT, BIAS, 4, MSE, true>(s, p, x, x_stride, y, y_stride, rows, stream, mse);
         if (rc == kTcNotApplicable && cap >= 3) rc = launch_fwd_pipe<T, ACT, BIAS, 3, MSE, true>(s, p, x, x_stride, y, y_stride, rows, stream, mse);
+        // networks of 18 layers and more, whose weights leave no room for the biases' operand tiles
+        if constexpr (BIAS)
+            if (rc == kTcNotApplicable && cap >= 3) rc = launch_fwd_pipe<T, ACT, BIAS, 3, MSE, true, false>(s, p, x, x_stride, y, y_stride, rows, stream, mse);
         return rc;
     }
     if (cap >= 4) rc = launch_fwd_pipe<T, ACT, BIAS, 4, MSE, false>(s, p, x, x_stride, y, y_stride, rows, stream, mse);

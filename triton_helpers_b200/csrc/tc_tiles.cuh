@@ -604,6 +604,14 @@ bool make_map(CUtensorMap *map, const void *base, long long rows, int cols, int 
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// One box of `map` from shared memory to element coordinates (x, y), clipped at the matrix's edges; its own bulk group.
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap *map, uint32_t smem_src, int x, int y) {
+    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(reinterpret_cast<uint64_t>(map)), "r"(smem_src),
+                 "r"(x), "r"(y)
+                 : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+
 // One box of `map` at element coordinates (x, y) into shared memory, completion counted on `mbar`.
 __device__ __forceinline__ void tma_load_2d(void *smem_dst, const CUtensorMap *map, int x, int y, uint32_t mbar) {
     asm volatile(
