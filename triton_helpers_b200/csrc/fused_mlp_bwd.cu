@@ -9,13 +9,19 @@
 //   * the wgrad warp issues the weight- and bias-gradient MMAs of every slot.  MMAs of one thread execute in order, so all
 //     slots accumulate into ONE shared set of TMEM columns instead of one set per tile in flight;
 //   * dz of layer l - 1 is written in place over the parked input of layer l once both MMAs that read it have finished;
-//   * when features and output gradient are at most 32 wide, the output-gradient rows of a slot live in the logical chunks
-//     4..7 of its feature tile (which uses chunks 0..3): depth + 1 tiles per slot.  The output layer's wgrad then reads the
-//     whole feature tile as its A operand, and the real gradient rows sit at rows 32.. of that layer's accumulator (rows
-//     0..31 are products nobody reads).
+//   * rows come and go through a ring of buffers (features, output gradient), one more than slots where that fits, kept by ROW
+//     WARPS: TMA fetches the next tile's rows while the slots work, and the input gradient, which the slot leaves in its buffer
+//     as rounded rows, goes out by TMA before the buffer is filled again.  Rows TMA cannot describe are copied by four row warps,
+//     a thread a row.  Rows of 16 or 32 columns lie 32 or 64 bytes apart (the tensor core's 32- and 64-byte swizzles).
+// The output layer's weight gradient is formed transposed, act^T . dz: an M = 64 MMA takes 27 + N / 2 cycles, and N is then the
+// padded output width (16: 35 instead of 60 cycles a K step) instead of the hidden one.
 // Bias gradient of a layer = column sums of dz = dz^T . ONES, a small MMA (N = 8) next to the weight gradient's.  SiLU' and
 // ReLU^2' want the pre-activation: the step that needs it issues that layer's forward GEMM again into a second accumulator
 // and rounds z to the storage dtype, as the forward pass did.
+//
+// Measured: rows fetched and stored by the slots themselves were 22 % of a slot's time (2^21 rows 32-64-64-16; a fence for the
+// tensor core also waits for the thread's own copies and stores in flight): 0.234 -> 0.209 ms; 2^20 rows 32-4x64-16 0.279 -> 0.265;
+// 300 007 rows 32-3x64-16 with biases, where the smaller row buffers make room for a third slot, 0.081 -> 0.069.
 //
 // Per slot three mbarriers: `ready` (one arrival: the operands of the slot's next backward step are in place), `acc` (the
 // slot's own MMAs of the step are done), `wdone` (the step's wgrad is done).  The wgrad warp polls all `ready` barriers at
@@ -31,9 +37,23 @@ namespace {
 constexpr int kSlotsMax = 4;
 constexpr int kStepsMax = 24;  // 2 depth + 1
 
+// Rows of at most 16, 32 or 64 columns lie 32, 64 or 128 bytes apart, in the tensor core's 32-, 64- or 128-byte swizzle.
+__host__ __device__ constexpr int row_pitch(int pad) { return pad <= 16 ? 32 : (pad <= 32 ? 64 : 128); }
+__host__ __device__ constexpr uint32_t desc_high(int pitch) {
+    return (static_cast<uint32_t>(8 * pitch) >> 4) | (1u << 14) | ((pitch == 128 ? 2u : (pitch == 64 ? 4u : 6u)) << 29);
+}
+__device__ __forceinline__ uint64_t desc_of(uint32_t low, uint32_t high) {
+    uint64_t d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(low), "r"(high));
+    return d;
+}
+
 struct SlotPlan {
-    int packed;          // the output gradient shares the feature tile
-    int tiles_per_slot;
+    int rings;           // buffers of rows: slots, or slots + 1
+    int x_pitch, go_pitch;
+    int ring;            // byte offset
+    int ring_bytes;      // a buffer: the rows, then the output gradient
+    int row_warps;       // 1: rows by TMA; 4: some of them by threads
     int ones;            // byte offset of the tile of ones (biases)
     int weights;         // byte offset of the weight tiles and biases
     int tables;          // byte offset of the barriers and step table
@@ -57,12 +77,17 @@ struct __align__(16) SlotStep {
     uint32_t za_off;   // pre-activation of the layer below: A operand
     uint32_t zb_addr;  //   B operand
     uint32_t z_k;      //   K steps; 0 = none
-    uint32_t unused;
+    uint32_t a_high;   // high words of the descriptors that are not a 128-byte tile's: the slot's own GEMM's A operand
+    uint32_t wa_high, wb_high;  // the weight gradient's operands
+    uint32_t wa_step, wb_step;  // bytes between K steps
+    uint32_t flags;    // operands in the row buffer: bit 1 the weight gradient's A, 2 its B, 3 the pre-activation's A; 4: B is dz (transposed)
+    uint32_t unused[2];
 };
 
 struct SlotTables {
     unsigned long long weights_bar;
     unsigned long long ready[kSlotsMax], acc[kSlotsMax], wdone[kSlotsMax];
+    unsigned long long full[kSlotsMax + 1], empty[kSlotsMax + 1];
     uint32_t tmem_holder;
     int abort_flag;
     SlotStep steps[kStepsMax];
@@ -70,24 +95,34 @@ struct SlotTables {
 
 __host__ __device__ constexpr bool needs_preact(int act) { return act == TH_ACT_SILU || act == TH_ACT_RELU2; }
 
-SlotPlan slot_plan(const MlpShape &s, int slots) {
+SlotPlan slot_plan(const MlpShape &s, int slots, int rings) {
     SlotPlan b{};
-    b.packed = (s.ki <= 32 && s.no <= 32) ? 1 : 0;
-    b.tiles_per_slot = s.depth + 1 + (b.packed ? 0 : 1);
-    int off = slots * b.tiles_per_slot * kTileBytes;
+    b.rings = rings;
+    b.x_pitch = row_pitch(s.ki);
+    b.go_pitch = row_pitch(s.no);
+    int off = slots * s.depth * kTileBytes;
+    b.ring = off;
+    b.ring_bytes = kTileRows * (b.x_pitch + b.go_pitch);
+    off += rings * b.ring_bytes;
     b.ones = off;
-    if (s.has_bias) off += kTileBytes;
+    if (s.has_bias) off += kTileRows * 32;
+    off = (off + 1023) & ~1023;
     b.weights = off;
     b.w = tc_plan(s, false, 0);
     off += s.has_bias ? b.w.total : b.w.bias_offset;  // the biases are the plan's last part
-    b.tables = off;
-    b.total = off + static_cast<int>(offsetof(SlotTables, steps)) + (2 * s.depth + 1) * static_cast<int>(sizeof(SlotStep));
+    b.tables = (off + 15) & ~15;
+    b.total = b.tables + static_cast<int>(offsetof(SlotTables, steps)) + (2 * s.depth + 1) * static_cast<int>(sizeof(SlotStep));
     b.acc_cols = kAccCols * (needs_preact(s.act) ? 2 : 1);
-    const int cols = slots * b.acc_cols + s.ki + s.depth * s.h + (s.has_bias ? 8 * (s.depth + 1) : 0);
+    const int cols = slots * b.acc_cols + s.ki + (s.depth - 1) * s.h + s.no + (s.has_bias ? 8 * (s.depth + 1) : 0);
     int alloc = 32;
     while (alloc < cols) alloc <<= 1;
     b.tmem_cols = alloc;
     return b;
+}
+
+// 16-byte chunk c of row r lies at chunk c ^ row_swizzle_of(r, pitch)
+__device__ __forceinline__ uint32_t row_swizzle_of(int r, int pitch) {
+    return pitch == 128 ? (r & 7) : (pitch == 64 ? ((r >> 1) & 3) : ((r >> 2) & 1));
 }
 
 __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
@@ -99,8 +134,8 @@ __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
     return done != 0;
 }
 
-__device__ __forceinline__ void mbar_init(const void *bar) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(1u) : "memory");
+__device__ __forceinline__ void mbar_init(const void *bar, uint32_t arrivals = 1) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(arrivals) : "memory");
 }
 
 // This thread's columns of a row of `pad` accumulator columns (all of them, or one half of them), 8 at a time:
@@ -119,12 +154,16 @@ __device__ __forceinline__ void for_row_pieces(uint32_t taddr, int pad, int half
     }
 }
 
+// Three slots of two warpgroups leave registers for one row warp: rows by TMA only
+template <int S, int W>
+constexpr int kRowWarps = S * W > 4 ? 1 : 4;
+
 template <typename T, int ACT, bool BIAS, int S, int W>
-__global__ void __launch_bounds__(128 * S * W + 32, 1)
+__global__ void __launch_bounds__(128 * S * W + 32 + 32 * kRowWarps<S, W>, 1)
 slots_mlp_bwd_tc_kernel(const MlpShape s, const MlpParams p, const __grid_constant__ WeightMaps maps, const int use_tma,
-                        const __grid_constant__ SlotPlan P, const T *__restrict__ x, long long x_stride, const T *__restrict__ go,
-                        long long go_stride, T *__restrict__ gx, long long gx_stride, float *__restrict__ workspace, long long n_rows, int x_vec,
-                        int go_vec, int gx_vec) {
+                        const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap go_map,
+                        const __grid_constant__ CUtensorMap gx_map, const int row_tma, const __grid_constant__ SlotPlan P, const T *__restrict__ x, long long x_stride, const T *__restrict__ go,
+                        long long go_stride, T *__restrict__ gx, long long gx_stride, float *__restrict__ workspace, long long n_rows) {
     constexpr bool kPreact = needs_preact(ACT);
     constexpr int kSlotThreads = 128 * W;
     constexpr int bf16 = std::is_same<T, __half>::value ? 0 : 1;
@@ -133,7 +172,7 @@ slots_mlp_bwd_tc_kernel(const MlpShape s, const MlpParams p, const __grid_consta
     SlotTables &tb = *reinterpret_cast<SlotTables *>(smem + P.tables);
     const int d = s.depth, n_steps = 2 * d + 1;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const bool is_wgrad_warp = warp == 4 * S * W;
+    const bool is_wgrad_warp = warp == 4 * S * W, is_row_warp = warp > 4 * S * W;
     unsigned char *wsmem = smem + P.weights;
     volatile int *abort_now = &tb.abort_flag;
 
@@ -146,17 +185,18 @@ slots_mlp_bwd_tc_kernel(const MlpShape s, const MlpParams p, const __grid_consta
             mbar_init(&tb.acc[i]);
             mbar_init(&tb.wdone[i]);
         }
+        for (int i = 0; i < P.rings; ++i) {
+            mbar_init(&tb.full[i], static_cast<uint32_t>(P.row_warps));
+            mbar_init(&tb.empty[i]);
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     // operand tiles start out as zeros: columns a layer does not use are still read as MMA rows
     for (int e = threadIdx.x; e < P.ones / 16; e += blockDim.x) reinterpret_cast<uint4 *>(smem)[e] = make_uint4(0, 0, 0, 0);
     if constexpr (BIAS) {
-        // 128 rows x 8 columns of ones (logical chunk 0 of every row)
+        // 128 rows of ones, 32 bytes apart
         const uint32_t one2 = pack_pair<T>(1.f, 1.f);
-        for (int e = threadIdx.x; e < kTileBytes / 16; e += blockDim.x) {
-            const int r = e >> 3, c = (e & 7) ^ (r & 7);
-            reinterpret_cast<uint4 *>(smem + P.ones)[e] = c == 0 ? make_uint4(one2, one2, one2, one2) : make_uint4(0, 0, 0, 0);
-        }
+        for (int e = threadIdx.x; e < kTileRows * 2; e += blockDim.x) reinterpret_cast<uint4 *>(smem + P.ones)[e] = make_uint4(one2, one2, one2, one2);
         stage_biases<T>(wsmem, P.w, s, p);
     }
     fence_async_smem();
@@ -187,35 +227,53 @@ slots_mlp_bwd_tc_kernel(const MlpShape s, const MlpParams p, const __grid_consta
     const long long first_tile = blockIdx.x, tile_stride = gridDim.x;
     const long long n_mine = first_tile < n_tiles ? (n_tiles - first_tile + tile_stride - 1) / tile_stride : 0;
     const uint32_t smem_base = smem_addr(smem);
-    const uint32_t slot_bytes = static_cast<uint32_t>(P.tiles_per_slot) * kTileBytes;
+    const uint32_t slot_bytes = static_cast<uint32_t>(d) * kTileBytes;
+    const uint32_t go_at = static_cast<uint32_t>(kTileRows * P.x_pitch);  // the output gradient in a row buffer
+    auto ring_of = [&](uint32_t b) { return smem_base + P.ring + b * P.ring_bytes; };
     auto dw_col = [&](int l) { return S * P.acc_cols + (l == 0 ? 0 : s.ki + (l - 1) * s.h); };
-    auto db_col = [&](int l) { return S * P.acc_cols + s.ki + d * s.h + 8 * l; };
-    // the output gradient of a slot: its own tile, or logical chunks 4.. of the slot's feature tile
-    const uint32_t go_off = P.packed ? 64u : static_cast<uint32_t>(d + 1) * kTileBytes;
+    auto db_col = [&](int l) { return S * P.acc_cols + s.ki + (d - 1) * s.h + s.no + 8 * l; };
     if (static_cast<int>(threadIdx.x) < n_steps) {  // steps 0 .. d - 1 recompute, step j >= d is the backward step of layer 2 d - j
         const int j = threadIdx.x;
         SlotStep st{};
+        st.a_high = st.wa_high = st.wb_high = kDescHigh;
+        st.wa_step = st.wb_step = 2048;
         if (j < d) {
-            st.a_off = static_cast<uint32_t>(j) * kTileBytes;
+            st.a_off = j == 0 ? 0u : static_cast<uint32_t>(j - 1) * kTileBytes;
+            if (j == 0) st.a_high = desc_high(P.x_pitch);
             st.b_addr = smem_addr(weight_tile(wsmem, P.w, s, j));
             st.idesc = instr_desc(128, s.h, bf16, 0, 0);
             st.k_steps = static_cast<uint32_t>((j == 0 ? s.ki : s.h) / 16);
         } else {
             const int l = 2 * d - j;
             const int in_pad = l == 0 ? s.ki : s.h, out_pad = l == d ? s.no : s.h;
-            const uint32_t dz = l == d ? go_off : static_cast<uint32_t>(l + 1) * kTileBytes;
+            const uint32_t dz = l == d ? go_at : static_cast<uint32_t>(l) * kTileBytes;
             if (l > 0 || gx != nullptr) {
                 st.a_off = dz;
                 st.b_addr = smem_addr(weight_tile(wsmem, P.w, s, l));
                 st.idesc = instr_desc(128, in_pad, bf16, 0, 1);
                 st.k_steps = static_cast<uint32_t>(out_pad / 16) | 256u;
             }
-            st.wa_off = (l == d && P.packed) ? 0u : dz;  // packed output gradient: the whole feature tile is the A operand
-            st.wb_off = static_cast<uint32_t>(l) * kTileBytes;
+            st.wa_off = dz;
+            st.wb_off = l == 0 ? 0u : static_cast<uint32_t>(l - 1) * kTileBytes;
             st.widesc = instr_desc(64, in_pad, bf16, 1, 1);
+            if (l == d) {  // transposed: act^T . dz
+                st.a_high = desc_high(P.go_pitch);
+                st.wa_off = st.wb_off;
+                st.wb_off = go_at;
+                st.flags |= 4u | 16u;
+                st.wb_high = desc_high(P.go_pitch);
+                st.wb_step = 16 * P.go_pitch;
+                st.widesc = instr_desc(64, out_pad, bf16, 1, 1);
+            }
+            if (l == 0) {
+                st.flags |= 4u;
+                st.wb_high = desc_high(P.x_pitch);
+                st.wb_step = 16 * P.x_pitch;
+            }
             st.dw_col = static_cast<uint32_t>(dw_col(l)) | (static_cast<uint32_t>(db_col(l)) << 16);
             if (kPreact && l > 0) {
-                st.za_off = static_cast<uint32_t>(l - 1) * kTileBytes;
+                st.za_off = l == 1 ? 0u : static_cast<uint32_t>(l - 2) * kTileBytes;
+                if (l == 1) st.flags |= 8u;
                 st.zb_addr = smem_addr(weight_tile(wsmem, P.w, s, l - 1));
                 st.z_k = static_cast<uint32_t>((l == 1 ? s.ki : s.h) / 16);
             }
@@ -228,6 +286,7 @@ slots_mlp_bwd_tc_kernel(const MlpShape s, const MlpParams p, const __grid_consta
         // ================= weight gradients of every slot =================
         // lane i < S keeps slot i's state: its next backward step, the tiles it still has, the parity to wait for
         int my_step = d;
+        uint32_t my_buf = static_cast<uint32_t>(lane) % static_cast<uint32_t>(P.rings);
         long long my_tiles = lane < S && lane < n_mine ? (n_mine - lane + S - 1) / S : 0;
         uint32_t my_parity = 0, started = 0;
         const uint32_t my_bar = smem_addr(&tb.ready[lane < S ? lane : 0]);
@@ -258,11 +317,22 @@ slots_mlp_bwd_tc_kernel(const MlpShape s, const MlpParams p, const __grid_consta
                 mask &= mask - 1;
                 const int j = __shfl_sync(0xffffffffu, my_step, i);
                 const uint4 w = *reinterpret_cast<const uint4 *>(&tb.steps[j].wa_off);
-                const uint32_t tile0 = smem_base + static_cast<uint32_t>(i) * slot_bytes;
+                const uint4 h = *reinterpret_cast<const uint4 *>(&tb.steps[j].wa_high);
+                const uint32_t flags = tb.steps[j].flags;
+                const uint32_t tile0 = smem_base + static_cast<uint32_t>(i) * slot_bytes, rows0 = ring_of(__shfl_sync(0xffffffffu, my_buf, i));
                 const bool more = (started >> (j - d)) & 1u;
-                issue_gemm(leader, tmem + (w.w & 0xffffu), tile0 + w.x, 2048, tile0 + w.y, 2048, kTileRows / 16, w.z, more);
-                if constexpr (BIAS)
-                    issue_gemm(leader, tmem + (w.w >> 16), tile0 + w.x, 2048, smem_base + P.ones, 2048, kTileRows / 16, instr_desc(64, 8, bf16, 1, 1), more);
+                if (leader) {
+                    const uint32_t a_low = desc_low((flags & 2u ? rows0 : tile0) + w.x), b_low = desc_low((flags & 4u ? rows0 : tile0) + w.y);
+                    for (int k = 0; k < kTileRows / 16; ++k)
+                        mma_f16(tmem + (w.w & 0xffffu), desc_of(a_low + k * (h.z >> 4), h.x), desc_of(b_low + k * (h.w >> 4), h.y), w.z, more || k > 0);
+                    if constexpr (BIAS) {
+                        const bool from_b = flags & 16u;
+                        const uint32_t dz_low = from_b ? b_low : a_low, dz_step = (from_b ? h.w : h.z) >> 4, dz_high = from_b ? h.y : h.x;
+                        for (int k = 0; k < kTileRows / 16; ++k)
+                            mma_f16(tmem + (w.w >> 16), desc_of(dz_low + k * dz_step, dz_high), desc_of(desc_low(smem_base + P.ones) + k * 32, desc_high(32)),
+                                    instr_desc(64, 8, bf16, 1, 1), more || k > 0);
+                    }
+                }
                 started |= 1u << (j - d);
                 if (leader) mma_commit(smem_addr(&tb.wdone[i]));
             }
@@ -272,11 +342,64 @@ slots_mlp_bwd_tc_kernel(const MlpShape s, const MlpParams p, const __grid_consta
                 if (++my_step == n_steps) {
                     my_step = d;
                     --my_tiles;
+                    my_buf = (my_buf + S) % static_cast<uint32_t>(P.rings);
                 }
             }
         }
+    } else if (is_row_warp) {
+        // ================= rows: the input gradient out of a buffer, the next tile's rows into it =================
+        const uint32_t x_bytes = static_cast<uint32_t>(kTileRows * P.x_pitch), go_bytes = static_cast<uint32_t>(kTileRows * P.go_pitch);
+        const bool x_tma = row_tma & 1, go_tma = row_tma & 2, gx_tma = row_tma & 4;
+        const int r_warp = warp - 4 * S * W - 1, r = 32 * r_warp + lane;  // a thread's row
+        // this thread's row, element by element
+        auto copy_row = [&](const T *src, long long grow, long long stride, int cols, int pad, int pitch, uint32_t tile) {
+            const unsigned short *from = reinterpret_cast<const unsigned short *>(src + (grow < n_rows ? grow * stride : 0));
+            const uint32_t at = tile + r * pitch, swz = row_swizzle_of(r, pitch);
+#pragma unroll 2
+            for (int c = 0; c < pad / 8; ++c)
+                st_shared_16(at + ((c ^ swz) << 4), gather8(from + 8 * c, 8 * c, grow < n_rows ? cols : 0));
+        };
+        bool alive = true;  // after an abort: the same sequence of barriers, no work
+        for (long long k = 0; r_warp < P.row_warps && k < n_mine + P.rings; ++k) {
+            const uint32_t b = static_cast<uint32_t>(k % P.rings), rows_at = ring_of(b);
+            const long long row0 = (first_tile + k * tile_stride) * kTileRows;
+            if (k >= P.rings) {
+                if (k - P.rings >= n_mine) continue;
+                const long long old0 = row0 - P.rings * tile_stride * kTileRows;
+                pipe_wait(smem_addr(&tb.empty[b]), static_cast<uint32_t>((k / P.rings - 1) & 1), &tb.abort_flag);
+                alive = alive && !__any_sync(0xffffffffu, *abort_now);
+                if (!alive) {
+                } else if (gx_tma) {
+                    if (r_warp == 0 && lane == 0) {
+                        tma_store_2d(&gx_map, rows_at, 0, static_cast<int>(old0));
+                        asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+                    }
+                } else if (gx != nullptr && old0 + r < n_rows) {
+                    const uint32_t at = rows_at + r * P.x_pitch, swz = row_swizzle_of(r, P.x_pitch);
+                    for (int c = 0; c < s.ki / 8; ++c) store_chunk_to_global<T>(gx + (old0 + r) * gx_stride, c, s.d_in, ld_shared_16(at + ((c ^ swz) << 4)), false);
+                }
+                __syncwarp();
+                if (P.row_warps > 1) asm volatile("bar.sync 15, 128;" ::: "memory");
+            }
+            if (k >= n_mine || !alive) continue;
+            if (P.row_warps > 1) {
+                if (!x_tma) copy_row(x, row0 + r, x_stride, s.d_in, s.ki, P.x_pitch, rows_at);
+                if (!go_tma) copy_row(go, row0 + r, go_stride, s.d_out, s.no, P.go_pitch, rows_at + go_at);
+                fence_async_smem();
+                __syncwarp();
+            }
+            if (lane == 0) {
+                const uint32_t full_bar = smem_addr(&tb.full[b]), bytes = r_warp == 0 ? (x_tma ? x_bytes : 0u) + (go_tma ? go_bytes : 0u) : 0u;
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full_bar), "r"(bytes) : "memory");
+                if (r_warp == 0 && x_tma) tma_load_2d(smem + P.ring + b * P.ring_bytes, &x_map, 0, static_cast<int>(row0), full_bar);
+                if (r_warp == 0 && go_tma) tma_load_2d(smem + P.ring + b * P.ring_bytes + go_at, &go_map, 0, static_cast<int>(row0), full_bar);
+            }
+            __syncwarp();
+        }
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+        if (*abort_now && r_warp == 0 && lane == 0) drain_copies(tb.full, P.rings);
     } else {
-        // ================= slots: loads, own MMAs, epilogues =================
+        // ================= slots: own MMAs, epilogues =================
         const int slot = warp / (4 * W), wq = warp & 3;
         const int tid = threadIdx.x - slot * kSlotThreads;
         const int row = tid & 127, half = W == 2 ? tid >> 7 : 0;
@@ -284,36 +407,14 @@ slots_mlp_bwd_tc_kernel(const MlpShape s, const MlpParams p, const __grid_consta
         const uint32_t taddr = acc + (static_cast<uint32_t>(32 * wq) << 16);
         const uint32_t acc_bar = smem_addr(&tb.acc[slot]), ready_bar = smem_addr(&tb.ready[slot]), wdone_bar = smem_addr(&tb.wdone[slot]);
         const uint32_t tile0 = smem_base + static_cast<uint32_t>(slot) * slot_bytes;
-        auto act_addr = [&](int l) { return tile0 + static_cast<uint32_t>(l) * kTileBytes; };
+        auto act_addr = [&](int l) { return tile0 + static_cast<uint32_t>(l - 1) * kTileBytes; };  // input of layer l > 0
         const float *bias = reinterpret_cast<const float *>(wsmem + P.w.bias_offset);
         const uint32_t row_off = row * 128, row_swizzle = (row & 7) << 4;
         const bool issuer = tid < 32;
         const bool leader = issuer && elect_one();
         uint32_t acc_phase = 0, wdone_phase = 0;
         auto slot_sync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(slot + 1), "n"(kSlotThreads) : "memory"); };
-        auto copy_rows = [&](const T *src, long long stride, long long row0, int cols, int chunks, uint32_t tile, int chunk0, int vec) {
-            if (vec) {
-#pragma unroll 2
-                for (int id = tid; id < kTileRows * chunks; id += kSlotThreads) {
-                    const int r = id / chunks, c = id - r * chunks;
-                    const long long grow = row0 + r;
-                    const bool inside = grow < n_rows && 8 * c < cols;
-                    const T *from = inside ? src + grow * stride + 8 * c : src;
-                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(tile + r * 128 + (((chunk0 + c) ^ (r & 7)) << 4)), "l"(from),
-                                 "r"(inside ? 16 : 0)
-                                 : "memory");
-                }
-            } else {
-#pragma unroll 1
-                for (int id = tid; id < kTileRows * chunks; id += kSlotThreads) {
-                    const int r = id / chunks, c = id - r * chunks;
-                    const long long grow = row0 + r;
-                    const bool inside = grow < n_rows && 8 * c < cols;
-                    const unsigned short *from = reinterpret_cast<const unsigned short *>(inside ? src + grow * stride + 8 * c : src);
-                    st_shared_16(tile + r * 128 + (((chunk0 + c) ^ (r & 7)) << 4), inside ? gather8(from, 8 * c, cols) : make_uint4(0, 0, 0, 0));
-                }
-            }
-        };
+        uint32_t buf = 0, rows0 = 0, prev_buf = 0, full_phase = 0, tiles_done = 0;
         // operands written -> the slot's warp 0 issues the step's own MMAs (and hands the wgrad to the wgrad warp)
         auto start_step = [&](int j) {
             fence_async_smem();
@@ -321,14 +422,36 @@ slots_mlp_bwd_tc_kernel(const MlpShape s, const MlpParams p, const __grid_consta
             slot_sync();
             if (issuer && !*abort_now) {
                 tc_fence_after();
+                if (j == 0) {
+                    // the buffer of the tile before holds its input gradient now; this tile's rows
+                    if (tiles_done > 0 && leader) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(&tb.empty[prev_buf])) : "memory");
+                    pipe_wait(smem_addr(&tb.full[buf]), full_phase, &tb.abort_flag);
+                    __syncwarp();
+                }
                 if (j >= d && leader) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(ready_bar) : "memory");
                 const SlotStep &st = tb.steps[j];
                 const uint4 own = *reinterpret_cast<const uint4 *>(&st.a_off);
                 if (own.z != 0) {
-                    issue_gemm(leader, acc, tile0 + own.x, 32, own.y, (own.w & 256u) ? 2048 : 32, static_cast<int>(own.w & 255u), own.z, false);
+                    if (j == 0 || j == d) {
+                        if (leader) {
+                            const uint32_t a_low = desc_low(rows0 + own.x), b_low = desc_low(own.y), b_step = (own.w & 256u) ? 128 : 2;
+                            for (int k = 0; k < static_cast<int>(own.w & 255u); ++k)
+                                mma_f16(acc, desc_of(a_low + 2 * k, st.a_high), smem_desc(b_low + k * b_step), own.z, k > 0);
+                        }
+                    } else {
+                        issue_gemm(leader, acc, tile0 + own.x, 32, own.y, (own.w & 256u) ? 2048 : 32, static_cast<int>(own.w & 255u), own.z, false);
+                    }
                     if constexpr (kPreact) {
                         if (st.z_k)
-                            issue_gemm(leader, acc + kAccCols, tile0 + st.za_off, 32, st.zb_addr, 32, static_cast<int>(st.z_k), instr_desc(128, s.h, bf16, 0, 0), false);
+{
+                            if (st.flags & 8u) {
+                                if (leader)
+                                    for (int k = 0; k < static_cast<int>(st.z_k); ++k)
+                                        mma_f16(acc + kAccCols, desc_of(desc_low(rows0) + 2 * k, desc_high(P.x_pitch)), smem_desc(desc_low(st.zb_addr) + 2 * k), instr_desc(128, s.h, bf16, 0, 0), k > 0);
+                            } else {
+                                issue_gemm(leader, acc + kAccCols, tile0 + st.za_off, 32, st.zb_addr, 32, static_cast<int>(st.z_k), instr_desc(128, s.h, bf16, 0, 0), false);
+                            }
+                        }
                     }
                     if (leader) mma_commit(acc_bar);
                 }
@@ -346,13 +469,9 @@ slots_mlp_bwd_tc_kernel(const MlpShape s, const MlpParams p, const __grid_consta
             return !*abort_now;
         };
         for (long long k = slot; k < n_mine; k += S) {
-            const long long row0 = (first_tile + k * tile_stride) * kTileRows;
-            if (!*abort_now) {
-                copy_rows(x, x_stride, row0, s.d_in, s.ki / 8, tile0, 0, x_vec);
-                copy_rows(go, go_stride, row0, s.d_out, s.no / 8, P.packed ? tile0 : act_addr(d + 1), P.packed ? 4 : 0, go_vec);
-                asm volatile("cp.async.commit_group;" ::: "memory");
-                async_tile_wait();
-            }
+            buf = static_cast<uint32_t>(k % P.rings);
+            full_phase = static_cast<uint32_t>((k / P.rings) & 1);
+            rows0 = ring_of(buf);
             for (int l = 0; l < d; ++l) {  // recomputed activation of layer l -> input tile of layer l + 1
                 start_step(l);
                 if (finish_step(true, false)) {
@@ -404,22 +523,27 @@ slots_mlp_bwd_tc_kernel(const MlpShape s, const MlpParams p, const __grid_consta
                         });
                     }
                 } else if (ok && gx != nullptr) {
-                    const bool live = row0 + row < n_rows;
-                    T *row_ptr = gx + (live ? row0 + row : 0) * gx_stride;
+                    // into the tile's row buffer, whose readers are done: the row warps send it off
+                    const uint32_t at = rows0 + row * P.x_pitch, swz = row_swizzle_of(row, P.x_pitch);
                     for_row_pieces<W>(taddr, in_pad, half, [&](int chunk, const uint32_t(&piece)[8]) {
-                        if (live) store_chunk_to_global<T>(row_ptr, chunk, s.d_in, finish8<T, TH_ACT_NONE, false>(piece, nullptr), gx_vec);
+                        st_shared_16(at + ((chunk ^ swz) << 4), finish8<T, TH_ACT_NONE, false>(piece, nullptr));
                     });
                     tc_fence_before();
                 }
             }
+            prev_buf = buf;
+            ++tiles_done;
         }
+        fence_async_smem();
+        slot_sync();
+        if (tiles_done > 0 && leader) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(&tb.empty[prev_buf])) : "memory");
     }
 
     // ---- flush the weight gradients (M = 64 layout: lanes 0..15 of warp quarter q hold rows 16 q ..); a warpgroup per layer ----
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    if (!tb.abort_flag && n_mine > 0 && !is_wgrad_warp) {
+    if (!tb.abort_flag && n_mine > 0 && !is_wgrad_warp && !is_row_warp) {
         const MlpGradWorkspace G = grad_workspace_layout(s, workspace);
         const int wq = warp & 3;
         const uint32_t lane_base = static_cast<uint32_t>(32 * wq) << 16;
@@ -427,9 +551,21 @@ slots_mlp_bwd_tc_kernel(const MlpShape s, const MlpParams p, const __grid_consta
             const int in_pad = l == 0 ? s.ki : s.h;
             const int in_dim = l == 0 ? s.d_in : s.d_hid, out_dim = l == d ? s.d_out : s.d_hid;
             float *dst = G.base + (l == 0 ? G.w_in : (l == d ? G.w_out : G.w_hid + (l - 1) * s.d_hid * s.d_hid));
-            const int o = 16 * wq + lane - ((l == d && P.packed) ? 32 : 0);  // output row this lane holds
+            const int o = 16 * wq + lane;  // gradient row this lane holds
+            if (l == d) {  // transposed: this lane holds input 16 wq + lane, a column an output
+                for (int first = 0; first < s.no; first += 16) {
+                    uint32_t raw[32];
+                    tmem_ld16(tmem + lane_base + dw_col(l) + first, raw);
+                    tmem_ld_wait();
+                    if (lane < 16 && o < in_dim) {
+#pragma unroll
+                        for (int c = 0; c < 16; ++c)
+                            if (first + c < out_dim) atomicAdd(dst + (first + c) * in_dim + o, __uint_as_float(raw[c]));
+                    }
+                }
+            }
             const bool quads = in_dim % 4 == 0 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0;
-            for (int first = 0; first < in_pad; first += 16) {
+            for (int first = 0; l < d && first < in_pad; first += 16) {
                 uint32_t raw[32];
                 tmem_ld16(tmem + lane_base + dw_col(l) + first, raw);
                 tmem_ld_wait();
@@ -473,18 +609,32 @@ bool one_slot_only() {
     return off;
 }
 
-// S slots of W warpgroups, if that fits one SM.  Measured (ms, B200), the most slots that fit are the fastest, two warpgroups
-// per slot when there are threads left: 2^21 rows 32-64-64-16 4 x 1 0.234, 3 x 2 0.269; 2^20 rows 32-4x64-16 2 x 2 0.277, 1 x 2 0.45;
-// with biases 32-64-64-16 3 x 2 0.158, 2 x 2 0.20; 300 007 rows 32-3x64-3 SiLU with biases 2 x 2 0.145 (0.218, and 1 x 2 0.40, with a division in the sigmoid).  The kernels this
-// one replaced (four one-warpgroup slots with a polling warp each; one tile per CTA for biases and SiLU): 0.271, 0.333, 0.340 and
-// 0.412.  Tried: dz in a tile of its own so that the chain waits for a weight gradient one step late, next rows fetched ahead into
-// it (0.290 at 32-4x64-16 against 0.284, and a slot less where it costs one); loops over 32 columns left rolled because
-// unrolled ones overflow the instruction cache (2^21 rows: 0.280 against 0.234).
+// A matrix of rows as boxes of 128 rows of a row buffer: `pitch` bytes of every row (zeros past the last column)
+bool make_rows_map(CUtensorMap *map, const void *base, long long rows, int cols, int pitch, long long row_stride) {
+    EncodeTiledFn encode = encode_tiled_fn();
+    memset(map, 0, sizeof(*map));
+    if (!encode || !base || cols % 8 != 0 || row_stride % 8 != 0 || !aligned_to(base, 16) || rows >= (1ll << 31) - kTileRows) return false;
+    const cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
+    const cuuint64_t strides[1] = {static_cast<cuuint64_t>(row_stride) * 2};
+    const cuuint32_t box[2] = {static_cast<cuuint32_t>(pitch / 2), kTileRows};
+    const cuuint32_t elem[2] = {1, 1};
+    return encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, const_cast<void *>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  pitch == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : (pitch == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B),
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// S slots of W warpgroups and `rings` row buffers, if that fits one SM.
 template <typename T, int ACT, bool BIAS, int S, int W>
-int launch_slots(const MlpShape &s, const MlpParams &p, const void *x, int64_t x_stride, const void *go, int64_t go_stride,
+int launch_slots(int rings, const MlpShape &s, const MlpParams &p, const void *x, int64_t x_stride, const void *go, int64_t go_stride,
                  void *gx, int64_t gx_stride, float *workspace, int64_t rows, cudaStream_t stream) {
-    const SlotPlan P = slot_plan(s, S);
+    SlotPlan P = slot_plan(s, S, rings);
     if (P.total > kSmemBudget || P.tmem_cols > 512 || 2 * s.depth + 1 > kStepsMax) return kTcNotApplicable;
+    CUtensorMap x_map, go_map, gx_map;
+    memset(&gx_map, 0, sizeof(gx_map));
+    const bool x_tma = make_rows_map(&x_map, x, rows, s.d_in, P.x_pitch, x_stride), go_tma = make_rows_map(&go_map, go, rows, s.d_out, P.go_pitch, go_stride);
+    const bool gx_tma = gx != nullptr && make_rows_map(&gx_map, gx, rows, s.d_in, P.x_pitch, gx_stride);
+    P.row_warps = x_tma && go_tma && (gx_tma || gx == nullptr) ? 1 : 4;
+    if (P.row_warps > kRowWarps<S, W>) return kTcNotApplicable;
     int smem = P.total;
     if (smem < kSmemBudget / 2 + 1024) smem = kSmemBudget / 2 + 1024;  // one CTA per SM
     WeightMaps maps;
@@ -494,19 +644,26 @@ int launch_slots(const MlpShape &s, const MlpParams &p, const void *x, int64_t x
                              "cudaFuncSetAttribute(slots_mlp_bwd_tc_kernel)")) return rc;
     const long long tiles = (rows + kTileRows - 1) / kTileRows;
     const long long cap = sm_count();
-    kernel<<<static_cast<unsigned>(tiles < cap ? tiles : cap), 128 * S * W + 32, smem, stream>>>(
-        s, p, maps, use_tma, P, static_cast<const T *>(x), x_stride, static_cast<const T *>(go), go_stride, static_cast<T *>(gx), gx_stride,
-        workspace, rows, rows_vector_ok(x, x_stride, s.d_in), rows_vector_ok(go, go_stride, s.d_out), gx ? rows_vector_ok(gx, gx_stride, s.d_in) : 0);
+    kernel<<<static_cast<unsigned>(tiles < cap ? tiles : cap), 128 * S * W + 32 + 32 * kRowWarps<S, W>, smem, stream>>>(
+        s, p, maps, use_tma, x_map, go_map, gx_map, (x_tma ? 1 : 0) | (go_tma ? 2 : 0) | (gx_tma ? 4 : 0), P, static_cast<const T *>(x), x_stride,
+        static_cast<const T *>(go), go_stride, static_cast<T *>(gx), gx_stride, workspace, rows);
     return launch_status("slots_mlp_bwd_tc_kernel launch");
 }
 
+// The most slots that fit are the fastest, two warpgroups per slot when there are threads left, and then one row buffer more than
+// slots (B200, ms; with / without the spare buffer): 2^21 rows 32-64-64-16 4 x 1 0.209 / 0.231, 3 x 2 0.250; 2^20 rows 32-4x64-16
+// 2 x 2 0.265 / 0.293; 300 007 rows 32-3x64-16 with biases 3 x 2 0.069, 2 x 2 0.081; 2^18 rows 32-64-64-16 with biases 4 x 1 0.043, 3 x 2
+// 0.048.  Tried: dz in a tile of its own so that the chain waits for a weight gradient one step late (0.287 at 32-4x64-16: MMAs run
+// in the order of issue, and the next step's queue behind the weight gradient's all the same); the chain's A operands in tensor memory
+// (0.304; the epilogue writes both places); unrolled loops over 32 columns (2^21 rows: 0.280 against 0.234).
 template <typename T, int ACT, bool BIAS>
 int launch_any_slots(const MlpShape &s, const MlpParams &p, const void *x, int64_t x_stride, const void *go, int64_t go_stride, void *gx,
                      int64_t gx_stride, float *workspace, int64_t rows, cudaStream_t stream) {
-#define TH_SLOTS(S, W)                                                                                                          \
-    if (const int rc = launch_slots<T, ACT, BIAS, S, W>(s, p, x, x_stride, go, go_stride, gx, gx_stride, workspace, rows, stream); \
-        rc != kTcNotApplicable)                                                                                                 \
-        return rc;
+#define TH_SLOTS(S, W)                                                                                                                        \
+    for (int rings = S + 1; rings >= S; --rings)                                                                                              \
+        if (const int rc = launch_slots<T, ACT, BIAS, S, W>(rings, s, p, x, x_stride, go, go_stride, gx, gx_stride, workspace, rows, stream); \
+            rc != kTcNotApplicable)                                                                                                           \
+            return rc;
     if (!one_slot_only()) {
         TH_SLOTS(4, 1)
         TH_SLOTS(3, 2)
