@@ -428,13 +428,13 @@ int launch_rev_bwd(const RevShape &s, const RevParams &p, const void *y, int64_t
     if (int rc = cuda_status(cudaFuncSetAttribute(rev_bwd_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, L.total),
                              "cudaFuncSetAttribute(rev_bwd_kernel)")) return rc;
     const int grid = rev_grid(rows);
-    const size_t bytes = sizeof(float) * rev_cta_floats(s) * grid;
-    if (int rc = cuda_status(cudaMemsetAsync(workspace, 0, bytes, stream), "cudaMemsetAsync(workspace)")) return rc;
     // tensor-core kernels first (they also reduce and write the gradients); mma.sync kernels otherwise
     const int tc = rows > 0 ? rev_bwd_tc(s, p, y, y_stride, go, go_stride, gx, gx_stride, x_rec, xr_stride, dw, db, workspace, grid,
                                          rows, std::is_same<T, __half>::value ? TH_F16 : TH_BF16, stream)
                             : kRevTcNotApplicable;
     if (tc != kRevTcNotApplicable) return tc;
+    const size_t bytes = sizeof(float) * rev_cta_floats(s) * grid;
+    if (int rc = cuda_status(cudaMemsetAsync(workspace, 0, bytes, stream), "cudaMemsetAsync(workspace)")) return rc;
     if (rows > 0) {
         rev_bwd_kernel<T><<<grid, kRevThreads, L.total, stream>>>(
             s, p, static_cast<const T *>(y), y_stride, static_cast<const T *>(go), go_stride, static_cast<T *>(gx),

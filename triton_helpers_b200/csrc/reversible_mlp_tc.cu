@@ -17,17 +17,22 @@
 //
 // Weights (4 matrices per block) stream block by block through a two-stage cp.async ring in the
 // operand-tile layout; the same tile is read K-major by the forward GEMMs and MN-major by dgrad.
-// Weight gradients of a (tile, block, branch) leave TMEM straight into the CTA's private fp32
-// accumulator in global memory (vector red.global.add, one owner per copy, L2 resident), carried
-// out by four extra warps while the other eight are already in the next branch; a reduction
-// kernel sums the copies.  The backward pass needs all 512 TMEM columns, so one CTA per SM; the
-// forward pass needs 192 (256 allocated), two CTAs per SM.
+// Weight gradients of a (tile, block, branch) leave TMEM for staging in shared memory and from there as bulk reductions
+// (cp.reduce.async.bulk, 4 KB each) for one of kRevCopies fp32 accumulators in global memory, carried out by four extra warps while
+// the other eight are already in the next branch; a reduction kernel sums the copies.  As vector reductions of the four warps they
+// shared the load / store pipe with the chain's stores: 32 KB a branch, 17 % of the kernel (2^19 rows, eight blocks of 64 -> 64 -> 64:
+// 0.872 -> 0.757 ms, 0.72 with no reductions at all).  How many CTAs add to one copy makes no difference to them (1 to 148 copies:
+// 0.87 to 0.88 ms), to the zero fill and the sum over the copies it does.
+//
+// The chain's A operands (U and DY, h and dz) lie in 64 TMEM columns besides their tiles, which the weight gradients read: an MMA
+// then takes 43 cycles instead of 76.  The two weight-gradient accumulators (M = 64) share 64 columns, one in lanes 0..15 and one in
+// lanes 16..31 of every quarter.  Backward 512 columns, one CTA per SM; forward 192 (256 allocated), two.
 //
 // Bias gradients are column sums of the DY and DZ tiles, formed by the flush warps while the chain goes on (in the chain's
 // epilogues they cost 2 us a pass): tensor memory has no columns left for the MMA with ones that the fused MLP uses.
 //
-// Measured with biases and SiLU, 2^17 rows, six blocks of 64 -> 64 -> 64: 0.431 ms (mma.sync 0.70); without biases, ReLU,
-// 2^20 rows, eight blocks: 2.22 ms.
+// Measured, backward: with biases and SiLU, 2^17 rows, six blocks of 64 -> 64 -> 64 0.397 -> 0.360 ms; without biases, ReLU, eight
+// blocks, 2^19 rows 0.933 -> 0.757 ms, 5 003 rows 56 -> 45 us.
 //
 // Covered here: float16 / bfloat16, 16-byte-aligned rows.  Everything else stays on the mma.sync kernels.
 #include "rev_shape.cuh"
@@ -46,12 +51,13 @@ constexpr int kStageBytes = 4 * kWTileBytes;     // [f1 | f2 | g1 | g2]
 constexpr int kS1 = 0, kS2 = 64;                 // the stream
 constexpr int kFwdHid = 128;                     // forward: hidden pre-activation
 constexpr int kFwdAU = 192, kFwdAH = 224;        // forward: 16-bit A operands (the branch's input, its hidden activation), 32 columns each
-constexpr int kD1 = 128, kD2 = 192, kZ = 256, kDH = 320, kDW1 = 384, kDW2 = 448;  // backward
+constexpr int kD1 = 128, kD2 = 192, kZ = 256, kDH = 320, kDW1 = 384, kDW2 = 384 + (16 << 16), kA0 = 448, kA1 = 480;  // backward; kDW2: lanes 16..31
 
 struct RevTcPlan {
     int tiles;     // operand tiles before the weight ring (2 forward, 8 backward)
     int ring;      // byte offset of the ring (2 stages)
     int bias;      // fp32 [2 stages][4][64]
+    int stage;     // backward: 8 KB of weight gradients per flush warp
     int total;
     int tmem_cols;
 };
@@ -61,7 +67,8 @@ __host__ __device__ inline RevTcPlan rev_tc_plan(bool backward) {
     p.tiles = backward ? 8 : 2;
     p.ring = p.tiles * kTileBytes;
     p.bias = p.ring + 2 * kStageBytes;
-    p.total = p.bias + 2 * 4 * kMaxDim * 4;
+    p.stage = p.bias + 2 * 4 * kMaxDim * 4;
+    p.total = p.stage + (backward ? 32768 : 0);
     p.tmem_cols = backward ? 512 : 256;
     return p;
 }
@@ -127,8 +134,8 @@ struct RevRowMaps {
 
 template <typename T, bool BIAS>
 __device__ __forceinline__ void prefetch_weights_tma(unsigned char *smem, const RevTcPlan &P, const RevShape &s, const RevParams &p,
-                                     const RevWeightMaps &maps, unsigned long long *ring_bars, int k, int stage) {
-    if (threadIdx.x == 64) {  // not warp 0, which is about to issue MMAs
+                                     const RevWeightMaps &maps, unsigned long long *ring_bars, int k, int stage, volatile int *abort_now = nullptr) {
+    if (threadIdx.x == 64 && !(abort_now && *abort_now)) {  // not warp 0, which is about to issue MMAs
         const uint32_t bar = smem_addr(&ring_bars[stage]);
         const uint32_t bytes = static_cast<uint32_t>(2 * (s.hid + s.half) * 128);  // four boxes of 64 columns
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
@@ -222,8 +229,8 @@ __device__ __forceinline__ bool commit_and_wait(bool leader, uint32_t bar, uint3
     return cta_wait_mma(bar, phase, abort_flag);
 }
 
-__device__ __forceinline__ void publish_tiles() {
-    fence_async_smem();
+__device__ __forceinline__ void publish(bool to_async_proxy) {
+    if (to_async_proxy) fence_async_smem();
     tc_fence_before();
     __syncthreads();
 }
@@ -238,8 +245,8 @@ rev_fwd_tc_kernel(const RevShape shape, const RevParams p, const __grid_constant
                   const T *__restrict__ x, long long x_stride, T *__restrict__ y, long long y_stride, long long n_rows) {
     constexpr bool kRolled = HALF == 0, kLines = HALF > 0 && HID == 0;
     const RevShape s = known_widths<HALF, HID>(shape);
-    extern __shared__ unsigned char smem_raw[];
-    unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    unsigned char *smem = smem_raw;
     __shared__ uint32_t tmem_holder;
     __shared__ __align__(8) unsigned long long mbar;
     __shared__ int abort_flag;
@@ -260,6 +267,9 @@ rev_fwd_tc_kernel(const RevShape shape, const RevParams p, const __grid_constant
         prefetch_weights_tma<T, BIAS>(smem, P, s, p, maps, ring_bars, 0, 0);
         ring_wait(ring_bars, 0, &abort_flag);
     }
+    // With the A operands in tensor memory and the weights by TMA nothing that an MMA reads is written by a thread, and the fence
+    // between the two proxies, which waits for the row loads and stores in flight, is left out (2^19 rows, eight blocks: 0.250 -> 0.229 ms)
+    const bool needs_fence = !TA || !use_tma;
     const uint32_t bar = smem_addr(&mbar);
     const Seat seat;
     const uint32_t taddr = tmem + seat.lane_base;
@@ -284,7 +294,7 @@ rev_fwd_tc_kernel(const RevShape shape, const RevParams p, const __grid_constant
                 tmem_st4(taddr + kFwdAU + 4 * (first + u), *reinterpret_cast<const uint4 *>(chunk_ptr(u_tile, seat.row, first + u)));
         }
         tmem_st_wait();
-        publish_tiles();
+        publish(needs_fence);
 
         for (int k = 0; k < s.blocks && !abort_flag; ++k, ++step) {
             const int stage = step & 1;
@@ -320,7 +330,7 @@ rev_fwd_tc_kernel(const RevShape shape, const RevParams p, const __grid_constant
                     });
                     if constexpr (TA) tmem_st_wait();
                 }
-                publish_tiles();
+                publish(needs_fence);
                 if (threadIdx.x < 32) {
                     leader = elect_one();
                     tc_fence_after();
@@ -340,7 +350,7 @@ rev_fwd_tc_kernel(const RevShape shape, const RevParams p, const __grid_constant
                     if (!use_tma) async_tile_wait();
                     else if (more) ring_wait(ring_bars, step + 1, &abort_flag);
                 }
-                publish_tiles();
+                publish(needs_fence);
             }
         }
     }
@@ -353,11 +363,8 @@ rev_fwd_tc_kernel(const RevShape shape, const RevParams p, const __grid_constant
 
 // ---- backward ----------------------------------------------------------------------------------
 
-// One weight-gradient accumulator (M = 64 layout) out of TMEM, added into this CTA's private copy.
-// The copy of a matrix is stored [column / 4][row][column % 4]: the 16 lanes of a warp that hold rows
-// m .. m + 15 of one column quad then add to 256 contiguous bytes (8 full sectors per instruction
-// instead of 16 half-used ones), which is what the L2's reduction rate is counted in.
-__host__ __device__ inline int dw_private_index(int row, int col) { return ((col >> 2) * 64 + row) * 4 + (col & 3); }
+// A copy of a matrix is stored [row / 16][column / 4][row % 16][column % 4]: what one flush warp holds of it is contiguous.
+constexpr int kRevCopies = 16;
 
 // The backward kernel runs 256 "main" threads (the chain: issue, wait, epilogue) and 128 "flush" threads
 // that carry the weight gradients of a pass out of TMEM while the main threads are already in the next pass.
@@ -382,47 +389,48 @@ __device__ __forceinline__ bool rev_wait(uint32_t bar, uint32_t parity, int *abo
             : "r"(bar), "r"(parity)
             : "memory");
         if (done) return true;
-        if ((poll & 63) == 63 && *reinterpret_cast<volatile int *>(abort_flag)) return false;
+        if (*reinterpret_cast<volatile int *>(abort_flag)) return false;
     }
     *reinterpret_cast<volatile int *>(abort_flag) = 1;
     return false;
 }
 
-// cta_wait_mma for the main threads: warp 0 polls, the others park at the main barrier
-__device__ __forceinline__ bool main_wait_mma(uint32_t mbar, uint32_t &phase, int *abort_flag) {
-    if (threadIdx.x < 32) {
-        rev_wait(mbar, phase, abort_flag);
-        tc_fence_after();
-        tc_fence_before();
-    }
+// The MMAs committed to `mbar` are done.  Every main warp polls: with one polling and the others parked at a barrier behind it
+// 0.805 against 0.757 ms (2^19 rows, eight blocks).
+__device__ __forceinline__ void main_wait_mma(uint32_t mbar, uint32_t &phase, int *abort_flag) {
+    rev_wait(mbar, phase, abort_flag);
+    __syncwarp();
     phase ^= 1;
-    main_sync();
     tc_fence_after();
-    return *reinterpret_cast<volatile int *>(abort_flag) == 0;
 }
 
-// One flush warp's share (TMEM lanes 32 q .. 32 q + 15 = gradient rows 16 q .. 16 q + 15) of one accumulator
-__device__ __forceinline__ void flush_dw_quadrant(uint32_t tmem, int q, uint32_t col, int out_dim, int in_dim, float *dst) {
+// One flush warp's share of both accumulators: TMEM lanes 32 q .. 32 q + 15 hold rows 16 q .. of the first matrix, the other sixteen
+// those of the second.  The accumulators are free once they are in registers.
+__device__ __forceinline__ void flush_dw_pair(uint32_t tmem, int q, uint32_t stage, float *dst, uint32_t flushed) {
     const int lane = threadIdx.x & 31;
-    const int m = 16 * q + lane;
-    const bool owner = lane < 16 && m < out_dim;
-    const uint32_t taddr = tmem + (static_cast<uint32_t>(32 * q) << 16) + col;
-    // The private copies (0.5 MB per CTA) are revisited once per row tile while a gigabyte of rows streams through
-    // L2: ask the L2 to keep their lines (evict-last), or most of the reductions end up in DRAM.
-    unsigned long long keep;
-    asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(keep));
-    for (int first = 0; first < in_dim; first += 16) {
-        uint32_t raw[32];
-        tmem_ld16(taddr + first, raw);
-        tmem_ld_wait();
-        if (owner) {
+    const uint32_t taddr = tmem + (static_cast<uint32_t>(32 * q) << 16) + kDW1;
+    uint32_t lo[32], hi[32];
+    tmem_ld32(taddr, lo);
+    tmem_ld32(taddr + 32, hi);
+    tmem_ld_wait();
+    tc_fence_before();
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // the reductions before have been read
+    __syncwarp();
+    if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(flushed) : "memory");
+    const uint32_t at = stage + (lane >> 4) * 4096 + (lane & 15) * 16;
 #pragma unroll
-            for (int h = 0; h < 4; ++h)
-                asm volatile("red.global.add.L2::cache_hint.v4.f32 [%0], {%1, %2, %3, %4}, %5;" ::"l"(dst + dw_private_index(m, first + 4 * h)),
-                             "f"(__uint_as_float(raw[4 * h])), "f"(__uint_as_float(raw[4 * h + 1])),
-                             "f"(__uint_as_float(raw[4 * h + 2])), "f"(__uint_as_float(raw[4 * h + 3])), "l"(keep)
-                             : "memory");
-        }
+    for (int h = 0; h < 8; ++h) st_shared_16(at + h * 256, make_uint4(lo[4 * h], lo[4 * h + 1], lo[4 * h + 2], lo[4 * h + 3]));
+#pragma unroll
+    for (int h = 0; h < 8; ++h) st_shared_16(at + 2048 + h * 256, make_uint4(hi[4 * h], hi[4 * h + 1], hi[4 * h + 2], hi[4 * h + 3]));
+    fence_async_smem();
+    __syncwarp();
+    if (lane == 0) {
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+            asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], 4096;" ::"l"(dst + m * kMatFloats + q * 1024),
+                         "r"(stage + m * 4096)
+                         : "memory");
+        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
     }
 }
 
@@ -465,8 +473,8 @@ rev_bwd_tc_kernel(const RevShape shape, const RevParams p, const __grid_constant
                   T *__restrict__ x_rec, long long xr_stride, float *__restrict__ workspace, long long n_rows) {
     constexpr bool kRolled = HALF == 0, kLines = HALF > 0 && HID == 0;
     const RevShape s = known_widths<HALF, HID>(shape);
-    extern __shared__ unsigned char smem_raw[];
-    unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    unsigned char *smem = smem_raw;
     __shared__ uint32_t tmem_holder;
     __shared__ __align__(8) unsigned long long mbar;
     __shared__ int abort_flag;
@@ -484,9 +492,11 @@ rev_bwd_tc_kernel(const RevShape shape, const RevParams p, const __grid_constant
     // operands_bar: h and dz of a pass are in place and the chain's MMAs on them issued (one arrival)
     // BIAS - summed_bar: the flush warps have summed the columns of dz and dy
     // rows_bar: the four TMA boxes of a row tile have landed
+    // the main threads' copy of the abort flag: written before a barrier of theirs and read behind it, so that all of them leave together
+    __shared__ int stop_flag;
     __shared__ __align__(8) unsigned long long wgrad_bar, flushed_bar, operands_bar, summed_bar, rows_bar;
     if (threadIdx.x == 0) {
-        abort_flag = 0;
+        abort_flag = stop_flag = 0;
         asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&ring_bars[0])), "r"(1u) : "memory");
         asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&ring_bars[1])), "r"(1u) : "memory");
         asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&wgrad_bar)), "r"(1u) : "memory");
@@ -499,13 +509,14 @@ rev_bwd_tc_kernel(const RevShape shape, const RevParams p, const __grid_constant
     const long long n_tiles = (n_rows + kTileRows - 1) / kTileRows;
     if (!is_flush && !use_tma && static_cast<long long>(blockIdx.x) < n_tiles) prefetch_weights<T>(smem, P, shape, p, s.blocks - 1, 0);
     const uint32_t tmem = cta_setup(&tmem_holder, &mbar, P.tmem_cols);  // publishes the barrier inits
-    float *cta_acc = workspace + static_cast<size_t>(blockIdx.x) * rev_cta_floats(s);
+    float *cta_acc = workspace + static_cast<size_t>(blockIdx.x % kRevCopies) * rev_cta_floats(s);
     const uint32_t wgrad_addr = smem_addr(&wgrad_bar), flushed_addr = smem_addr(&flushed_bar);
     const uint32_t operands_addr = smem_addr(&operands_bar), summed_addr = smem_addr(&summed_bar);
 
     if (is_flush) {
         // ================= weight gradients out of TMEM, one pass behind the main threads =================
         const int q = (threadIdx.x >> 5) & 3;
+        const uint32_t stage = smem_addr(smem + P.stage) + q * 8192;
         const uint32_t id_dw2 = instr_desc(64, s.hid, bf16, 1, 1), id_dw1 = instr_desc(64, s.half, bf16, 1, 1);  // both operands MN-major, M = 64
         uint32_t n = 0;  // passes flushed so far
         bool alive = true;
@@ -540,14 +551,11 @@ rev_bwd_tc_kernel(const RevShape shape, const RevParams p, const __grid_constant
                     if (!alive) break;
                     tc_fence_after();
                     const int m1 = pass == 0 ? 2 : 0;
-                    flush_dw_quadrant(tmem, q, kDW1, s.hid, s.half, block_acc + m1 * kMatFloats);
-                    flush_dw_quadrant(tmem, q, kDW2, s.half, s.hid, block_acc + (m1 + 1) * kMatFloats);
-                    tc_fence_before();
-                    __syncwarp();
-                    if ((threadIdx.x & 31) == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(flushed_addr) : "memory");
+                    flush_dw_pair(tmem, q, stage, block_acc + m1 * kMatFloats, flushed_addr);
                 }
             }
         }
+        if ((threadIdx.x & 31) == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     } else {
         // ================= the chain =================
         if (use_tma && static_cast<long long>(blockIdx.x) < n_tiles) {
@@ -573,7 +581,7 @@ rev_bwd_tc_kernel(const RevShape shape, const RevParams p, const __grid_constant
         auto fetch_rows = [&](long long row0, uint32_t copy) {
             unsigned char *u_in = u_tiles + copy * kTileBytes, *dy_in = dy_tiles + copy * kTileBytes;
             if (use_tma) {
-                if (threadIdx.x == 64) {
+                if (threadIdx.x == 64 && !*abort_now) {
                     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(rows_addr), "r"(4u * kTileBytes) : "memory");
                     const int at = static_cast<int>(row0);
                     tma_load_2d(u_in, &row_maps.y1, 0, at, rows_addr);
@@ -591,7 +599,8 @@ rev_bwd_tc_kernel(const RevShape shape, const RevParams p, const __grid_constant
         uint32_t rows_phase = 0;
         if (static_cast<long long>(blockIdx.x) < n_tiles) fetch_rows(static_cast<long long>(blockIdx.x) * kTileRows, 0);
 
-        for (long long tile = blockIdx.x; tile < n_tiles && !*abort_now; tile += gridDim.x) {
+        volatile int *stop = &stop_flag;
+        for (long long tile = blockIdx.x; tile < n_tiles && !*stop; tile += gridDim.x) {
             const long long row0 = tile * kTileRows;
             const bool live = row0 + seat.row < n_rows;
             unsigned char *u_in = u_tiles + (n & 1u) * kTileBytes, *dy_in = dy_tiles + (n & 1u) * kTileBytes;
@@ -606,14 +615,21 @@ rev_bwd_tc_kernel(const RevShape shape, const RevParams p, const __grid_constant
             tile_row_to_tmem<T>(y2_tile, seat, s.half, taddr + kS2);
             tile_row_to_tmem<T>(go1_tile, seat, s.half, taddr + kD1);
             tile_row_to_tmem<T>(dy_in, seat, s.half, taddr + kD2);
+            {
+                const int count = s.half / (8 * kGroups), first = seat.group * count;
+                for (int u = 0; u < count; ++u) {
+                    tmem_st4(taddr + kA0 + 4 * (first + u), *reinterpret_cast<const uint4 *>(chunk_ptr(u_in, seat.row, first + u)));
+                    tmem_st4(taddr + kA1 + 4 * (first + u), *reinterpret_cast<const uint4 *>(chunk_ptr(dy_in, seat.row, first + u)));
+                }
+            }
             tmem_st_wait();
             main_publish();
 
-            for (int k = s.blocks - 1; k >= 0 && !*abort_now; --k, ++step) {
+            for (int k = s.blocks - 1; k >= 0 && !*stop; --k, ++step) {
                 const int stage = step & 1;
                 const bool more = k > 0 || tile + gridDim.x < n_tiles;
                 if (more) {
-                    if (use_tma) prefetch_weights_tma<T, BIAS>(smem, P, s, p, maps, ring_bars, k > 0 ? k - 1 : s.blocks - 1, stage ^ 1);
+                    if (use_tma) prefetch_weights_tma<T, BIAS>(smem, P, s, p, maps, ring_bars, k > 0 ? k - 1 : s.blocks - 1, stage ^ 1, abort_now);
                     else prefetch_weights<T>(smem, P, shape, p, k > 0 ? k - 1 : s.blocks - 1, stage ^ 1);
                 }
                 const unsigned char *w = smem + P.ring + stage * kStageBytes;
@@ -631,8 +647,8 @@ rev_bwd_tc_kernel(const RevShape shape, const RevParams p, const __grid_constant
                     if (threadIdx.x < 32) {
                         const bool leader = elect_one();
                         tc_fence_after();
-                        issue_gemm<kLines>(leader, tmem + kZ, u_cur, 32, w1, 32, s.half / 16, id_z, false);
-                        issue_gemm<kLines>(leader, tmem + kDH, dy_cur, 32, w2, 2048, s.half / 16, id_dh, false);
+                        issue_gemm_ta<kLines>(leader, tmem + kZ, tmem + kA0, w1, 32, s.half / 16, id_z, false);
+                        issue_gemm_ta<kLines>(leader, tmem + kDH, tmem + kA1, w2, 2048, s.half / 16, id_dh, false);
                         if (leader) mma_commit(bar);
                         __syncwarp();
                     }
@@ -648,10 +664,10 @@ rev_bwd_tc_kernel(const RevShape shape, const RevParams p, const __grid_constant
                             tmem_st8(taddr + out_col + seat.group * nh + 8 * u, v);
                         });
                         tmem_st_wait();
-                        if (threadIdx.x < 32 && n > 0) rev_wait(summed_addr, (n - 1) & 1u, &abort_flag);
+                        if (n > 0) rev_wait(summed_addr, (n - 1) & 1u, &abort_flag);
                     }
                     // the previous pass's weight-gradient MMAs read the h and dz tiles the epilogue below overwrites
-                    if (threadIdx.x < 32 && n > 0) rev_wait(wgrad_addr, (n - 1) & 1u, &abort_flag);
+                    if (n > 0) rev_wait(wgrad_addr, (n - 1) & 1u, &abort_flag);
                     main_wait_mma(bar, phase, &abort_flag);
                     const bool last = k == 0 && pass == 1;
                     if (last && tile + gridDim.x < n_tiles) fetch_rows(row0 + static_cast<long long>(gridDim.x) * kTileRows, (n + 1) & 1u);
@@ -661,43 +677,70 @@ rev_bwd_tc_kernel(const RevShape shape, const RevParams p, const __grid_constant
                         const uint32_t row_off = seat.row * 128, row_swizzle = (seat.row & 7) << 4;
                         const uint32_t h_row = smem_addr(h_tile) + row_off, dz_row = smem_addr(dz_tile) + row_off;
                         const float *bias1 = block_bias + m1 * kMaxDim;
-                        for_each_piece<kRolled>(taddr + kZ + seat.group * nn, nn, [&](int u, const uint32_t(&piece)[8]) {
-                            st_shared_16(h_row + (((first + u) << 4) ^ row_swizzle), finish8<T, ACT, BIAS>(piece, bias1 + 8 * (first + u)));
-                        });
+                        auto store_h = [&](int u, uint4 q) {
+                            st_shared_16(h_row + (((first + u) << 4) ^ row_swizzle), q);
+                            tmem_st4(taddr + kA0 + 4 * (first + u), q);
+                        };
                         auto store_dz = [&](int u, uint4 g) {
                             st_shared_16(dz_row + (((first + u) << 4) ^ row_swizzle), g);
+                            tmem_st4(taddr + kA1 + 4 * (first + u), g);
                         };
-                        if constexpr (ACT == TH_ACT_SILU || ACT == TH_ACT_RELU2) {
-                            // the derivative is taken at the pre-activation rounded to the storage type
-#pragma unroll 1
-                            for (int u = 0; u < nn / 8; ++u) {
-                                uint32_t dh[8], zz[8];
-                                tmem_ld8(taddr + kDH + seat.group * nn + 8 * u, dh);
-                                tmem_ld8(taddr + kZ + seat.group * nn + 8 * u, zz);
-                                tmem_ld_wait();
-                                float g[8];
+                        if constexpr (HALF == 64 && HID == 64 && (ACT == TH_ACT_RELU || ACT == TH_ACT_NONE)) {
+                            // both accumulators in flight together, the mask from registers
+                            uint32_t zz[32], dh[32];
+                            tmem_ld32(taddr + kZ + seat.group * 32, zz);
+                            tmem_ld32(taddr + kDH + seat.group * 32, dh);
+                            tmem_ld_wait();
 #pragma unroll
-                                for (int e = 0; e < 8; ++e) {
-                                    float z = __uint_as_float(zz[e]);
-                                    if constexpr (BIAS) z += bias1[8 * (first + u) + e];
-                                    z = to_float<T>(from_float<T>(z));
-                                    g[e] = activate_grad(ACT, z, __uint_as_float(dh[e]));
-                                }
-                                store_dz(u, make_uint4(pack_pair<T>(g[0], g[1]), pack_pair<T>(g[2], g[3]), pack_pair<T>(g[4], g[5]), pack_pair<T>(g[6], g[7])));
-                            }
-                        } else {
-                            for_each_piece<kRolled>(taddr + kDH + seat.group * nn, nn, [&](int u, const uint32_t(&piece)[8]) {
-                                uint4 g = finish8<T, TH_ACT_NONE, false>(piece, nullptr);
+                            for (int u = 0; u < 4; ++u) {
+                                const uint4 h = finish8<T, ACT, BIAS>(zz + 8 * u, bias1 + 8 * (first + u));
+                                store_h(u, h);
+                                uint4 g = finish8<T, TH_ACT_NONE, false>(dh + 8 * u, nullptr);
                                 if constexpr (ACT == TH_ACT_RELU) {
-                                    const uint4 h = ld_shared_16(h_row + (((first + u) << 4) ^ row_swizzle));  // this thread's own store above
                                     g.x = keep_where_positive<T>(g.x, h.x);
                                     g.y = keep_where_positive<T>(g.y, h.y);
                                     g.z = keep_where_positive<T>(g.z, h.z);
                                     g.w = keep_where_positive<T>(g.w, h.w);
                                 }
                                 store_dz(u, g);
+                            }
+                        } else {
+                            for_each_piece<kRolled>(taddr + kZ + seat.group * nn, nn, [&](int u, const uint32_t(&piece)[8]) {
+                                store_h(u, finish8<T, ACT, BIAS>(piece, bias1 + 8 * (first + u)));
                             });
+                            if constexpr (ACT == TH_ACT_SILU || ACT == TH_ACT_RELU2) {
+                                // the derivative is taken at the pre-activation rounded to the storage type
+#pragma unroll 1
+                                for (int u = 0; u < nn / 8; ++u) {
+                                    uint32_t dh[8], zz[8];
+                                    tmem_ld8(taddr + kDH + seat.group * nn + 8 * u, dh);
+                                    tmem_ld8(taddr + kZ + seat.group * nn + 8 * u, zz);
+                                    tmem_ld_wait();
+                                    float g[8];
+#pragma unroll
+                                    for (int e = 0; e < 8; ++e) {
+                                        float z = __uint_as_float(zz[e]);
+                                        if constexpr (BIAS) z += bias1[8 * (first + u) + e];
+                                        z = to_float<T>(from_float<T>(z));
+                                        g[e] = activate_grad(ACT, z, __uint_as_float(dh[e]));
+                                    }
+                                    store_dz(u, make_uint4(pack_pair<T>(g[0], g[1]), pack_pair<T>(g[2], g[3]), pack_pair<T>(g[4], g[5]), pack_pair<T>(g[6], g[7])));
+                                }
+                            } else {
+                                for_each_piece<kRolled>(taddr + kDH + seat.group * nn, nn, [&](int u, const uint32_t(&piece)[8]) {
+                                    uint4 g = finish8<T, TH_ACT_NONE, false>(piece, nullptr);
+                                    if constexpr (ACT == TH_ACT_RELU) {
+                                        const uint4 h = ld_shared_16(h_row + (((first + u) << 4) ^ row_swizzle));  // this thread's own store above
+                                        g.x = keep_where_positive<T>(g.x, h.x);
+                                        g.y = keep_where_positive<T>(g.y, h.y);
+                                        g.z = keep_where_positive<T>(g.z, h.z);
+                                        g.w = keep_where_positive<T>(g.w, h.w);
+                                    }
+                                    store_dz(u, g);
+                                });
+                            }
                         }
+                        tmem_st_wait();
                     }
                     main_publish();
                     // step B: undo the branch and push the gradient through.  Then the flush warps may issue the two weight gradients:
@@ -706,8 +749,8 @@ rev_bwd_tc_kernel(const RevShape shape, const RevParams p, const __grid_constant
                     if (threadIdx.x < 32) {
                         const bool leader = elect_one();
                         tc_fence_after();
-                        issue_gemm<kLines>(leader, tmem + out_col, smem_addr(h_tile), 32, w2, 32, s.hid / 16, id_undo, true);
-                        issue_gemm<kLines>(leader, tmem + in_d_col, smem_addr(dz_tile), 32, w1, 2048, s.hid / 16, id_din, true);
+                        issue_gemm_ta<kLines>(leader, tmem + out_col, tmem + kA0, w2, 32, s.hid / 16, id_undo, true);
+                        issue_gemm_ta<kLines>(leader, tmem + in_d_col, tmem + kA1, w1, 2048, s.hid / 16, id_din, true);
                         if (leader) mma_commit(bar);
                         if (leader) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(operands_addr) : "memory");
                         __syncwarp();
@@ -715,18 +758,48 @@ rev_bwd_tc_kernel(const RevShape shape, const RevParams p, const __grid_constant
                     main_wait_mma(bar, phase, &abort_flag);
                     // next pass: its input is the stream just reconstructed, its output gradient the one just updated
                     if (!last) {
-                        stream_epilogue<T, false, kRolled>(taddr + out_col, seat, s.half, nullptr, u_next, nullptr, false);
-                        stream_epilogue<T, false, kRolled>(taddr + in_d_col, seat, s.half, nullptr, dy_next, nullptr, false);
+                        if constexpr (HALF == 64) {
+                            uint32_t su[32], sd[32];
+                            tmem_ld32(taddr + out_col + seat.group * 32, su);
+                            tmem_ld32(taddr + in_d_col + seat.group * 32, sd);
+                            tmem_ld_wait();
+                            const uint32_t row_off = seat.row * 128, row_swizzle = (seat.row & 7) << 4;
+                            const uint32_t u_row = smem_addr(u_next) + row_off, dy_row = smem_addr(dy_next) + row_off;
+#pragma unroll
+                            for (int u = 0; u < 4; ++u) {
+                                const int c = 4 * seat.group + u;
+                                const uint4 a = finish8<T, TH_ACT_NONE, false>(su + 8 * u, nullptr), g = finish8<T, TH_ACT_NONE, false>(sd + 8 * u, nullptr);
+                                st_shared_16(u_row + ((c << 4) ^ row_swizzle), a);
+                                st_shared_16(dy_row + ((c << 4) ^ row_swizzle), g);
+                                tmem_st4(taddr + kA0 + 4 * c, a);
+                                tmem_st4(taddr + kA1 + 4 * c, g);
+                            }
+                            tmem_st_wait();
+                        } else {
+                            auto both = [&](uint32_t from, unsigned char *tile, uint32_t a_col) {
+                                const int n8 = s.half / kGroups, first = seat.group * (n8 / 8);
+                                const uint32_t row_addr = smem_addr(tile) + seat.row * 128, row_swizzle = (seat.row & 7) << 4;
+                                for_each_piece<kRolled>(taddr + from + seat.group * n8, n8, [&](int u, const uint32_t(&piece)[8]) {
+                                    const uint4 q = finish8<T, TH_ACT_NONE, false>(piece, nullptr);
+                                    st_shared_16(row_addr + (((first + u) << 4) ^ row_swizzle), q);
+                                    tmem_st4(taddr + a_col + 4 * (first + u), q);
+                                });
+                            };
+                            both(out_col, u_next, kA0);
+                            both(in_d_col, dy_next, kA1);
+                            tmem_st_wait();
+                        }
                     }
                     if (pass == 1) {  // next block's weights have landed
                         if (!use_tma) async_tile_wait();
                         else if (more) ring_wait(ring_bars, step + 1, &abort_flag);
+                        if (threadIdx.x == 0) *stop = *abort_now;
                     }
                     main_publish();
                 }
             }
             // the stream is now the reconstructed input, the gradient stream the input gradient
-            if (!*abort_now) {
+            if (!*stop) {
 #pragma unroll 1
                 for (int q = 0; q < 4; ++q) {
                     // q: 0 = dx1 (D1), 1 = dx2 (D2), 2 = x1 (S1), 3 = x2 (S2)
@@ -750,36 +823,56 @@ rev_bwd_tc_kernel(const RevShape shape, const RevParams p, const __grid_constant
     cta_teardown(tmem, P.tmem_cols);
 }
 
-// Sum the per-CTA accumulators ([cta][block][matrix][64][64], then [block][4][64] bias sums) into the gradient tensors.
+// Sum the accumulators ([copy][block][matrix][column / 4][row][column % 4], then [block][4][64] bias sums) into the gradient
+// tensors: a thread sums one quad of every 8th copy, the block's eight shares meet in shared memory in a fixed order.
+constexpr int kReduceQuads = 32, kReduceShares = 8;
 template <typename T>
-__global__ void rev_grad_reduce_tc_kernel(const RevShape s, const float *__restrict__ workspace, int n_ctas, T *dw_f1, T *dw_f2, T *dw_g1,
+__global__ void __launch_bounds__(kReduceQuads * kReduceShares)
+rev_grad_reduce_tc_kernel(const RevShape s, const float *__restrict__ workspace, int copies, T *dw_f1, T *dw_f2, T *dw_g1,
                                           T *dw_g2, T *db_f1, T *db_f2, T *db_g1, T *db_g2) {
-    const size_t per_cta = rev_cta_floats(s);
-    const size_t mat_total = static_cast<size_t>(s.blocks) * 4 * kMatFloats;
-    const size_t total = s.has_bias ? per_cta : mat_total;
-    T *dw[4] = {dw_f1, dw_f2, dw_g1, dw_g2};
-    T *db[4] = {db_f1, db_f2, db_g1, db_g2};
-    for (size_t e = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; e < total;
-         e += static_cast<size_t>(gridDim.x) * blockDim.x) {
-        size_t at = e;
-        T *dst;
-        if (e < mat_total) {
-            const int k = static_cast<int>(e / (4 * kMatFloats));
-            const int m = static_cast<int>((e / kMatFloats) % 4);
-            const int row = static_cast<int>((e % kMatFloats) / 64), col = static_cast<int>(e % 64);
-            const int out_dim = (m & 1) ? s.half : s.hid, in_dim = (m & 1) ? s.hid : s.half;
-            if (row >= out_dim || col >= in_dim || !dw[m]) continue;
-            at = (e / kMatFloats) * kMatFloats + dw_private_index(row, col);
-            dst = dw[m] + (static_cast<size_t>(k) * out_dim + row) * in_dim + col;
-        } else {
-            const int b = static_cast<int>(e - mat_total), k = b / 256, m = (b / 64) % 4, c = b % 64;
-            const int width = (m & 1) ? s.half : s.hid;
-            if (c >= width || !db[m]) continue;
-            dst = db[m] + static_cast<size_t>(k) * width + c;
+    const size_t per_cta = rev_cta_floats(s), mat_total = static_cast<size_t>(s.blocks) * 4 * kMatFloats, total = s.has_bias ? per_cta : mat_total;
+    const int lane = threadIdx.x % kReduceQuads, share = threadIdx.x / kReduceQuads;
+    const size_t e = (static_cast<size_t>(blockIdx.x) * kReduceQuads + lane) * 4;
+    __shared__ float4 part[kReduceShares][kReduceQuads];
+    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+    T *dst = nullptr;
+    if (e < mat_total) {
+        const int k = static_cast<int>(e / (4 * kMatFloats)), m = static_cast<int>((e / kMatFloats) % 4);
+        const int at = static_cast<int>(e % kMatFloats), row = at / 1024 * 16 + at / 4 % 16, col = at / 64 % 16 * 4;
+        const int out_dim = (m & 1) ? s.half : s.hid, in_dim = (m & 1) ? s.hid : s.half;
+        T *dw = m == 0 ? dw_f1 : (m == 1 ? dw_f2 : (m == 2 ? dw_g1 : dw_g2));
+        if (dw && row < out_dim && col < in_dim) dst = dw + (static_cast<size_t>(k) * out_dim + row) * in_dim + col;
+    } else if (e < total) {
+        const int b = static_cast<int>(e - mat_total), k = b / 256, m = (b / 64) % 4, c = b % 64;
+        const int width = (m & 1) ? s.half : s.hid;
+        T *db = m == 0 ? db_f1 : (m == 1 ? db_f2 : (m == 2 ? db_g1 : db_g2));
+        if (db && c < width) dst = db + static_cast<size_t>(k) * width + c;
+    }
+    if (dst) {
+#pragma unroll 4
+        for (int c = share; c < copies; c += kReduceShares) {
+            const float4 v = __ldcs(reinterpret_cast<const float4 *>(workspace + c * per_cta + e));
+            sum.x += v.x;
+            sum.y += v.y;
+            sum.z += v.z;
+            sum.w += v.w;
         }
-        float sum = 0.f;
-        for (int c = 0; c < n_ctas; ++c) sum += workspace[c * per_cta + at];
-        *dst = from_float<T>(sum);
+    }
+    part[share][lane] = sum;
+    __syncthreads();
+    if (share == 0 && dst) {
+#pragma unroll
+        for (int i = 1; i < kReduceShares; ++i) {
+            const float4 v = part[i][lane];
+            sum.x += v.x;
+            sum.y += v.y;
+            sum.z += v.z;
+            sum.w += v.w;
+        }
+        dst[0] = from_float<T>(sum.x);
+        dst[1] = from_float<T>(sum.y);
+        dst[2] = from_float<T>(sum.z);
+        dst[3] = from_float<T>(sum.w);
     }
 }
 
@@ -797,7 +890,7 @@ bool rows16_ok(const void *p, int64_t stride) { return p && stride % 8 == 0 && a
 
 // Dynamic shared memory to request so that no more than `ctas` CTAs share an SM.
 int smem_request(const RevTcPlan &P, int ctas) {
-    const int need = P.total + 1024;
+    const int need = P.total;
     const int floor_bytes = kSmemBudget / (ctas + 1) + 1;
     return need > floor_bytes ? need : floor_bytes;
 }
@@ -901,12 +994,14 @@ int launch_rev_bwd_t(const RevShape &s, const RevParams &p, const void *y, int64
                         make_map(&row_maps.y2, y_rows + s.half, rows, s.half, kTileRows, y_stride) &&
                         make_map(&row_maps.go1, go_rows, rows, s.half, kTileRows, go_stride) &&
                         make_map(&row_maps.go2, go_rows + s.half, rows, s.half, kTileRows, go_stride);
+    const int copies = n_ctas < kRevCopies ? n_ctas : kRevCopies;
+    if (int rc = cuda_status(cudaMemsetAsync(workspace, 0, sizeof(float) * rev_cta_floats(s) * copies, stream), "cudaMemsetAsync(workspace)")) return rc;
     kernel<<<n_ctas, kTcThreads + kRevFlushThreads, smem, stream>>>(s, p, maps, row_maps, use_tma, static_cast<const T *>(y), y_stride,
                                                 static_cast<const T *>(go), go_stride, static_cast<T *>(gx), gx_stride,
                                                 static_cast<T *>(x_rec), xr_stride, workspace, rows);
     if (int rc = launch_status("rev_bwd_tc_kernel launch")) return rc;
-    rev_grad_reduce_tc_kernel<T><<<static_cast<unsigned>((rev_cta_floats(s) + 255) / 256), 256, 0, stream>>>(
-        s, workspace, n_ctas, static_cast<T *>(dw[0]), static_cast<T *>(dw[1]), static_cast<T *>(dw[2]),
+    rev_grad_reduce_tc_kernel<T><<<static_cast<unsigned>((rev_cta_floats(s) / 4 + kReduceQuads - 1) / kReduceQuads), kReduceQuads * kReduceShares, 0, stream>>>(
+        s, workspace, copies, static_cast<T *>(dw[0]), static_cast<T *>(dw[1]), static_cast<T *>(dw[2]),
         static_cast<T *>(dw[3]), static_cast<T *>(db[0]), static_cast<T *>(db[1]), static_cast<T *>(db[2]), static_cast<T *>(db[3]));
     return launch_status("rev_grad_reduce_tc_kernel launch");
 }
