@@ -20,8 +20,9 @@
 // and rounds z to the storage dtype, as the forward pass did.
 //
 // Measured: rows fetched and stored by the slots themselves were 22 % of a slot's time (2^21 rows 32-64-64-16; a fence for the
-// tensor core also waits for the thread's own copies and stores in flight): 0.234 -> 0.209 ms; 2^20 rows 32-4x64-16 0.279 -> 0.265;
-// 300 007 rows 32-3x64-16 with biases, where the smaller row buffers make room for a third slot, 0.081 -> 0.069.
+// tensor core also waits for the thread's own copies and stores in flight).  With the ring 0.234 -> 0.209 ms, 2^20 rows 32-4x64-16
+// 0.279 -> 0.265, 300 007 rows 32-3x64-16 with biases, where the smaller row buffers make room for a third slot, 0.081 -> 0.069; with the
+// issuers on schedulers of their own and their lanes elected where they issue, 0.189, 0.226 and 0.063.
 //
 // Per slot three mbarriers: `ready` (one arrival: the operands of the slot's next backward step are in place), `acc` (the
 // slot's own MMAs of the step are done), `wdone` (the step's wgrad is done).  The wgrad warp polls all `ready` barriers at
@@ -180,6 +181,7 @@ slots_mlp_bwd_tc_kernel(const MlpShape s, const MlpParams p, const __grid_consta
     if (threadIdx.x == 0) {
         tb.abort_flag = (smem_addr(smem) & 1023u) ? 1 : 0;  // operand tiles need their alignment
         if (tb.abort_flag) g_tc_status = 1;
+        mbar_init(&tb.weights_bar);
         for (int i = 0; i < S; ++i) {
             mbar_init(&tb.ready[i]);
             mbar_init(&tb.acc[i]);
@@ -201,13 +203,11 @@ slots_mlp_bwd_tc_kernel(const MlpShape s, const MlpParams p, const __grid_consta
         stage_biases<T>(wsmem, P.w, s, p);
     }
     fence_async_smem();
-    bool weights_ok = true;
-    if (use_tma) {
-        weights_ok = tma_stage_weights(wsmem, P.w, s, maps, &tb.weights_bar);  // contains the barrier that publishes the inits
-    } else {
+    if (!use_tma) {
         stage_all_weights<T>(wsmem, P.w, s, p);
         fence_async_smem();
-        __syncthreads();
+    } else if (threadIdx.x == 0) {
+        tma_issue_weights(wsmem, P.w, s, maps, &tb.weights_bar);  // awaited by the issuers, ahead of their first MMA
     }
     if (is_wgrad_warp) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&tb.tmem_holder)),
@@ -215,15 +215,6 @@ slots_mlp_bwd_tc_kernel(const MlpShape s, const MlpParams p, const __grid_consta
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    if (!weights_ok) {
-        tb.abort_flag = 1;
-        g_tc_status = 1;
-    }
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem = tb.tmem_holder;
-
     const long long n_tiles = (n_rows + kTileRows - 1) / kTileRows;
     const long long first_tile = blockIdx.x, tile_stride = gridDim.x;
     const long long n_mine = first_tile < n_tiles ? (n_tiles - first_tile + tile_stride - 1) / tile_stride : 0;
@@ -281,7 +272,10 @@ slots_mlp_bwd_tc_kernel(const MlpShape s, const MlpParams p, const __grid_consta
         }
         tb.steps[j] = st;
     }
+    tc_fence_before();
     __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tb.tmem_holder;
 
     if (is_wgrad_warp) {
         // ================= weight gradients of every slot =================
@@ -411,8 +405,8 @@ slots_mlp_bwd_tc_kernel(const MlpShape s, const MlpParams p, const __grid_consta
         auto act_addr = [&](int l) { return tile0 + static_cast<uint32_t>(l - 1) * kTileBytes; };  // input of layer l > 0
         const float *bias = reinterpret_cast<const float *>(wsmem + P.w.bias_offset);
         const uint32_t row_off = row * 128, row_swizzle = (row & 7) << 4;
-        const bool issuer = tid < 32;
-        const bool leader = issuer && elect_one();
+        // on another scheduler than other slots' issuers and the wgrad warp (all on its scheduler: 0.261 against 0.243 ms)
+        const bool issuer = (tid >> 5) == ((slot + 1) & 3);
         uint32_t acc_phase = 0, wdone_phase = 0;
         auto slot_sync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(slot + 1), "n"(kSlotThreads) : "memory"); };
         uint32_t buf = 0, rows0 = 0, prev_buf = 0, full_phase = 0, tiles_done = 0;
@@ -422,10 +416,14 @@ slots_mlp_bwd_tc_kernel(const MlpShape s, const MlpParams p, const __grid_consta
             tc_fence_before();
             slot_sync();
             if (issuer && !*abort_now) {
+                // elected here and not ahead of the loop, or the MMAs do not go through uniform registers (2^20 rows 32-4x64-16: 0.243 -> 0.226
+                // ms; the weight gradients' MMAs, which the chain's wait behind, are the better for the longer way: 0.228)
+                const bool leader = elect_one();
                 tc_fence_after();
                 if (j == 0) {
                     // the buffer of the tile before holds its input gradient now; this tile's rows
                     if (tiles_done > 0 && leader) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(&tb.empty[prev_buf])) : "memory");
+                    if (tiles_done == 0 && use_tma) pipe_wait(smem_addr(&tb.weights_bar), 0, &tb.abort_flag);
                     pipe_wait(smem_addr(&tb.full[buf]), full_phase, &tb.abort_flag);
                     __syncwarp();
                 }
@@ -537,13 +535,16 @@ slots_mlp_bwd_tc_kernel(const MlpShape s, const MlpParams p, const __grid_consta
         }
         fence_async_smem();
         slot_sync();
-        if (tiles_done > 0 && leader) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(&tb.empty[prev_buf])) : "memory");
+        if (tiles_done > 0 && issuer && elect_one()) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(&tb.empty[prev_buf])) : "memory");
     }
 
     // ---- flush the weight gradients (M = 64 layout: lanes 0..15 of warp quarter q hold rows 16 q ..); a warpgroup per layer ----
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
+    // (the slots have waited for every weight gradient; the row warps may still be sending the last rows off)
+    if (!is_wgrad_warp && !is_row_warp) {
+        tc_fence_before();
+        asm volatile("bar.sync 14, %0;" ::"n"(128 * S * W) : "memory");
+        tc_fence_after();
+    }
     if (!tb.abort_flag && n_mine > 0 && !is_wgrad_warp && !is_row_warp) {
         const MlpGradWorkspace G = grad_workspace_layout(s, workspace);
         const int wq = warp & 3;
@@ -652,16 +653,16 @@ int launch_slots(int rings, const MlpShape &s, const MlpParams &p, const void *x
 }
 
 // The most slots that fit are the fastest, two warpgroups per slot when there are threads left, and then one row buffer more than
-// slots (B200, ms; with / without the spare buffer): 2^21 rows 32-64-64-16 4 x 1 0.209 / 0.231, 3 x 2 0.250; 2^20 rows 32-4x64-16
-// 2 x 2 0.265 / 0.293; 300 007 rows 32-3x64-16 with biases 3 x 2 0.069, 2 x 2 0.081; 2^18 rows 32-64-64-16 with biases 4 x 1 0.043, 3 x 2
-// 0.048.  Tried: dz in a tile of its own so that the chain waits for a weight gradient one step late (0.287 at 32-4x64-16: MMAs run
-// in the order of issue, and the next step's queue behind the weight gradient's all the same); the chain's A operands in tensor memory
-// (0.304; the epilogue writes both places); unrolled loops over 32 columns (2^21 rows: 0.280 against 0.234).
+// slots (B200, ms; with / without the spare buffer, before the issuers were spread): 2^21 rows 32-64-64-16 4 x 1 0.209 / 0.231, 3 x 2
+// 0.250; 2^20 rows 32-4x64-16 2 x 2 0.265 / 0.293; 300 007 rows 32-3x64-16 with biases 3 x 2 0.069, 2 x 2 0.081; 2^18 rows 32-64-64-16
+// with biases 4 x 1 0.043, 3 x 2 0.048.  Tried: dz in a tile of its own so that the chain waits for a weight gradient one step late (0.287
+// at 32-4x64-16: MMAs run in the order of issue, and the next step's queue behind the weight gradient's all the same); the chain's A
+// operands in tensor memory (0.304; the epilogue writes both places); unrolled loops over 32 columns (2^21 rows: 0.280 against 0.234).
 template <typename T, int ACT, bool BIAS>
 int launch_any_slots(const MlpShape &s, const MlpParams &p, const void *x, int64_t x_stride, const void *go, int64_t go_stride, void *gx,
                      int64_t gx_stride, float *workspace, int64_t rows, cudaStream_t stream) {
-    // One or two tiles per CTA: two warpgroups walk a tile's chain faster than one (2^14 rows 32-64-64-16 with biases: 13.2 us as
-    // 1 x 2, 16 as 4 x 1), and there is nothing for more slots to do.
+    // One or two tiles per CTA: two warpgroups walk a tile's chain faster than one, and there is nothing for more slots to do (2^14
+    // rows 32-64-64-16 with biases: 13.6 us as 1 x 2, 14.6 as 2 x 2).
     const int64_t tiles_per_cta = ((rows + kTileRows - 1) / kTileRows + sm_count() - 1) / sm_count();
 #define TH_SLOTS(S, W)                                                                                                                        \
     for (int rings = S + 1; rings >= S; --rings)                                                                                              \

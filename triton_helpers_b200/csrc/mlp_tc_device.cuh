@@ -108,8 +108,16 @@ struct WeightMaps {
     CUtensorMap w_in, w_hid, w_out;
 };
 
-// All weight tiles of the network by TMA: thread 0 arms the barrier with the byte count and issues
-// one box per layer; everybody waits (bounded) for the bytes to land.  Returns false on a timeout.
+// All weight tiles of the network by TMA, by one thread: arms the barrier with the byte count and issues one box per layer.
+__device__ __forceinline__ void tma_issue_weights(unsigned char *smem, const TcPlan &P, const MlpShape &s, const WeightMaps &maps, unsigned long long *wbar) {
+    const uint32_t bar = smem_addr(wbar), bytes = static_cast<uint32_t>((s.h + (s.depth - 1) * s.h + s.no) * 128);
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+    tma_load_2d(smem + P.w_offset[0], &maps.w_in, 0, 0, bar);
+    for (int i = 0; i < s.depth - 1; ++i) tma_load_2d(smem + P.w_offset[1] + i * P.w_hid_each, &maps.w_hid, 0, i * s.d_hid, bar);
+    tma_load_2d(smem + P.w_offset[2], &maps.w_out, 0, 0, bar);
+}
+
+// The same with everybody waiting (bounded) for the bytes to land.  Returns false on a timeout.
 __device__ bool tma_stage_weights(unsigned char *smem, const TcPlan &P, const MlpShape &s, const WeightMaps &maps,
                                   unsigned long long *wbar) {
     const uint32_t bar = smem_addr(wbar);
@@ -118,13 +126,7 @@ __device__ bool tma_stage_weights(unsigned char *smem, const TcPlan &P, const Ml
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        const uint32_t bytes = static_cast<uint32_t>((s.h + (s.depth - 1) * s.h + s.no) * 128);
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-        tma_load_2d(smem + P.w_offset[0], &maps.w_in, 0, 0, bar);
-        for (int i = 0; i < s.depth - 1; ++i) tma_load_2d(smem + P.w_offset[1] + i * P.w_hid_each, &maps.w_hid, 0, i * s.d_hid, bar);
-        tma_load_2d(smem + P.w_offset[2], &maps.w_out, 0, 0, bar);
-    }
+    if (threadIdx.x == 0) tma_issue_weights(smem, P, s, maps, wbar);
     return mbar_wait(bar, 0);
 }
 

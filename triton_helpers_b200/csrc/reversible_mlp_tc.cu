@@ -264,8 +264,7 @@ rev_fwd_tc_kernel(const RevShape shape, const RevParams p, const __grid_constant
     if (!use_tma && static_cast<long long>(blockIdx.x) < n_tiles) prefetch_weights<T>(smem, P, shape, p, 0, 0);
     const uint32_t tmem = cta_setup(&tmem_holder, &mbar, P.tmem_cols);  // publishes the barrier inits
     if (use_tma && static_cast<long long>(blockIdx.x) < n_tiles) {
-        prefetch_weights_tma<T, BIAS>(smem, P, s, p, maps, ring_bars, 0, 0);
-        ring_wait(ring_bars, 0, &abort_flag);
+        prefetch_weights_tma<T, BIAS>(smem, P, s, p, maps, ring_bars, 0, 0);  // awaited behind the first rows
     }
     // With the A operands in tensor memory and the weights by TMA nothing that an MMA reads is written by a thread, and the fence
     // between the two proxies, which waits for the row loads and stores in flight, is left out (2^19 rows, eight blocks: 0.250 -> 0.229 ms)
@@ -285,6 +284,7 @@ rev_fwd_tc_kernel(const RevShape shape, const RevParams p, const __grid_constant
         async_tile_load<T>(h_tile, x, x_stride, row0, n_rows, s.half, s.half);
         async_tile_load<T>(u_tile, x + s.half, x_stride, row0, n_rows, s.half, s.half);
         async_tile_wait();  // also the weights queued for this step
+        if (use_tma && step == 0) ring_wait(ring_bars, 0, &abort_flag);
         __syncthreads();
         tile_row_to_tmem<T>(h_tile, seat, s.half, taddr + kS1);
         tile_row_to_tmem<T>(u_tile, seat, s.half, taddr + kS2);
@@ -365,6 +365,7 @@ rev_fwd_tc_kernel(const RevShape shape, const RevParams p, const __grid_constant
 
 // A copy of a matrix is stored [row / 16][column / 4][row % 16][column % 4]: what one flush warp holds of it is contiguous.
 constexpr int kRevCopies = 16;
+constexpr int kWgradIssuer = 2;  // the flush warp that issues the weight gradients: on another scheduler than the chain's issuer
 
 // The backward kernel runs 256 "main" threads (the chain: issue, wait, epilogue) and 128 "flush" threads
 // that carry the weight gradients of a pass out of TMEM while the main threads are already in the next pass.
@@ -525,13 +526,13 @@ rev_bwd_tc_kernel(const RevShape shape, const RevParams p, const __grid_constant
                 float *block_acc = cta_acc + static_cast<size_t>(k) * 4 * kMatFloats;
                 for (int pass = 0; pass < 2; ++pass, ++n) {
                     const uint32_t dy_cur = smem_addr(dy_tiles + (n & 1u) * kTileBytes);
-                    if (BIAS || q == 0) {
+                    if (BIAS || q == kWgradIssuer) {
                         alive = __all_sync(0xffffffffu, rev_wait(operands_addr, n & 1u, &abort_flag));
                         // the accumulators hold the previous pass's sums until all four flush warps have read them
-                        if (q == 0 && alive && n > 0) alive = __all_sync(0xffffffffu, rev_wait(flushed_addr, (n - 1) & 1u, &abort_flag));
+                        if (q == kWgradIssuer && alive && n > 0) alive = __all_sync(0xffffffffu, rev_wait(flushed_addr, (n - 1) & 1u, &abort_flag));
                         if (!alive) break;
                     }
-                    if (q == 0) {
+                    if (q == kWgradIssuer) {
                         const bool leader = elect_one();
                         tc_fence_after();
                         const uint32_t u_cur = smem_addr(u_tiles + (n & 1u) * kTileBytes);
