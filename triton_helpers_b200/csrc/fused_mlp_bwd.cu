@@ -408,6 +408,7 @@ slots_mlp_bwd_tc_kernel(const MlpShape s, const MlpParams p, const __grid_consta
         // on another scheduler than other slots' issuers and the wgrad warp (all on its scheduler: 0.261 against 0.243 ms)
         const bool issuer = (tid >> 5) == ((slot + 1) & 3);
         uint32_t acc_phase = 0, wdone_phase = 0;
+        bool alive = true;
         auto slot_sync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(slot + 1), "n"(kSlotThreads) : "memory"); };
         uint32_t buf = 0, rows0 = 0, prev_buf = 0, full_phase = 0, tiles_done = 0;
         // operands written -> the slot's warp 0 issues the step's own MMAs (and hands the wgrad to the wgrad warp)
@@ -415,7 +416,7 @@ slots_mlp_bwd_tc_kernel(const MlpShape s, const MlpParams p, const __grid_consta
             fence_async_smem();
             tc_fence_before();
             slot_sync();
-            if (issuer && !*abort_now) {
+            if (issuer && alive) {
                 // elected here and not ahead of the loop, or the MMAs do not go through uniform registers (2^20 rows 32-4x64-16: 0.243 -> 0.226
                 // ms; the weight gradients' MMAs, which the chain's wait behind, are the better for the longer way: 0.228)
                 const bool leader = elect_one();
@@ -459,13 +460,13 @@ slots_mlp_bwd_tc_kernel(const MlpShape s, const MlpParams p, const __grid_consta
         };
         auto finish_step = [&](bool own, bool wgrad) {
             // every warp polls: parking three of four warps at a barrier behind the polling one measured 2-6 % slower
-            if (own) pipe_wait(acc_bar, acc_phase, &tb.abort_flag);
-            if (wgrad) pipe_wait(wdone_bar, wdone_phase, &tb.abort_flag);
+            if (own) alive = pipe_wait(acc_bar, acc_phase, &tb.abort_flag) && alive;
+            if (wgrad) alive = pipe_wait(wdone_bar, wdone_phase, &tb.abort_flag) && alive;
             __syncwarp();
             if (own) acc_phase ^= 1u;
             if (wgrad) wdone_phase ^= 1u;
             tc_fence_after();
-            return !*abort_now;
+            return alive;
         };
         for (long long k = slot; k < n_mine; k += S) {
             buf = static_cast<uint32_t>(k % P.rings);

@@ -390,7 +390,7 @@ __device__ __forceinline__ bool rev_wait(uint32_t bar, uint32_t parity, int *abo
             : "r"(bar), "r"(parity)
             : "memory");
         if (done) return true;
-        if (*reinterpret_cast<volatile int *>(abort_flag)) return false;
+        if ((poll & 63) == 63 && *reinterpret_cast<volatile int *>(abort_flag)) return false;
     }
     *reinterpret_cast<volatile int *>(abort_flag) = 1;
     return false;
