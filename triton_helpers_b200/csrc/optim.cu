@@ -92,6 +92,19 @@ __device__ __forceinline__ T adam_one(T p, T g_in, float &m, float &v, const Ada
     return from_float<T>(to_float<T>(p) - (a.lr / a.bias1) * (m / denom));
 }
 
+// Elements of a parameter in one 16-byte packet, and the matching moments (float32: four, for twice the threads and half their
+// registers of eight: 3.3 M parameters 34.2 -> 26.4 us)
+template <typename T>
+constexpr int kPacket = 16 / sizeof(T);
+template <typename T>
+struct __align__(16) Packet16 {
+    T v[kPacket<T>];
+};
+template <int N>
+struct __align__(16) Moments {
+    float v[N];
+};
+
 // The same update for several tensors of one dtype in one launch: a small network's tensors are a few blocks each, and
 // a launch per tensor (seven for a table and a biased MLP: 43 us of kernels and 100 us of host time in a training step)
 // costs more than the update.  Every block walks every tensor with the whole grid's stride.
@@ -109,27 +122,28 @@ struct AdamTensors {
 template <typename T>
 __device__ __forceinline__ int adam_walk(T *__restrict__ param, T *__restrict__ grad, float *__restrict__ exp_avg, float *__restrict__ exp_avg_sq,
                                          long long n, const AdamScalars &a) {
+    constexpr int N = kPacket<T>;
     int skipped = 0;
-    const long long packets = n / 8;
+    const long long packets = n / N;
     for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < packets;
          i += static_cast<long long>(gridDim.x) * blockDim.x) {
-        Vec8<T> p = reinterpret_cast<Vec8<T> *>(param)[i];
-        const Vec8<T> g = reinterpret_cast<const Vec8<T> *>(grad)[i];
-        Vec8<float> m = reinterpret_cast<Vec8<float> *>(exp_avg)[i];
-        Vec8<float> v = reinterpret_cast<Vec8<float> *>(exp_avg_sq)[i];
+        Packet16<T> p = reinterpret_cast<Packet16<T> *>(param)[i];
+        const Packet16<T> g = reinterpret_cast<const Packet16<T> *>(grad)[i];
+        Moments<N> m = reinterpret_cast<Moments<N> *>(exp_avg)[i];
+        Moments<N> v = reinterpret_cast<Moments<N> *>(exp_avg_sq)[i];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) p.v[k] = adam_one<T>(p.v[k], g.v[k], m.v[k], v.v[k], a, skipped);
-        reinterpret_cast<Vec8<T> *>(param)[i] = p;
-        reinterpret_cast<Vec8<float> *>(exp_avg)[i] = m;
-        reinterpret_cast<Vec8<float> *>(exp_avg_sq)[i] = v;
+        for (int k = 0; k < N; ++k) p.v[k] = adam_one<T>(p.v[k], g.v[k], m.v[k], v.v[k], a, skipped);
+        reinterpret_cast<Packet16<T> *>(param)[i] = p;
+        reinterpret_cast<Moments<N> *>(exp_avg)[i] = m;
+        reinterpret_cast<Moments<N> *>(exp_avg_sq)[i] = v;
         if (a.zero_grad) {
-            Vec8<T> z;
+            Packet16<T> z;
 #pragma unroll
-            for (int k = 0; k < 8; ++k) z.v[k] = from_float<T>(0.f);
-            reinterpret_cast<Vec8<T> *>(grad)[i] = z;
+            for (int k = 0; k < N; ++k) z.v[k] = from_float<T>(0.f);
+            reinterpret_cast<Packet16<T> *>(grad)[i] = z;
         }
     }
-    for (long long i = packets * 8 + static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
+    for (long long i = packets * N + static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
          i += static_cast<long long>(gridDim.x) * blockDim.x) {
         param[i] = adam_one<T>(param[i], grad[i], exp_avg[i], exp_avg_sq[i], a, skipped);
         if (a.zero_grad) grad[i] = from_float<T>(0.f);
@@ -188,9 +202,9 @@ scale_cast_kernel(const float *__restrict__ src, T *__restrict__ dst, long long 
         dst[i] = from_float<T>(src[i] * scale);
 }
 
-unsigned stream_grid(long long n) {
-    const long long blocks = (n / 8 + kOptThreads - 1) / kOptThreads + 1;
-    const long long cap = static_cast<long long>(sm_count()) * 8;
+unsigned stream_grid(long long n, int packet = 8, int per_sm = 8) {
+    const long long blocks = (n / packet + kOptThreads - 1) / kOptThreads + 1;
+    const long long cap = static_cast<long long>(sm_count()) * per_sm;
     return static_cast<unsigned>(blocks < cap ? blocks : cap);
 }
 
@@ -253,7 +267,7 @@ extern "C" int th_adam_steps(int n_tensors, void *const *param_dev, void *const 
     a.bias1 = static_cast<float>(1.0 - pow(static_cast<double>(beta1), step));
     a.bias2_sqrt = static_cast<float>(sqrt(1.0 - pow(static_cast<double>(beta2), step)));
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const unsigned grid = stream_grid(most);
+    const unsigned grid = dtype == TH_F32 ? stream_grid(most, 4, 24) : stream_grid(most);
     switch (dtype) {
         case TH_F32: adam_many_kernel<float><<<grid, kOptThreads, 0, st>>>(t, a, skipped_dev); break;
         case TH_F16: adam_many_kernel<__half><<<grid, kOptThreads, 0, st>>>(t, a, skipped_dev); break;
