@@ -288,9 +288,8 @@ int th_rev_fwd(const void *x_dev, int64_t x_stride, const void *w_f1_dev, const 
  * out and results are invalid).  Synchronises the device. */
 int th_rev_tc_status(void);
 
-/* Bytes of fp32 scratch th_rev_bwd needs for `rows` rows: room for one copy of all weight-gradient
- * accumulators per resident CTA (about 0.5 MB per CTA for 8 blocks of 64 x 64); the tensor-core kernel
- * uses at most sixteen of them. */
+/* Bytes of fp32 scratch th_rev_bwd needs for `rows` rows: one private copy of all weight-gradient
+ * accumulators per resident CTA (about 0.5 MB per CTA for 8 blocks of 64 x 64). */
 int64_t th_rev_workspace_bytes(int64_t rows, int d_model, int d_hidden, int blocks);
 
 /* Backward from the stack's OUTPUT y (no stored activations): reconstructs the inputs block by

@@ -1,4 +1,4 @@
-r"""The reversible backward's weight gradients on their way out: several CTAs to one accumulator, several row tiles per CTA, every
+r"""The reversible backward's weight gradients on their way out: several row tiles per CTA, every
 pair of widths (the two accumulators of a branch share tensor-memory columns), with and without biases."""
 import pytest
 import torch
@@ -46,3 +46,18 @@ def test_weight_gradients_of_every_width_and_batch(rows, half, hidden, bias):
             s = slice(b * per_block, (b + 1) * per_block)
             assert nerr(have[s], want[s]) <= 5 * TIGHT[dtype], (b, nerr(have[s], want[s]))
     assert _lib.lib().th_rev_tc_status() == 0
+
+
+@pytest.mark.parametrize("rows,blocks", [(128 * 148 * 3 + 5, 2), (128 * 148 * 4, 1), (128 * 40, 8)])
+def test_weight_gradients_repeat_bit_for_bit(rows, blocks):
+    # an accumulator has one owner that adds to it in order, and the copies are summed in order: no call differs from another
+    dtype, half = torch.float16, 64
+    weights, _ = make_params(blocks, half, half, False, dtype, seed=3)
+    g = torch.Generator().manual_seed(rows)
+    x, go = torch.randn(rows, 2 * half, generator=g).to(dtype).cuda(), torch.randn(rows, 2 * half, generator=g).to(dtype).cuda()
+    wc, bc = to_cuda(weights), to_cuda((None,) * 4)
+    y = reversible_mlp_forward(x, wc, bc, "relu")
+    first = reversible_mlp_backward(y, go, wc, bc, "relu")
+    for _ in range(8):
+        for want, have in zip(first, reversible_mlp_backward(y, go, wc, bc, "relu")):
+            assert want is None or torch.equal(want, have)

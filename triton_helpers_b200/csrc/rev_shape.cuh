@@ -33,8 +33,8 @@ constexpr int kRevTcNotApplicable = -1000;
 int rev_fwd_tc(const RevShape &s, const RevParams &p, const void *x, int64_t x_stride, void *y, int64_t y_stride,
                int64_t rows, int dtype, cudaStream_t stream);
 
-// Backward from the output; `workspace` has room for `n_ctas` fp32 copies of all weight gradients, some of which the launch
-// clears and uses; writes the gradient tensors itself.
+// Backward from the output; `workspace` has room for one fp32 copy of all weight gradients per CTA, `n_ctas` of them (at most
+// one per 128 rows), of any content; writes the gradient tensors itself.
 int rev_bwd_tc(const RevShape &s, const RevParams &p, const void *y, int64_t y_stride, const void *go,
                int64_t go_stride, void *gx, int64_t gx_stride, void *x_rec, int64_t xr_stride, void *const dw[4],
                void *const db[4], float *workspace, int n_ctas, int64_t rows, int dtype, cudaStream_t stream);

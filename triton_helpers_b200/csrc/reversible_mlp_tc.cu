@@ -18,11 +18,13 @@
 // Weights (4 matrices per block) stream block by block through a two-stage cp.async ring in the
 // operand-tile layout; the same tile is read K-major by the forward GEMMs and MN-major by dgrad.
 // Weight gradients of a (tile, block, branch) leave TMEM for staging in shared memory and from there as bulk reductions
-// (cp.reduce.async.bulk, 4 KB each) for one of kRevCopies fp32 accumulators in global memory, carried out by four extra warps while
-// the other eight are already in the next branch; a reduction kernel sums the copies.  As vector reductions of the four warps they
+// (cp.reduce.async.bulk, 4 KB each) for the CTA's own fp32 accumulators in global memory, carried out by four extra warps while
+// the other eight are already in the next branch; a reduction kernel sums the CTAs' copies.  As vector reductions of the four warps they
 // shared the load / store pipe with the chain's stores: 32 KB a branch, 17 % of the kernel (2^19 rows, eight blocks of 64 -> 64 -> 64:
-// 0.872 -> 0.757 ms, 0.72 with no reductions at all).  How many CTAs add to one copy makes no difference to them (1 to 148 copies:
-// 0.87 to 0.88 ms), to the zero fill and the sum over the copies it does.
+// 0.872 -> 0.757 ms, 0.72 with no reductions at all).  An accumulator has one owner, whose first tile writes it and whose later ones add
+// to it in order, so the weight gradients are the same bits at every call.  (Sixteen copies that all CTAs add to in the order of
+// arrival: 1 to 6 % less time from 20 000 rows on, up to 11 % at ten blocks, for the shorter sum over the copies; gradients that vary from
+// call to call.  Cleared copies, only added to: 3 to 34 % more.)
 //
 // The chain's A operands (U and DY, h and dz) lie in 64 TMEM columns besides their tiles, which the weight gradients read: an MMA
 // then takes 43 cycles instead of 76.  The two weight-gradient accumulators (M = 64) share 64 columns, one in lanes 0..15 and one in
@@ -363,8 +365,7 @@ rev_fwd_tc_kernel(const RevShape shape, const RevParams p, const __grid_constant
 
 // ---- backward ----------------------------------------------------------------------------------
 
-// A copy of a matrix is stored [row / 16][column / 4][row % 16][column % 4]: what one flush warp holds of it is contiguous.
-constexpr int kRevCopies = 16;
+// An accumulator matrix is stored [row / 16][column / 4][row % 16][column % 4]: what one flush warp holds of it is contiguous.
 constexpr int kWgradIssuer = 2;  // the flush warp that issues the weight gradients: on another scheduler than the chain's issuer
 
 // The backward kernel runs 256 "main" threads (the chain: issue, wait, epilogue) and 128 "flush" threads
@@ -406,8 +407,8 @@ __device__ __forceinline__ void main_wait_mma(uint32_t mbar, uint32_t &phase, in
 }
 
 // One flush warp's share of both accumulators: TMEM lanes 32 q .. 32 q + 15 hold rows 16 q .. of the first matrix, the other sixteen
-// those of the second.  The accumulators are free once they are in registers.
-__device__ __forceinline__ void flush_dw_pair(uint32_t tmem, int q, uint32_t stage, float *dst, uint32_t flushed) {
+// those of the second.  The accumulators are free once they are in registers.  `first`: nothing has been written to dst yet.
+__device__ __forceinline__ void flush_dw_pair(uint32_t tmem, int q, uint32_t stage, float *dst, uint32_t flushed, bool first) {
     const int lane = threadIdx.x & 31;
     const uint32_t taddr = tmem + (static_cast<uint32_t>(32 * q) << 16) + kDW1;
     uint32_t lo[32], hi[32];
@@ -426,11 +427,23 @@ __device__ __forceinline__ void flush_dw_pair(uint32_t tmem, int q, uint32_t sta
     fence_async_smem();
     __syncwarp();
     if (lane == 0) {
+        // Bulk copies and reductions in flight together arrive in no order.  The next ones to the same addresses are two passes or more
+        // away (the other branch lies between), so these are sent once all but the last pass's have been performed.
+        asm volatile("cp.async.bulk.wait_group 1;" ::: "memory");
+        // The copies (0.5 MB per CTA) are revisited once per row tile while a gigabyte of rows streams through L2: ask it to keep them
+        unsigned long long keep;
+        asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(keep));
 #pragma unroll
-        for (int m = 0; m < 2; ++m)
-            asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], 4096;" ::"l"(dst + m * kMatFloats + q * 1024),
-                         "r"(stage + m * 4096)
-                         : "memory");
+        for (int m = 0; m < 2; ++m) {
+            float *at_dst = dst + m * kMatFloats + q * 1024;
+            if (first)
+                asm volatile("cp.async.bulk.global.shared::cta.bulk_group.L2::cache_hint [%0], [%1], 4096, %2;" ::"l"(at_dst), "r"(stage + m * 4096), "l"(keep)
+                             : "memory");
+            else
+                asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.L2::cache_hint.add.f32 [%0], [%1], 4096, %2;" ::"l"(at_dst),
+                             "r"(stage + m * 4096), "l"(keep)
+                             : "memory");
+        }
         asm volatile("cp.async.bulk.commit_group;" ::: "memory");
     }
 }
@@ -510,7 +523,7 @@ rev_bwd_tc_kernel(const RevShape shape, const RevParams p, const __grid_constant
     const long long n_tiles = (n_rows + kTileRows - 1) / kTileRows;
     if (!is_flush && !use_tma && static_cast<long long>(blockIdx.x) < n_tiles) prefetch_weights<T>(smem, P, shape, p, s.blocks - 1, 0);
     const uint32_t tmem = cta_setup(&tmem_holder, &mbar, P.tmem_cols);  // publishes the barrier inits
-    float *cta_acc = workspace + static_cast<size_t>(blockIdx.x % kRevCopies) * rev_cta_floats(s);
+    float *cta_acc = workspace + static_cast<size_t>(blockIdx.x) * rev_cta_floats(s);
     const uint32_t wgrad_addr = smem_addr(&wgrad_bar), flushed_addr = smem_addr(&flushed_bar);
     const uint32_t operands_addr = smem_addr(&operands_bar), summed_addr = smem_addr(&summed_bar);
 
@@ -552,7 +565,7 @@ rev_bwd_tc_kernel(const RevShape shape, const RevParams p, const __grid_constant
                     if (!alive) break;
                     tc_fence_after();
                     const int m1 = pass == 0 ? 2 : 0;
-                    flush_dw_pair(tmem, q, stage, block_acc + m1 * kMatFloats, flushed_addr);
+                    flush_dw_pair(tmem, q, stage, block_acc + m1 * kMatFloats, flushed_addr, tile == blockIdx.x);
                 }
             }
         }
@@ -824,8 +837,8 @@ rev_bwd_tc_kernel(const RevShape shape, const RevParams p, const __grid_constant
     cta_teardown(tmem, P.tmem_cols);
 }
 
-// Sum the accumulators ([copy][block][matrix][column / 4][row][column % 4], then [block][4][64] bias sums) into the gradient
-// tensors: a thread sums one quad of every 8th copy, the block's eight shares meet in shared memory in a fixed order.
+// Sum the accumulators ([CTA][block][matrix][row / 16][column / 4][row % 16][column % 4], then [block][4][64] bias sums) into the
+// gradient tensors: a thread sums one quad of every 8th copy, the block's eight shares meet in shared memory in a fixed order.
 constexpr int kReduceQuads = 32, kReduceShares = 8;
 template <typename T>
 __global__ void __launch_bounds__(kReduceQuads * kReduceShares)
@@ -995,14 +1008,18 @@ int launch_rev_bwd_t(const RevShape &s, const RevParams &p, const void *y, int64
                         make_map(&row_maps.y2, y_rows + s.half, rows, s.half, kTileRows, y_stride) &&
                         make_map(&row_maps.go1, go_rows, rows, s.half, kTileRows, go_stride) &&
                         make_map(&row_maps.go2, go_rows + s.half, rows, s.half, kTileRows, go_stride);
-    const int copies = n_ctas < kRevCopies ? n_ctas : kRevCopies;
-    if (int rc = cuda_status(cudaMemsetAsync(workspace, 0, sizeof(float) * rev_cta_floats(s) * copies, stream), "cudaMemsetAsync(workspace)")) return rc;
+    // the matrices are written by a CTA's first tile (it has one: n_ctas is at most the number of tiles), the bias sums only added to
+    if constexpr (BIAS) {
+        const size_t pitch = sizeof(float) * rev_cta_floats(s), sums = sizeof(float) * s.blocks * 4 * kMaxDim;
+        if (int rc = cuda_status(cudaMemset2DAsync(reinterpret_cast<unsigned char *>(workspace) + pitch - sums, pitch, 0, sums, n_ctas, stream),
+                                 "cudaMemset2DAsync(workspace)")) return rc;
+    }
     kernel<<<n_ctas, kTcThreads + kRevFlushThreads, smem, stream>>>(s, p, maps, row_maps, use_tma, static_cast<const T *>(y), y_stride,
                                                 static_cast<const T *>(go), go_stride, static_cast<T *>(gx), gx_stride,
                                                 static_cast<T *>(x_rec), xr_stride, workspace, rows);
     if (int rc = launch_status("rev_bwd_tc_kernel launch")) return rc;
     rev_grad_reduce_tc_kernel<T><<<static_cast<unsigned>((rev_cta_floats(s) / 4 + kReduceQuads - 1) / kReduceQuads), kReduceQuads * kReduceShares, 0, stream>>>(
-        s, workspace, copies, static_cast<T *>(dw[0]), static_cast<T *>(dw[1]), static_cast<T *>(dw[2]),
+        s, workspace, n_ctas, static_cast<T *>(dw[0]), static_cast<T *>(dw[1]), static_cast<T *>(dw[2]),
         static_cast<T *>(dw[3]), static_cast<T *>(db[0]), static_cast<T *>(db[1]), static_cast<T *>(db[2]), static_cast<T *>(db[3]));
     return launch_status("rev_grad_reduce_tc_kernel launch");
 }
