@@ -17,7 +17,8 @@
 // padded output width (16: 35 instead of 60 cycles a K step) instead of the hidden one.
 // Bias gradient of a layer = column sums of dz = dz^T . ONES, a small MMA (N = 8) next to the weight gradient's.  SiLU' and
 // ReLU^2' want the pre-activation: the step that needs it issues that layer's forward GEMM again into a second accumulator
-// and rounds z to the storage dtype, as the forward pass did.
+// and rounds z to the storage dtype, as the forward pass did.  Biases are in the accumulators before a recompute GEMM is issued, as in
+// the forward kernels: the backward opens the ReLUs that the forward opened.
 //
 // Measured: rows fetched and stored by the slots themselves were 22 % of a slot's time (2^21 rows 32-64-64-16; a fence for the
 // tensor core also waits for the thread's own copies and stores in flight).  With the ring 0.234 -> 0.209 ms, 2^20 rows 32-4x64-16
@@ -414,6 +415,7 @@ slots_mlp_bwd_tc_kernel(const MlpShape s, const MlpParams p, const __grid_consta
         // operands written -> the slot's warp 0 issues the step's own MMAs (and hands the wgrad to the wgrad warp)
         auto start_step = [&](int j) {
             fence_async_smem();
+            if constexpr (BIAS) tmem_st_wait();
             tc_fence_before();
             slot_sync();
             if (issuer && alive) {
@@ -436,10 +438,10 @@ slots_mlp_bwd_tc_kernel(const MlpShape s, const MlpParams p, const __grid_consta
                         if (leader) {
                             const uint32_t a_low = desc_low(rows0 + own.x), b_low = desc_low(own.y), b_step = (own.w & 256u) ? 128 : 2;
                             for (int k = 0; k < static_cast<int>(own.w & 255u); ++k)
-                                mma_f16(acc, desc_of(a_low + 2 * k, st.a_high), smem_desc(b_low + k * b_step), own.z, k > 0);
+                                mma_f16(acc, desc_of(a_low + 2 * k, st.a_high), smem_desc(b_low + k * b_step), own.z, k > 0 || (BIAS && j == 0));
                         }
                     } else {
-                        issue_gemm(leader, acc, tile0 + own.x, 32, own.y, (own.w & 256u) ? 2048 : 32, static_cast<int>(own.w & 255u), own.z, false);
+                        issue_gemm(leader, acc, tile0 + own.x, 32, own.y, (own.w & 256u) ? 2048 : 32, static_cast<int>(own.w & 255u), own.z, BIAS && j < d);
                     }
                     if constexpr (kPreact) {
                         if (st.z_k)
@@ -447,9 +449,9 @@ slots_mlp_bwd_tc_kernel(const MlpShape s, const MlpParams p, const __grid_consta
                             if (st.flags & 8u) {
                                 if (leader)
                                     for (int k = 0; k < static_cast<int>(st.z_k); ++k)
-                                        mma_f16(acc + kAccCols, desc_of(desc_low(rows0) + 2 * k, desc_high(P.x_pitch)), smem_desc(desc_low(st.zb_addr) + 2 * k), instr_desc(128, s.h, bf16, 0, 0), k > 0);
+                                        mma_f16(acc + kAccCols, desc_of(desc_low(rows0) + 2 * k, desc_high(P.x_pitch)), smem_desc(desc_low(st.zb_addr) + 2 * k), instr_desc(128, s.h, bf16, 0, 0), BIAS || k > 0);
                             } else {
-                                issue_gemm(leader, acc + kAccCols, tile0 + st.za_off, 32, st.zb_addr, 32, static_cast<int>(st.z_k), instr_desc(128, s.h, bf16, 0, 0), false);
+                                issue_gemm(leader, acc + kAccCols, tile0 + st.za_off, 32, st.zb_addr, 32, static_cast<int>(st.z_k), instr_desc(128, s.h, bf16, 0, 0), BIAS);
                             }
                         }
                     }
@@ -468,7 +470,14 @@ slots_mlp_bwd_tc_kernel(const MlpShape s, const MlpParams p, const __grid_consta
             tc_fence_after();
             return alive;
         };
+        [[maybe_unused]] int read = s.h;  // BIAS: accumulator columns that the slot has read last, half of them by each warpgroup
         for (long long k = slot; k < n_mine; k += S) {
+            if constexpr (BIAS) {
+                if constexpr (W == 2) start_half_from_bias(taddr, half, read, s.h, bias);
+                else start_from_bias(taddr, 0, s.h, bias);
+                if constexpr (kPreact) start_from_bias(taddr + kAccCols, half * (s.h / W), (half + 1) * (s.h / W), bias + (d - 1) * kMaxDim);
+                if (gx != nullptr) read = s.ki;
+            }
             buf = static_cast<uint32_t>(k % P.rings);
             full_phase = static_cast<uint32_t>((k / P.rings) & 1);
             rows0 = ring_of(buf);
@@ -476,10 +485,10 @@ slots_mlp_bwd_tc_kernel(const MlpShape s, const MlpParams p, const __grid_consta
                 start_step(l);
                 if (finish_step(true, false)) {
                     const uint32_t dst = act_addr(l + 1) + row_off;
-                    const float *layer_bias = bias + l * kMaxDim;
                     for_row_pieces<W>(taddr, s.h, half, [&](int chunk, const uint32_t(&piece)[8]) {
-                        st_shared_16(dst + ((chunk << 4) ^ row_swizzle), finish8<T, ACT, BIAS>(piece, layer_bias + 8 * chunk));
+                        st_shared_16(dst + ((chunk << 4) ^ row_swizzle), finish8<T, ACT, false>(piece, nullptr));
                     });
+                    if (BIAS && l + 1 < d) start_from_bias(taddr, half * (s.h / W), (half + 1) * (s.h / W), bias + (l + 1) * kMaxDim);
                 }
             }
             for (int l = d; l >= 0; --l) {
@@ -489,7 +498,6 @@ slots_mlp_bwd_tc_kernel(const MlpShape s, const MlpParams p, const __grid_consta
                 if (l > 0 && ok) {  // dz of the layer below = dy * act', in place over that layer's parked output
                     const uint32_t parked = act_addr(l) + row_off;
                     if constexpr (kPreact) {
-                        const float *layer_bias = bias + (l - 1) * kMaxDim;
 #pragma unroll 1
                         for (int u = 0; u < in_pad / (8 * W); ++u) {
                             const int chunk = half * (in_pad / 16) + u;
@@ -500,14 +508,13 @@ slots_mlp_bwd_tc_kernel(const MlpShape s, const MlpParams p, const __grid_consta
                             float g[8];
 #pragma unroll
                             for (int e = 0; e < 8; ++e) {
-                                float z = __uint_as_float(zz[e]);
-                                if constexpr (BIAS) z += layer_bias[8 * chunk + e];
-                                z = to_float<T>(from_float<T>(z));  // the forward pass stored z rounded
+                                const float z = to_float<T>(from_float<T>(__uint_as_float(zz[e])));  // the forward pass stored z rounded
                                 g[e] = activate_grad(ACT, z, __uint_as_float(dy[e]));
                             }
                             st_shared_16(parked + ((chunk << 4) ^ row_swizzle),
                                          make_uint4(pack_pair<T>(g[0], g[1]), pack_pair<T>(g[2], g[3]), pack_pair<T>(g[4], g[5]), pack_pair<T>(g[6], g[7])));
                         }
+                        if (BIAS && l > 1) start_from_bias(taddr + kAccCols, half * (s.h / W), (half + 1) * (s.h / W), bias + (l - 2) * kMaxDim);
                     } else {
                         for_row_pieces<W>(taddr, in_pad, half, [&](int chunk, const uint32_t(&piece)[8]) {
                             const uint32_t off = (chunk << 4) ^ row_swizzle;

@@ -70,6 +70,10 @@ mlp_fwd_tc_kernel(const MlpShape s, const MlpParams p, const __grid_constant__ W
     const float *bias = reinterpret_cast<const float *>(smem + P.bias_offset);
     const Seat seat;
     const uint32_t taddr = tmem + seat.lane_base;
+    if constexpr (BIAS) {
+        start_half_from_bias(taddr, seat.group, s.h, s.h, bias);
+        tmem_st_wait();
+    }
     uint32_t phase = 0;
     const long long n_tiles = (n_rows + kTileRows - 1) / kTileRows;
 
@@ -105,7 +109,7 @@ mlp_fwd_tc_kernel(const MlpShape s, const MlpParams p, const __grid_constant__ W
                 const bool leader = elect_one();
                 tc_fence_after();
                 issue_gemm(leader, tmem, act_addr, 32, smem_addr(weight_tile(smem, P, s, l)), 32, in_pad / 16,
-                           instr_desc(128, out_pad, bf16, 0, 0), false);
+                           instr_desc(128, out_pad, bf16, 0, 0), BIAS);
                 if (leader) mma_commit(bar);
                 __syncwarp();
             }
@@ -113,11 +117,15 @@ mlp_fwd_tc_kernel(const MlpShape s, const MlpParams p, const __grid_constant__ W
             if (!ok) {
                 g_tc_status = 1;
             } else if (l < s.depth) {
-                hidden_epilogue<T, ACT, BIAS>(taddr, seat, out_pad, bias + l * kMaxDim, act_tile);
+                hidden_epilogue<T, ACT>(taddr, seat, out_pad, act_tile);
             } else {
                 const bool live = row0 + seat.row < n_rows;
-                output_epilogue<T, BIAS>(taddr, seat, out_pad, bias + l * kMaxDim, y + (live ? row0 + seat.row : 0) * y_stride,
-                                         s.d_out, live, y_vec);
+                output_epilogue<T>(taddr, seat, out_pad, y + (live ? row0 + seat.row : 0) * y_stride, s.d_out, live, y_vec);
+            }
+            if constexpr (BIAS) {  // of the next layer, or of the next tile's first one
+                const int next = l == s.depth ? 0 : l + 1;
+                start_half_from_bias(taddr, seat.group, out_pad, next == s.depth ? s.no : s.h, bias + next * kMaxDim);
+                tmem_st_wait();
             }
             if (l < s.depth) {
                 fence_async_smem();
@@ -203,7 +211,8 @@ __device__ __forceinline__ void slot_barrier(int slot) {
 // BM: a layer's bias is one more K step of its GEMM, ahead of the others: A is a constant in tensor memory (element 0 of every row
 // is one), B an operand tile whose element 16 (l % 4) of row n is b_l[n].  The elements beside it are zeros, so that no other layer's
 // bias (it may be infinite) is multiplied by anything.  The additions in the epilogue it replaces cost 64 instructions and 16
-// shared loads a row and layer, 600 of 2 900 cycles (2^18 rows, ten 64-wide layers: 0.0434 -> 0.0339 ms).
+// shared loads a row and layer, 600 of 2 900 cycles (2^18 rows, ten 64-wide layers: 0.0434 -> 0.0339 ms).  Without BM the epilogue
+// of the layer before writes the biases into the accumulator.
 template <typename T, int ACT, bool BIAS, int S, bool MSE, bool TA, bool H64, bool BM>
 __global__ void __launch_bounds__(128 * S, 1)
 mlp_fwd_pipe_kernel(const MlpShape shape, const MlpParams p, const __grid_constant__ WeightMaps maps,
@@ -286,6 +295,11 @@ mlp_fwd_pipe_kernel(const MlpShape shape, const MlpParams p, const __grid_consta
             tmem_st8(one_tmem + (static_cast<uint32_t>(32 * warp) << 16), one);
             tmem_st_wait();
         }
+    } else if constexpr (BIAS) {
+        start_from_bias(tmem + (warp >> 2) * kAccCols + (static_cast<uint32_t>(32 * (warp & 3)) << 16), 0, s.h, bias);
+        tmem_st_wait();
+    }
+    if constexpr (BIAS) {
         tc_fence_before();
         __syncthreads();
         tc_fence_after();
@@ -377,9 +391,9 @@ mlp_fwd_pipe_kernel(const MlpShape shape, const MlpParams p, const __grid_consta
                         if (leader) mma_f16_ta(acc, one_tmem, smem_desc(desc_low(smem_addr(smem + plan.bias) + (l >> 2) * 64 * 128) + 2 * (l & 3)), idesc, 0);
                     }
                     if (TA && l > 0)
-                        issue_gemm_ta(leader, acc, act_tmem, w_addr, 32, H64 ? 4 : in_pad / 16, idesc, kBiasMma);
+                        issue_gemm_ta(leader, acc, act_tmem, w_addr, 32, H64 ? 4 : in_pad / 16, idesc, BIAS);
                     else
-                        issue_gemm(leader, acc, tile_addr, 32, w_addr, 32, in_pad / 16, idesc, kBiasMma);
+                        issue_gemm(leader, acc, tile_addr, 32, w_addr, 32, in_pad / 16, idesc, BIAS);
                     if (leader) mma_commit(acc_bar);
                     __syncwarp();
                     pipe_wait(acc_bar, acc_phase, &abort_flag);
@@ -390,13 +404,12 @@ mlp_fwd_pipe_kernel(const MlpShape shape, const MlpParams p, const __grid_consta
             slot_barrier(slot);
             if (!given_up) {
                 tc_fence_after();
-                const float *layer_bias = bias + l * kMaxDim;
                 if (l < s.depth) {
                     if constexpr (TA) {
-                        drain_row<T, ACT, BIAS && !BM>(taddr, H64 ? 64 : out_pad, layer_bias, [&](int chunk, uint4 packed) { tmem_st4(act_taddr + 4 * chunk, packed); });
+                        drain_row<T, ACT>(taddr, H64 ? 64 : out_pad, [&](int chunk, uint4 packed) { tmem_st4(act_taddr + 4 * chunk, packed); });
                         tmem_st_wait();
                     } else {
-                        drain_row<T, ACT, BIAS && !BM>(taddr, out_pad, layer_bias, [&](int chunk, uint4 packed) {
+                        drain_row<T, ACT>(taddr, out_pad, [&](int chunk, uint4 packed) {
                             st_shared_16(row_addr + ((chunk << 4) ^ row_swizzle), packed);
                         });
                         fence_async_smem();
@@ -410,7 +423,7 @@ mlp_fwd_pipe_kernel(const MlpShape shape, const MlpParams p, const __grid_consta
                         const float *target_row_f32 = static_cast<const float *>(mse.target) + target_at * mse.target_stride;
                         T *grad_row = static_cast<T *>(mse.grad) + r * mse.grad_stride;
                         T *out_row = y ? y + r * y_stride : nullptr;
-                        drain_row<T, TH_ACT_NONE, BIAS && !BM>(taddr, out_pad, layer_bias, [&](int chunk, uint4 packed) {
+                        drain_row<T, TH_ACT_NONE>(taddr, out_pad, [&](int chunk, uint4 packed) {
                             if (live && 8 * chunk < s.d_out) {
                                 if (out_row) __stcs(reinterpret_cast<uint4 *>(out_row + 8 * chunk), packed);
                                 uint4 g;
@@ -435,17 +448,22 @@ mlp_fwd_pipe_kernel(const MlpShape shape, const MlpParams p, const __grid_consta
                                 tmem_ld_wait();
 #pragma unroll
                                 for (int u = 0; u < 4; ++u)
-                                    st_shared_16(stage_row + ((u << 4) ^ stage_swizzle), finish8<T, TH_ACT_NONE, BIAS && !BM>(raw + 8 * u, layer_bias + first + 8 * u));
+                                    st_shared_16(stage_row + ((u << 4) ^ stage_swizzle), finish8<T, TH_ACT_NONE, false>(raw + 8 * u, nullptr));
                                 fence_async_smem();
                                 __syncwarp();
                                 if (lane == 0 && row0 + 32 * (warp & 3) < n_rows) tma_store_2d(&y_map, stage, first, static_cast<int>(row0) + 32 * (warp & 3));
                             }
                         } else {
-                            drain_row<T, TH_ACT_NONE, BIAS && !BM>(taddr, out_pad, layer_bias, [&](int chunk, uint4 packed) {
+                            drain_row<T, TH_ACT_NONE>(taddr, out_pad, [&](int chunk, uint4 packed) {
                                 if (live) store_chunk_to_global<T>(out_row, chunk, s.d_out, packed, y_vec);
                             });
                         }
                     }
+                }
+                if constexpr (BIAS && !BM) {  // of the next layer, or of the next tile's first one
+                    const int next = l == s.depth ? 0 : l + 1;
+                    start_from_bias(taddr, 0, next == s.depth ? s.no : s.h, bias + next * kMaxDim);
+                    tmem_st_wait();
                 }
                 tc_fence_before();
             }

@@ -162,37 +162,60 @@ __device__ void stage_all_weights(unsigned char *smem, const TcPlan &P, const Ml
     stage_weight_tile<T>(smem + P.w_offset[2], static_cast<const T *>(p.w_out), s.d_out, s.d_hid, s.no, s.h);
 }
 
+// ---- biases ------------------------------------------------------------------------------------
+//
+// In every kernel a layer's sum STARTS from its bias: as the value its accumulator holds when the GEMM is issued, or as a first K
+// step (mlp_fwd_pipe_kernel), which leaves the same value there.  Float32 sums depend on their order, so a backward kernel that
+// recomputes a layer gets the forward's pre-activations, and opens the same ReLUs, only if both do.
+
+// Columns [first, end) of this thread's accumulator row, multiples of eight.  To be followed by tmem_st_wait() ahead of the fence that
+// hands the accumulator to the issuer.
+__device__ __forceinline__ void start_from_bias(uint32_t taddr, int first, int end, const float *bias) {
+#pragma unroll 4
+    for (int c = first; c < end; c += 8) {
+        const uint4 lo = *reinterpret_cast<const uint4 *>(bias + c), hi = *reinterpret_cast<const uint4 *>(bias + c + 4);
+        const uint32_t v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+        tmem_st8(taddr + c, v);
+    }
+}
+
+// The same where two threads share a row: between them all `next` columns, and this one none that the other, which has read (or is still
+// reading) its half of `read` columns, may not have read yet.
+__device__ __forceinline__ void start_half_from_bias(uint32_t taddr, int half, int read, int next, const float *bias) {
+    const int middle = read / 2 < next ? read / 2 : next;
+    start_from_bias(taddr, half ? middle : 0, half ? next : middle, bias);
+}
+
 // ---- epilogues: forward ------------------------------------------------------------------------
 
-// A hidden layer's accumulator -> bias, activation, rounding -> this thread's chunks of the next operand tile
-template <typename T, int ACT, bool BIAS>
-__device__ __forceinline__ void hidden_epilogue(uint32_t taddr, const Seat &seat, int pad, const float *bias,
-                                                unsigned char *next_tile) {
+// A hidden layer's accumulator -> activation, rounding -> this thread's chunks of the next operand tile
+template <typename T, int ACT>
+__device__ __forceinline__ void hidden_epilogue(uint32_t taddr, const Seat &seat, int pad, unsigned char *next_tile) {
     const int n = pad / kGroups, first = seat.group * (n / 8);  // this thread's columns / first 8-column piece
     const uint32_t row_addr = smem_addr(next_tile) + seat.row * 128, row_swizzle = (seat.row & 7) << 4;
     for_each_piece(taddr + seat.group * n, n, [&](int u, const uint32_t(&piece)[8]) {
-        st_shared_16(row_addr + (((first + u) << 4) ^ row_swizzle), finish8<T, ACT, BIAS>(piece, bias + 8 * (first + u)));
+        st_shared_16(row_addr + (((first + u) << 4) ^ row_swizzle), finish8<T, ACT, false>(piece, nullptr));
     });
 }
 
-template <typename T, bool BIAS>
-__device__ __forceinline__ void output_epilogue(uint32_t taddr, const Seat &seat, int pad, const float *bias, T *row_ptr,
-                                                int cols, bool live, bool vector_ok) {
+template <typename T>
+__device__ __forceinline__ void output_epilogue(uint32_t taddr, const Seat &seat, int pad, T *row_ptr, int cols, bool live, bool vector_ok) {
     const int n = pad / kGroups, first = seat.group * (n / 8);
     for_each_piece(taddr + seat.group * n, n, [&](int u, const uint32_t(&piece)[8]) {
-        if (live)
-            store_chunk_to_global<T>(row_ptr, first + u, cols, finish8<T, TH_ACT_NONE, BIAS>(piece, bias + 8 * (first + u)), vector_ok);
+        if (live) store_chunk_to_global<T>(row_ptr, first + u, cols, finish8<T, TH_ACT_NONE, false>(piece, nullptr), vector_ok);
     });
 }
 
-template <typename T, int ACT, bool BIAS, typename Sink>
-__device__ __forceinline__ void drain_row(uint32_t taddr, int out_pad, const float *bias, Sink sink) {
+// One accumulator row (out_pad a multiple of 16 columns) -> activation, rounding -> 16-byte chunks handed to
+// `sink(chunk index, packed values)`
+template <typename T, int ACT, typename Sink>
+__device__ __forceinline__ void drain_row(uint32_t taddr, int out_pad, Sink sink) {
     uint32_t raw[32];
     if (out_pad == 16) {
         tmem_ld16(taddr, raw);
         tmem_ld_wait();
 #pragma unroll
-        for (int u = 0; u < 2; ++u) sink(u, finish8<T, ACT, BIAS>(raw + 8 * u, bias + 8 * u));
+        for (int u = 0; u < 2; ++u) sink(u, finish8<T, ACT, false>(raw + 8 * u, nullptr));
         return;
     }
 #pragma unroll 1
@@ -200,7 +223,7 @@ __device__ __forceinline__ void drain_row(uint32_t taddr, int out_pad, const flo
         tmem_ld32(taddr + first, raw);
         tmem_ld_wait();
 #pragma unroll
-        for (int u = 0; u < 4; ++u) sink(first / 8 + u, finish8<T, ACT, BIAS>(raw + 8 * u, bias + first + 8 * u));
+        for (int u = 0; u < 4; ++u) sink(first / 8 + u, finish8<T, ACT, false>(raw + 8 * u, nullptr));
     }
 }
 

@@ -85,16 +85,16 @@ __device__ __forceinline__ bool rows_wait_mma(uint32_t mbar, uint32_t &phase, vo
     return *abort_flag == 0;
 }
 
-// One accumulator row (out_pad a multiple of 16 columns) -> bias, activation, rounding -> 16-byte chunks handed
+// One accumulator row (out_pad a multiple of 16 columns) -> activation, rounding -> 16-byte chunks handed
 // to `sink(chunk index, packed values)`, 16 columns per TMEM load: half the registers of the 32-column form.
-template <typename T, int ACT, bool BIAS, typename Sink>
-__device__ __forceinline__ void drain_row16(uint32_t taddr, int out_pad, const float *bias, Sink sink) {
+template <typename T, int ACT, typename Sink>
+__device__ __forceinline__ void drain_row16(uint32_t taddr, int out_pad, Sink sink) {
     for (int first = 0; first < out_pad; first += 16) {
         uint32_t raw[32];
         tmem_ld16(taddr + first, raw);
         tmem_ld_wait();
 #pragma unroll
-        for (int u = 0; u < 2; ++u) sink(first / 8 + u, finish8<T, ACT, BIAS>(raw + 8 * u, bias + first + 8 * u));
+        for (int u = 0; u < 2; ++u) sink(first / 8 + u, finish8<T, ACT, false>(raw + 8 * u, nullptr));
     }
 }
 
@@ -293,6 +293,11 @@ field_fwd_kernel(const __grid_constant__ LevelParams P, const CoordView cv, cons
         const float *bias = reinterpret_cast<const float *>(smem + PL.bias_offset);
         uint32_t phase = 0;
         float loss = 0.f;
+        if constexpr (BIAS) {
+            start_from_bias(taddr, 0, s.h, bias);
+            tmem_st_wait();
+            tc_fence_before();
+        }
         for (long long q = g; q < n_mine; q += kRowGroups) {
             const int r = static_cast<int>(q % kRing);
             unsigned char *tile = smem + r * kTileBytes;
@@ -308,15 +313,14 @@ field_fwd_kernel(const __grid_constant__ LevelParams P, const CoordView cv, cons
                     const bool leader = elect_one();
                     tc_fence_after();
                     issue_gemm(leader, acc, tile_addr, 32, smem_addr(weight_tile(smem, PL, s, l)), 32, in_pad / 16,
-                               instr_desc(128, out_pad, bf16, 0, 0), false);
+                               instr_desc(128, out_pad, bf16, 0, 0), BIAS);
                     if (leader) mma_commit(bar);
                     __syncwarp();
                     issued = true;
                 }
                 const bool ok = rows_wait_mma(bar, phase, abort_now, bar_rows(g), issued);
-                const float *layer_bias = bias + l * kMaxDim;
                 if (ok && l < s.depth) {
-                    drain_row16<T, ACT, BIAS>(taddr, out_pad, layer_bias, [&](int chunk, uint4 packed) {
+                    drain_row16<T, ACT>(taddr, out_pad, [&](int chunk, uint4 packed) {
                         st_shared_16(row_addr + ((chunk << 4) ^ row_swizzle), packed);
                     });
                     fence_async_smem();
@@ -328,7 +332,7 @@ field_fwd_kernel(const __grid_constant__ LevelParams P, const CoordView cv, cons
                         const T *target_row = static_cast<const T *>(mse.target) + rr * mse.target_stride;
                         T *grad_row = static_cast<T *>(mse.grad) + rr * mse.grad_stride;
                         T *out_row = y ? y + rr * y_stride : nullptr;
-                        drain_row16<T, TH_ACT_NONE, BIAS>(taddr, out_pad, layer_bias, [&](int chunk, uint4 packed) {
+                        drain_row16<T, TH_ACT_NONE>(taddr, out_pad, [&](int chunk, uint4 packed) {
                             if (live && 8 * chunk < s.d_out) {
                                 if (out_row) __stcs(reinterpret_cast<uint4 *>(out_row + 8 * chunk), packed);
                                 const uint4 tg = __ldcs(reinterpret_cast<const uint4 *>(target_row + 8 * chunk));
@@ -337,10 +341,15 @@ field_fwd_kernel(const __grid_constant__ LevelParams P, const CoordView cv, cons
                         });
                     } else {
                         T *out_row = y + rr * y_stride;
-                        drain_row16<T, TH_ACT_NONE, BIAS>(taddr, out_pad, layer_bias, [&](int chunk, uint4 packed) {
+                        drain_row16<T, TH_ACT_NONE>(taddr, out_pad, [&](int chunk, uint4 packed) {
                             if (live) store_chunk_to_global<T>(out_row, chunk, s.d_out, packed, y_vec);
                         });
                     }
+                }
+                if constexpr (BIAS) {  // of the next layer, or of the next tile's first one
+                    const int next = l == s.depth ? 0 : l + 1;
+                    start_from_bias(taddr, 0, next == s.depth ? s.no : s.h, bias + next * kMaxDim);
+                    tmem_st_wait();
                 }
                 tc_fence_before();
                 named_barrier(bar_rows(g), kRowThreads);  // next layer reads what the group wrote; the accumulator is free again
@@ -561,7 +570,7 @@ field_bwd_kernel(const __grid_constant__ LevelParams P, const CoordView cv, cons
                     issued = true;
                 }
                 if (group_wait_mma(bar, phase, abort_now, bar_mlp, issued))
-                    hidden_epilogue<T, ACT, false>(taddr, seat, s.h, nullptr, act_tile(l + 1));
+                    hidden_epilogue<T, ACT>(taddr, seat, s.h, act_tile(l + 1));
                 fence_async_smem();
                 tc_fence_before();
                 named_barrier(bar_mlp, kTcThreads);
@@ -587,7 +596,7 @@ field_bwd_kernel(const __grid_constant__ LevelParams P, const CoordView cv, cons
                         dz_epilogue<T, ACT>(taddr, seat, in_pad, act_tile(l), act_tile(l));  // in place: mask from the parked activation
                     } else {
                         // the tile's feature gradient, rounded to T, in the operand layout in act[1]'s buffer
-                        hidden_epilogue<T, TH_ACT_NONE, false>(taddr, seat, in_pad, nullptr, act_tile(1));
+                        hidden_epilogue<T, TH_ACT_NONE>(taddr, seat, in_pad, act_tile(1));
                         if (gx) {
                             const bool live = row0 + seat.row < n_points;
                             dx_epilogue<T>(taddr, seat, in_pad, gx + (live ? row0 + seat.row : 0) * gx_stride, s.d_in, live, gx_vec);
