@@ -202,7 +202,12 @@ __device__ __forceinline__ uint4 finish_piece(const uint32_t (&raw)[8], const fl
         v[0] += b0.x; v[1] += b0.y; v[2] += b0.z; v[3] += b0.w;
         v[4] += b1.x; v[5] += b1.y; v[6] += b1.z; v[7] += b1.w;
     }
-    if constexpr (ACT == TH_ACT_SILU || ACT == TH_ACT_RELU2) {
+    if constexpr (ACT == TH_ACT_SILU) {
+        float s[8];
+        sigmoid8(v, s);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[k] *= s[k];
+    } else if constexpr (ACT == TH_ACT_RELU2) {
 #pragma unroll
         for (int k = 0; k < 8; ++k) v[k] = activate(ACT, v[k]);
     }
