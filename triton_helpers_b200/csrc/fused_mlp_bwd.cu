@@ -11,8 +11,8 @@
 //   * dz of layer l - 1 is written in place over the parked input of layer l once both MMAs that read it have finished;
 //   * rows come and go through a ring of buffers (features, output gradient), one more than slots where that fits, kept by ROW
 //     WARPS: TMA fetches the next tile's rows while the slots work, and the input gradient, which the slot leaves in its buffer
-//     as rounded rows, goes out by TMA before the buffer is filled again.  Rows TMA cannot describe are copied by four row warps,
-//     a thread a row.  Rows of 16 or 32 columns lie 32 or 64 bytes apart (the tensor core's 32- and 64-byte swizzles).
+//     as rounded rows, goes out by TMA before the buffer is filled again: one row warp; where TMA cannot describe some of the rows
+//     four, which copy them.  Rows of 16 or 32 columns lie 32 or 64 bytes apart (the tensor core's 32- and 64-byte swizzles).
 // The output layer's weight gradient is formed transposed, act^T . dz: an M = 64 MMA takes 27 + N / 2 cycles, and N is then the
 // padded output width (16: 35 instead of 60 cycles a K step) instead of the hidden one.
 // Bias gradient of a layer = column sums of dz = dz^T . ONES, a small MMA (N = 8) next to the weight gradient's.  SiLU' and
@@ -55,7 +55,6 @@ struct SlotPlan {
     int x_pitch, go_pitch;
     int ring;            // byte offset
     int ring_bytes;      // a buffer: the rows, then the output gradient
-    int row_warps;       // 1: rows by TMA; 4: some of them by threads
     int ones;            // byte offset of the tile of ones (biases)
     int weights;         // byte offset of the weight tiles and biases
     int tables;          // byte offset of the barriers and step table
@@ -156,12 +155,61 @@ __device__ __forceinline__ void for_row_pieces(uint32_t taddr, int pad, int half
     }
 }
 
-// Three slots of two warpgroups leave registers for one row warp: rows by TMA only
-template <int S, int W>
-constexpr int kRowWarps = S * W > 4 ? 1 : 4;
+// ---- rows that TMA cannot describe ----
+//
+// The row warps copy them, a warp its 32 rows of a tile, a thread a 16-byte chunk of a row at a time, the warp's chunks side by side, so that
+// an access touches five lines.  A chunk is eight accesses at fixed distances from one address, and two chunks are in flight.  Measured, 300 007
+// rows, one layer, rows off their alignment by an element, backward (a thread a row, whose accesses touch 32 lines / this): 64-64
+// 350 / 200 us, 32-64 186 / 88, 32-16 114 / 61, 27-3 96 / 65.  Lanes along a row, whose addresses are worked out for every element: 230
+// to 460, 188 to 290, 157, 143.
 
-template <typename T, int ACT, bool BIAS, int S, int W>
-__global__ void __launch_bounds__(128 * S * W + 32 + 32 * kRowWarps<S, W>, 1)
+// Chunk i of the warp's 32 rows of `chunks` chunks each
+struct RowChunk {
+    int row, chunk;
+    __device__ __forceinline__ RowChunk(int i, int chunks, int r0) {
+        const int r = (i * (65536 / chunks + 1)) >> 16;  // i / chunks: i < 256, chunks <= 8
+        row = r0 + r;
+        chunk = i - r * chunks;
+    }
+    __device__ __forceinline__ uint32_t at(int pitch) const { return row * pitch + ((chunk ^ row_swizzle_of(row, pitch)) << 4); }
+};
+
+// Rows r0 .. r0 + 31 of the tile whose first row is src, `live` of the tile's rows exist -> row buffer, zero padded to `pad` columns
+__device__ __forceinline__ void copy_rows_in(const unsigned short *src, long long stride, int r0, int live, int cols, int pad, int pitch, uint32_t buffer) {
+    if (cols <= 8) {
+        const int r = r0 + (threadIdx.x & 31);
+        const uint32_t at = buffer + r * pitch, swz = row_swizzle_of(r, pitch);
+        const uint4 v = gather8(src + (r < live ? r * stride : 0), 0, r < live ? cols : 0);
+        for (int c = 0; c < pad / 8; ++c) st_shared_16(at + ((c ^ swz) << 4), c == 0 ? v : make_uint4(0, 0, 0, 0));
+        return;
+    }
+    const int chunks = pad / 8;
+#pragma unroll 1
+    for (int i = threadIdx.x & 31; i < 32 * chunks; i += 64) {
+        const RowChunk c(i, chunks, r0), e(i + 32, chunks, r0);  // an even number of chunks
+        const uint4 u = gather8(src + (c.row < live ? c.row * stride : 0) + 8 * c.chunk, 8 * c.chunk, c.row < live ? cols : 0);
+        const uint4 v = gather8(src + (e.row < live ? e.row * stride : 0) + 8 * e.chunk, 8 * e.chunk, e.row < live ? cols : 0);
+        st_shared_16(buffer + c.at(pitch), u);
+        st_shared_16(buffer + e.at(pitch), v);
+    }
+}
+
+// The other way, without the padding
+__device__ __forceinline__ void copy_rows_out(unsigned short *dst, long long stride, int r0, int live, int cols, int pitch, uint32_t buffer) {
+    const int chunks = (cols + 7) / 8;
+#pragma unroll 1
+    for (int i = threadIdx.x & 31; i < 32 * chunks; i += 32) {
+        const RowChunk c(i, chunks, r0);
+        if (c.row < live) store_chunk_to_global(dst + c.row * stride, c.chunk, cols, ld_shared_16(buffer + c.at(pitch)), false);
+    }
+}
+
+// COPIED: some rows are copied by four row warps; otherwise one asks for boxes
+template <bool COPIED>
+constexpr int kRowWarps = COPIED ? 4 : 1;
+
+template <typename T, int ACT, bool BIAS, int S, int W, bool COPIED>
+__global__ void __launch_bounds__(128 * S * W + 32 + 32 * kRowWarps<COPIED>, 1)
 slots_mlp_bwd_tc_kernel(const MlpShape s, const MlpParams p, const __grid_constant__ WeightMaps maps, const int use_tma,
                         const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap go_map,
                         const __grid_constant__ CUtensorMap gx_map, const int row_tma, const __grid_constant__ SlotPlan P, const T *__restrict__ x, long long x_stride, const T *__restrict__ go,
@@ -189,7 +237,7 @@ slots_mlp_bwd_tc_kernel(const MlpShape s, const MlpParams p, const __grid_consta
             mbar_init(&tb.wdone[i]);
         }
         for (int i = 0; i < P.rings; ++i) {
-            mbar_init(&tb.full[i], static_cast<uint32_t>(P.row_warps));
+            mbar_init(&tb.full[i], static_cast<uint32_t>(kRowWarps<COPIED>));
             mbar_init(&tb.empty[i]);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -345,18 +393,11 @@ slots_mlp_bwd_tc_kernel(const MlpShape s, const MlpParams p, const __grid_consta
     } else if (is_row_warp) {
         // ================= rows: the input gradient out of a buffer, the next tile's rows into it =================
         const uint32_t x_bytes = static_cast<uint32_t>(kTileRows * P.x_pitch), go_bytes = static_cast<uint32_t>(kTileRows * P.go_pitch);
-        const bool x_tma = row_tma & 1, go_tma = row_tma & 2, gx_tma = row_tma & 4;
-        const int r_warp = warp - 4 * S * W - 1, r = 32 * r_warp + lane;  // a thread's row
-        // this thread's row, element by element
-        auto copy_row = [&](const T *src, long long grow, long long stride, int cols, int pad, int pitch, uint32_t tile) {
-            const unsigned short *from = reinterpret_cast<const unsigned short *>(src + (grow < n_rows ? grow * stride : 0));
-            const uint32_t at = tile + r * pitch, swz = row_swizzle_of(r, pitch);
-#pragma unroll 2
-            for (int c = 0; c < pad / 8; ++c)
-                st_shared_16(at + ((c ^ swz) << 4), gather8(from + 8 * c, 8 * c, grow < n_rows ? cols : 0));
-        };
+        const bool x_tma = !COPIED || (row_tma & 1), go_tma = !COPIED || (row_tma & 2), gx_tma = COPIED ? (row_tma & 4) != 0 : gx != nullptr;
+        const int r_warp = warp - 4 * S * W - 1;
+        auto live_rows = [&](long long first) { return static_cast<int>(n_rows - first < kTileRows ? n_rows - first : kTileRows); };
         bool alive = true;  // after an abort: the same sequence of barriers, no work
-        for (long long k = 0; r_warp < P.row_warps && k < n_mine + P.rings; ++k) {
+        for (long long k = 0; k < n_mine + P.rings; ++k) {
             const uint32_t b = static_cast<uint32_t>(k % P.rings), rows_at = ring_of(b);
             const long long row0 = (first_tile + k * tile_stride) * kTileRows;
             if (k >= P.rings) {
@@ -370,17 +411,19 @@ slots_mlp_bwd_tc_kernel(const MlpShape s, const MlpParams p, const __grid_consta
                         tma_store_2d(&gx_map, rows_at, 0, static_cast<int>(old0));
                         asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
                     }
-                } else if (gx != nullptr && old0 + r < n_rows) {
-                    const uint32_t at = rows_at + r * P.x_pitch, swz = row_swizzle_of(r, P.x_pitch);
-                    for (int c = 0; c < s.ki / 8; ++c) store_chunk_to_global<T>(gx + (old0 + r) * gx_stride, c, s.d_in, ld_shared_16(at + ((c ^ swz) << 4)), false);
+                } else if (COPIED && gx != nullptr) {
+                    copy_rows_out(reinterpret_cast<unsigned short *>(gx + old0 * gx_stride), gx_stride, 32 * r_warp, live_rows(old0), s.d_in, P.x_pitch, rows_at);
                 }
                 __syncwarp();
-                if (P.row_warps > 1) asm volatile("bar.sync 15, 128;" ::: "memory");
+                if constexpr (COPIED) asm volatile("bar.sync 15, 128;" ::: "memory");
             }
             if (k >= n_mine || !alive) continue;
-            if (P.row_warps > 1) {
-                if (!x_tma) copy_row(x, row0 + r, x_stride, s.d_in, s.ki, P.x_pitch, rows_at);
-                if (!go_tma) copy_row(go, row0 + r, go_stride, s.d_out, s.no, P.go_pitch, rows_at + go_at);
+            if constexpr (COPIED) {
+                if (!x_tma)
+                    copy_rows_in(reinterpret_cast<const unsigned short *>(x + row0 * x_stride), x_stride, 32 * r_warp, live_rows(row0), s.d_in, s.ki, P.x_pitch, rows_at);
+                if (!go_tma)
+                    copy_rows_in(reinterpret_cast<const unsigned short *>(go + row0 * go_stride), go_stride, 32 * r_warp, live_rows(row0), s.d_out, s.no, P.go_pitch,
+                                 rows_at + go_at);
                 fence_async_smem();
                 __syncwarp();
             }
@@ -637,24 +680,28 @@ bool make_rows_map(CUtensorMap *map, const void *base, long long rows, int cols,
 template <typename T, int ACT, bool BIAS, int S, int W>
 int launch_slots(int rings, const MlpShape &s, const MlpParams &p, const void *x, int64_t x_stride, const void *go, int64_t go_stride,
                  void *gx, int64_t gx_stride, float *workspace, int64_t rows, cudaStream_t stream) {
-    SlotPlan P = slot_plan(s, S, rings);
+    const SlotPlan P = slot_plan(s, S, rings);
     if (P.total > kSmemBudget || P.tmem_cols > 512 || 2 * s.depth + 1 > kStepsMax) return kTcNotApplicable;
     CUtensorMap x_map, go_map, gx_map;
     memset(&gx_map, 0, sizeof(gx_map));
     const bool x_tma = make_rows_map(&x_map, x, rows, s.d_in, P.x_pitch, x_stride), go_tma = make_rows_map(&go_map, go, rows, s.d_out, P.go_pitch, go_stride);
     const bool gx_tma = gx != nullptr && make_rows_map(&gx_map, gx, rows, s.d_in, P.x_pitch, gx_stride);
-    P.row_warps = x_tma && go_tma && (gx_tma || gx == nullptr) ? 1 : 4;
-    if (P.row_warps > kRowWarps<S, W>) return kTcNotApplicable;
+    // three slots of two warpgroups leave registers for one row warp
+    constexpr bool kMayCopy = S * W <= 4;
+    const bool copied = !(x_tma && go_tma && (gx_tma || gx == nullptr));
+    if (copied && !kMayCopy) return kTcNotApplicable;
     int smem = P.total;
     if (smem < kSmemBudget / 2 + 1024) smem = kSmemBudget / 2 + 1024;  // one CTA per SM
     WeightMaps maps;
     const int use_tma = make_weight_maps(maps, s, p);
-    auto kernel = slots_mlp_bwd_tc_kernel<T, ACT, BIAS, S, W>;
+    auto kernel = slots_mlp_bwd_tc_kernel<T, ACT, BIAS, S, W, false>;
+    if constexpr (kMayCopy)
+        if (copied) kernel = slots_mlp_bwd_tc_kernel<T, ACT, BIAS, S, W, true>;
     if (int rc = cuda_status(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
                              "cudaFuncSetAttribute(slots_mlp_bwd_tc_kernel)")) return rc;
     const long long tiles = (rows + kTileRows - 1) / kTileRows;
     const long long cap = sm_count();
-    kernel<<<static_cast<unsigned>(tiles < cap ? tiles : cap), 128 * S * W + 32 + 32 * kRowWarps<S, W>, smem, stream>>>(
+    kernel<<<static_cast<unsigned>(tiles < cap ? tiles : cap), 128 * S * W + 32 + 32 * (copied ? kRowWarps<true> : kRowWarps<false>), smem, stream>>>(
         s, p, maps, use_tma, x_map, go_map, gx_map, (x_tma ? 1 : 0) | (go_tma ? 2 : 0) | (gx_tma ? 4 : 0), P, static_cast<const T *>(x), x_stride,
         static_cast<const T *>(go), go_stride, static_cast<T *>(gx), gx_stride, workspace, rows);
     return launch_status("slots_mlp_bwd_tc_kernel launch");
