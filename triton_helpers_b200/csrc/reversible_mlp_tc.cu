@@ -64,7 +64,7 @@ struct RevTcPlan {
     int tmem_cols;
 };
 
-__host__ __device__ inline RevTcPlan rev_tc_plan(bool backward) {
+__host__ __device__ constexpr RevTcPlan rev_tc_plan(bool backward) {
     RevTcPlan p{};
     p.tiles = backward ? 8 : 2;
     p.ring = p.tiles * kTileBytes;
@@ -74,6 +74,8 @@ __host__ __device__ inline RevTcPlan rev_tc_plan(bool backward) {
     p.tmem_cols = backward ? 512 : 256;
     return p;
 }
+// one backward CTA per SM, two forward ones, beside 1 KB of the kernels' static variables each
+static_assert(rev_tc_plan(true).total + 1024 <= kSmemBudget && 2 * (rev_tc_plan(false).total + 1024) <= kSmemBudget);
 
 // Queue block k's four weight matrices into ring stage `stage` (cp.async, operand-tile layout).
 // A call, not inlined: the kernels live on their instruction cache and almost never come here.
@@ -258,14 +260,14 @@ rev_fwd_tc_kernel(const RevShape shape, const RevParams p, const __grid_constant
 
     __shared__ __align__(8) unsigned long long ring_bars[2];
     if (threadIdx.x == 0) {
-        abort_flag = 0;
+        abort_flag = (smem_addr(smem) & 1023u) ? 1 : 0;  // operand tiles need their alignment
         asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&ring_bars[0])), "r"(1u) : "memory");
         asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&ring_bars[1])), "r"(1u) : "memory");
     }
     const long long n_tiles = (n_rows + kTileRows - 1) / kTileRows;
     if (!use_tma && static_cast<long long>(blockIdx.x) < n_tiles) prefetch_weights<T>(smem, P, shape, p, 0, 0);
     const uint32_t tmem = cta_setup(&tmem_holder, &mbar, P.tmem_cols);  // publishes the barrier inits
-    if (use_tma && static_cast<long long>(blockIdx.x) < n_tiles) {
+    if (use_tma && !abort_flag && static_cast<long long>(blockIdx.x) < n_tiles) {
         prefetch_weights_tma<T, BIAS>(smem, P, s, p, maps, ring_bars, 0, 0);  // awaited behind the first rows
     }
     // With the A operands in tensor memory and the weights by TMA nothing that an MMA reads is written by a thread, and the fence
@@ -510,7 +512,7 @@ rev_bwd_tc_kernel(const RevShape shape, const RevParams p, const __grid_constant
     __shared__ int stop_flag;
     __shared__ __align__(8) unsigned long long wgrad_bar, flushed_bar, operands_bar, summed_bar, rows_bar;
     if (threadIdx.x == 0) {
-        abort_flag = stop_flag = 0;
+        abort_flag = stop_flag = (smem_addr(smem) & 1023u) ? 1 : 0;  // operand tiles need their alignment
         asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&ring_bars[0])), "r"(1u) : "memory");
         asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&ring_bars[1])), "r"(1u) : "memory");
         asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&wgrad_bar)), "r"(1u) : "memory");
@@ -572,7 +574,7 @@ rev_bwd_tc_kernel(const RevShape shape, const RevParams p, const __grid_constant
         if ((threadIdx.x & 31) == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     } else {
         // ================= the chain =================
-        if (use_tma && static_cast<long long>(blockIdx.x) < n_tiles) {
+        if (use_tma && !stop_flag && static_cast<long long>(blockIdx.x) < n_tiles) {
             prefetch_weights_tma<T, BIAS>(smem, P, s, p, maps, ring_bars, s.blocks - 1, 0);
             ring_wait(ring_bars, 0, &abort_flag);
         }
