@@ -77,6 +77,14 @@ __host__ __device__ constexpr RevTcPlan rev_tc_plan(bool backward) {
 // one backward CTA per SM, two forward ones, beside 1 KB of the kernels' static variables each
 static_assert(rev_tc_plan(true).total + 1024 <= kSmemBudget && 2 * (rev_tc_plan(false).total + 1024) <= kSmemBudget);
 
+// Operand tiles need their alignment, which the shared memory's declaration asks for: should the base be another one, all threads leave
+// before anything is set up, with the status word raised.
+__device__ __forceinline__ bool misplaced(const unsigned char *smem) {
+    if ((smem_addr(smem) & 1023u) == 0) return false;
+    g_tc_status = 1;
+    return true;
+}
+
 // Queue block k's four weight matrices into ring stage `stage` (cp.async, operand-tile layout).
 // A call, not inlined: the kernels live on their instruction cache and almost never come here.
 template <typename T>
@@ -251,6 +259,7 @@ rev_fwd_tc_kernel(const RevShape shape, const RevParams p, const __grid_constant
     const RevShape s = known_widths<HALF, HID>(shape);
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char *smem = smem_raw;
+    if (misplaced(smem)) return;
     __shared__ uint32_t tmem_holder;
     __shared__ __align__(8) unsigned long long mbar;
     __shared__ int abort_flag;
@@ -260,14 +269,14 @@ rev_fwd_tc_kernel(const RevShape shape, const RevParams p, const __grid_constant
 
     __shared__ __align__(8) unsigned long long ring_bars[2];
     if (threadIdx.x == 0) {
-        abort_flag = (smem_addr(smem) & 1023u) ? 1 : 0;  // operand tiles need their alignment
+        abort_flag = 0;
         asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&ring_bars[0])), "r"(1u) : "memory");
         asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&ring_bars[1])), "r"(1u) : "memory");
     }
     const long long n_tiles = (n_rows + kTileRows - 1) / kTileRows;
     if (!use_tma && static_cast<long long>(blockIdx.x) < n_tiles) prefetch_weights<T>(smem, P, shape, p, 0, 0);
     const uint32_t tmem = cta_setup(&tmem_holder, &mbar, P.tmem_cols);  // publishes the barrier inits
-    if (use_tma && !abort_flag && static_cast<long long>(blockIdx.x) < n_tiles) {
+    if (use_tma && static_cast<long long>(blockIdx.x) < n_tiles) {
         prefetch_weights_tma<T, BIAS>(smem, P, s, p, maps, ring_bars, 0, 0);  // awaited behind the first rows
     }
     // With the A operands in tensor memory and the weights by TMA nothing that an MMA reads is written by a thread, and the fence
@@ -491,6 +500,7 @@ rev_bwd_tc_kernel(const RevShape shape, const RevParams p, const __grid_constant
     const RevShape s = known_widths<HALF, HID>(shape);
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char *smem = smem_raw;
+    if (misplaced(smem)) return;
     __shared__ uint32_t tmem_holder;
     __shared__ __align__(8) unsigned long long mbar;
     __shared__ int abort_flag;
@@ -512,7 +522,7 @@ rev_bwd_tc_kernel(const RevShape shape, const RevParams p, const __grid_constant
     __shared__ int stop_flag;
     __shared__ __align__(8) unsigned long long wgrad_bar, flushed_bar, operands_bar, summed_bar, rows_bar;
     if (threadIdx.x == 0) {
-        abort_flag = stop_flag = (smem_addr(smem) & 1023u) ? 1 : 0;  // operand tiles need their alignment
+        abort_flag = stop_flag = 0;
         asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&ring_bars[0])), "r"(1u) : "memory");
         asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&ring_bars[1])), "r"(1u) : "memory");
         asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&wgrad_bar)), "r"(1u) : "memory");
@@ -574,7 +584,7 @@ rev_bwd_tc_kernel(const RevShape shape, const RevParams p, const __grid_constant
         if ((threadIdx.x & 31) == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     } else {
         // ================= the chain =================
-        if (use_tma && !stop_flag && static_cast<long long>(blockIdx.x) < n_tiles) {
+        if (use_tma && static_cast<long long>(blockIdx.x) < n_tiles) {
             prefetch_weights_tma<T, BIAS>(smem, P, s, p, maps, ring_bars, s.blocks - 1, 0);
             ring_wait(ring_bars, 0, &abort_flag);
         }
