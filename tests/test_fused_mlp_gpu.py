@@ -27,7 +27,7 @@ def rows_outside(got, want, tol) -> float:
     r"""Fraction of rows whose largest error exceeds ``tol * max|want|``."""
     got, want = got.detach().double().cpu(), want.detach().double().cpu()
     err = (got - want).abs().reshape(-1, want.shape[-1]).amax(-1) / want.abs().max().clamp_min(1e-300)
-    return float((err > tol).double().mean())
+    return float((~(err <= tol)).double().mean())  # a NaN is outside
 
 
 def make_params(d_in, d_hid, d_out, depth, dtype, bias=True, seed=0):
