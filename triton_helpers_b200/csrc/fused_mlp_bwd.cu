@@ -4,7 +4,7 @@
 // layer by layer backwards), each a round trip "operands written -> barrier -> issue -> commit -> mbarrier -> tcgen05.ld ->
 // convert -> st.shared" of about a microsecond of which the MMAs are a tenth.  Throughput is row tiles in flight over
 // chain length.  ONE CTA per SM runs S independent SLOTS of 128 W threads plus one WGRAD warp:
-//   * warp 0 of a slot issues the slot's recompute and dgrad MMAs into the slot's own accumulator columns, so that chain
+//   * a warp of a slot issues the slot's recompute and dgrad MMAs into the slot's own accumulator columns, so that chain
 //     never leaves the slot; the W warpgroups of a slot share a tile's columns (thread = tile row = TMEM lane, column half);
 //   * the wgrad warp issues the weight- and bias-gradient MMAs of every slot.  MMAs of one thread execute in order, so all
 //     slots accumulate into ONE shared set of TMEM columns instead of one set per tile in flight;
@@ -23,7 +23,8 @@
 // Measured: rows fetched and stored by the slots themselves were 22 % of a slot's time (2^21 rows 32-64-64-16; a fence for the
 // tensor core also waits for the thread's own copies and stores in flight).  With the ring 0.234 -> 0.209 ms, 2^20 rows 32-4x64-16
 // 0.279 -> 0.265, 300 007 rows 32-3x64-16 with biases, where the smaller row buffers make room for a third slot, 0.081 -> 0.069; with the
-// issuers on schedulers of their own and their lanes elected where they issue, 0.189, 0.226 and 0.063.
+// issuers spread over the schedulers, their lanes elected where they issue and no load of the abort flag ahead of a wait that is over,
+// 0.186, 0.220 and 0.062.
 //
 // Per slot three mbarriers: `ready` (one arrival: the operands of the slot's next backward step are in place), `acc` (the
 // slot's own MMAs of the step are done), `wdone` (the step's wgrad is done).  The wgrad warp polls all `ready` barriers at
@@ -81,7 +82,7 @@ struct __align__(16) SlotStep {
     uint32_t a_high;   // high words of the descriptors that are not a 128-byte tile's: the slot's own GEMM's A operand
     uint32_t wa_high, wb_high;  // the weight gradient's operands
     uint32_t wa_step, wb_step;  // bytes between K steps
-    uint32_t flags;    // operands in the row buffer: bit 1 the weight gradient's A, 2 its B, 3 the pre-activation's A; 4: B is dz (transposed)
+    uint32_t flags;    // operands in the row buffer: bit 2 the weight gradient's B, 3 the pre-activation's A; 4: B is dz (transposed)
     uint32_t unused[2];
 };
 
@@ -366,7 +367,7 @@ slots_mlp_bwd_tc_kernel(const MlpShape s, const MlpParams p, const __grid_consta
                 const uint32_t tile0 = smem_base + static_cast<uint32_t>(i) * slot_bytes, rows0 = ring_of(__shfl_sync(0xffffffffu, my_buf, i));
                 const bool more = (started >> (j - d)) & 1u;
                 if (leader) {
-                    const uint32_t a_low = desc_low((flags & 2u ? rows0 : tile0) + w.x), b_low = desc_low((flags & 4u ? rows0 : tile0) + w.y);
+                    const uint32_t a_low = desc_low(tile0 + w.x), b_low = desc_low((flags & 4u ? rows0 : tile0) + w.y);
                     for (int k = 0; k < kTileRows / 16; ++k)
                         mma_f16(tmem + (w.w & 0xffffu), desc_of(a_low + k * (h.z >> 4), h.x), desc_of(b_low + k * (h.w >> 4), h.y), w.z, more || k > 0);
                     if constexpr (BIAS) {
@@ -449,21 +450,25 @@ slots_mlp_bwd_tc_kernel(const MlpShape s, const MlpParams p, const __grid_consta
         auto act_addr = [&](int l) { return tile0 + static_cast<uint32_t>(l - 1) * kTileBytes; };  // input of layer l > 0
         const float *bias = reinterpret_cast<const float *>(wsmem + P.w.bias_offset);
         const uint32_t row_off = row * 128, row_swizzle = (row & 7) << 4;
-        // on another scheduler than other slots' issuers and the wgrad warp (all on its scheduler: 0.261 against 0.243 ms)
+        // spread over the schedulers, slots 0 to 2 on others than the wgrad warp's, which slot 3 shares (all on it: 0.261 against 0.243 ms)
         const bool issuer = (tid >> 5) == ((slot + 1) & 3);
         uint32_t acc_phase = 0, wdone_phase = 0;
         bool alive = true;
         auto slot_sync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(slot + 1), "n"(kSlotThreads) : "memory"); };
         uint32_t buf = 0, rows0 = 0, prev_buf = 0, full_phase = 0, tiles_done = 0;
-        // operands written -> the slot's warp 0 issues the step's own MMAs (and hands the wgrad to the wgrad warp)
+        // Biases and two accumulators: the recompute steps alternate between them, the last one in the first, so that a step's biases are
+        // written while the step before it waits for its MMAs (2^20 rows 64-64-64-64 SiLU 304 -> 297 us, 300 007 rows
+        // 32-3x64-3 132.2 -> 130.9)
+        auto recompute_col = [&](int l) { return BIAS && kPreact && ((d - 1 - l) & 1) ? kAccCols : 0; };
+        // operands written -> the slot's issuing warp issues the step's own MMAs (and hands the wgrad to the wgrad warp)
         auto start_step = [&](int j) {
             fence_async_smem();
             if constexpr (BIAS) tmem_st_wait();
             tc_fence_before();
             slot_sync();
             if (issuer && alive) {
-                // elected here and not ahead of the loop, or the MMAs do not go through uniform registers (2^20 rows 32-4x64-16: 0.243 -> 0.226
-                // ms; the weight gradients' MMAs, which the chain's wait behind, are the better for the longer way: 0.228)
+                // elected here and not ahead of the loop: 2^20 rows 32-4x64-16 0.243 -> 0.226 ms (by the time; presumably the descriptors then
+                // stay in uniform registers); the weight gradients' MMAs, which the chain's wait behind, are the better for not being: 0.228
                 const bool leader = elect_one();
                 tc_fence_after();
                 if (j == 0) {
@@ -481,14 +486,13 @@ slots_mlp_bwd_tc_kernel(const MlpShape s, const MlpParams p, const __grid_consta
                         if (leader) {
                             const uint32_t a_low = desc_low(rows0 + own.x), b_low = desc_low(own.y), b_step = (own.w & 256u) ? 128 : 2;
                             for (int k = 0; k < static_cast<int>(own.w & 255u); ++k)
-                                mma_f16(acc, desc_of(a_low + 2 * k, st.a_high), smem_desc(b_low + k * b_step), own.z, k > 0 || (BIAS && j == 0));
+                                mma_f16(acc + (j == 0 ? recompute_col(0) : 0), desc_of(a_low + 2 * k, st.a_high), smem_desc(b_low + k * b_step), own.z, k > 0 || (BIAS && j == 0));
                         }
                     } else {
-                        issue_gemm(leader, acc, tile0 + own.x, 32, own.y, (own.w & 256u) ? 2048 : 32, static_cast<int>(own.w & 255u), own.z, BIAS && j < d);
+                        issue_gemm(leader, acc + (j < d ? recompute_col(j) : 0), tile0 + own.x, 32, own.y, (own.w & 256u) ? 2048 : 32, static_cast<int>(own.w & 255u), own.z, BIAS && j < d);
                     }
                     if constexpr (kPreact) {
-                        if (st.z_k)
-{
+                        if (st.z_k) {
                             if (st.flags & 8u) {
                                 if (leader)
                                     for (int k = 0; k < static_cast<int>(st.z_k); ++k)
@@ -516,9 +520,8 @@ slots_mlp_bwd_tc_kernel(const MlpShape s, const MlpParams p, const __grid_consta
         [[maybe_unused]] int read = s.h;  // BIAS: accumulator columns that the slot has read last, half of them by each warpgroup
         for (long long k = slot; k < n_mine; k += S) {
             if constexpr (BIAS) {
-                if constexpr (W == 2) start_half_from_bias(taddr, half, read, s.h, bias);
-                else start_from_bias(taddr, 0, s.h, bias);
-                if constexpr (kPreact) start_from_bias(taddr + kAccCols, half * (s.h / W), (half + 1) * (s.h / W), bias + (d - 1) * kMaxDim);
+                if constexpr (W == 2) start_half_from_bias(taddr + recompute_col(0), half, recompute_col(0) ? s.h : read, s.h, bias);
+                else start_from_bias(taddr + recompute_col(0), 0, s.h, bias);
                 if (gx != nullptr) read = s.ki;
             }
             buf = static_cast<uint32_t>(k % P.rings);
@@ -526,12 +529,17 @@ slots_mlp_bwd_tc_kernel(const MlpShape s, const MlpParams p, const __grid_consta
             rows0 = ring_of(buf);
             for (int l = 0; l < d; ++l) {  // recomputed activation of layer l -> input tile of layer l + 1
                 start_step(l);
+                if constexpr (BIAS && kPreact) {
+                    // under the step's MMAs: the other accumulator is free, for the next step or for the pre-activation of the last layer
+                    const int col = l + 1 < d ? recompute_col(l + 1) : kAccCols, layer = l + 1 < d ? l + 1 : d - 1;
+                    start_from_bias(taddr + col, half * (s.h / W), (half + 1) * (s.h / W), bias + layer * kMaxDim);
+                }
                 if (finish_step(true, false)) {
                     const uint32_t dst = act_addr(l + 1) + row_off;
-                    for_row_pieces<W>(taddr, s.h, half, [&](int chunk, const uint32_t(&piece)[8]) {
+                    for_row_pieces<W>(taddr + recompute_col(l), s.h, half, [&](int chunk, const uint32_t(&piece)[8]) {
                         st_shared_16(dst + ((chunk << 4) ^ row_swizzle), finish8<T, ACT, false>(piece, nullptr));
                     });
-                    if (BIAS && l + 1 < d) start_from_bias(taddr, half * (s.h / W), (half + 1) * (s.h / W), bias + (l + 1) * kMaxDim);
+                    if (BIAS && !kPreact && l + 1 < d) start_from_bias(taddr, half * (s.h / W), (half + 1) * (s.h / W), bias + (l + 1) * kMaxDim);
                 }
             }
             for (int l = d; l >= 0; --l) {
@@ -622,7 +630,7 @@ slots_mlp_bwd_tc_kernel(const MlpShape s, const MlpParams p, const __grid_consta
                 uint32_t raw[32];
                 tmem_ld16(tmem + lane_base + dw_col(l) + first, raw);
                 tmem_ld_wait();
-                if (lane < 16 && o >= 0 && o < out_dim) {
+                if (lane < 16 && o < out_dim) {
 #pragma unroll
                     for (int c = 0; c < 16; c += 4) {
                         if (quads) {
@@ -643,7 +651,7 @@ slots_mlp_bwd_tc_kernel(const MlpShape s, const MlpParams p, const __grid_consta
                 uint32_t raw[8];
                 tmem_ld8(tmem + lane_base + db_col(l), raw);
                 tmem_ld_wait();
-                if (lane < 16 && o >= 0 && o < out_dim) atomicAdd(bdst + o, __uint_as_float(raw[0]));
+                if (lane < 16 && o < out_dim) atomicAdd(bdst + o, __uint_as_float(raw[0]));
             }
         }
     }
@@ -717,7 +725,8 @@ template <typename T, int ACT, bool BIAS>
 int launch_any_slots(const MlpShape &s, const MlpParams &p, const void *x, int64_t x_stride, const void *go, int64_t go_stride, void *gx,
                      int64_t gx_stride, float *workspace, int64_t rows, cudaStream_t stream) {
     // One or two tiles per CTA: two warpgroups walk a tile's chain faster than one, and there is nothing for more slots to do (2^14
-    // rows 32-64-64-16 with biases: 13.6 us as 1 x 2, 14.6 as 2 x 2).
+    // rows 32-64-64-16 with biases: 13.6 us as 1 x 2, 14.6 as 2 x 2; two tiles, 18 945 to 37 888 rows, 2 x 2 against the most slots that
+    // fit with rows fetched by the slots: 32-64-16 12.4 to 13.6 / 14.2 to 15.4, 32-64-64-16 16.8 / 19.1, 32-3x64-16 18.2 / 20.5).
     const int64_t tiles_per_cta = ((rows + kTileRows - 1) / kTileRows + sm_count() - 1) / sm_count();
 #define TH_SLOTS(S, W)                                                                                                                        \
     for (int rings = S + 1; rings >= S; --rings)                                                                                              \

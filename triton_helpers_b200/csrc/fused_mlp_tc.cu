@@ -149,7 +149,7 @@ mlp_fwd_tc_kernel(const MlpShape s, const MlpParams p, const __grid_constant__ W
 // where those stay in shared memory) and its mbarriers, and walks its row tiles layer by layer - but the slots share the weights, and they never meet at a
 // CTA-wide barrier after set-up, so one slot's MMAs run under the other slots' epilogues:
 //
-//   warp 0 of the slot  : fetches the slot's next input tile by TMA (a box of 64 columns x 128 rows
+//   its issuing warp    : fetches the slot's next input tile by TMA (a box of 64 columns x 128 rows
 //                         lands in the operand-tile layout; rows past the end and columns past
 //                         d_in arrive as zeros), waits for the current one, issues each layer's
 //                         GEMM, commits it to `acc_full` and polls that barrier;
@@ -202,8 +202,6 @@ __device__ __forceinline__ void slot_barrier(int slot) {
     asm volatile("bar.sync %0, 128;" ::"r"(slot + 1) : "memory");
 }
 
-// One accumulator row (out_pad = 16, 32 or 64 columns) -> bias, activation, rounding -> 16-byte
-// chunks, each handed to `sink(chunk index, packed values)`; 32 columns per TMEM load.
 // TA: hidden activations go back to the tensor core through tensor memory (32 more columns per slot) instead of
 // the operand tile in shared memory; the first layer still reads the TMA-fetched input tile.
 // H64: the hidden width (padded) is 64 at compile time: one form of the hidden layers' epilogue and of their GEMMs' issue
@@ -311,9 +309,9 @@ mlp_fwd_pipe_kernel(const MlpShape shape, const MlpParams p, const __grid_consta
 
     // ---- the slot's life; nothing below depends on other slots ----
     const int slot = warp >> 2;
-    // The issuing warps of different slots on different schedulers, and the lane that issues elected where it issues: the MMAs then
-    // take the short way through uniform registers (2^20 rows 32-4x64-16: 0.0497 -> 0.0477 ms; with the lane elected once, ahead of the
-    // loop, 0.0514 and 0.0560).
+    // The issuing warps of the slots spread over the schedulers (the fifth shares the first's), and the lane that issues elected where it
+    // issues: 2^20 rows 32-4x64-16 0.0497 -> 0.0477 ms; with the lane elected once, ahead of the loop, 0.0514 and 0.0560 (by the time;
+    // presumably the descriptors then miss the uniform registers).
     const bool issuer = (warp & 3) == (slot & 3);
     const int row = 32 * (warp & 3) + lane;
     const uint32_t stage = smem_addr(smem + plan.staging) + static_cast<uint32_t>(warp) * kStageBytes;

@@ -361,8 +361,5 @@ bool tc_disabled() {
     return off;
 }
 
-// The pipelined kernel needs TMA for the weights and for the input rows, and enough shared memory
-// for two operand tiles per slot; anything else goes to the one-tile-per-CTA kernel below.
-
 }  // namespace
 }  // namespace th
