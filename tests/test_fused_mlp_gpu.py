@@ -173,8 +173,8 @@ def test_many_row_tiles_per_cta(dtype, depth, d_hid):
 
 @pytest.mark.parametrize("d_in,d_hid,d_out,depth", [(64, 64, 64, 2), (64, 32, 16, 3), (16, 64, 32, 1), (48, 64, 8, 2)])
 def test_many_row_tiles_when_the_output_gradient_has_its_own_tile(d_in, d_hid, d_out, depth):
-    # the backward with several row tiles per CTA packs the output gradient into the feature tile only when both are
-    # at most 32 wide; wider ones take a tile of their own (and d_in = 48 is padded to 64 columns)
+    # features and output gradient lie side by side in a row buffer, 32, 64 or 128 bytes a row each: the wide ones, and mixed
+    # (48 columns lie in 128 bytes)
     dtype = torch.float16
     rows = 148 * 4 * 128 * 2 + 333
     p = make_params(d_in, d_hid, d_out, depth, dtype, bias=False, seed=d_in + depth)
